@@ -282,8 +282,9 @@ int build_sublist(dvm_ctx* c, SubList& sl, Plan& pl, bool f32_pairs = false) {
         e.poff = poff;
         e.roff = roff;
         e.cofs = cofs;
+        e.noff = 2 * coff / kLeaf + (uint64_t)kNodeSlack * k;
         coff += e.cap;  // caps are multiples of kCapAlign
-        if (s->h.precision != kF32)  // the FP32 path sums in fixed point, without partials
+        if (s->h.precision != kF32)  // the FP32 path has no chunk partials
             poff += (uint64_t)e.chunks * e.cap;
         roff += (uint64_t)e.rhs_chunks * e.npad;
         cofs += (uint64_t)e.rhs_chunks;
@@ -334,6 +335,7 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
         c->ws_block = nullptr;
     }
     const size_t cub = cub_sort_bytes(cap);
+    const uint64_t nodes = 2 * cap / kLeaf + (uint64_t)kNodeSlack * lists;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -343,7 +345,8 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     const size_t o_keys_in = take(8 * cap), o_keys_out = take(8 * cap), o_vals = take(4 * cap),
                  o_perm = take(4 * cap), o_packed = take(32 * cap),
                  o_meta = take(sizeof(TileMeta) * (cap / kBsST + 1)), o_part = take(16 * part),
-                 o_macc = take(16 * cap), o_mexp = take(sizeof(int) * 4 * kTableCap),
+                 o_nodes = take(sizeof(TreeNode) * nodes), o_mom = take(16 * kTerms * nodes),
+                 o_loc = take(16 * kTerms * nodes), o_arr = take(4 * nodes),
                  o_rhs = take(16 * rhs), o_circ = take(8 * circ + 8), o_cub = take(cub + 256),
                  o_work = take(64 * sizeof(unsigned)), o_flags = take(cap),
                  o_tiles = take(4 * (cap / 1024 + 1)),
@@ -370,8 +373,10 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     w.packed_cap = cap;
     w.meta = reinterpret_cast<TileMeta*>(b + o_meta);
     w.part = reinterpret_cast<double2*>(b + o_part);
-    w.macc = reinterpret_cast<unsigned long long*>(b + o_macc);
-    w.mexp = reinterpret_cast<int*>(b + o_mexp);
+    w.nodes = reinterpret_cast<TreeNode*>(b + o_nodes);
+    w.mom = reinterpret_cast<double2*>(b + o_mom);
+    w.loc = reinterpret_cast<double2*>(b + o_loc);
+    w.arrived = reinterpret_cast<unsigned*>(b + o_arr);
     w.rhs_part = reinterpret_cast<double2*>(b + o_rhs);
     w.circ_part = reinterpret_cast<double*>(b + o_circ);
     w.cub_tmp = b + o_cub;
@@ -2152,9 +2157,8 @@ int dvm_ctx_autotune(dvm_ctx* c, dvm_sim* const* sims, int nsims, int reps, dvm_
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     auto launch = [&](const dvm_pair_config& p) {
-        cudaMemsetAsync(ws.work, 0, sizeof(unsigned), c->stream);
         biot_savart_compute(T, S, p.order == 1 ? c->d_tune_list : sl.d_list, sl.n, kF32, ws,
-                            c->sms, c->stream, to_internal(p));
+                            c->sms, c->stream, to_internal(p), true);
     };
     int err = DVM_OK;
     // one untimed launch (module load, caches)
@@ -2166,10 +2170,10 @@ int dvm_ctx_autotune(dvm_ctx* c, dvm_sim* const* sims, int nsims, int reps, dvm_
     for (int k = 0; k < kNumCandidates && !err; ++k) {
         double ms = 0.0;
         for (int r = 0; r < reps; ++r) {
-            cudaMemsetAsync(ws.work, 0, sizeof(unsigned), c->stream);
             cudaEventRecord(a, c->stream);
             biot_savart_compute(T, S, kCandidates[k].order == 1 ? c->d_tune_list : sl.d_list,
-                                sl.n, kF32, ws, c->sms, c->stream, to_internal(kCandidates[k]));
+                                sl.n, kF32, ws, c->sms, c->stream, to_internal(kCandidates[k]),
+                                true);
             cudaEventRecord(b, c->stream);
             float t = 0.f;
             if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&t, a, b) != cudaSuccess) {
@@ -2217,7 +2221,7 @@ static int raw_reserve(dvm_ctx* c, size_t bytes) {
 // Runs the batched self-induced kernel on caller buffers through table slot 0.
 static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* circ,
                     const double* sigma, uint64_t n, double* u, double* w, int precision,
-                    double kx0, double kz0, double kinv) {
+                    double kx0, double kz0, double kinv) {  // kinv 0: domain from the blobs
     if (n == 0) return DVM_OK;
     if (n > 0xF0000000ull) return fail(DVM_ERR_ARG, "too many particles");
     const uint64_t cap = align_up(n, kCapAlign);
@@ -2256,6 +2260,7 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     Workspace ws = c->ws;
     ws.key_bits = key_bits_for(1);
     ws.total_cap = cap;
+    if (!(kinv > 0.0)) set_domain(c->d_table, x, z, (uint32_t)n, ws, c->sms, c->stream);
     biot_savart_self(c->d_table, c->d_state, d_list, 1, precision, ws, c->sms, c->stream,
                      tuned_config(c, shape_class(cap, 1)));
     g_launches += 4;  // keys, pack, pair kernel, combine
@@ -2270,7 +2275,7 @@ int dvm_biot_savart_self_device(dvm_ctx* c, const double* x, const double* z, co
     if (precision != DVM_F64 && precision != DVM_F32) return fail(DVM_ERR_ARG, "bad precision");
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    return raw_self(c, x, z, circ, sigma, n, u, w, precision, -64.0, -64.0, 65536.0 / 128.0);
+    return raw_self(c, x, z, circ, sigma, n, u, w, precision, 0.0, 0.0, 0.0);
 }
 
 int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velocity* out,

@@ -47,6 +47,21 @@ constexpr int kCapAlign = 1024;                // capacities are multiples of th
 constexpr int kMaxBatch = 1024;                // simulations per batched step
 constexpr int kTableCap = 4096;                // simulation slots per context
 
+constexpr int kLeaf = 64;                      // blobs per leaf of the far-field tree
+constexpr int kTerms = 24;                     // terms of its expansions
+constexpr int kNodeSlack = 32;                 // nodes per simulation beyond 2 per leaf
+
+// Node of the far-field tree (dvm_tree.cuh): the box and circle around its
+// blobs, their largest 10 sigma^2, and the exponent of its moments' scale.
+struct __align__(16) TreeNode {
+    double cx, cz;  // centre of the box
+    double R;       // radius around it
+    double thr;
+    double hx, hz;  // half extents of the box
+    int e, pad;
+    double pad2;
+};
+
 // Sources per work item of a simulation's blob-on-collocation right-hand side:
 // a power of two in [512, kAtChunk], the smallest that still leaves about 600
 // items (four per SM) when the simulation is evaluated alone, so a single
@@ -135,6 +150,7 @@ struct ListEntry {
     uint64_t poff;     // N-body partials offset (double2): sum chunks * cap
     uint64_t roff;     // at-target partials offset (double2): sum rhs_chunks * npad
     uint64_t cofs;     // circulation partials offset (double): sum rhs_chunks
+    uint64_t noff;     // first node of the far-field tree: sum 2 cap / kLeaf + kNodeSlack
 };
 
 // Per-tile bounds of a 256-blob tile of the spatially sorted sources.
@@ -154,13 +170,12 @@ struct Workspace {
     uint64_t packed_cap = 0;       // slots of `packed`
     TileMeta* meta = nullptr;      // total_cap / kBsST
     double2* part = nullptr;       // N-body partials
-    // FP32 N-body, mutual far tiles: per sorted blob two 64-bit fixed-point sums
-    // (Gamma_i K dz, Gamma_i K dx over the targets i whose tile evaluated this blob as a
-    // source), 2 * total_cap; and per simulation slot the exponent bounds of
-    // their scale (max |Gamma|, 1 / min core radius, max |coordinate|, one unused:
-    // 4 * kTableCap)
-    unsigned long long* macc = nullptr;
-    int* mexp = nullptr;
+    // FP32 N-body: the far-field tree of the sorted blobs (ListEntry::noff)
+    TreeNode* nodes = nullptr;
+    double2* mom = nullptr;        // kTerms moments per node
+    double2* loc = nullptr;        // kTerms local coefficients per node that is a target group
+    unsigned* arrived = nullptr;   // children done, per node
+    uint64_t nodes_cap = 0;
     double2* rhs_part = nullptr;   // at-target partials
     double* circ_part = nullptr;
     void* cub_tmp = nullptr;
@@ -191,7 +206,8 @@ struct PairConfig {
 };
 
 // Self-induced Biot-Savart (src/VelocityKernel.cpp:30-67) for every listed sim:
-// FP32 + compensated sums over spatially sorted blobs, or FP64 in blob order.
+// FP32 near pairs and FP64 far-field expansions over spatially sorted blobs, or
+// FP64 pairs.
 void biot_savart_self(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                       int precision, const Workspace& ws, int sms, cudaStream_t s,
                       const PairConfig& cfg = PairConfig());
@@ -201,9 +217,12 @@ void biot_savart_prepare(const InstDesc* table, InstState* st, const ListEntry* 
                          int precision, const Workspace& ws, int sms, cudaStream_t s);
 void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                          int precision, const Workspace& ws, int sms, cudaStream_t s,
-                         const PairConfig& cfg = PairConfig());
+                         const PairConfig& cfg = PairConfig(), bool dry = false);
 void biot_savart_finish(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                         int precision, const Workspace& ws, int sms, cudaStream_t s);
+// The sort domain of descriptor d (device) from the box of n device points.
+void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const Workspace& ws,
+                int sms, cudaStream_t s);
 // Blob-on-collocation right-hand side b (src/VortexSheet.cpp:171-210).
 void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s);

@@ -6,24 +6,19 @@
 //               u_i = -(1/2pi) sum_j K dz Gamma_j,  w_i = (1/2pi) sum_j K dx Gamma_j
 //
 // FP32 path (the throughput path): blobs of every listed simulation are sorted
-// along a Morton curve, packed as FP64 (x, z) + FP32 (Gamma, 10 sigma^2,
-// 1/sigma^2) and split into 256-blob tiles with bounding boxes.  A work item is
-// (simulation, 256 or 128 sorted targets, one source chunk); every warp pulls
-// items from an atomic counter on its own and stages 256 sources at a time in
-// its slice of shared memory.  Per staged tile the warp checks once, from the
-// boxes of its 256-target block and of the tile, whether any pair can fall
-// inside the 10 sigma^2 core: far tiles (almost all) run packed FP32x2
-// arithmetic with one MUFU reciprocal per pair and no test; near tiles run the
-// same packed arithmetic plus the exact per-pair test, the core kernel
-// evaluated as (1/sigma^2) phi(r^2/sigma^2) with the r -> 0 limit built in
-// (core_kernel).  Coordinates
-// are FP32 offsets from the first target of the enclosing 256-target block,
-// sums are FP32 within a stage and Kahan-compensated across stages, and chunk
-// partials are combined in FP64 in chunk order: deterministic, and independent
-// of the batch a simulation runs in and of the launch shape.
+// along a Hilbert curve, packed as FP64 (x, z) + FP32 (Gamma, 10 sigma^2,
+// 1/sigma^2) and cut into leaves of 64 blobs.  A binary tree over the leaves
+// carries FP64 expansions of the field outside the cores (dvm_tree.cuh).  A block
+// takes one leaf of targets: it walks the tree, translates every node that is
+// far enough into a local expansion about the leaf, and sums the few leaves
+// that remain pair by pair in packed FP32x2 arithmetic, each with the core
+// test only where a core can reach.  Coordinates are FP32 offsets from the
+// target leaf's first blob; sums are FP32 within a source leaf and FP64 across
+// leaves, in an order that the simulation's own blobs fix: deterministic, and
+// independent of the batch a simulation runs in and of the launch shape.
 //
-// FP64 path (the parity path): same work decomposition in original blob order
-// and the reference's exact operation sequence (no FMA contraction).
+// FP64 path (the parity path): every pair with the reference's operation
+// sequence (no FMA contraction), over 256-blob tiles of the same sorted order.
 #include <cfloat>
 #include <mutex>
 #include <string>
@@ -32,28 +27,78 @@
 
 #include "dvm_device.cuh"
 #include "dvm_internal.h"
+#include "dvm_tree.cuh"
 
 namespace dvmk {
 namespace {
 
 constexpr int kMaxList = kMaxBatch;  // simulations per batched launch
 
-__device__ __forceinline__ uint32_t spread16(uint32_t v) {
-    v &= 0xFFFFu;
-    v = (v | (v << 8)) & 0x00FF00FFu;
-    v = (v | (v << 4)) & 0x0F0F0F0Fu;
-    v = (v | (v << 2)) & 0x33333333u;
-    v = (v | (v << 1)) & 0x55555555u;
-    return v;
-}
-
-__device__ __forceinline__ uint32_t morton_key(double x, double z, double x0, double z0,
-                                               double inv) {
+// Index along a Hilbert curve over 2^16 x 2^16 cells (the standard quadrant
+// recursion: rotate and reflect the lower bits by the quadrant taken).  Runs of
+// consecutive blobs are spatially connected, so the boxes of sort tiles and
+// leaves stay compact where Morton order jumps.
+__device__ __forceinline__ uint32_t curve_key(double x, double z, double x0, double z0,
+                                              double inv) {
     double fx = (x - x0) * inv, fz = (z - z0) * inv;
     fx = fmin(fmax(fx, 0.0), 65535.0);
     fz = fmin(fmax(fz, 0.0), 65535.0);
-    const uint32_t key = spread16((uint32_t)fx) | (spread16((uint32_t)fz) << 1);
+    uint32_t a = (uint32_t)fx, b = (uint32_t)fz, key = 0;
+#pragma unroll 4
+    for (int k = 15; k >= 0; --k) {
+        const uint32_t ra = (a >> k) & 1u, rb = (b >> k) & 1u;
+        key = (key << 2) | ((3u * ra) ^ rb);
+        if (!rb) {
+            if (ra) {
+                a = ~a;
+                b = ~b;
+            }
+            const uint32_t t = a;
+            a = b;
+            b = t;
+        }
+    }
     return key == 0xFFFFFFFFu ? 0xFFFFFFFEu : key;
+}
+
+// Bounding box of n points as order-preserving bits: dom[0..3] = max of x, z,
+// -x, -z over the finite points (0: none yet).
+__device__ __forceinline__ unsigned long long ordered_bits(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double from_ordered_bits(unsigned long long o) {
+    return __longlong_as_double((long long)((o >> 63) ? (o & 0x7FFFFFFFFFFFFFFFull) : ~o));
+}
+__global__ void __launch_bounds__(256) k_domain(const double* __restrict__ x,
+                                                const double* __restrict__ z, uint32_t n,
+                                                unsigned long long* __restrict__ dom) {
+    double m[4] = {-DBL_MAX, -DBL_MAX, -DBL_MAX, -DBL_MAX};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double a = x[i], b = z[i];
+        if (fabs(a) < 1e300 && fabs(b) < 1e300) {
+            m[0] = fmax(m[0], a);
+            m[1] = fmax(m[1], b);
+            m[2] = fmax(m[2], -a);
+            m[3] = fmax(m[3], -b);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        for (int o = 16; o > 0; o >>= 1) m[k] = fmax(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+        if ((threadIdx.x & 31) == 0 && m[k] > -DBL_MAX) atomicMax(&dom[k], ordered_bits(m[k]));
+    }
+}
+
+// The sort domain of a simulation's descriptor from k_domain's box.
+__global__ void k_set_domain(InstDesc* __restrict__ d, const unsigned long long* __restrict__ dom) {
+    if (dom[0] == 0ull) return;  // no finite point: the domain is as good as any
+    const double x1 = from_ordered_bits(dom[0]), z1 = from_ordered_bits(dom[1]);
+    const double x0 = -from_ordered_bits(dom[2]), z0 = -from_ordered_bits(dom[3]);
+    const double L = fmax(x1 - x0, z1 - z0);
+    d->kx0 = x0;
+    d->kz0 = z0;
+    d->kinv = L > 0.0 ? 65535.0 / L : 1.0;
 }
 
 __device__ __forceinline__ int entry_of_slot(const ListEntry* list, int nlist, uint64_t g) {
@@ -66,7 +111,7 @@ __device__ __forceinline__ int entry_of_slot(const ListEntry* list, int nlist, u
     return lo;
 }
 
-// Sort keys over the concatenated capacity space: (entry << 32 | morton);
+// Sort keys over the concatenated capacity space: (entry << 32 | curve index);
 // unused slots sort to the end of their simulation's range.
 __global__ void k_keys(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
                        const ListEntry* __restrict__ list, int nlist, uint64_t total,
@@ -78,33 +123,23 @@ __global__ void k_keys(const InstDesc* __restrict__ table, const InstState* __re
         const uint32_t i = (uint32_t)(g - e.coff);
         const InstDesc& d = table[e.inst];
         uint32_t mk = 0xFFFFFFFFu;
-        if (i < st[e.inst].n) mk = morton_key(d.x[i], d.z[i], d.kx0, d.kz0, d.kinv);
+        if (i < st[e.inst].n) mk = curve_key(d.x[i], d.z[i], d.kx0, d.kz0, d.kinv);
         keys[g] = ((uint64_t)k << 32) | mk;
         vals[g] = i;
     }
 }
 
-// Gather (x, z, Gamma, sigma) into sorted order and record per-tile bounds.
+// Gather (x, z, Gamma, sigma) into sorted order and record per-tile bounds (FP64
+// path).
 __global__ void __launch_bounds__(kBsST) k_pack(const InstDesc* __restrict__ table,
                                                 const InstState* __restrict__ st,
                                                 const ListEntry* __restrict__ list, int nlist,
                                                 const uint32_t* __restrict__ perm,
                                                 double4* __restrict__ packed,
-                                                double2* __restrict__ pxz,
-                                                float4* __restrict__ pf,
-                                                TileMeta* __restrict__ meta,
-                                                int* __restrict__ mexp) {
+                                                TileMeta* __restrict__ meta) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    __shared__ double s_red[7][kBsST / 32];
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += (st[list[k].inst].n + kBsST - 1) / kBsST;
-        }
-        s_pre[nlist] = acc;
-    }
-    __syncthreads();
+    __shared__ double s_red[5][kBsST / 32];
+    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kBsST - 1) / kBsST; });
     const unsigned total = s_pre[nlist];
     for (unsigned item = blockIdx.x; item < total; item += gridDim.x) {
         const int k = locate(s_pre, nlist, item);
@@ -113,21 +148,13 @@ __global__ void __launch_bounds__(kBsST) k_pack(const InstDesc* __restrict__ tab
         const uint32_t n = st[e.inst].n;
         const uint32_t i = (item - s_pre[k]) * kBsST + threadIdx.x;
         double xmin = DBL_MAX, xmax = -DBL_MAX, zmin = DBL_MAX, zmax = -DBL_MAX, thr = 0.0;
-        double gmax = 0.0, tmin = DBL_MAX;  // max |Gamma| (as the FP32 path rounds it), min 10 sigma^2
         if (i < n) {
-            const uint32_t p = perm ? perm[e.coff + i] : i;
+            const uint32_t p = perm[e.coff + i];
             const double4 v = make_double4(d.x[p], d.z[p], d.circ[p], d.sigma[p]);
-            if (pxz) {  // FP32 path: positions in FP64, per-source constants in FP32
-                const double s2 = v.w * v.w;
-                pxz[e.coff + i] = make_double2(v.x, v.y);
-                pf[e.coff + i] = make_float4((float)v.z, (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
-            } else {
-                packed[e.coff + i] = v;
-            }
+            packed[e.coff + i] = v;
             xmin = xmax = v.x;
             zmin = zmax = v.y;
-            thr = tmin = 10.0 * (v.w * v.w);
-            gmax = fabs((double)(float)v.z);
+            thr = 10.0 * (v.w * v.w);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -136,8 +163,6 @@ __global__ void __launch_bounds__(kBsST) k_pack(const InstDesc* __restrict__ tab
             zmin = fmin(zmin, __shfl_xor_sync(0xffffffffu, zmin, o));
             zmax = fmax(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
             thr = fmax(thr, __shfl_xor_sync(0xffffffffu, thr, o));
-            gmax = fmax(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-            tmin = fmin(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
         }
         const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (lane == 0) {
@@ -146,8 +171,6 @@ __global__ void __launch_bounds__(kBsST) k_pack(const InstDesc* __restrict__ tab
             s_red[2][wid] = zmin;
             s_red[3][wid] = zmax;
             s_red[4][wid] = thr;
-            s_red[5][wid] = gmax;
-            s_red[6][wid] = tmin;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -166,37 +189,205 @@ __global__ void __launch_bounds__(kBsST) k_pack(const InstDesc* __restrict__ tab
             }
             m.pad0 = m.pad1 = m.pad2 = 0.0;
             meta[(e.coff + (uint64_t)(item - s_pre[k]) * kBsST) / kBsST] = m;
-            if (mexp) {  // exponent bounds of the simulation's mutual sums (order-free max)
-                double gm = s_red[5][0], tm = s_red[6][0];
-                for (int q = 1; q < kBsST / 32; ++q) {
-                    gm = fmax(gm, s_red[5][q]);
-                    tm = fmin(tm, s_red[6][q]);
-                }
-                const int eg = gm > 0.0 ? ilogb(gm) + 1 : -1100;  // max |Gamma| < 2^eg
-                const int es = (1 - ilogb(fmax(tm, 1e-30))) >> 1;  // 1 / sqrt(min) <= 2^es
-                const double cm = fmax(fmax(fabs(m.xmin), fabs(m.xmax)),
-                                       fmax(fabs(m.zmin), fabs(m.zmax)));
-                const int ec = cm > 0.0 ? ilogb(cm) + 1 : -1100;  // |coordinates| < 2^ec
-                atomicMax(&mexp[4 * e.inst], eg);
-                atomicMax(&mexp[4 * e.inst + 1], es);
-                atomicMax(&mexp[4 * e.inst + 2], ec);
-            }
         }
         __syncthreads();
     }
 }
 
-__device__ __forceinline__ void item_prefix_f64(unsigned* s_pre, const InstState* st,
-                                                 const ListEntry* list, int nlist) {
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += ((st[list[k].inst].n + kBsTT - 1) / kBsTT) * (unsigned)list[k].chunks;
+// ---- far-field tree of the sorted blobs ----------------------------------------
+// Sum over the warp of 8 complex values per lane: each step halves the values a
+// lane holds and the lanes that share one, so 8 sums cost 9 complex shuffles
+// instead of 40.  Returns value ((lane >> 2) & 7, bit-reversed as the exchanges
+// take them) complete in every lane.
+__device__ __forceinline__ Cplx warp_sum8(Cplx (&v)[8], int lane) {
+    const unsigned all = 0xffffffffu;
+#pragma unroll
+    for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const Cplx give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k].x = keep.x + __shfl_xor_sync(all, give.x, o);
+            v[k].y = keep.y + __shfl_xor_sync(all, give.y, o);
         }
-        s_pre[nlist] = acc;
     }
-    __syncthreads();
+#pragma unroll
+    for (int o = 2; o >= 1; o >>= 1) {
+        v[0].x += __shfl_xor_sync(all, v[0].x, o);
+        v[0].y += __shfl_xor_sync(all, v[0].y, o);
+    }
+    return v[0];
+}
+
+__device__ __forceinline__ int scale_exp(double R) {  // 2^e > R, clamped
+    return R > 0.0 ? max(-300, min(300, ilogb(R) + 1)) : -300;
+}
+
+// Gather the blobs in sorted order, and build the tree bottom up: a warp makes one
+// leaf (box, radius, moments), and the warp that completes a node's second half
+// goes on to make that node from its halves (moment-to-moment translations as a
+// convolution with the factorials divided out).  Nobody waits: the warp that
+// arrives first at a node leaves.  The halves are added in index order, so the
+// result does not depend on who arrives when.
+__global__ void __launch_bounds__(128) k_tree(const InstDesc* __restrict__ table,
+                                              const InstState* __restrict__ st,
+                                              const ListEntry* __restrict__ list, int nlist,
+                                              const uint32_t* __restrict__ perm,
+                                              double2* __restrict__ pxz, float4* __restrict__ pf,
+                                              TreeNode* __restrict__ nodes,
+                                              double2* __restrict__ mom,
+                                              unsigned* __restrict__ arrived) {
+    __shared__ unsigned s_pre[kMaxList + 1];
+    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
+    const unsigned total = s_pre[nlist], all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    double fact = 1.0;  // lane!
+    for (int k = 2; k <= lane; ++k) fact *= (double)k;
+    const double ifact = 1.0 / fact;
+    for (unsigned item = blockIdx.x * 4 + (threadIdx.x >> 5); item < total; item += gridDim.x * 4) {
+        const int k = locate(s_pre, nlist, item);
+        const ListEntry e = list[k];
+        const InstDesc& d = table[e.inst];
+        const uint32_t n = st[e.inst].n, C = e.cap / kLeaf;
+        const uint32_t nl = (n + kLeaf - 1) / kLeaf;
+        uint32_t idx = item - s_pre[k];
+        TreeNode* __restrict__ N = nodes + e.noff;
+        double2* __restrict__ A = mom + e.noff * kTerms;
+        unsigned* __restrict__ cnt = arrived + e.noff;
+        double px[2], pz[2], g[2];
+        double x0 = DBL_MAX, x1 = -DBL_MAX, z0 = DBL_MAX, z1 = -DBL_MAX, thr = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = idx * kLeaf + h * 32 + lane;
+            px[h] = pz[h] = g[h] = 0.0;
+            if (i < n) {
+                const uint32_t p = perm[e.coff + i];
+                const double sg = d.sigma[p], s2 = sg * sg;
+                px[h] = d.x[p];
+                pz[h] = d.z[p];
+                g[h] = d.circ[p];
+                pxz[e.coff + i] = make_double2(px[h], pz[h]);
+                pf[e.coff + i] = make_float4((float)g[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
+                x0 = fmin(x0, px[h]);
+                x1 = fmax(x1, px[h]);
+                z0 = fmin(z0, pz[h]);
+                z1 = fmax(z1, pz[h]);
+                thr = fmax(thr, 10.0 * s2);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            x0 = fmin(x0, __shfl_xor_sync(all, x0, o));
+            x1 = fmax(x1, __shfl_xor_sync(all, x1, o));
+            z0 = fmin(z0, __shfl_xor_sync(all, z0, o));
+            z1 = fmax(z1, __shfl_xor_sync(all, z1, o));
+            thr = fmax(thr, __shfl_xor_sync(all, thr, o));
+        }
+        TreeNode m;
+        m.cx = 0.5 * (x0 + x1);
+        m.cz = 0.5 * (z0 + z1);
+        m.hx = 0.5 * (x1 - x0);
+        m.hz = 0.5 * (z1 - z0);
+        m.thr = thr;
+        double r2 = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (idx * kLeaf + h * 32 + lane < n) {
+                px[h] -= m.cx;
+                pz[h] -= m.cz;
+                r2 = fmax(r2, px[h] * px[h] + pz[h] * pz[h]);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(all, r2, o));
+        m.R = sqrt(r2) * (1.0 + 1e-12);
+        m.e = scale_exp(m.R);
+        m.pad = 0;
+        m.pad2 = 0.0;
+        {
+            const double is = exp2_int(-m.e);
+            const Cplx q0{px[0] * is, pz[0] * is}, q1{px[1] * is, pz[1] * is};
+            Cplx t0{g[0], 0.0}, t1{g[1], 0.0};
+            const int own = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+            double2* __restrict__ out = A + (uint64_t)idx * kTerms;
+#pragma unroll
+            for (int c = 0; c < kTerms / 8; ++c) {
+                Cplx v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    v[q] = Cplx{t0.x + t1.x, t0.y + t1.y};
+                    t0 = cmul(t0, q0);
+                    t1 = cmul(t1, q1);
+                }
+                const Cplx sum = warp_sum8(v, lane);
+                if ((lane & 3) == 0) out[c * 8 + own] = make_double2(sum.x, sum.y);
+            }
+        }
+        if (lane == 0) N[idx] = m;
+        // the nodes above
+        for (int l = 0;; ++l) {
+            if (((nl + (1u << l) - 1) >> l) <= 1u) break;  // the root is done
+            const uint32_t par = idx >> 1, cl = (nl + (1u << l) - 1) >> l;
+            const unsigned kids = 2 * par + 1 < cl ? 2u : 1u;
+            __threadfence();
+            __syncwarp();
+            unsigned before = 0;
+            if (lane == 0) before = atomicAdd(&cnt[node_level(C, l + 1) + par], 1u);
+            before = __shfl_sync(all, before, 0);
+            if (before + 1 < kids) break;
+            __threadfence();
+            const uint64_t c0 = node_level(C, l) + 2ull * par;
+            // (__ldcg: the halves were written by other SMs during this launch)
+            auto node_in = [&](uint64_t at) {
+                TreeNode r;
+                const double2* q = reinterpret_cast<const double2*>(N + at);
+                const double2 a = __ldcg(q), b = __ldcg(q + 1), c = __ldcg(q + 2);
+                const int2 ee = __ldcg(reinterpret_cast<const int2*>(q + 3));
+                r.cx = a.x;
+                r.cz = a.y;
+                r.R = b.x;
+                r.thr = b.y;
+                r.hx = c.x;
+                r.hz = c.y;
+                r.e = ee.x;
+                return r;
+            };
+            const TreeNode a = node_in(c0), b = kids == 2 ? node_in(c0 + 1) : a;
+            const double bx0 = fmin(a.cx - a.hx, b.cx - b.hx), bx1 = fmax(a.cx + a.hx, b.cx + b.hx);
+            const double bz0 = fmin(a.cz - a.hz, b.cz - b.hz), bz1 = fmax(a.cz + a.hz, b.cz + b.hz);
+            m.cx = 0.5 * (bx0 + bx1);
+            m.cz = 0.5 * (bz0 + bz1);
+            m.hx = 0.5 * (bx1 - bx0);
+            m.hz = 0.5 * (bz1 - bz0);
+            m.thr = fmax(a.thr, b.thr);
+            const double ra = a.R + sqrt((a.cx - m.cx) * (a.cx - m.cx) + (a.cz - m.cz) * (a.cz - m.cz));
+            const double rb = b.R + sqrt((b.cx - m.cx) * (b.cx - m.cx) + (b.cz - m.cz) * (b.cz - m.cz));
+            m.R = fmin(fmax(ra, rb), sqrt(m.hx * m.hx + m.hz * m.hz)) * (1.0 + 1e-12);
+            m.e = scale_exp(m.R);
+            const double is = exp2_int(-m.e);
+            Cplx acc{0.0, 0.0};
+            for (unsigned q = 0; q < kids; ++q) {
+                const TreeNode& ch = q ? b : a;
+                Cplx v{0.0, 0.0};
+                if (lane < kTerms) {
+                    const double2 w = __ldcg(&A[(c0 + q) * kTerms + lane]);
+                    const double f = exp2_int((ch.e - m.e) * lane) * ifact;
+                    v = Cplx{w.x * f, w.y * f};
+                }
+                Cplx h = cpow_lane(Cplx{(ch.cx - m.cx) * is, (ch.cz - m.cz) * is}, lane);
+                h.x *= ifact;
+                h.y *= ifact;
+#pragma unroll 4
+                for (int j = 0; j < kTerms; ++j) {
+                    const Cplx aj = cshfl(v, j), hj = cshfl(h, (lane - j) & 31);
+                    if (lane >= j) acc = cfma(aj, hj, acc);
+                }
+            }
+            idx = par;
+            if (lane < kTerms)
+                A[(node_level(C, l + 1) + par) * kTerms + lane] = make_double2(acc.x * fact, acc.y * fact);
+            if (lane == 0) N[node_level(C, l + 1) + par] = m;
+        }
+    }
 }
 
 __device__ __forceinline__ uint32_t chunk_size(uint32_t n, int chunks) {
@@ -205,158 +396,26 @@ __device__ __forceinline__ uint32_t chunk_size(uint32_t n, int chunks) {
 }
 
 // ---- FP32 pair loops --------------------------------------------------------
-// A work item belongs to ONE warp: one 256-blob sort tile of targets (8
-// consecutive ones per lane, 4 packed FP32x2 target pairs) against one source
-// chunk.  The warp stages its own source tiles in shared memory and never waits
-// for other warps, so far-path and near-path warps of a block do not hold each
-// other up at barriers.
-//
-// Tile pairs.  A (target tile a, source tile b) stage is
-//   mutual far  when the two tiles' boxes are farther apart than both tiles'
-//               core radii (every pair, either way round, has K = 1/r2): the
-//               item of the lower tile evaluates it once for both directions
-//               and the item of the upper tile skips it;
-//   far         when only the source cores are out of reach (no core test);
-//   near        otherwise (the exact core test per pair; a == b is near).
-constexpr int kWWarps = 4;            // independent warps per block
-constexpr int kSelfMinBlocks = 4;     // blocks per SM the registers allow (128 each)
-constexpr int kWR = 8;                // targets per lane
-constexpr int kWP = kWR / 2;          // packed target pairs per lane
+// A warp sums one staged source leaf at the 64 targets of a leaf, two targets
+// per lane.  Two SOURCES share a packed FP32x2 instruction: their values come
+// out of shared memory as register pairs (no duplicating moves), the targets'
+// are duplicated once per item.
+constexpr int kNearWarps = 4;   // warps of a block
+constexpr int kNearBlocks = 5;  // blocks per SM at full occupancy
+constexpr int kNearSlots = 8;   // partial sums of an item: list entries q, q + 8, ...
 
-// A warp's staged source tile: pos2[i] = (x, z) of sources 2i and 2i+1 (FP32
-// offsets), gam2[i] = (Gamma, Gamma) of both, core[j] = (10 sigma^2,
-// 1/sigma^2).  The loops read two sources with two 16-byte loads and duplicate
-// x and z into packed register pairs themselves (half the shared-memory loads
-// of one 32-byte record per source: 0.6 % faster, same results).
-struct StagedTile {
-    float4 pos2[kBsST / 2];
-    float4 gam2[kBsST / 2];
-    float2 core[kBsST];
+__device__ __forceinline__ void split_hi_lo(double v, float& hi, float& lo) {
+    hi = (float)v;
+    lo = (float)(v - (double)hi);
+}
+
+struct StagedLeaf {
+    float4 pos[kLeaf / 2];   // (x a, x b, z a, z b) of sources 2i, 2i + 1 (offsets)
+    float2 gam[kLeaf / 2];   // Gamma of both
+    float2 thr[kLeaf / 2];   // 10 sigma^2 of both
+    float2 rs[kLeaf / 2];    // 1 / sigma^2 of both
+    float4 low[kLeaf / 2];   // WIDE: what pos leaves of the offsets, same order
 };
-
-// One staged source against the warp's targets (far: no core test).
-template <int WP>
-__device__ __forceinline__ void far_pair(uint64_t sx, uint64_t sz, uint64_t sg,
-                                         const uint64_t (&tx2)[WP], const uint64_t (&tz2)[WP],
-                                         uint64_t (&nu2)[WP], uint64_t (&w2)[WP]) {
-#pragma unroll
-    for (int q = 0; q < WP; ++q) {
-        const uint64_t dx = f2sub(tx2[q], sx);
-        const uint64_t dz = f2sub(tz2[q], sz);
-        const uint64_t r2 = f2fma(dx, dx, f2mul(dz, dz));
-        // one MUFU reciprocal per pair (padded sources: rcp of ~2e36, Gamma 0)
-        const uint64_t inv = f2pack(rcp_approx(f2lo(r2)), rcp_approx(f2hi(r2)));
-        const uint64_t g = f2mul(inv, sg);
-        nu2[q] = f2fma(g, dz, nu2[q]);
-        w2[q] = f2fma(g, dx, w2[q]);
-    }
-}
-
-// Far pairs: no core test.  Accumulates -u (so every update is one FMA) and w.
-// (Sharing one reciprocal between the two targets of a packed pair, 1/a = b/(ab),
-// trades one MUFU operation for three FP32 multiplications; it measured 1-4 %
-// slower for 1/8 to 1/2 of the sources, the FMA pipe being nearly as loaded as
-// the MUFU pipe.  So did a Newton reciprocal on the FMA pipe for one source in
-// sixteen: 3.5 % slower at N = 2^20.)
-template <int WP>
-__device__ __forceinline__ void stage_far(const StagedTile& __restrict__ src,
-                                          const uint64_t (&tx2)[WP], const uint64_t (&tz2)[WP],
-                                          uint64_t (&nu2)[WP], uint64_t (&w2)[WP]) {
-#pragma unroll 4  // 8 sources per unrolled body
-    for (int i = 0; i < kBsST / 2; ++i) {
-        const float4 P = src.pos2[i];
-        const float4 G = src.gam2[i];
-        far_pair(f2pack(P.x, P.x), f2pack(P.y, P.y), f2pack(G.x, G.y), tx2, tz2, nu2, w2);
-        far_pair(f2pack(P.z, P.z), f2pack(P.w, P.w), f2pack(G.z, G.w), tx2, tz2, nu2, w2);
-    }
-}
-
-// Mutual far pairs: one reciprocal per pair serves both directions.  Besides
-// the targets' sums (as far_pair), the lane adds Gamma_i K (dz_ij, dx_ij) of its
-// targets i to source j's packed sums snu, sw; the source's own velocity takes
-// them with the opposite sign (dx_ji = -dx_ij).  Padding targets carry Gamma 0.
-__device__ __forceinline__ void mutual_pair(uint64_t sx, uint64_t sz, uint64_t sg,
-                                            const uint64_t (&tx2)[kWP],
-                                            const uint64_t (&tz2)[kWP],
-                                            const uint64_t (&tg2)[kWP], uint64_t (&nu2)[kWP],
-                                            uint64_t (&w2)[kWP], uint64_t& snu, uint64_t& sw) {
-#pragma unroll
-    for (int q = 0; q < kWP; ++q) {
-        const uint64_t dx = f2sub(tx2[q], sx);
-        const uint64_t dz = f2sub(tz2[q], sz);
-        const uint64_t r2 = f2fma(dx, dx, f2mul(dz, dz));
-        const uint64_t inv = f2pack(rcp_approx(f2lo(r2)), rcp_approx(f2hi(r2)));
-        const uint64_t g = f2mul(inv, sg);
-        nu2[q] = f2fma(g, dz, nu2[q]);
-        w2[q] = f2fma(g, dx, w2[q]);
-        const uint64_t h = f2mul(inv, tg2[q]);
-        snu = f2fma(h, dz, snu);
-        sw = f2fma(h, dx, sw);
-    }
-}
-
-// v 2^shift rounded to a 64-bit integer (two's complement in the unsigned
-// accumulator; the conversion saturates outside the 64-bit range).
-__device__ __forceinline__ unsigned long long to_fixed(double v, double scale) {
-    return (unsigned long long)__double2ll_rn(v * scale);
-}
-
-// A mutual far stage.  The staged sources form 64 groups of four, taken in
-// two rounds of 32.  In step s of a round lane l evaluates group (l + s) mod 32
-// against its 8 targets, adding to the group's packed sums (Gamma_i K dz,
-// Gamma_i K dx per source; low and high halves from the even and odd targets),
-// then hands the sums to lane l - 1, which takes that group in step s + 1.
-// After 32 steps lane l holds the sums of group l over all 256 targets, in a
-// fixed order, and adds them to the sources' 64-bit fixed-point accumulators
-// acc[2 j], acc[2 j + 1] (value x 2^shift, rounded; integer addition is exact
-// and order-free, so the sums do not depend on which warp adds first).  The
-// hand-over costs 16 shuffles per 32 pairs and no arithmetic (a shuffle-tree
-// reduction per batch of sources was 3.5 % slower).  Sources j >= n are padding.
-__device__ __forceinline__ void stage_mutual(const StagedTile& __restrict__ src,
-                                             const uint64_t (&tx2)[kWP],
-                                             const uint64_t (&tz2)[kWP],
-                                             const uint64_t (&tg2)[kWP], uint64_t (&nu2)[kWP],
-                                             uint64_t (&w2)[kWP],
-                                             unsigned long long* __restrict__ acc,
-                                             uint32_t nsrc, double scale, int lane) {
-    const unsigned all = 0xffffffffu;
-    const int next = (lane + 1) & 31;
-#pragma unroll 1
-    for (int rnd = 0; rnd < kBsST / 128; ++rnd) {
-        uint64_t au[4], aw[4];  // packed sums of the group this lane holds
-#pragma unroll
-        for (int b = 0; b < 4; ++b) au[b] = aw[b] = 0ull;
-#pragma unroll 1
-        for (int s = 0; s < 32; ++s) {
-            const int gi = rnd * 32 + ((lane + s) & 31);  // group of 4 sources
-            const float4 P0 = src.pos2[2 * gi], P1 = src.pos2[2 * gi + 1];
-            const float4 G0 = src.gam2[2 * gi], G1 = src.gam2[2 * gi + 1];
-            mutual_pair(f2pack(P0.x, P0.x), f2pack(P0.y, P0.y), f2pack(G0.x, G0.y), tx2, tz2,
-                        tg2, nu2, w2, au[0], aw[0]);
-            mutual_pair(f2pack(P0.z, P0.z), f2pack(P0.w, P0.w), f2pack(G0.z, G0.w), tx2, tz2,
-                        tg2, nu2, w2, au[1], aw[1]);
-            mutual_pair(f2pack(P1.x, P1.x), f2pack(P1.y, P1.y), f2pack(G1.x, G1.y), tx2, tz2,
-                        tg2, nu2, w2, au[2], aw[2]);
-            mutual_pair(f2pack(P1.z, P1.z), f2pack(P1.w, P1.w), f2pack(G1.z, G1.w), tx2, tz2,
-                        tg2, nu2, w2, au[3], aw[3]);
-            // the group moves on to the lane that takes it next (lane - 1)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                au[b] = __shfl_sync(all, au[b], next);
-                aw[b] = __shfl_sync(all, aw[b], next);
-            }
-        }
-        // after 32 steps every lane's targets have passed over the group this lane holds
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t j = 4 * (rnd * 32 + lane) + b;
-            if (j < nsrc) {  // u_j += sum Gamma_i K dz_ij, w_j -= sum Gamma_i K dx_ij
-                atomicAdd(&acc[2 * j], to_fixed((double)(f2lo(au[b]) + f2hi(au[b])), scale));
-                atomicAdd(&acc[2 * j + 1], to_fixed(-(double)(f2lo(aw[b]) + f2hi(aw[b])), scale));
-            }
-        }
-    }
-}
 
 // Core kernel (1 - exp(-r2/sigma^2)) / r2 in FP32, written as rs phi(t) with
 // t = r2 rs, rs = 1/sigma^2 and phi(t) = (1 - e^-t) / t.  For t < 1/2 phi is
@@ -389,56 +448,65 @@ __device__ __forceinline__ float core_kernel_expm1(float r2, float rs, float rcp
     return r2 > 1e-30f ? -e * rcp_r2 : rs;
 }
 
-// One staged source against the warp's targets with the exact core test.  SELF
-// (the target tile's own sources): a pair at r2 == 0 adds nothing, which is the
+// The staged leaf against the lane's two targets.  MODE 0: no core reaches (the
+// 1/r^2 branch without a test); 1: the reference's exact test per pair; 2: the
+// same for the targets' own leaf, where a pair at r2 == 0 adds nothing -- the
 // reference's i != j skip for the self pair whatever the core size (sigma = 0
-// would otherwise give 1/0 times dz = 0).
-template <int WP, bool SELF>
-__device__ __forceinline__ void near_pair(uint64_t sx, uint64_t sz, uint64_t sg, float2 C,
-                                          const uint64_t (&tx2)[WP], const uint64_t (&tz2)[WP],
-                                          uint64_t (&nu2)[WP], uint64_t (&w2)[WP]) {
+// would otherwise give 1/0 times dz = 0).  A pair outside the core gets the
+// same bits in every mode; the core kernel runs for both halves, branch-free,
+// whenever any lane of the warp has a pair inside a core, and a select keeps it
+// only for those pairs, so a pair's value does not depend on its neighbours.
+// Accumulates -u and w, even and odd sources apart.
+//
+// WIDE: for a target leaf much wider than the source leaf, or than its
+// neighbours (blobs of two distant clusters, a sparse fringe).  Offsets from
+// its first blob would carry the rounding of its extent into close pairs, so
+// they are kept in two FP32 parts, hi + low: dx = (t_hi - s_hi) + (t_low -
+// s_low), exact before its last rounding for close pairs.
+template <int MODE, bool WIDE>
+__device__ __forceinline__ void leaf_sum(const StagedLeaf& __restrict__ src,
+                                         const uint64_t (&tx2)[2], const uint64_t (&tz2)[2],
+                                         const uint64_t (&lx2)[2], const uint64_t (&lz2)[2],
+                                         uint64_t (&nu2)[2], uint64_t (&w2)[2]) {
+#pragma unroll 4
+    for (int i = 0; i < kLeaf / 2; ++i) {
+        const float4 P = src.pos[i];
+        const float2 G = src.gam[i];
+        const uint64_t sx = f2pack(P.x, P.y), sz = f2pack(P.z, P.w), sg = f2pack(G.x, G.y);
+        const float4 L = WIDE ? src.low[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 T = make_float2(0.f, 0.f), S = make_float2(0.f, 0.f);
+        if (MODE) {
+            T = src.thr[i];
+            S = src.rs[i];
+        }
 #pragma unroll
-    for (int q = 0; q < WP; ++q) {
-        const uint64_t dx = f2sub(tx2[q], sx);
-        const uint64_t dz = f2sub(tz2[q], sz);
-        const uint64_t r2 = f2fma(dx, dx, f2mul(dz, dz));
-        const float ra = f2lo(r2), rb = f2hi(r2);
-        float ka = rcp_approx(ra), kb = rcp_approx(rb);
-        const bool ca = ra < C.x, cb = rb < C.x;
-        if (__any_sync(0xffffffffu, ca || cb)) {
-            const float qa = core_kernel(ra, C.y, ka), qb = core_kernel(rb, C.y, kb);
-            ka = ca ? qa : ka;
-            kb = cb ? qb : kb;
+        for (int t = 0; t < 2; ++t) {
+            uint64_t dx = f2sub(tx2[t], sx);
+            uint64_t dz = f2sub(tz2[t], sz);
+            if (WIDE) {
+                dx = f2add(dx, f2sub(lx2[t], f2pack(L.x, L.y)));
+                dz = f2add(dz, f2sub(lz2[t], f2pack(L.z, L.w)));
+            }
+            const uint64_t r2 = f2fma(dx, dx, f2mul(dz, dz));
+            const float ra = f2lo(r2), rb = f2hi(r2);
+            // one MUFU reciprocal per pair (padded sources: rcp of ~2e36, Gamma 0)
+            float ka = rcp_approx(ra), kb = rcp_approx(rb);
+            if (MODE) {
+                const bool ca = ra < T.x, cb = rb < T.y;
+                if (__any_sync(0xffffffffu, ca || cb)) {
+                    const float qa = core_kernel(ra, S.x, ka), qb = core_kernel(rb, S.y, kb);
+                    ka = ca ? qa : ka;
+                    kb = cb ? qb : kb;
+                }
+                if (MODE == 2) {
+                    ka = ra > 0.0f ? ka : 0.0f;
+                    kb = rb > 0.0f ? kb : 0.0f;
+                }
+            }
+            const uint64_t g = f2mul(f2pack(ka, kb), sg);
+            nu2[t] = f2fma(g, dz, nu2[t]);
+            w2[t] = f2fma(g, dx, w2[t]);
         }
-        if (SELF) {
-            ka = ra > 0.0f ? ka : 0.0f;
-            kb = rb > 0.0f ? kb : 0.0f;
-        }
-        const uint64_t g = f2mul(f2pack(ka, kb), sg);
-        nu2[q] = f2fma(g, dz, nu2[q]);
-        w2[q] = f2fma(g, dx, w2[q]);
-    }
-}
-
-// Near pairs: the reference's exact test per pair.  The shared arithmetic is
-// packed like the far path (each half rounds like the scalar instruction, so a
-// pair outside the core gets the same bits on either path); the core kernel
-// runs for both halves of a packed pair, branch-free, whenever any lane of the
-// warp has a pair inside the core, and a select keeps it only for those pairs,
-// so a pair's value does not depend on its neighbours in the warp.
-template <int WP, bool SELF>
-__device__ __forceinline__ void stage_near(const StagedTile& __restrict__ src,
-                                           const uint64_t (&tx2)[WP], const uint64_t (&tz2)[WP],
-                                           uint64_t (&nu2)[WP], uint64_t (&w2)[WP]) {
-#pragma unroll 1
-    for (int i = 0; i < kBsST / 2; ++i) {
-        const float4 P = src.pos2[i];
-        const float4 G = src.gam2[i];
-        const float2 C0 = src.core[2 * i], C1 = src.core[2 * i + 1];
-        near_pair<WP, SELF>(f2pack(P.x, P.x), f2pack(P.y, P.y), f2pack(G.x, G.y), C0, tx2, tz2,
-                            nu2, w2);
-        near_pair<WP, SELF>(f2pack(P.z, P.z), f2pack(P.w, P.w), f2pack(G.z, G.w), C1, tx2, tz2,
-                            nu2, w2);
     }
 }
 
@@ -449,164 +517,292 @@ __device__ __forceinline__ void kahan(float& s, float& c, float x) {
     s = t;
 }
 
-// Scale exponent of a simulation's fixed-point velocity sums.  One pair adds at
-// most |Gamma_j| K r: 1/r <= 1/sqrt(10 sigma_j^2) outside the core and at most
-// 0.64/sigma_j = 2.02/sqrt(10 sigma_j^2) inside it, so every sum is below
-// 2.02 n max|Gamma| / r_min with r_min = sqrt(min 10 sigma^2); k_pack bounds
-// max|Gamma| < 2^mexp[0] and 1/sqrt(min) <= 2^mexp[1].  Cores far smaller than
-// the blobs' spacing (sigma = 0 above all: 1/r^2 for every pair) would make that
-// bound meaningless and round every sum to zero, so r_min is floored at 2^-20 of
-// the coordinates' magnitude (|x|, |z| < 2^mexp[2]).  With the shift below
-// |sum| 2^shift < 2^58, well inside 64 bits, and one unit is 2^-56 of the bound
-// (below 2e-17 of it; the FP32 terms carry 6e-8).  Under the floor a sum can
-// leave the 64-bit range (32 times the bound) only through a pair closer than
-// 2^-26 / n of 2^mexp[2] with a core smaller still: point vortices closer than
-// the FP32 offsets (relative to a 256-blob tile) resolve in most layouts.
-__device__ __forceinline__ int mutual_shift(const int* __restrict__ mexp, int inst, uint32_t n) {
-    const int lgn = n > 1 ? 32 - __clz(n - 1) : 0;
-    const long long es = min((long long)mexp[4 * inst + 1], 20ll - mexp[4 * inst + 2]);
-    const long long e = (long long)lgn + mexp[4 * inst] + es;
-    return (int)max(-1000ll, min(1000ll, 56 - e));
+// Local expansions of every target group of every listed simulation: one block
+// per group (the wide groups first, they have the most to translate), each warp
+// translating every fourth node of its list; the warps' sums are added in order.
+struct FarShared {
+    TreeWalk walk;
+    Cplx buf[kWalk / 32][kTerms];
+    double2 at[kLeaf];
+};
+constexpr int kFarBlocks = 4;  // blocks per SM (the translation matrix's row: 48 registers)
+
+__device__ __forceinline__ uint32_t groups_at(uint32_t nl, int c) {  // groups of chain place c
+    return c < chain_length(nl) ? (nl + (1u << (kFarStep * c)) - 1) >> (kFarStep * c) : 0u;
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(32 * kWWarps, MINB)
-    k_self_f32(const InstState* __restrict__ st, const ListEntry* __restrict__ list, int nlist,
-               const double2* __restrict__ pxz, const float4* __restrict__ pf,
-               const TileMeta* __restrict__ meta, unsigned long long* __restrict__ macc,
-               const int* __restrict__ mexp, unsigned* __restrict__ work) {
+__global__ void __launch_bounds__(kWalk, kFarBlocks)
+    k_far(const InstState* __restrict__ st, const ListEntry* __restrict__ list, int nlist,
+          const double2* __restrict__ pxz, const TreeNode* __restrict__ nodes,
+          const double2* __restrict__ mom, double2* __restrict__ loc,
+          unsigned* __restrict__ work) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    __shared__ StagedTile s_src[kWWarps];
-    // Kahan sums of -u and w per lane, in shared memory rather than registers
-    // (touched once per stage; the registers go to the pair arithmetic: 4 CTAs per
-    // SM at 128 registers, 6 % faster than 3 CTAs with the sums in registers)
-    __shared__ float s_kahan[kWWarps][4][kWR][32];
-    constexpr int kWTT = 32 * kWR;
-    static_assert(kWTT == kBsST, "a work item's targets are one sort tile");
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += ((st[list[k].inst].n + kWTT - 1) / kWTT) * (unsigned)list[k].chunks;
-        }
-        s_pre[nlist] = acc;
-    }
-    __syncthreads();
+    __shared__ FarShared S;
+    __shared__ unsigned s_item;
+    list_prefix(s_pre, nlist, [&](int k) {
+        const uint32_t nl = (st[list[k].inst].n + kLeaf - 1) / kLeaf;
+        uint32_t g = 0;
+        for (int c = 0; c < kChainMax; ++c) g += groups_at(nl, c);
+        return g;
+    });
     const unsigned total = s_pre[nlist];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    StagedTile& wsrc = s_src[wid];
-    float2* __restrict__ wpos = reinterpret_cast<float2*>(wsrc.pos2);
-    float2* __restrict__ wgam = reinterpret_cast<float2*>(wsrc.gam2);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double row[kTerms];
+    binomial_row(row, lane);
     for (;;) {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(work, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
+        __syncthreads();
+        if (tid == 0) s_item = atomicAdd(work, 1u);
+        __syncthreads();
+        const unsigned item = s_item;
         if (item >= total) break;
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
-        const uint32_t n = st[e.inst].n;
-        const unsigned local = item - s_pre[k];
-        const uint32_t tile = local / e.chunks, c = local % e.chunks;
-        const uint32_t t0 = tile * kWTT;
-        const uint32_t cs = chunk_size(n, e.chunks);
-        const uint32_t j0 = c * cs, j1 = min(n, j0 + cs);
-        const double2* __restrict__ X = pxz + e.coff;
-        const float4* __restrict__ F = pf + e.coff;
-        // FP32 offsets from the tile's first target
-        const double2 o = X[t0];
-        const double scale = ldexp(1.0, mutual_shift(mexp, e.inst, n));
-
-        uint64_t tx2[kWP], tz2[kWP], tg2[kWP];
-        const uint32_t tb = t0 + lane * kWR;
-#pragma unroll
-        for (int q = 0; q < kWP; ++q) {
-            float xs[2], zs[2], gs[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                xs[h] = 0.0f;  // padding targets sit on the origin (a real target), Gamma 0
-                zs[h] = 0.0f;
-                gs[h] = 0.0f;
-                const uint32_t t = tb + 2 * q + h;
-                if (t < n) {
-                    const double2 p = X[t];
-                    xs[h] = (float)(p.x - o.x);
-                    zs[h] = (float)(p.y - o.y);
-                    gs[h] = F[t].x;
-                }
+        const uint32_t n = st[e.inst].n, C = e.cap / kLeaf;
+        const uint32_t nl = (n + kLeaf - 1) / kLeaf;
+        const TreeNode* __restrict__ N = nodes + e.noff;
+        const double2* __restrict__ A = mom + e.noff * kTerms;
+        uint32_t idx = item - s_pre[k];
+        int c = chain_length(nl) - 1;
+        while (idx >= groups_at(nl, c)) idx -= groups_at(nl, c--);
+        const int level = kFarStep * c;
+        const uint32_t t0 = idx * kLeaf;  // (a leaf's)
+        if (c == 0 && tid < kLeaf) S.at[tid] = pxz[e.coff + min(t0 + tid, n - 1)];
+        walk_begin(S.walk, N, C, nl, level, idx, c == 0 ? (int)min((uint32_t)kLeaf, n - t0) : 0, S.at);
+        const TargetBox tb = S.walk.chain[0];
+        Cplx b{0.0, 0.0};  // lane l: local coefficient l, this warp's share
+        for (bool more = true; more;) {
+            do more = walk_step<true>(S.walk, N, C, nl);  // until the list could overflow
+            while (more && S.walk.n[0] + kWalk <= kListCap);
+            const int nfar = S.walk.n[0];
+            for (int q = wid; q < nfar; q += kWalk / 32) {
+                const uint32_t id = S.walk.list[0][q];
+                const uint64_t at = node_level(C, (int)(id >> 27)) + (id & ((1u << 27) - 1));
+                translate(N[at], A + at * kTerms, tb, row, S.buf[wid], lane, b);
             }
-            tx2[q] = f2pack(xs[0], xs[1]);
-            tz2[q] = f2pack(zs[0], zs[1]);
-            tg2[q] = f2pack(gs[0], gs[1]);
+            __syncthreads();
+            if (tid == 0) S.walk.n[0] = 0;
+            __syncthreads();
         }
-        const TileMeta& tm = meta[(e.coff + t0) / kBsST];
-        float (*kh)[kWR][32] = s_kahan[wid];  // [0] -u, [1] its compensation, [2] w, [3]
-#pragma unroll
-        for (int r = 0; r < kWR; ++r)
-            kh[0][r][lane] = kh[1][r][lane] = kh[2][r][lane] = kh[3][r][lane] = 0.0f;
-
-        for (uint32_t s0 = j0; s0 < j1; s0 += kBsST) {
-            const TileMeta m = meta[(e.coff + s0) / kBsST];
-            const double gx = fmax(0.0, fmax(m.xmin - tm.xmax, tm.xmin - m.xmax));
-            const double gz = fmax(0.0, fmax(m.zmin - tm.zmax, tm.zmin - m.zmax));
-            const double g2 = gx * gx + gz * gz;
-            // the same test in both tiles' items (symmetric in the two tiles)
-            const bool mutual = g2 > fmax(m.thr, tm.thr) * 1.001 + 1e-30;
-            if (mutual && s0 < t0) continue;  // the source tile's item adds this stage
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < kBsST / 32; ++q) {
-                const uint32_t jj = q * 32 + lane, j = s0 + jj;
-                if (j < j1) {
-                    const double2 p = X[j];
-                    const float4 f = F[j];  // (circ, 10 sigma^2, 1/sigma^2, -)
-                    wpos[jj] = make_float2((float)(p.x - o.x), (float)(p.y - o.y));
-                    wgam[jj] = make_float2(f.x, f.x);
-                    wsrc.core[jj] = make_float2(f.y, f.z);
-                } else {  // padding: far away, no circulation, never in a core
-                    wpos[jj] = make_float2(1e18f, 1e18f);
-                    wgam[jj] = make_float2(0.0f, 0.0f);
-                    wsrc.core[jj] = make_float2(-1.0f, 0.0f);
-                }
+        __syncwarp();
+        if (lane < kTerms) S.buf[wid][lane] = b;
+        __syncthreads();
+        if (tid < kTerms) {
+            Cplx v = S.buf[0][tid];
+            for (int q = 1; q < kWalk / 32; ++q) {
+                v.x += S.buf[q][tid].x;
+                v.y += S.buf[q][tid].y;
             }
-            __syncwarp();
-            uint64_t nu2[kWP], w2[kWP];
-#pragma unroll
-            for (int q = 0; q < kWP; ++q) nu2[q] = w2[q] = 0ull;  // +0.0f in both halves
-            if (mutual) {
-                stage_mutual(wsrc, tx2, tz2, tg2, nu2, w2, macc + 2 * (e.coff + s0),
-                             min((uint32_t)kBsST, j1 - s0), scale, lane);
-            } else if (g2 > m.thr * 1.001 + 1e-30) {
-                stage_far(wsrc, tx2, tz2, nu2, w2);
-            } else if (s0 == t0) {
-                stage_near<kWP, true>(wsrc, tx2, tz2, nu2, w2);
-            } else {
-                stage_near<kWP, false>(wsrc, tx2, tz2, nu2, w2);
-            }
-#pragma unroll
-            for (int q = 0; q < kWP; ++q) {  // Kahan fold of the stage partials
-                kahan(kh[0][2 * q][lane], kh[1][2 * q][lane], f2lo(nu2[q]));
-                kahan(kh[0][2 * q + 1][lane], kh[1][2 * q + 1][lane], f2hi(nu2[q]));
-                kahan(kh[2][2 * q][lane], kh[3][2 * q][lane], f2lo(w2[q]));
-                kahan(kh[2][2 * q + 1][lane], kh[3][2 * q + 1][lane], f2hi(w2[q]));
-            }
+            loc[(e.noff + node_level(C, level) + idx) * kTerms + tid] = make_double2(v.x, v.y);
         }
-        // the item's sums join the targets' fixed-point sums (exact, order-free)
-        unsigned long long* __restrict__ ta = macc + 2 * (e.coff + tb);
-#pragma unroll
-        for (int r = 0; r < kWR; ++r)
-            if (tb + r < n) {
-                atomicAdd(&ta[2 * r],
-                          to_fixed(-((double)kh[0][r][lane] - (double)kh[1][r][lane]), scale));
-                atomicAdd(&ta[2 * r + 1],
-                          to_fixed((double)kh[2][r][lane] - (double)kh[3][r][lane], scale));
-            }
     }
 }
+
+// Near pairs, and the sum of everything: one block per leaf of 64 targets, taken
+// from a counter.  The walk's lists are worked off whenever they fill and at its
+// end; their entries go to kNearSlots partial sums by their place in the list (a
+// warp serves several slots in turn), which are added in slot order.  The local
+// expansions of the leaf's chain are evaluated at the targets at the end.
+//
+// Measured (B200, wake of 2^20 blobs, sigma 0.0169): the whole velocity call
+// 2.56 ms, of which this kernel 1.34, k_far 0.82 and k_tree 0.28, against
+// 215 ms for all pairs in mutual FP32x2 tiles at 80 % of the FP32 peak;
+// 2^16: 0.33 against 1.21 ms; 5003 blobs: 0.21 against 0.28 ms.  Relative L2
+// error against FP64 1.3e-7 (all pairs: 5.7e-7 to 7.6e-7) at 2^18.
+struct NearShared {
+    TreeWalk walk;
+    StagedLeaf src[kNearWarps];
+    Cplx buf[kNearWarps][kTerms];
+    double2 at[kLeaf];
+    double2 sum[kNearSlots][kLeaf];
+};
+
+template <int MINB>
+__global__ void __launch_bounds__(32 * kNearWarps, MINB)
+    k_self_f32(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
+               const ListEntry* __restrict__ list, int nlist, const double2* __restrict__ pxz,
+               const float4* __restrict__ pf, const uint32_t* __restrict__ perm,
+               const TreeNode* __restrict__ nodes, const double2* __restrict__ mom,
+               const double2* __restrict__ loc, double* __restrict__ dry_u,
+               double* __restrict__ dry_w, unsigned* __restrict__ work) {
+    __shared__ unsigned s_pre[kMaxList + 1];
+    __shared__ NearShared S;
+    __shared__ unsigned s_item;
+    static_assert(32 * kNearWarps == kWalk, "the whole block walks");
+    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
+    const unsigned total = s_pre[nlist];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_item = atomicAdd(work, 1u);
+        __syncthreads();
+        const unsigned item = s_item;
+        if (item >= total) break;
+        const int k = locate(s_pre, nlist, item);
+        const ListEntry e = list[k];
+        const uint32_t n = st[e.inst].n, C = e.cap / kLeaf;
+        const uint32_t nl = (n + kLeaf - 1) / kLeaf, leaf = item - s_pre[k];
+        const TreeNode* __restrict__ N = nodes + e.noff;
+        const double2* __restrict__ X = pxz + e.coff;
+        const float4* __restrict__ F = pf + e.coff;
+        const uint32_t t0 = leaf * kLeaf;
+        const int nchain = chain_length(nl);
+        const double2 o = X[t0];  // FP32 offsets from the leaf's first blob
+        uint64_t tx2[2], tz2[2];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const uint32_t i = t0 + t * 32 + lane;
+            float x = 0.0f, z = 0.0f;  // padding targets sit on the origin
+            if (i < n) {
+                const double2 p = X[i];
+                x = (float)(p.x - o.x);
+                z = (float)(p.y - o.y);
+            }
+            tx2[t] = f2pack(x, x);
+            tz2[t] = f2pack(z, z);
+        }
+        if (tid < kLeaf) S.at[tid] = X[min(t0 + tid, n - 1)];
+        for (int q = tid; q < kNearSlots * kLeaf; q += 32 * kNearWarps)
+            S.sum[q / kLeaf][q % kLeaf] = make_double2(0.0, 0.0);
+        walk_begin(S.walk, N, C, nl, 0, leaf, (int)min((uint32_t)kLeaf, n - t0), S.at);
+        const double tr = N[leaf].R;
+        const double nr = fmin(leaf > 0 ? N[leaf - 1].R : DBL_MAX,
+                               leaf + 1 < nl ? N[leaf + 1].R : DBL_MAX);
+        for (bool more = true; more;) {
+            do more = walk_step<false>(S.walk, N, C, nl);  // until a list could overflow
+            while (more && max(S.walk.n[0], S.walk.n[1]) + kWalk <= kListCap);
+            const int nnear = S.walk.n[0], nmid = S.walk.n[1];
+            for (int slot = wid; slot < kNearSlots && slot < max(nnear, nmid); slot += kNearWarps) {
+                double su[2] = {0.0, 0.0}, sw[2] = {0.0, 0.0};
+                for (int q = slot; q < nmid; q += kNearSlots) {
+                    const uint32_t id = S.walk.list[1][q];
+                    const uint64_t at = node_level(C, (int)(id >> 27)) + (id & ((1u << 27) - 1));
+                    const TreeNode& m = N[at];
+                    __syncwarp();
+                    if (lane < kTerms) {
+                        const double2 v = mom[(e.noff + at) * kTerms + lane];
+                        S.buf[wid][lane] = Cplx{v.x, v.y};
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const double2 p = S.at[t * 32 + lane];
+                        const Cplx f = moment_value(S.buf[wid], exp2_int(m.e), p.x - m.cx, p.y - m.cz);
+                        su[t] -= f.y;
+                        sw[t] += f.x;
+                    }
+                }
+                for (int q = slot; q < nnear; q += kNearSlots) {
+                    const uint32_t sl = S.walk.list[0][q], j0 = sl * kLeaf;
+                    const bool wide = tr > kSpread * (sl == leaf ? nr : N[sl].R);
+                    const bool far = box_gap2(N[sl], S.walk.chain[0]) > N[sl].thr * 1.001 + 1e-30;
+                    float4 P = make_float4(1e18f, 1e18f, 1e18f, 1e18f);  // padding: far away
+                    float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float2 G = make_float2(0.f, 0.f), T = make_float2(-1.f, -1.f), R = G;
+                    const uint32_t ja = j0 + 2 * lane, jb = ja + 1;
+                    if (ja < n) {
+                        const double2 p = X[ja];
+                        const float4 f = F[ja];
+                        split_hi_lo(p.x - o.x, P.x, L.x);
+                        split_hi_lo(p.y - o.y, P.z, L.z);
+                        G.x = f.x;
+                        T.x = f.y;
+                        R.x = f.z;
+                    }
+                    if (jb < n) {
+                        const double2 p = X[jb];
+                        const float4 f = F[jb];
+                        split_hi_lo(p.x - o.x, P.y, L.y);
+                        split_hi_lo(p.y - o.y, P.w, L.w);
+                        G.y = f.x;
+                        T.y = f.y;
+                        R.y = f.z;
+                    }
+                    StagedLeaf& w = S.src[wid];
+                    __syncwarp();
+                    w.pos[lane] = P;
+                    w.gam[lane] = G;
+                    w.thr[lane] = T;
+                    w.rs[lane] = R;
+                    if (wide) w.low[lane] = L;
+                    __syncwarp();
+                    uint64_t nu2[2] = {0ull, 0ull}, w2[2] = {0ull, 0ull};
+                    if (wide) {
+                        uint64_t lx2[2], lz2[2];
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            const double2 p = S.at[t * 32 + lane];
+                            float h, lo;
+                            split_hi_lo(p.x - o.x, h, lo);
+                            lx2[t] = f2pack(lo, lo);
+                            split_hi_lo(p.y - o.y, h, lo);
+                            lz2[t] = f2pack(lo, lo);
+                        }
+                        if (sl != leaf) leaf_sum<1, true>(w, tx2, tz2, lx2, lz2, nu2, w2);
+                        else leaf_sum<2, true>(w, tx2, tz2, lx2, lz2, nu2, w2);
+                    } else if (far) {
+                        leaf_sum<0, false>(w, tx2, tz2, tx2, tz2, nu2, w2);
+                    } else if (sl != leaf) {
+                        leaf_sum<1, false>(w, tx2, tz2, tx2, tz2, nu2, w2);
+                    } else {
+                        leaf_sum<2, false>(w, tx2, tz2, tx2, tz2, nu2, w2);
+                    }
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        su[t] += (double)(f2lo(nu2[t]) + f2hi(nu2[t]));
+                        sw[t] += (double)(f2lo(w2[t]) + f2hi(w2[t]));
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {  // only this warp touches the slot
+                    double2& v = S.sum[slot][t * 32 + lane];
+                    v.x += su[t];
+                    v.y += sw[t];
+                }
+            }
+            __syncthreads();
+            if (tid == 0) S.walk.n[0] = S.walk.n[1] = 0;
+            __syncthreads();
+        }
+        for (int q = tid; q < nchain * kTerms; q += 32 * kNearWarps) {
+            const int c = q / kTerms, up = kFarStep * c;
+            const double2 v = loc[(e.noff + node_level(C, up) + (leaf >> up)) * kTerms + q % kTerms];
+            S.buf[c][q % kTerms] = Cplx{v.x, v.y};
+        }
+        __syncthreads();
+        const uint32_t i = t0 + tid;
+        if (tid < kLeaf && i < n) {
+            const double2 p = S.at[tid];
+            double nu = 0.0, w = 0.0;
+            for (int c = 0; c < nchain; ++c) {
+                const TargetBox& t = S.walk.chain[c];
+                const Cplx f = local_value(S.buf[c], p.x - t.cx, p.y - t.cz, t.e);
+                nu -= f.y;
+                w += f.x;
+            }
+            for (int q = 0; q < kNearSlots; ++q) {
+                nu += S.sum[q][tid].x;
+                w += S.sum[q][tid].y;
+            }
+            const double u = -nu * kRpi2;
+            w *= kRpi2;
+            if (dry_u) {  // timing runs leave the simulations alone
+                dry_u[e.coff + i] = u;
+                dry_w[e.coff + i] = w;
+            } else {
+                const InstDesc& d = table[e.inst];
+                const uint32_t g = perm[e.coff + i];
+                d.u[g] = u;
+                d.w[g] = w;
+            }
+        }
+    }
+}
+static_assert(kChainMax <= kNearWarps, "a chain's expansions fit the warps' buffers");
 
 // ---- FP64, the reference's per-pair arithmetic -------------------------------
 // Every pair is evaluated with the reference's operations (src/VelocityKernel.cpp:
 // 44-60: IEEE division and exp inside the core, 1/r2 outside), over the same
-// Morton-sorted tiles as the FP32 path.  A source stage whose tile box is beyond
+// sorted tiles as the FP32 path.  A source stage whose tile box is beyond
 // 10 sigma^2 of the item's target box (the union of its sort tiles) holds no core
 // pair and no self pair, and runs the 1/r2 branch without the per-pair test; in
 // blob order nearly every warp met a core pair somewhere and ran both branches.
@@ -622,7 +818,9 @@ __global__ void __launch_bounds__(kBsThreads, kF64Ctas)
     __shared__ double s_rs[kBsST];
     __shared__ double s_box[4];  // the item's target box: xmin, xmax, zmin, zmax
     __shared__ unsigned s_item;
-    item_prefix_f64(s_pre, st, list, nlist);
+    list_prefix(s_pre, nlist, [&](int k) {
+        return ((st[list[k].inst].n + kBsTT - 1) / kBsTT) * (unsigned)list[k].chunks;
+    });
     const unsigned total = s_pre[nlist];
     const int tid = threadIdx.x;
     for (;;) {
@@ -717,25 +915,16 @@ __global__ void __launch_bounds__(kBsThreads, kF64Ctas)
     }
 }
 
-// Per blob: the FP32 path's fixed-point sums, or the FP64 path's chunk partials
-// in chunk order; scale by 1/(2 pi), scatter to blob order.
+// FP64 path, per blob: the chunk partials in chunk order, scaled by 1/(2 pi),
+// scattered to blob order.
 __global__ void k_self_combine(const InstDesc* __restrict__ table,
                                const InstState* __restrict__ st,
                                const ListEntry* __restrict__ list, int nlist,
                                const uint32_t* __restrict__ perm,
-                               const double2* __restrict__ part,
-                               const unsigned long long* __restrict__ macc,
-                               const int* __restrict__ mexp) {
+                               const double2* __restrict__ part) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += (st[list[k].inst].n + blockDim.x - 1) / blockDim.x;
-        }
-        s_pre[nlist] = acc;
-    }
-    __syncthreads();
+    list_prefix(s_pre, nlist,
+                [&](int k) { return (st[list[k].inst].n + blockDim.x - 1) / blockDim.x; });
     const unsigned total = s_pre[nlist];
     for (unsigned item = blockIdx.x; item < total; item += gridDim.x) {
         const int k = locate(s_pre, nlist, item);
@@ -744,20 +933,13 @@ __global__ void k_self_combine(const InstDesc* __restrict__ table,
         const uint32_t t = (item - s_pre[k]) * blockDim.x + threadIdx.x;
         if (t >= n) continue;
         double su = 0.0, sw = 0.0;
-        if (macc) {  // FP32: the blob's fixed-point sums
-            const double inv = ldexp(1.0, -mutual_shift(mexp, e.inst, n));
-            const uint64_t g = 2 * (e.coff + t);
-            su = (double)(long long)macc[g] * inv;
-            sw = (double)(long long)macc[g + 1] * inv;
-        } else {  // FP64: the chunk partials in chunk order
-            for (int c = 0; c < e.chunks; ++c) {
-                const double2 v = part[e.poff + (uint64_t)c * e.cap + t];
-                su += v.x;
-                sw += v.y;
-            }
+        for (int c = 0; c < e.chunks; ++c) {
+            const double2 v = part[e.poff + (uint64_t)c * e.cap + t];
+            su += v.x;
+            sw += v.y;
         }
         const InstDesc& d = table[e.inst];
-        const uint32_t p = perm ? perm[e.coff + t] : t;
+        const uint32_t p = perm[e.coff + t];
         d.u[p] = su * kRpi2;
         d.w[p] = sw * kRpi2;
     }
@@ -819,11 +1001,6 @@ struct AtStage {
     float4 cst[128];     // (circ a, circ b, 10 sigma^2 a, 10 sigma^2 b)
     float2 rs[128];      // (1/sigma^2 a, 1/sigma^2 b)
 };
-
-__device__ __forceinline__ void split_hi_lo(double v, float& hi, float& lo) {
-    hi = (float)v;
-    lo = (float)(v - (double)hi);
-}
 
 template <bool F32>
 __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int njobs) {
@@ -1080,6 +1257,14 @@ __global__ void k_build_rhs_jobs(const InstDesc* __restrict__ table, InstState* 
 
 }  // namespace
 
+void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const Workspace& ws,
+                int sms, cudaStream_t s) {
+    unsigned long long* dom = reinterpret_cast<unsigned long long*>(ws.work + 32);
+    cudaMemsetAsync(dom, 0, 4 * sizeof(*dom), s);
+    k_domain<<<std::min<uint32_t>((n + 1023) / 1024, sms * 4), 256, 0, s>>>(x, z, n, dom);
+    k_set_domain<<<1, 1, 0, s>>>(d, dom);
+}
+
 size_t cub_sort_bytes(uint64_t total) {
     size_t bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
@@ -1090,36 +1275,41 @@ size_t cub_sort_bytes(uint64_t total) {
 
 void biot_savart_prepare(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                          int precision, const Workspace& ws, int sms, cudaStream_t s) {
-    {  // both precisions evaluate over Morton-sorted tiles
+    {  // both precisions evaluate over sorted tiles
         const int g = (int)std::min<uint64_t>((ws.total_cap + 255) / 256, (uint64_t)sms * 16);
         k_keys<<<g, 256, 0, s>>>(table, st, list, nlist, ws.total_cap, ws.keys_in, ws.vals_in);
         size_t bytes = ws.cub_bytes;
         cub::DeviceRadixSort::SortPairs(ws.cub_tmp, bytes, ws.keys_in, ws.keys_out, ws.vals_in,
                                         ws.perm, (int64_t)ws.total_cap, 0, ws.key_bits, s);
     }
-    const uint32_t* perm = ws.perm;
-    double2* pxz = precision == kF32 ? reinterpret_cast<double2*>(ws.packed) : nullptr;
-    float4* pf = precision == kF32 ? reinterpret_cast<float4*>(ws.packed + ws.packed_cap / 2)
-                                   : nullptr;
-    if (precision == kF32)  // 0x80808080 per exponent: below any bound k_pack writes
-        cudaMemsetAsync(ws.mexp, 0x80, sizeof(int) * 4 * kTableCap, s);
-    k_pack<<<sms * 8, kBsST, 0, s>>>(table, st, list, nlist, perm, ws.packed, pxz, pf, ws.meta,
-                                     precision == kF32 ? ws.mexp : nullptr);
-    cudaMemsetAsync(ws.work, 0, sizeof(unsigned), s);
+    if (precision == kF32) {
+        cudaMemsetAsync(ws.arrived, 0, sizeof(unsigned) * (2 * ws.total_cap / kLeaf + (uint64_t)kNodeSlack * nlist), s);
+        k_tree<<<sms * 8, 128, 0, s>>>(table, st, list, nlist, ws.perm,
+                                       reinterpret_cast<double2*>(ws.packed),
+                                       reinterpret_cast<float4*>(ws.packed + ws.packed_cap / 2),
+                                       ws.nodes, ws.mom, ws.arrived);
+    } else {
+        k_pack<<<sms * 8, kBsST, 0, s>>>(table, st, list, nlist, ws.perm, ws.packed, ws.meta);
+    }
 }
 
 void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                          int precision, const Workspace& ws, int sms, cudaStream_t s,
-                         const PairConfig& cfg) {
-    (void)table;
+                         const PairConfig& cfg, bool dry) {
     if (precision == kF32) {
+        // cfg.ctas = 1 .. 4 quarters of full occupancy
+        const int g = std::max(1, sms * kNearBlocks * std::max(1, std::min(cfg.ctas, 4)) / 4);
         const double2* pxz = reinterpret_cast<const double2*>(ws.packed);
-        const float4* pf = reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2);
-        const int g = sms * std::max(1, std::min(cfg.ctas, kSelfMinBlocks));
-        cudaMemsetAsync(ws.macc, 0, 16 * ws.total_cap, s);
-        k_self_f32<kSelfMinBlocks><<<g, 32 * kWWarps, 0, s>>>(st, list, nlist, pxz, pf, ws.meta,
-                                                             ws.macc, ws.mexp, ws.work);
+        cudaMemsetAsync(ws.work, 0, 2 * sizeof(unsigned), s);
+        k_far<<<sms * kFarBlocks, kWalk, 0, s>>>(st, list, nlist, pxz, ws.nodes, ws.mom, ws.loc,
+                                                 ws.work + 1);
+        k_self_f32<kNearBlocks><<<g, 32 * kNearWarps, 0, s>>>(
+            table, st, list, nlist, pxz,
+            reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.perm, ws.nodes,
+            ws.mom, ws.loc, dry ? reinterpret_cast<double*>(ws.keys_in) : nullptr,
+            dry ? reinterpret_cast<double*>(ws.keys_out) : nullptr, ws.work);
     } else {
+        cudaMemsetAsync(ws.work, 0, sizeof(unsigned), s);
         k_self_f64<<<sms * kF64Ctas, kBsThreads, 0, s>>>(st, list, nlist, ws.packed, ws.meta,
                                                              ws.part, ws.work);
     }
@@ -1127,9 +1317,8 @@ void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* 
 
 void biot_savart_finish(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                         int precision, const Workspace& ws, int sms, cudaStream_t s) {
-    const bool f32 = precision == kF32;
-    k_self_combine<<<sms * 8, 256, 0, s>>>(table, st, list, nlist, ws.perm, ws.part,
-                                           f32 ? ws.macc : nullptr, ws.mexp);
+    if (precision == kF32) return;  // the pair kernel writes the blobs' velocities itself
+    k_self_combine<<<sms * 8, 256, 0, s>>>(table, st, list, nlist, ws.perm, ws.part);
 }
 
 void biot_savart_self(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
