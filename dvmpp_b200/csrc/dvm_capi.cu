@@ -347,6 +347,7 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
                  o_meta = take(sizeof(TileMeta) * (cap / kBsST + 1)), o_part = take(16 * part),
                  o_nodes = take(sizeof(TreeNode) * nodes), o_mom = take(16 * kTerms * nodes),
                  o_loc = take(16 * kTerms * nodes), o_arr = take(4 * nodes),
+                 o_near = take(sizeof(NearRow) * (cap / kLeaf + 1)),
                  o_rhs = take(16 * rhs), o_circ = take(8 * circ + 8), o_cub = take(cub + 256),
                  o_work = take(64 * sizeof(unsigned)), o_flags = take(cap),
                  o_tiles = take(4 * (cap / 1024 + 1)),
@@ -376,6 +377,7 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     w.nodes = reinterpret_cast<TreeNode*>(b + o_nodes);
     w.mom = reinterpret_cast<double2*>(b + o_mom);
     w.loc = reinterpret_cast<double2*>(b + o_loc);
+    w.near = reinterpret_cast<NearRow*>(b + o_near);
     w.arrived = reinterpret_cast<unsigned*>(b + o_arr);
     w.rhs_part = reinterpret_cast<double2*>(b + o_rhs);
     w.circ_part = reinterpret_cast<double*>(b + o_circ);
@@ -398,8 +400,8 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     return DVM_OK;
 }
 
-int key_bits_for(int nlist) {
-    int b = 1;
+int key_bits_for(int nlist) {  // (an odd bit more costs a whole 8-bit sort pass)
+    int b = 0;
     while ((1 << b) < nlist) ++b;
     return 32 + b;
 }

@@ -62,6 +62,15 @@ struct __align__(16) TreeNode {
     double pad2;
 };
 
+// What a leaf of targets sums itself: leaves pair by pair (from the front) and
+// nodes whose moments it evaluates at every target (from the back).
+constexpr uint32_t kNearRow = 126;
+constexpr uint32_t kNearOver = 0xFFFFFFFFu;  // as nnear: the row is too short
+struct __align__(16) NearRow {
+    uint32_t nnear, nmid;
+    uint32_t id[kNearRow];
+};
+
 // Sources per work item of a simulation's blob-on-collocation right-hand side:
 // a power of two in [512, kAtChunk], the smallest that still leaves about 600
 // items (four per SM) when the simulation is evaluated alone, so a single
@@ -175,6 +184,7 @@ struct Workspace {
     double2* mom = nullptr;        // kTerms moments per node
     double2* loc = nullptr;        // kTerms local coefficients per node that is a target group
     unsigned* arrived = nullptr;   // children done, per node
+    NearRow* near = nullptr;       // per leaf
     uint64_t nodes_cap = 0;
     double2* rhs_part = nullptr;   // at-target partials
     double* circ_part = nullptr;

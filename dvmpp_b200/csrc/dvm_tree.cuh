@@ -142,127 +142,113 @@ __device__ __forceinline__ bool takes_each(const TargetBox& t, const TreeNode& m
            (1.0 - kTheta) * (1.0 - kTheta) * d2 > m.thr * 1.001 + 1e-30;
 }
 
-// Walks the tree for one target group with the block's kWalk threads and fills
-// the block's lists: for FAR the nodes that this group translates, else the
-// leaves to sum and the nodes to evaluate (chain[0] is then the leaf's own).
-// chain[0 .. nchain): the group and the wider ones above it; a stack entry keeps
-// the place in the chain that its node is to meet.  Every thread of
-// the block must call step(); it returns false when the walk is over.  The
-// lists' order depends on the tree and the chain only.  A step adds at most kWalk
-// entries to each list.  The stack holds at most kWalk nodes left over per level
-// (a step takes kWalk from the top and adds twice that one level down), and a
-// walk starts at most 20 levels up (2^27 leaves under kWalk nodes).
-constexpr int kWalk = 128;
-constexpr int kListCap = 512;                // entries of a list before it is worked off
-constexpr int kWalkStack = kWalk * 22;
-struct TreeWalk {
-    TargetBox chain[kChainMax];
-    uint32_t stack[kWalkStack];
-    uint8_t place[kWalkStack];
-    uint32_t list[2][kListCap];  // FAR: [0] nodes to translate; else [0] leaves to sum, [1] nodes
-                                 // to evaluate at every target (ids: level << 27 | index)
-    unsigned cnt[3][kWalk / 32];
-    int sp, n[2];
-};
-
 __device__ __forceinline__ TargetBox target_box(const TreeNode& m) {
     return TargetBox{m.cx, m.cz, m.R, m.hx, m.hz, m.e, 0, nullptr};
 }
 
-// Chain of node (level, idx); the targets' positions are needed for a leaf only.
-__device__ __forceinline__ void walk_begin(TreeWalk& W, const TreeNode* __restrict__ nodes,
-                                           uint32_t C, uint32_t nleaves, int level, uint32_t idx,
-                                           int ntargets, const double2* at) {
+// A warp's walk of the tree for one target group.  chain[0 .. nchain): the group
+// and the wider ones above it; a stack entry keeps the place in the chain that
+// its node is to meet.  step() takes up to 32 nodes from the stack, tells each
+// lane what becomes of its node, and pushes the halves of those to be split.
+// The order of the outcomes depends on the tree and the chain only.  The
+// stack starts with at most kWalkTop nodes and holds at most 32 left over per
+// level below (a step takes 32 from the top and adds twice that one level down;
+// 20 levels: 2^26 leaves under kWalkTop nodes).
+constexpr int kWalkTop = 128;
+constexpr int kWalkStack = kWalkTop + 32 * 22;
+enum WalkKind : int { kWalkNone = -1, kWalkFar = 0, kWalkNear = 1, kWalkMid = 2, kWalkSplit = 3 };
+struct TreeWalk {
+    TargetBox chain[kChainMax];
+    uint32_t stack[kWalkStack];  // level << 27 | index
+    uint8_t place[kWalkStack];
+};
+
+__host__ __device__ __forceinline__ uint32_t level_count(uint32_t nleaves, int l) {
+    return (nleaves + (1u << l) - 1) >> l;
+}
+
+// Starts the walk of node (level, idx), a chain member; ntargets, at: a leaf's
+// targets.  Returns the stack's height.
+__device__ __forceinline__ int walk_begin(TreeWalk& W, const TreeNode* __restrict__ nodes,
+                                          uint32_t C, uint32_t nleaves, int level, uint32_t idx,
+                                          int ntargets, const double2* at, int lane) {
     int l0 = 0;
-    while (((nleaves + (1u << l0) - 1) >> l0) > (unsigned)kWalk) ++l0;
-    const int top = (int)((nleaves + (1u << l0) - 1) >> l0);
+    while (level_count(nleaves, l0) > (uint32_t)kWalkTop) ++l0;
+    const int top = (int)level_count(nleaves, l0);
     const int nchain = chain_length(nleaves) - level / kFarStep;
-    for (int i = threadIdx.x; i < top; i += blockDim.x) {
+    __syncwarp();
+    for (int i = lane; i < top; i += 32) {
         W.stack[i] = ((uint32_t)l0 << 27) | (uint32_t)i;
         W.place[i] = (uint8_t)(nchain - 1);
     }
-    if ((int)threadIdx.x < nchain) {
-        const int up = kFarStep * (int)threadIdx.x;
+    if (lane < nchain) {
+        const int up = kFarStep * lane;
         TargetBox t = target_box(nodes[node_level(C, level + up) + (idx >> up)]);
-        if (threadIdx.x == 0) {
+        if (lane == 0) {
             t.n = ntargets;
             t.at = at;
         }
-        W.chain[threadIdx.x] = t;
+        W.chain[lane] = t;
     }
-    if (threadIdx.x == 0) {
-        W.sp = top;
-        W.n[0] = W.n[1] = 0;
-    }
-    __syncthreads();
+    __syncwarp();
+    return top;
 }
 
-template <bool FAR>
-__device__ __forceinline__ bool walk_step(TreeWalk& W, const TreeNode* __restrict__ nodes,
-                                          uint32_t C, uint32_t nleaves) {
-    const int sp = W.sp;
-    if (sp == 0) return false;  // block-uniform
-    const int take = min(kWalk, sp), base = sp - take;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint32_t id = 0;
-    int kind = -1, c = 0;  // 0, 1: to that list; 2: split; -1: another group's
-    if (tid < take) {
-        id = W.stack[base + tid];
-        c = W.place[base + tid];
+// What the walk's own group (chain[0]) makes of the lane's node: translate (far),
+// sum its pairs (near, a leaf), evaluate its moments at every target (mid); none:
+// another group's, or no node.
+__device__ __forceinline__ int walk_step(TreeWalk& W, const TreeNode* __restrict__ nodes,
+                                         uint32_t C, uint32_t nleaves, int& sp, uint32_t& id,
+                                         int lane) {
+    const int take = min(32, sp), base = sp - take;
+    int kind = kWalkNone, c = 0;
+    id = 0;
+    if (lane < take) {
+        id = W.stack[base + lane];
+        c = W.place[base + lane];
         const int l = (int)(id >> 27);
         const uint32_t i = id & ((1u << 27) - 1);
-        if (i < ((nleaves + (1u << l) - 1) >> l)) {
+        if (i < level_count(nleaves, l)) {
             const TreeNode m = nodes[node_level(C, l) + i];
-            bool met = false;  // taken, or to be split
+            bool met = false;  // taken by a wider group, or to be split
             while (c > 0 && !met) {
                 const TargetBox& t = W.chain[c];
                 if (takes(t, m)) {
                     met = true;
                 } else if (l > 0 && m.R >= t.R) {
                     met = true;
-                    kind = 2;
+                    kind = kWalkSplit;
                 } else {
                     --c;
                 }
             }
             if (!met) {
                 const TargetBox& t = W.chain[0];
-                if (takes(t, m)) kind = FAR ? 0 : -1;
-                else if (t.n == 0) kind = l > 0 && m.R >= t.R ? 2 : -1;  // a wide group
-                else if (t.R > kSpread * m.R && takes_each(t, m)) kind = FAR ? -1 : 1;
-                else kind = l > 0 ? 2 : (FAR ? -1 : 0);
+                if (takes(t, m)) kind = kWalkFar;
+                else if (t.n == 0) kind = l > 0 && m.R >= t.R ? kWalkSplit : kWalkNone;  // a wide group
+                else if (t.R > kSpread * m.R && takes_each(t, m)) kind = kWalkMid;
+                else kind = l > 0 ? kWalkSplit : kWalkNear;
             }
         }
     }
-    unsigned ball[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        ball[k] = __ballot_sync(0xffffffffu, kind == k);
-        if (lane == 0) W.cnt[k][wid] = __popc(ball[k]);
+    const unsigned split = __ballot_sync(0xffffffffu, kind == kWalkSplit);  // (all have read)
+    if (kind == kWalkSplit) {
+        const int at = base + 2 * __popc(split & ((1u << lane) - 1u));
+        const uint32_t child = (((id >> 27) - 1) << 27) | ((id & ((1u << 27) - 1)) << 1);
+        W.stack[at] = child;
+        W.stack[at + 1] = child + 1;
+        W.place[at] = W.place[at + 1] = (uint8_t)c;
     }
-    __syncthreads();
-    if (kind >= 0) {
-        const unsigned b = kind == 0 ? ball[0] : kind == 1 ? ball[1] : ball[2];
-        int at = __popc(b & ((1u << lane) - 1u));
-        for (int q = 0; q < wid; ++q) at += (int)W.cnt[kind][q];
-        if (kind < 2) {
-            W.list[kind][W.n[kind] + at] = id;
-        } else {
-            const uint32_t child = (((id >> 27) - 1) << 27) | ((id & ((1u << 27) - 1)) << 1);
-            W.stack[base + 2 * at] = child;
-            W.stack[base + 2 * at + 1] = child + 1;
-            W.place[base + 2 * at] = W.place[base + 2 * at + 1] = (uint8_t)c;
-        }
-    }
-    __syncthreads();
-    if (tid < 3) {
-        int n = 0;
-        for (int q = 0; q < kWalk / 32; ++q) n += (int)W.cnt[tid][q];
-        if (tid < 2) W.n[tid] += n;
-        else W.sp = base + 2 * n;
-    }
-    __syncthreads();
-    return true;
+    sp = base + 2 * __popc(split);
+    __syncwarp();
+    return kind;
+}
+
+// The place of this lane's item among the warp's, and how many there are.
+__device__ __forceinline__ int warp_place(bool mine, int lane, int& count) {
+    const unsigned b = __ballot_sync(0xffffffffu, mine);
+    count = __popc(b);
+    return __popc(b & ((1u << lane) - 1u));
 }
 
 // Translation matrix C(l + k, k), exact in FP64: row k holds lanes l = 0 .. 31.
@@ -295,40 +281,75 @@ __device__ __forceinline__ Cplx moment_value(const Cplx* __restrict__ A, double 
     return cmul(v, Cplx{dx * r, -(dz * r)});
 }
 
-// One moment-to-local translation by a warp: lane l adds node m's contribution
-// to local coefficient l (scaled by 2^(e l) of the target group).  buf: the
-// warp's kTerms entries of shared memory.
-__device__ __forceinline__ void translate(const TreeNode& m, const double2* __restrict__ mom,
+// Moment-to-local translations by a warp, kBatch nodes at a time.  Four lanes per
+// node first write c_k = a_k (s_node / d)^k and f_l = (-s_group / d)^l / d to
+// shared memory, a quarter of the powers each; then lane l adds f_l times its row
+// of the translation matrix times c, two nodes side by side.  (Forming both powers
+// in every lane for one node at a time took 500 instructions per node, walk
+// included; this takes 210, 36 % of them FP64.)
+constexpr int kBatch = 8;
+constexpr int kPowStride = kTerms + 1;  // 400-byte rows: the quarters' stores meet no bank twice
+struct TransBuf {
+    Cplx c[kBatch][kPowStride];
+    Cplx f[kBatch][kPowStride];
+};
+
+// Nodes list[0 .. cnt), cnt <= kBatch; N, mom: the simulation's.
+__device__ __forceinline__ void translate(const TreeNode* __restrict__ N,
+                                          const double2* __restrict__ mom, uint32_t C,
+                                          const uint32_t* __restrict__ list, int cnt,
                                           const TargetBox& t, const double (&row)[kTerms],
-                                          Cplx* __restrict__ buf, int lane, Cplx& b) {
-    Cplx a{0.0, 0.0};
-    if (lane < kTerms) {
-        const double2 v = mom[lane];
-        a = Cplx{v.x, v.y};
-    }
-    const double dx = t.cx - m.cx, dz = t.cz - m.cz;
-    const int e = max(m.e, t.e);
-    const double s = exp2_int(e);
-    const double inv = s / fma(dx, dx, dz * dz);
-    const Cplx q{dx * inv, -(dz * inv)};  // s / d
-    const Cplx pw = cpow_lane(q, lane);
-    const double fs = exp2_int((m.e - e) * lane);
-    const Cplx c = cmul(a, pw);
-    __syncwarp();  // the previous translation's reads of buf
-    if (lane < kTerms) buf[lane] = Cplx{c.x * fs, c.y * fs};
-    __syncwarp();
-    Cplx s0{0.0, 0.0}, s1{0.0, 0.0};
+                                          TransBuf& buf, int lane, Cplx& b) {
+    constexpr int Q = kTerms / 4;
+    const int n = lane >> 2, part = lane & 3;
+    __syncwarp();  // the previous batch's reads
+    if (n < cnt) {
+        const uint32_t id = list[n];
+        const uint64_t at = node_level(C, (int)(id >> 27)) + (id & ((1u << 27) - 1));
+        const double2* __restrict__ A = mom + at * kTerms + part * Q;
+        double2 a[Q];
 #pragma unroll
-    for (int k = 0; k < kTerms; k += 2) {
-        const Cplx c0 = buf[k], c1 = buf[k + 1];
-        s0.x = fma(row[k], c0.x, s0.x);
-        s0.y = fma(row[k], c0.y, s0.y);
-        s1.x = fma(row[k + 1], c1.x, s1.x);
-        s1.y = fma(row[k + 1], c1.y, s1.y);
+        for (int k = 0; k < Q; ++k) a[k] = A[k];
+        const double dx = t.cx - N[at].cx, dz = t.cz - N[at].cz;
+        const int en = N[at].e;
+        const double inv = 1.0 / fma(dx, dx, dz * dz);
+        const Cplx r{dx * inv, -(dz * inv)};  // 1 / d
+        const double sn = exp2_int(en), st = -exp2_int(t.e);
+        const Cplx qn{r.x * sn, r.y * sn}, qt{r.x * st, r.y * st};
+        auto start = [&](Cplx q) {  // q^(part Q)
+            static_assert(Q == 6, "powers of six");
+            const Cplx q3 = cmul(cmul(q, q), q), q6 = cmul(q3, q3), q12 = cmul(q6, q6);
+            Cplx p = (part & 1) ? q6 : Cplx{1.0, 0.0};
+            const Cplx h = cmul(p, q12);
+            if (part & 2) p = h;
+            return p;
+        };
+        Cplx pn = start(qn), pt = cmul(start(qt), r);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            buf.c[n][part * Q + k] = cmul(Cplx{a[k].x, a[k].y}, pn);
+            buf.f[n][part * Q + k] = pt;
+            pn = cmul(pn, qn);
+            pt = cmul(pt, qt);
+        }
     }
-    const double ft = exp2_int((t.e - e) * lane) * ((lane & 1) ? -1.0 : 1.0) / s;
-    const Cplx f = cmul(pw, Cplx{q.x * ft, q.y * ft});
-    b = cfma(Cplx{s0.x + s1.x, s0.y + s1.y}, f, b);
+    __syncwarp();
+    for (int q = 0; q < cnt; q += 2) {  // two nodes side by side (an odd last one twice, once unused)
+        const int p = min(q + 1, cnt - 1);
+        Cplx s0{0.0, 0.0}, s1{0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < kTerms; ++k) {
+            const Cplx c0 = buf.c[q][k], c1 = buf.c[p][k];
+            s0.x = fma(row[k], c0.x, s0.x);
+            s0.y = fma(row[k], c0.y, s0.y);
+            s1.x = fma(row[k], c1.x, s1.x);
+            s1.y = fma(row[k], c1.y, s1.y);
+        }
+        if (lane < kTerms) {
+            b = cfma(s0, buf.f[q][lane], b);
+            if (p > q) b = cfma(s1, buf.f[p][lane], b);
+        }
+    }
 }
 
 // Value of a local expansion at offset (dx, dz) from the group's centre.

@@ -223,170 +223,247 @@ __device__ __forceinline__ int scale_exp(double R) {  // 2^e > R, clamped
     return R > 0.0 ? max(-300, min(300, ilogb(R) + 1)) : -300;
 }
 
-// Gather the blobs in sorted order, and build the tree bottom up: a warp makes one
-// leaf (box, radius, moments), and the warp that completes a node's second half
-// goes on to make that node from its halves (moment-to-moment translations as a
-// convolution with the factorials divided out).  Nobody waits: the warp that
-// arrives first at a node leaves.  The halves are added in index order, so the
-// result does not depend on who arrives when.
-__global__ void __launch_bounds__(128) k_tree(const InstDesc* __restrict__ table,
-                                              const InstState* __restrict__ st,
-                                              const ListEntry* __restrict__ list, int nlist,
-                                              const uint32_t* __restrict__ perm,
-                                              double2* __restrict__ pxz, float4* __restrict__ pf,
-                                              TreeNode* __restrict__ nodes,
-                                              double2* __restrict__ mom,
-                                              unsigned* __restrict__ arrived) {
+// Gather the blobs in sorted order, and build the tree bottom up.  A block makes
+// 32 consecutive leaves (box, radius, moments; one warp each at a time) and the
+// five levels above them in shared memory, one warp per node (moment-to-moment
+// translations as a convolution with the factorials divided out).  Of 16
+// neighbouring blocks the one that finishes last goes on with their 16 top nodes
+// in the same way, and so on up to the root; nobody waits.  A node is always
+// made from its halves in index order, so the result does not depend on who
+// finishes when.
+//
+// What bounds it is latency (a gather, then a chain of small FP64 steps), so the
+// levels inside a block meet no memory fence: with one arrival counter per
+// node and a fence at each the kernel took 284 us for 2^20 blobs, 93 for 250 k and
+// 38 for 5003, against 174, 55 and 29 us this way (32 leaves per block: 143, 75
+// and 36).
+constexpr int kFan = 16;  // nodes of the lowest level of a block's share
+constexpr int kFanLevels = 4;
+struct TreeShared {
+    TreeNode node[2 * kFan - 1];
+    Cplx mom[2 * kFan - 1][kTerms];  // level j of the share starts at 2 kFan - (2 kFan >> j)
+};
+
+// A leaf's node and moments from its (up to) two blobs per lane, as offsets from
+// its centre.
+__device__ __forceinline__ void leaf_moments(const double (&px)[2], const double (&pz)[2],
+                                             const double (&g)[2], int e, Cplx* __restrict__ out,
+                                             int lane) {
+    const double is = exp2_int(-e);
+    const Cplx q0{px[0] * is, pz[0] * is}, q1{px[1] * is, pz[1] * is};
+    // (even and odd powers as chains of their own, stepping by q^2)
+    const Cplx s0 = cmul(q0, q0), s1 = cmul(q1, q1);
+    Cplx t0[2] = {Cplx{g[0], 0.0}, Cplx{g[0] * q0.x, g[0] * q0.y}};
+    Cplx t1[2] = {Cplx{g[1], 0.0}, Cplx{g[1] * q1.x, g[1] * q1.y}};
+    const int own = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+#pragma unroll
+    for (int c = 0; c < kTerms / 8; ++c) {
+        Cplx v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            v[q] = Cplx{t0[q & 1].x + t1[q & 1].x, t0[q & 1].y + t1[q & 1].y};
+            t0[q & 1] = cmul(t0[q & 1], s0);
+            t1[q & 1] = cmul(t1[q & 1], s1);
+        }
+        const Cplx sum = warp_sum8(v, lane);
+        if ((lane & 3) == 0) out[c * 8 + own] = sum;
+    }
+}
+
+// A node from its halves (b == a when there is one), by a warp; fact = lane!.
+__device__ __forceinline__ void parent_node(const TreeNode& a, const TreeNode& b,
+                                            const Cplx* __restrict__ ma,
+                                            const Cplx* __restrict__ mb, bool two, double fact,
+                                            double ifact, int lane, TreeNode& m, Cplx& acc) {
+    const double bx0 = fmin(a.cx - a.hx, b.cx - b.hx), bx1 = fmax(a.cx + a.hx, b.cx + b.hx);
+    const double bz0 = fmin(a.cz - a.hz, b.cz - b.hz), bz1 = fmax(a.cz + a.hz, b.cz + b.hz);
+    m.cx = 0.5 * (bx0 + bx1);
+    m.cz = 0.5 * (bz0 + bz1);
+    m.hx = 0.5 * (bx1 - bx0);
+    m.hz = 0.5 * (bz1 - bz0);
+    m.thr = fmax(a.thr, b.thr);
+    const double ra = a.R + sqrt((a.cx - m.cx) * (a.cx - m.cx) + (a.cz - m.cz) * (a.cz - m.cz));
+    const double rb = b.R + sqrt((b.cx - m.cx) * (b.cx - m.cx) + (b.cz - m.cz) * (b.cz - m.cz));
+    m.R = fmin(fmax(ra, rb), sqrt(m.hx * m.hx + m.hz * m.hz)) * (1.0 + 1e-12);
+    m.e = scale_exp(m.R);
+    m.pad = 0;
+    m.pad2 = 0.0;
+    const double is = exp2_int(-m.e);
+    // both halves side by side: four independent chains of sums
+    Cplx v[2], h[2], sum[4];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const TreeNode& ch = q ? b : a;
+        v[q] = Cplx{0.0, 0.0};
+        if (lane < kTerms && (q == 0 || two)) {
+            const Cplx w = (q ? mb : ma)[lane];
+            const double f = exp2_int((ch.e - m.e) * lane) * ifact;
+            v[q] = Cplx{w.x * f, w.y * f};
+        }
+        h[q] = cpow_lane(Cplx{(ch.cx - m.cx) * is, (ch.cz - m.cz) * is}, lane);
+        h[q].x *= ifact;
+        h[q].y *= ifact;
+        sum[2 * q] = sum[2 * q + 1] = Cplx{0.0, 0.0};
+    }
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const Cplx aj = cshfl(v[q], j), hj = cshfl(h[q], (lane - j) & 31);
+            Cplx& t = sum[2 * q + (j & 1)];
+            if (lane >= j) t = cfma(aj, hj, t);
+        }
+    acc.x = ((sum[0].x + sum[1].x) + (sum[2].x + sum[3].x)) * fact;
+    acc.y = ((sum[0].y + sum[1].y) + (sum[2].y + sum[3].y)) * fact;
+}
+
+constexpr int kTreeWarps = 8;
+__global__ void __launch_bounds__(32 * kTreeWarps, 2)
+    k_tree(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
+           const ListEntry* __restrict__ list, int nlist, const uint32_t* __restrict__ perm,
+           double2* __restrict__ pxz, float4* __restrict__ pf, TreeNode* __restrict__ nodes,
+           double2* __restrict__ mom, unsigned* __restrict__ arrived) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
+    __shared__ TreeShared S;
+    __shared__ unsigned s_last;
+    list_prefix(s_pre, nlist, [&](int k) {
+        return (st[list[k].inst].n + kLeaf * kFan - 1) / (kLeaf * kFan);
+    });
     const unsigned total = s_pre[nlist], all = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double fact = 1.0;  // lane!
     for (int k = 2; k <= lane; ++k) fact *= (double)k;
     const double ifact = 1.0 / fact;
-    for (unsigned item = blockIdx.x * 4 + (threadIdx.x >> 5); item < total; item += gridDim.x * 4) {
+    for (unsigned item = blockIdx.x; item < total; item += gridDim.x) {
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
         const InstDesc& d = table[e.inst];
         const uint32_t n = st[e.inst].n, C = e.cap / kLeaf;
         const uint32_t nl = (n + kLeaf - 1) / kLeaf;
-        uint32_t idx = item - s_pre[k];
         TreeNode* __restrict__ N = nodes + e.noff;
         double2* __restrict__ A = mom + e.noff * kTerms;
-        unsigned* __restrict__ cnt = arrived + e.noff;
-        double px[2], pz[2], g[2];
-        double x0 = DBL_MAX, x1 = -DBL_MAX, z0 = DBL_MAX, z1 = -DBL_MAX, thr = 0.0;
+        uint32_t g = item - s_pre[k];  // the block's share: nodes kFan g .. of its lowest level
+        uint32_t next[2];  // the next leaf's blobs, ahead of its gather
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint32_t i = idx * kLeaf + h * 32 + lane;
-            px[h] = pz[h] = g[h] = 0.0;
-            if (i < n) {
-                const uint32_t p = perm[e.coff + i];
-                const double sg = d.sigma[p], s2 = sg * sg;
-                px[h] = d.x[p];
-                pz[h] = d.z[p];
-                g[h] = d.circ[p];
-                pxz[e.coff + i] = make_double2(px[h], pz[h]);
-                pf[e.coff + i] = make_float4((float)g[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
-                x0 = fmin(x0, px[h]);
-                x1 = fmax(x1, px[h]);
-                z0 = fmin(z0, pz[h]);
-                z1 = fmax(z1, pz[h]);
-                thr = fmax(thr, 10.0 * s2);
-            }
+            const uint32_t i = (g * kFan + wid) * kLeaf + h * 32 + lane;
+            next[h] = i < n ? perm[e.coff + i] : 0u;
         }
+        for (int w = wid; w < kFan && g * kFan + w < nl; w += kTreeWarps) {
+            const uint32_t idx = g * kFan + w;
+            const uint32_t here[2] = {next[0], next[1]};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x0 = fmin(x0, __shfl_xor_sync(all, x0, o));
-            x1 = fmax(x1, __shfl_xor_sync(all, x1, o));
-            z0 = fmin(z0, __shfl_xor_sync(all, z0, o));
-            z1 = fmax(z1, __shfl_xor_sync(all, z1, o));
-            thr = fmax(thr, __shfl_xor_sync(all, thr, o));
-        }
-        TreeNode m;
-        m.cx = 0.5 * (x0 + x1);
-        m.cz = 0.5 * (z0 + z1);
-        m.hx = 0.5 * (x1 - x0);
-        m.hz = 0.5 * (z1 - z0);
-        m.thr = thr;
-        double r2 = 0.0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (idx * kLeaf + h * 32 + lane < n) {
-                px[h] -= m.cx;
-                pz[h] -= m.cz;
-                r2 = fmax(r2, px[h] * px[h] + pz[h] * pz[h]);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t i = (idx + kTreeWarps) * kLeaf + h * 32 + lane;
+                next[h] = i < n ? perm[e.coff + i] : 0u;
             }
+            double px[2], pz[2], gc[2];
+            double x0 = DBL_MAX, x1 = -DBL_MAX, z0 = DBL_MAX, z1 = -DBL_MAX, thr = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(all, r2, o));
-        m.R = sqrt(r2) * (1.0 + 1e-12);
-        m.e = scale_exp(m.R);
-        m.pad = 0;
-        m.pad2 = 0.0;
-        {
-            const double is = exp2_int(-m.e);
-            const Cplx q0{px[0] * is, pz[0] * is}, q1{px[1] * is, pz[1] * is};
-            Cplx t0{g[0], 0.0}, t1{g[1], 0.0};
-            const int own = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-            double2* __restrict__ out = A + (uint64_t)idx * kTerms;
-#pragma unroll
-            for (int c = 0; c < kTerms / 8; ++c) {
-                Cplx v[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    v[q] = Cplx{t0.x + t1.x, t0.y + t1.y};
-                    t0 = cmul(t0, q0);
-                    t1 = cmul(t1, q1);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t i = idx * kLeaf + h * 32 + lane;
+                px[h] = pz[h] = gc[h] = 0.0;
+                if (i < n) {
+                    const uint32_t p = here[h];
+                    const double sg = d.sigma[p], s2 = sg * sg;
+                    px[h] = d.x[p];
+                    pz[h] = d.z[p];
+                    gc[h] = d.circ[p];
+                    pxz[e.coff + i] = make_double2(px[h], pz[h]);
+                    pf[e.coff + i] =
+                        make_float4((float)gc[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
+                    x0 = fmin(x0, px[h]);
+                    x1 = fmax(x1, px[h]);
+                    z0 = fmin(z0, pz[h]);
+                    z1 = fmax(z1, pz[h]);
+                    thr = fmax(thr, 10.0 * s2);
                 }
-                const Cplx sum = warp_sum8(v, lane);
-                if ((lane & 3) == 0) out[c * 8 + own] = make_double2(sum.x, sum.y);
             }
-        }
-        if (lane == 0) N[idx] = m;
-        // the nodes above
-        for (int l = 0;; ++l) {
-            if (((nl + (1u << l) - 1) >> l) <= 1u) break;  // the root is done
-            const uint32_t par = idx >> 1, cl = (nl + (1u << l) - 1) >> l;
-            const unsigned kids = 2 * par + 1 < cl ? 2u : 1u;
-            __threadfence();
-            __syncwarp();
-            unsigned before = 0;
-            if (lane == 0) before = atomicAdd(&cnt[node_level(C, l + 1) + par], 1u);
-            before = __shfl_sync(all, before, 0);
-            if (before + 1 < kids) break;
-            __threadfence();
-            const uint64_t c0 = node_level(C, l) + 2ull * par;
-            // (__ldcg: the halves were written by other SMs during this launch)
-            auto node_in = [&](uint64_t at) {
-                TreeNode r;
-                const double2* q = reinterpret_cast<const double2*>(N + at);
-                const double2 a = __ldcg(q), b = __ldcg(q + 1), c = __ldcg(q + 2);
-                const int2 ee = __ldcg(reinterpret_cast<const int2*>(q + 3));
-                r.cx = a.x;
-                r.cz = a.y;
-                r.R = b.x;
-                r.thr = b.y;
-                r.hx = c.x;
-                r.hz = c.y;
-                r.e = ee.x;
-                return r;
-            };
-            const TreeNode a = node_in(c0), b = kids == 2 ? node_in(c0 + 1) : a;
-            const double bx0 = fmin(a.cx - a.hx, b.cx - b.hx), bx1 = fmax(a.cx + a.hx, b.cx + b.hx);
-            const double bz0 = fmin(a.cz - a.hz, b.cz - b.hz), bz1 = fmax(a.cz + a.hz, b.cz + b.hz);
-            m.cx = 0.5 * (bx0 + bx1);
-            m.cz = 0.5 * (bz0 + bz1);
-            m.hx = 0.5 * (bx1 - bx0);
-            m.hz = 0.5 * (bz1 - bz0);
-            m.thr = fmax(a.thr, b.thr);
-            const double ra = a.R + sqrt((a.cx - m.cx) * (a.cx - m.cx) + (a.cz - m.cz) * (a.cz - m.cz));
-            const double rb = b.R + sqrt((b.cx - m.cx) * (b.cx - m.cx) + (b.cz - m.cz) * (b.cz - m.cz));
-            m.R = fmin(fmax(ra, rb), sqrt(m.hx * m.hx + m.hz * m.hz)) * (1.0 + 1e-12);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                x0 = fmin(x0, __shfl_xor_sync(all, x0, o));
+                x1 = fmax(x1, __shfl_xor_sync(all, x1, o));
+                z0 = fmin(z0, __shfl_xor_sync(all, z0, o));
+                z1 = fmax(z1, __shfl_xor_sync(all, z1, o));
+                thr = fmax(thr, __shfl_xor_sync(all, thr, o));
+            }
+            TreeNode m;
+            m.cx = 0.5 * (x0 + x1);
+            m.cz = 0.5 * (z0 + z1);
+            m.hx = 0.5 * (x1 - x0);
+            m.hz = 0.5 * (z1 - z0);
+            m.thr = thr;
+            double r2 = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (idx * kLeaf + h * 32 + lane < n) {
+                    px[h] -= m.cx;
+                    pz[h] -= m.cz;
+                    r2 = fmax(r2, px[h] * px[h] + pz[h] * pz[h]);
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(all, r2, o));
+            m.R = sqrt(r2) * (1.0 + 1e-12);
             m.e = scale_exp(m.R);
-            const double is = exp2_int(-m.e);
-            Cplx acc{0.0, 0.0};
-            for (unsigned q = 0; q < kids; ++q) {
-                const TreeNode& ch = q ? b : a;
-                Cplx v{0.0, 0.0};
-                if (lane < kTerms) {
-                    const double2 w = __ldcg(&A[(c0 + q) * kTerms + lane]);
-                    const double f = exp2_int((ch.e - m.e) * lane) * ifact;
-                    v = Cplx{w.x * f, w.y * f};
-                }
-                Cplx h = cpow_lane(Cplx{(ch.cx - m.cx) * is, (ch.cz - m.cz) * is}, lane);
-                h.x *= ifact;
-                h.y *= ifact;
-#pragma unroll 4
-                for (int j = 0; j < kTerms; ++j) {
-                    const Cplx aj = cshfl(v, j), hj = cshfl(h, (lane - j) & 31);
-                    if (lane >= j) acc = cfma(aj, hj, acc);
-                }
-            }
-            idx = par;
+            m.pad = 0;
+            m.pad2 = 0.0;
+            leaf_moments(px, pz, gc, m.e, S.mom[w], lane);
+            __syncwarp();
             if (lane < kTerms)
-                A[(node_level(C, l + 1) + par) * kTerms + lane] = make_double2(acc.x * fact, acc.y * fact);
-            if (lane == 0) N[node_level(C, l + 1) + par] = m;
+                A[(uint64_t)idx * kTerms + lane] = make_double2(S.mom[w][lane].x, S.mom[w][lane].y);
+            if (lane == 0) S.node[w] = N[idx] = m;
         }
+        __syncthreads();
+        for (int base = 0;; base += kFanLevels) {  // level of the share's lowest nodes
+            int l = base;
+            for (int j = 1; j <= kFanLevels; ++j) {
+                const uint32_t below = (nl + (1u << l) - 1) >> l;
+                if (below <= 1u) break;  // the root is done
+                ++l;
+                const uint32_t here = (nl + (1u << l) - 1) >> l, first = g * (kFan >> j);
+                const int at = 2 * kFan - (2 * kFan >> j), child = 2 * kFan - (2 * kFan >> (j - 1));
+                for (int w = wid; w < (kFan >> j) && first + w < here; w += kTreeWarps) {
+                    const bool two = 2 * (first + w) + 1 < below;
+                    const int c0 = child + 2 * w, c1 = two ? c0 + 1 : c0;
+                    TreeNode m;
+                    Cplx a;
+                    parent_node(S.node[c0], S.node[c1], S.mom[c0], S.mom[c1], two, fact, ifact,
+                                lane, m, a);
+                    const uint64_t to = node_level(C, l) + first + w;
+                    if (lane < kTerms) {
+                        S.mom[at + w][lane] = a;
+                        A[to * kTerms + lane] = make_double2(a.x, a.y);
+                    }
+                    if (lane == 0) S.node[at + w] = N[to] = m;
+                }
+                __syncthreads();
+            }
+            const uint32_t tops = (nl + (1u << l) - 1) >> l;
+            if (tops <= 1u) break;  // (then l is the root's level)
+            // kFan neighbouring shares: the last to finish takes their top nodes
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const uint32_t up = g / kFan, want = min((uint32_t)kFan, tops - up * kFan);
+                s_last = atomicAdd(&arrived[e.noff + node_level(C, l + kFanLevels) + up], 1u) + 1 == want;
+            }
+            __syncthreads();
+            if (!s_last) break;
+            __threadfence();
+            g /= kFan;
+            // (__ldcg: written by other SMs during this launch)
+            const uint32_t have = min((uint32_t)kFan, tops - g * kFan);
+            const uint64_t from = node_level(C, l) + (uint64_t)g * kFan;
+            for (uint32_t q = threadIdx.x; q < have * kTerms; q += blockDim.x) {
+                const double2 v = __ldcg(&A[from * kTerms + q]);
+                S.mom[q / kTerms][q % kTerms] = Cplx{v.x, v.y};
+            }
+            for (uint32_t q = threadIdx.x; q < have * (sizeof(TreeNode) / 16); q += blockDim.x)
+                reinterpret_cast<double2*>(S.node)[q] =
+                    __ldcg(reinterpret_cast<const double2*>(N + from) + q);
+            __syncthreads();
+        }
+        __syncthreads();
     }
 }
 
@@ -427,17 +504,20 @@ struct StagedLeaf {
 // gives, and distinct blobs closer than FP32 resolves stay finite, as the
 // FP64 reference is.  For t >= 1/2 it is (1 - e) / r2 with e = 2^(-t log2 e)
 // from one MUFU ex2; 1 - e >= 0.39 there, so the ex2 error stays below 4e-7
-// relative.
-__device__ __forceinline__ float core_kernel(float r2, float rs, float rcp_r2) {
-    const float t = r2 * rs;
-    float p = -1.121634850e-03f;
-    p = fmaf(p, t, 8.187386207e-03f);
-    p = fmaf(p, t, -4.162909091e-02f);
-    p = fmaf(p, t, 1.666622460e-01f);
-    p = fmaf(p, t, -4.999998212e-01f);
-    p = fmaf(p, t, 1.0f);
-    const float e = ex2_approx(-t * 1.44269504088896341f);
-    return t < 0.5f ? rs * p : (1.0f - e) * rcp_r2;
+// relative.  Two pairs at once, packed.
+__device__ __forceinline__ uint64_t core_kernel2(uint64_t r2, uint64_t rs, uint64_t rcp_r2) {
+    auto dup = [](float v) { return f2pack(v, v); };
+    const uint64_t t = f2mul(r2, rs);
+    uint64_t p = dup(-1.121634850e-03f);
+    p = f2fma(p, t, dup(8.187386207e-03f));
+    p = f2fma(p, t, dup(-4.162909091e-02f));
+    p = f2fma(p, t, dup(1.666622460e-01f));
+    p = f2fma(p, t, dup(-4.999998212e-01f));
+    p = f2fma(p, t, dup(1.0f));
+    const uint64_t m = f2mul(t, dup(-1.44269504088896341f));
+    const uint64_t e = f2pack(ex2_approx(f2lo(m)), ex2_approx(f2hi(m)));
+    const uint64_t in = f2mul(rs, p), out = f2mul(f2sub(dup(1.0f), e), rcp_r2);
+    return f2pack(f2lo(t) < 0.5f ? f2lo(in) : f2lo(out), f2hi(t) < 0.5f ? f2hi(in) : f2hi(out));
 }
 
 // The same core kernel through expm1f (about 1 ulp): the blob-on-collocation
@@ -494,9 +574,9 @@ __device__ __forceinline__ void leaf_sum(const StagedLeaf& __restrict__ src,
             if (MODE) {
                 const bool ca = ra < T.x, cb = rb < T.y;
                 if (__any_sync(0xffffffffu, ca || cb)) {
-                    const float qa = core_kernel(ra, S.x, ka), qb = core_kernel(rb, S.y, kb);
-                    ka = ca ? qa : ka;
-                    kb = cb ? qb : kb;
+                    const uint64_t q = core_kernel2(r2, f2pack(S.x, S.y), f2pack(ka, kb));
+                    ka = ca ? f2lo(q) : ka;
+                    kb = cb ? f2hi(q) : kb;
                 }
                 if (MODE == 2) {
                     ka = ra > 0.0f ? ka : 0.0f;
@@ -517,28 +597,34 @@ __device__ __forceinline__ void kahan(float& s, float& c, float x) {
     s = t;
 }
 
-// Local expansions of every target group of every listed simulation: one block
-// per group (the wide groups first, they have the most to translate), each warp
-// translating every fourth node of its list; the warps' sums are added in order.
+// Local expansions of every target group of every listed simulation, one warp per
+// group (the wide groups first, they have the most to translate).  A leaf's walk
+// also meets the leaves to be summed pair by pair and the nodes to be evaluated
+// at every target; it leaves them to k_self_f32 in the leaf's row of `near`:
+// leaves from the front, nodes from the back.  A row that is too short (cores
+// that reach over hundreds of leaves) has kNearOver as its count, and k_self_f32
+// walks again.
+constexpr int kFarWarps = 4;
+constexpr int kFarBlocks = 4;  // blocks per SM (the translation matrix's row: 48 registers)
+constexpr int kFarList = 64;   // at least kBatch + 32
 struct FarShared {
     TreeWalk walk;
-    Cplx buf[kWalk / 32][kTerms];
+    TransBuf buf;
     double2 at[kLeaf];
+    uint32_t far[kFarList];
 };
-constexpr int kFarBlocks = 4;  // blocks per SM (the translation matrix's row: 48 registers)
 
 __device__ __forceinline__ uint32_t groups_at(uint32_t nl, int c) {  // groups of chain place c
-    return c < chain_length(nl) ? (nl + (1u << (kFarStep * c)) - 1) >> (kFarStep * c) : 0u;
+    return c < chain_length(nl) ? level_count(nl, kFarStep * c) : 0u;
 }
 
-__global__ void __launch_bounds__(kWalk, kFarBlocks)
+__global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
     k_far(const InstState* __restrict__ st, const ListEntry* __restrict__ list, int nlist,
           const double2* __restrict__ pxz, const TreeNode* __restrict__ nodes,
-          const double2* __restrict__ mom, double2* __restrict__ loc,
+          const double2* __restrict__ mom, double2* __restrict__ loc, NearRow* __restrict__ near,
           unsigned* __restrict__ work) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    __shared__ FarShared S;
-    __shared__ unsigned s_item;
+    extern __shared__ __align__(16) unsigned char s_far[];  // FarShared per warp
     list_prefix(s_pre, nlist, [&](int k) {
         const uint32_t nl = (st[list[k].inst].n + kLeaf - 1) / kLeaf;
         uint32_t g = 0;
@@ -546,14 +632,14 @@ __global__ void __launch_bounds__(kWalk, kFarBlocks)
         return g;
     });
     const unsigned total = s_pre[nlist];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int lane = threadIdx.x & 31;
+    FarShared& S = reinterpret_cast<FarShared*>(s_far)[threadIdx.x >> 5];
     double row[kTerms];
     binomial_row(row, lane);
     for (;;) {
-        __syncthreads();
-        if (tid == 0) s_item = atomicAdd(work, 1u);
-        __syncthreads();
-        const unsigned item = s_item;
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(work, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= total) break;
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
@@ -566,54 +652,66 @@ __global__ void __launch_bounds__(kWalk, kFarBlocks)
         while (idx >= groups_at(nl, c)) idx -= groups_at(nl, c--);
         const int level = kFarStep * c;
         const uint32_t t0 = idx * kLeaf;  // (a leaf's)
-        if (c == 0 && tid < kLeaf) S.at[tid] = pxz[e.coff + min(t0 + tid, n - 1)];
-        walk_begin(S.walk, N, C, nl, level, idx, c == 0 ? (int)min((uint32_t)kLeaf, n - t0) : 0, S.at);
+        NearRow* row_out = c == 0 ? near + e.coff / kLeaf + idx : nullptr;
+        if (c == 0)
+            for (int q = lane; q < kLeaf; q += 32) S.at[q] = pxz[e.coff + min(t0 + q, n - 1)];
+        int sp = walk_begin(S.walk, N, C, nl, level, idx, c == 0 ? (int)min((uint32_t)kLeaf, n - t0) : 0,
+                            S.at, lane);
         const TargetBox tb = S.walk.chain[0];
-        Cplx b{0.0, 0.0};  // lane l: local coefficient l, this warp's share
-        for (bool more = true; more;) {
-            do more = walk_step<true>(S.walk, N, C, nl);  // until the list could overflow
-            while (more && S.walk.n[0] + kWalk <= kListCap);
-            const int nfar = S.walk.n[0];
-            for (int q = wid; q < nfar; q += kWalk / 32) {
-                const uint32_t id = S.walk.list[0][q];
-                const uint64_t at = node_level(C, (int)(id >> 27)) + (id & ((1u << 27) - 1));
-                translate(N[at], A + at * kTerms, tb, row, S.buf[wid], lane, b);
+        Cplx b{0.0, 0.0};  // lane l: local coefficient l
+        int nfar = 0, nnear = 0, nmid = 0;
+        while (sp > 0) {
+            uint32_t id;
+            const int kind = walk_step(S.walk, N, C, nl, sp, id, lane);
+            int cnt;
+            int at = warp_place(kind == kWalkFar, lane, cnt);
+            if (kind == kWalkFar) S.far[nfar + at] = id;
+            nfar += cnt;
+            if (row_out) {
+                at = warp_place(kind == kWalkNear, lane, cnt);
+                if (kind == kWalkNear && nnear + at < kNearRow) row_out->id[nnear + at] = id;
+                nnear += cnt;
+                at = warp_place(kind == kWalkMid, lane, cnt);
+                if (kind == kWalkMid && nmid + at < kNearRow) row_out->id[kNearRow - 1 - (nmid + at)] = id;
+                nmid += cnt;
             }
-            __syncthreads();
-            if (tid == 0) S.walk.n[0] = 0;
-            __syncthreads();
+            __syncwarp();
+            while (nfar >= kBatch || (sp == 0 && nfar > 0)) {  // from the list's end
+                const int m = min(kBatch, nfar);
+                nfar -= m;
+                translate(N, A, C, S.far + nfar, m, tb, row, S.buf, lane, b);
+            }
         }
-        __syncwarp();
-        if (lane < kTerms) S.buf[wid][lane] = b;
-        __syncthreads();
-        if (tid < kTerms) {
-            Cplx v = S.buf[0][tid];
-            for (int q = 1; q < kWalk / 32; ++q) {
-                v.x += S.buf[q][tid].x;
-                v.y += S.buf[q][tid].y;
-            }
-            loc[(e.noff + node_level(C, level) + idx) * kTerms + tid] = make_double2(v.x, v.y);
+        if (lane < kTerms)
+            loc[(e.noff + node_level(C, level) + idx) * kTerms + lane] = make_double2(b.x, b.y);
+        if (row_out && lane == 0) {
+            const bool fits = nnear + nmid <= kNearRow;
+            row_out->nnear = fits ? (uint32_t)nnear : kNearOver;
+            row_out->nmid = (uint32_t)nmid;
         }
     }
 }
 
 // Near pairs, and the sum of everything: one block per leaf of 64 targets, taken
-// from a counter.  The walk's lists are worked off whenever they fill and at its
-// end; their entries go to kNearSlots partial sums by their place in the list (a
-// warp serves several slots in turn), which are added in slot order.  The local
-// expansions of the leaf's chain are evaluated at the targets at the end.
+// from a counter.  The list's entries go to kNearSlots partial sums by their place
+// in it (a warp serves several slots in turn), which are added in slot order.
+// The local expansions of the leaf's chain are evaluated at the targets at the
+// end.
 //
 // Measured (B200, wake of 2^20 blobs, sigma 0.0169): the whole velocity call
-// 2.56 ms, of which this kernel 1.34, k_far 0.82 and k_tree 0.28, against
-// 215 ms for all pairs in mutual FP32x2 tiles at 80 % of the FP32 peak;
-// 2^16: 0.33 against 1.21 ms; 5003 blobs: 0.21 against 0.28 ms.  Relative L2
-// error against FP64 1.3e-7 (all pairs: 5.7e-7 to 7.6e-7) at 2^18.
+// 1.99 ms, of which this kernel 1.15, k_far 0.49 and k_tree 0.17, against
+// 215 ms for all pairs in mutual FP32x2 tiles at 80 % of the FP32 peak.  Relative
+// L2 error against FP64 1.3e-7 (all pairs: 5.7e-7 to 7.6e-7) at 2^18.  At 2^18
+// the MUFU pipe is 60 % and the FMA pipe 53 % busy, issue 57 %: latency bounds
+// it (6 blocks per SM at 80 registers were no faster at 2^20 and slower below).
 struct NearShared {
-    TreeWalk walk;
     StagedLeaf src[kNearWarps];
     Cplx buf[kNearWarps][kTerms];
     double2 at[kLeaf];
     double2 sum[kNearSlots][kLeaf];
+    uint32_t near[kNearRow], mid[kNearRow];
+    TreeWalk walk;  // for rows that overflowed
+    int count[2], more;
 };
 
 template <int MINB>
@@ -622,12 +720,12 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                const ListEntry* __restrict__ list, int nlist, const double2* __restrict__ pxz,
                const float4* __restrict__ pf, const uint32_t* __restrict__ perm,
                const TreeNode* __restrict__ nodes, const double2* __restrict__ mom,
-               const double2* __restrict__ loc, double* __restrict__ dry_u,
-               double* __restrict__ dry_w, unsigned* __restrict__ work) {
+               const double2* __restrict__ loc, const NearRow* __restrict__ near,
+               double* __restrict__ dry_u, double* __restrict__ dry_w,
+               unsigned* __restrict__ work) {
     __shared__ unsigned s_pre[kMaxList + 1];
     __shared__ NearShared S;
     __shared__ unsigned s_item;
-    static_assert(32 * kNearWarps == kWalk, "the whole block walks");
     list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
     const unsigned total = s_pre[nlist];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -645,7 +743,9 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
         const double2* __restrict__ X = pxz + e.coff;
         const float4* __restrict__ F = pf + e.coff;
         const uint32_t t0 = leaf * kLeaf;
-        const int nchain = chain_length(nl);
+        const int nchain = chain_length(nl), nt = (int)min((uint32_t)kLeaf, n - t0);
+        const NearRow& R = near[e.coff / kLeaf + leaf];
+        const bool over = R.nnear == kNearOver;
         const double2 o = X[t0];  // FP32 offsets from the leaf's first blob
         uint64_t tx2[2], tz2[2];
 #pragma unroll
@@ -663,18 +763,49 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
         if (tid < kLeaf) S.at[tid] = X[min(t0 + tid, n - 1)];
         for (int q = tid; q < kNearSlots * kLeaf; q += 32 * kNearWarps)
             S.sum[q / kLeaf][q % kLeaf] = make_double2(0.0, 0.0);
-        walk_begin(S.walk, N, C, nl, 0, leaf, (int)min((uint32_t)kLeaf, n - t0), S.at);
-        const double tr = N[leaf].R;
+        const TargetBox tb = target_box(N[leaf]);
         const double nr = fmin(leaf > 0 ? N[leaf - 1].R : DBL_MAX,
                                leaf + 1 < nl ? N[leaf + 1].R : DBL_MAX);
-        for (bool more = true; more;) {
-            do more = walk_step<false>(S.walk, N, C, nl);  // until a list could overflow
-            while (more && max(S.walk.n[0], S.walk.n[1]) + kWalk <= kListCap);
-            const int nnear = S.walk.n[0], nmid = S.walk.n[1];
+        int sp = 0;
+        if (over) {
+            __syncthreads();  // S.at is complete
+            if (wid == 0) sp = walk_begin(S.walk, N, C, nl, 0, leaf, nt, S.at, lane);
+        } else {
+            const uint32_t a = R.nnear, m = R.nmid;
+            for (uint32_t q = tid; q < a; q += 32 * kNearWarps) S.near[q] = R.id[q];
+            for (uint32_t q = tid; q < m; q += 32 * kNearWarps) S.mid[q] = R.id[kNearRow - 1 - q];
+            if (tid == 0) {
+                S.count[0] = (int)a;
+                S.count[1] = (int)m;
+                S.more = 0;
+            }
+        }
+        for (;;) {
+            if (over && wid == 0) {  // the next part of the walk
+                int a = 0, m = 0;
+                while (sp > 0 && max(a, m) + 32 <= kNearRow) {
+                    uint32_t id;
+                    const int kind = walk_step(S.walk, N, C, nl, sp, id, lane);
+                    int cnt;
+                    int at = warp_place(kind == kWalkNear, lane, cnt);
+                    if (kind == kWalkNear) S.near[a + at] = id;
+                    a += cnt;
+                    at = warp_place(kind == kWalkMid, lane, cnt);
+                    if (kind == kWalkMid) S.mid[m + at] = id;
+                    m += cnt;
+                }
+                if (lane == 0) {
+                    S.count[0] = a;
+                    S.count[1] = m;
+                    S.more = sp > 0;
+                }
+            }
+            __syncthreads();
+            const int nnear = S.count[0], nmid = S.count[1];
             for (int slot = wid; slot < kNearSlots && slot < max(nnear, nmid); slot += kNearWarps) {
                 double su[2] = {0.0, 0.0}, sw[2] = {0.0, 0.0};
                 for (int q = slot; q < nmid; q += kNearSlots) {
-                    const uint32_t id = S.walk.list[1][q];
+                    const uint32_t id = S.mid[q];
                     const uint64_t at = node_level(C, (int)(id >> 27)) + (id & ((1u << 27) - 1));
                     const TreeNode& m = N[at];
                     __syncwarp();
@@ -692,12 +823,13 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                     }
                 }
                 for (int q = slot; q < nnear; q += kNearSlots) {
-                    const uint32_t sl = S.walk.list[0][q], j0 = sl * kLeaf;
-                    const bool wide = tr > kSpread * (sl == leaf ? nr : N[sl].R);
-                    const bool far = box_gap2(N[sl], S.walk.chain[0]) > N[sl].thr * 1.001 + 1e-30;
+                    const uint32_t sl = S.near[q], j0 = sl * kLeaf;
+                    const TreeNode& sm = N[sl];
+                    const bool wide = tb.R > kSpread * (sl == leaf ? nr : sm.R);
+                    const bool far = box_gap2(sm, tb) > sm.thr * 1.001 + 1e-30;
                     float4 P = make_float4(1e18f, 1e18f, 1e18f, 1e18f);  // padding: far away
                     float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
-                    float2 G = make_float2(0.f, 0.f), T = make_float2(-1.f, -1.f), R = G;
+                    float2 G = make_float2(0.f, 0.f), T = make_float2(-1.f, -1.f), V = G;
                     const uint32_t ja = j0 + 2 * lane, jb = ja + 1;
                     if (ja < n) {
                         const double2 p = X[ja];
@@ -706,7 +838,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                         split_hi_lo(p.y - o.y, P.z, L.z);
                         G.x = f.x;
                         T.x = f.y;
-                        R.x = f.z;
+                        V.x = f.z;
                     }
                     if (jb < n) {
                         const double2 p = X[jb];
@@ -715,14 +847,14 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                         split_hi_lo(p.y - o.y, P.w, L.w);
                         G.y = f.x;
                         T.y = f.y;
-                        R.y = f.z;
+                        V.y = f.z;
                     }
                     StagedLeaf& w = S.src[wid];
                     __syncwarp();
                     w.pos[lane] = P;
                     w.gam[lane] = G;
                     w.thr[lane] = T;
-                    w.rs[lane] = R;
+                    w.rs[lane] = V;
                     if (wide) w.low[lane] = L;
                     __syncwarp();
                     uint64_t nu2[2] = {0ull, 0ull}, w2[2] = {0ull, 0ull};
@@ -759,9 +891,9 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                     v.y += sw[t];
                 }
             }
+            const int more = S.more;
             __syncthreads();
-            if (tid == 0) S.walk.n[0] = S.walk.n[1] = 0;
-            __syncthreads();
+            if (!more) break;
         }
         for (int q = tid; q < nchain * kTerms; q += 32 * kNearWarps) {
             const int c = q / kTerms, up = kFarStep * c;
@@ -769,12 +901,11 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             S.buf[c][q % kTerms] = Cplx{v.x, v.y};
         }
         __syncthreads();
-        const uint32_t i = t0 + tid;
-        if (tid < kLeaf && i < n) {
+        if (tid < nt) {
             const double2 p = S.at[tid];
             double nu = 0.0, w = 0.0;
             for (int c = 0; c < nchain; ++c) {
-                const TargetBox& t = S.walk.chain[c];
+                const TreeNode& t = N[node_level(C, kFarStep * c) + (leaf >> (kFarStep * c))];
                 const Cplx f = local_value(S.buf[c], p.x - t.cx, p.y - t.cz, t.e);
                 nu -= f.y;
                 w += f.x;
@@ -785,6 +916,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             }
             const double u = -nu * kRpi2;
             w *= kRpi2;
+            const uint32_t i = t0 + tid;
             if (dry_u) {  // timing runs leave the simulations alone
                 dry_u[e.coff + i] = u;
                 dry_w[e.coff + i] = w;
@@ -1284,7 +1416,7 @@ void biot_savart_prepare(const InstDesc* table, InstState* st, const ListEntry* 
     }
     if (precision == kF32) {
         cudaMemsetAsync(ws.arrived, 0, sizeof(unsigned) * (2 * ws.total_cap / kLeaf + (uint64_t)kNodeSlack * nlist), s);
-        k_tree<<<sms * 8, 128, 0, s>>>(table, st, list, nlist, ws.perm,
+        k_tree<<<sms * 2, 32 * kTreeWarps, 0, s>>>(table, st, list, nlist, ws.perm,
                                        reinterpret_cast<double2*>(ws.packed),
                                        reinterpret_cast<float4*>(ws.packed + ws.packed_cap / 2),
                                        ws.nodes, ws.mom, ws.arrived);
@@ -1301,12 +1433,15 @@ void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* 
         const int g = std::max(1, sms * kNearBlocks * std::max(1, std::min(cfg.ctas, 4)) / 4);
         const double2* pxz = reinterpret_cast<const double2*>(ws.packed);
         cudaMemsetAsync(ws.work, 0, 2 * sizeof(unsigned), s);
-        k_far<<<sms * kFarBlocks, kWalk, 0, s>>>(st, list, nlist, pxz, ws.nodes, ws.mom, ws.loc,
-                                                 ws.work + 1);
+        constexpr size_t far_smem = sizeof(FarShared) * kFarWarps;
+        cudaFuncSetAttribute(k_far, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)far_smem);
+        k_far<<<sms * kFarBlocks, 32 * kFarWarps, far_smem, s>>>(st, list, nlist, pxz, ws.nodes,
+                                                                 ws.mom, ws.loc, ws.near,
+                                                                 ws.work + 1);
         k_self_f32<kNearBlocks><<<g, 32 * kNearWarps, 0, s>>>(
             table, st, list, nlist, pxz,
             reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.perm, ws.nodes,
-            ws.mom, ws.loc, dry ? reinterpret_cast<double*>(ws.keys_in) : nullptr,
+            ws.mom, ws.loc, ws.near, dry ? reinterpret_cast<double*>(ws.keys_in) : nullptr,
             dry ? reinterpret_cast<double*>(ws.keys_out) : nullptr, ws.work);
     } else {
         cudaMemsetAsync(ws.work, 0, sizeof(unsigned), s);
