@@ -54,16 +54,20 @@ constexpr size_t kPoolPerPlan = 6144;  // list entries per plan: 4 partitions + 
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Source chunks of a simulation's pair kernel.  Fixed by the capacity alone, so
-// a simulation's sums are associated the same way alone and inside any batch:
-// at least one chunk per 32 k sources (up to 32), and for small simulations
-// enough chunks (~2^23 / cap per 256-target tile, ~32 k work items) to occupy
-// the GPU when stepped alone, but never chunks shorter than 512 sources.  In
-// FP32 a chunk costs two 64-bit atomic adds per target (FP64: a partial sum).
+// Source chunks of a simulation's FP64 pair kernel, at most.  Fixed by the capacity
+// alone, so a simulation's sums are associated the same way alone and inside
+// any batch: one chunk per 32 k sources (up to 32); for small simulations enough
+// for about 4800 work items of 256 targets (five rounds of blocks) when stepped
+// alone, and up to 64 while 2^23 / cap allows, which keeps a chunk's sum short
+// (40 k blobs: 30 chunks gave 1.4e-15 against 64 bits, 64 give 1.0e-15 at the
+// same speed); never chunks shorter than 64 sources.  A chunk costs a partial sum
+// per target.
 int nbody_chunks(uint32_t cap) {
+    const uint32_t c = std::max<uint32_t>(cap, 1);
     const int by_size = (int)std::min<uint32_t>(32, (cap + 32767) / 32768);
-    const int by_fill = (int)((8u << 20) / std::max<uint32_t>(cap, 1));
-    const int most = (int)std::max<uint32_t>(1, std::min<uint32_t>(64, cap / 512));
+    const int by_fill = (int)std::max<uint32_t>((4800u * 256u + c - 1) / c,
+                                                std::min<uint32_t>(64, (8u << 20) / c));
+    const int most = (int)std::max<uint32_t>(1, cap / 64);
     return std::max(1, std::min(most, std::max(by_size, by_fill)));
 }
 

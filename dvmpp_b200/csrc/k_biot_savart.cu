@@ -17,8 +17,8 @@
 // leaves, in an order that the simulation's own blobs fix: deterministic, and
 // independent of the batch a simulation runs in and of the launch shape.
 //
-// FP64 path (the parity path): every pair with the reference's operation
-// sequence (no FMA contraction), over 256-blob tiles of the same sorted order.
+// FP64 path (the parity path): every pair with the reference's formula in FP64,
+// over 256-blob tiles of the same sorted order.
 #include <cfloat>
 #include <mutex>
 #include <string>
@@ -467,9 +467,14 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
     }
 }
 
+// FP64 path: sources per chunk (a multiple of 64) of n blobs cut into at most
+// `chunks`, and how many chunks that makes.
 __device__ __forceinline__ uint32_t chunk_size(uint32_t n, int chunks) {
-    uint32_t cs = (n + chunks - 1) / chunks;
-    return (cs + kBsST - 1) / kBsST * kBsST;
+    return max(64u, ((n + chunks - 1) / chunks + 63) / 64 * 64);
+}
+__device__ __forceinline__ uint32_t chunk_count(uint32_t n, int chunks) {
+    const uint32_t cs = chunk_size(n, chunks);
+    return (n + cs - 1) / cs;
 }
 
 // ---- FP32 pair loops --------------------------------------------------------
@@ -477,8 +482,7 @@ __device__ __forceinline__ uint32_t chunk_size(uint32_t n, int chunks) {
 // per lane.  Two SOURCES share a packed FP32x2 instruction: their values come
 // out of shared memory as register pairs (no duplicating moves), the targets'
 // are duplicated once per item.
-constexpr int kNearWarps = 4;   // warps of a block
-constexpr int kNearBlocks = 5;  // blocks per SM at full occupancy
+constexpr int kNearThreads = 640;  // per SM at full occupancy (96 registers)
 constexpr int kNearSlots = 8;   // partial sums of an item: list entries q, q + 8, ...
 
 __device__ __forceinline__ void split_hi_lo(double v, float& hi, float& lo) {
@@ -704,9 +708,14 @@ __global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
 // L2 error against FP64 1.3e-7 (all pairs: 5.7e-7 to 7.6e-7) at 2^18.  At 2^18
 // the MUFU pipe is 60 % and the FMA pipe 53 % busy, issue 57 %: latency bounds
 // it (6 blocks per SM at 80 registers were no faster at 2^20 and slower below).
+//
+// WARPS does not change a result; few leaves take eight, so that a leaf's chain of
+// near sums is half as long (k_far and this kernel, 5003 blobs: 78 -> 60 us; 20 k:
+// 118 -> 86).
+template <int WARPS>
 struct NearShared {
-    StagedLeaf src[kNearWarps];
-    Cplx buf[kNearWarps][kTerms];
+    StagedLeaf src[WARPS];
+    Cplx buf[WARPS][kTerms];
     double2 at[kLeaf];
     double2 sum[kNearSlots][kLeaf];
     uint32_t near[kNearRow], mid[kNearRow];
@@ -714,8 +723,8 @@ struct NearShared {
     int count[2], more;
 };
 
-template <int MINB>
-__global__ void __launch_bounds__(32 * kNearWarps, MINB)
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, kNearThreads / (32 * WARPS))
     k_self_f32(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
                const ListEntry* __restrict__ list, int nlist, const double2* __restrict__ pxz,
                const float4* __restrict__ pf, const uint32_t* __restrict__ perm,
@@ -724,7 +733,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
                double* __restrict__ dry_u, double* __restrict__ dry_w,
                unsigned* __restrict__ work) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    __shared__ NearShared S;
+    __shared__ NearShared<WARPS> S;
     __shared__ unsigned s_item;
     list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
     const unsigned total = s_pre[nlist];
@@ -761,7 +770,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             tz2[t] = f2pack(z, z);
         }
         if (tid < kLeaf) S.at[tid] = X[min(t0 + tid, n - 1)];
-        for (int q = tid; q < kNearSlots * kLeaf; q += 32 * kNearWarps)
+        for (int q = tid; q < kNearSlots * kLeaf; q += 32 * WARPS)
             S.sum[q / kLeaf][q % kLeaf] = make_double2(0.0, 0.0);
         const TargetBox tb = target_box(N[leaf]);
         const double nr = fmin(leaf > 0 ? N[leaf - 1].R : DBL_MAX,
@@ -772,8 +781,8 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             if (wid == 0) sp = walk_begin(S.walk, N, C, nl, 0, leaf, nt, S.at, lane);
         } else {
             const uint32_t a = R.nnear, m = R.nmid;
-            for (uint32_t q = tid; q < a; q += 32 * kNearWarps) S.near[q] = R.id[q];
-            for (uint32_t q = tid; q < m; q += 32 * kNearWarps) S.mid[q] = R.id[kNearRow - 1 - q];
+            for (uint32_t q = tid; q < a; q += 32 * WARPS) S.near[q] = R.id[q];
+            for (uint32_t q = tid; q < m; q += 32 * WARPS) S.mid[q] = R.id[kNearRow - 1 - q];
             if (tid == 0) {
                 S.count[0] = (int)a;
                 S.count[1] = (int)m;
@@ -802,7 +811,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             }
             __syncthreads();
             const int nnear = S.count[0], nmid = S.count[1];
-            for (int slot = wid; slot < kNearSlots && slot < max(nnear, nmid); slot += kNearWarps) {
+            for (int slot = wid; slot < kNearSlots && slot < max(nnear, nmid); slot += WARPS) {
                 double su[2] = {0.0, 0.0}, sw[2] = {0.0, 0.0};
                 for (int q = slot; q < nmid; q += kNearSlots) {
                     const uint32_t id = S.mid[q];
@@ -895,7 +904,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
             __syncthreads();
             if (!more) break;
         }
-        for (int q = tid; q < nchain * kTerms; q += 32 * kNearWarps) {
+        for (int q = tid; q < nchain * kTerms; q += 32 * WARPS) {
             const int c = q / kTerms, up = kFarStep * c;
             const double2 v = loc[(e.noff + node_level(C, up) + (leaf >> up)) * kTerms + q % kTerms];
             S.buf[c][q % kTerms] = Cplx{v.x, v.y};
@@ -929,29 +938,57 @@ __global__ void __launch_bounds__(32 * kNearWarps, MINB)
         }
     }
 }
-static_assert(kChainMax <= kNearWarps, "a chain's expansions fit the warps' buffers");
+static_assert(kChainMax <= 4, "a chain's expansions fit the warps' buffers");
 
-// ---- FP64, the reference's per-pair arithmetic -------------------------------
-// Every pair is evaluated with the reference's operations (src/VelocityKernel.cpp:
-// 44-60: IEEE division and exp inside the core, 1/r2 outside), over the same
-// sorted tiles as the FP32 path.  A source stage whose tile box is beyond
-// 10 sigma^2 of the item's target box (the union of its sort tiles) holds no core
-// pair and no self pair, and runs the 1/r2 branch without the per-pair test; in
-// blob order nearly every warp met a core pair somewhere and ran both branches.
-// 3 CTAs of 8 warps per SM (80 registers): the FP64 division / exp chains need
-// the warps (1 CTA per SM ran 2.2x slower)
-constexpr int kF64Ctas = 3;
-__global__ void __launch_bounds__(kBsThreads, kF64Ctas)
+// ---- FP64 pairs ---------------------------------------------------------------
+// 1 / v in FP64: the hardware's approximation (about 20 bits) and two steps of
+// Newton's iteration y += y (1 - v y), each error the square of the one before;
+// the last step's rounding is all that is left (within one ulp; an IEEE
+// reciprocal takes three times the instructions).  For v in [1e-290, 1e290].
+__device__ __forceinline__ double rcp_newton(double v) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    y = fma(y, fma(-v, y, 1.0), y);
+    return fma(y, fma(-v, y, 1.0), y);
+}
+// The same for any v: IEEE where the iteration has no range (zero, infinite, NaN or
+// near the ends of the exponents).
+__device__ __forceinline__ double rcp_f64(double v) {
+    const unsigned h = (unsigned)__double2hiint(v);
+    return h - 0x03d00000u < 0x78000000u ? rcp_newton(v) : __drcp_rn(v);
+}
+
+// K(r2) of src/VelocityKernel.cpp:51-57 with rs = 1 / sigma^2, thr = 10 sigma^2.
+__device__ __forceinline__ double kernel_f64(double r2, double thr, double rs) {
+    const double y = rcp_f64(r2);
+    return r2 < thr ? dmul(dsub(1.0, exp(dmul(-r2, rs))), y) : y;
+}
+
+// Every pair, over the 256-blob tiles of the sorted order; each pair is the
+// reference's formula (src/VelocityKernel.cpp:44-60) in FP64.  A source stage
+// whose tile box is beyond 10 sigma^2 of the target tile's box holds no core pair
+// and no self pair, and runs the 1/r^2 branch without the per-pair test.
+//
+// The FP64 pipe bounds it (64 lanes per clock and SM): 12 operations per far
+// pair, where an IEEE reciprocal and unfused products took 27; 72 % busy at 40 k.  A work item is one
+// tile of targets (two per thread) against one source chunk; chunks are as
+// short as leaves a single simulation about five rounds of blocks
+// (nbody_chunks).  Measured (whole call): 40 k blobs 2.55 -> 1.52 ms, 262 k 75 -> 51,
+// 5003 blobs 0.64 -> 0.16 (before: items of 1024 targets, at least 256 sources).
+constexpr int kF64Threads = 128;
+constexpr int kF64Ctas = 6;
+__global__ void __launch_bounds__(kF64Threads, kF64Ctas)
     k_self_f64(const InstState* __restrict__ st, const ListEntry* __restrict__ list, int nlist,
                const double4* __restrict__ packed, const TileMeta* __restrict__ meta,
                double2* __restrict__ part, unsigned* __restrict__ work) {
+    static_assert(2 * kF64Threads == kBsST, "a work item's targets are one sort tile");
     __shared__ unsigned s_pre[kMaxList + 1];
     __shared__ double4 s_src[kBsST];  // x, z, circ, threshold
     __shared__ double s_rs[kBsST];
-    __shared__ double s_box[4];  // the item's target box: xmin, xmax, zmin, zmax
     __shared__ unsigned s_item;
     list_prefix(s_pre, nlist, [&](int k) {
-        return ((st[list[k].inst].n + kBsTT - 1) / kBsTT) * (unsigned)list[k].chunks;
+        const uint32_t n = st[list[k].inst].n;
+        return (n + kBsST - 1) / kBsST * chunk_count(n, list[k].chunks);
     });
     const unsigned total = s_pre[nlist];
     const int tid = threadIdx.x;
@@ -964,86 +1001,71 @@ __global__ void __launch_bounds__(kBsThreads, kF64Ctas)
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
         const uint32_t n = st[e.inst].n;
-        const unsigned local = item - s_pre[k];
-        const uint32_t tile = local / e.chunks, c = local % e.chunks;
+        const unsigned local = item - s_pre[k], chunks = chunk_count(n, e.chunks);
+        const uint32_t tile = local / chunks, c = local % chunks;
         const uint32_t cs = chunk_size(n, e.chunks);
         const uint32_t j0 = c * cs, j1 = min(n, j0 + cs);
         const double4* __restrict__ P = packed + e.coff;
-        const uint32_t tb = tile * kBsTT + tid * kBsR;
-        double tx[kBsR], tz[kBsR], uu[kBsR], ww[kBsR];
+        const TileMeta tm = meta[(e.coff + (uint64_t)tile * kBsST) / kBsST];
+        const uint32_t tb = tile * kBsST + tid;
+        double tx[2], tz[2], uu[2], ww[2];
 #pragma unroll
-        for (int r = 0; r < kBsR; ++r) {
-            const double4 p = (tb + r < n) ? P[tb + r] : make_double4(0, 0, 0, 1);
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t t = tb + r * kF64Threads;
+            const double4 p = t < n ? P[t] : make_double4(0, 0, 0, 1);
             tx[r] = p.x;
             tz[r] = p.y;
             uu[r] = ww[r] = 0.0;
         }
-        if (tid == 0) {  // the item's target box (read after the next barrier)
-            double b0 = DBL_MAX, b1 = -DBL_MAX, b2 = DBL_MAX, b3 = -DBL_MAX;
-            for (int q = 0; q < kBsTT / kBsST; ++q) {
-                const uint32_t t = tile * kBsTT + q * kBsST;
-                if (t < n) {
-                    const TileMeta& m = meta[(e.coff + t) / kBsST];
-                    b0 = fmin(b0, m.xmin);
-                    b1 = fmax(b1, m.xmax);
-                    b2 = fmin(b2, m.zmin);
-                    b3 = fmax(b3, m.zmax);
-                }
-            }
-            s_box[0] = b0;
-            s_box[1] = b1;
-            s_box[2] = b2;
-            s_box[3] = b3;
-        }
-        for (uint32_t s0 = j0; s0 < j1; s0 += kBsST) {
-            __syncthreads();
+        for (uint32_t s0 = j0; s0 < j1;) {
+            const int cnt = (int)min((uint32_t)kBsST - s0 % kBsST, j1 - s0);  // within one tile
             const TileMeta& m = meta[(e.coff + s0) / kBsST];
-            const double gx = fmax(0.0, fmax(m.xmin - s_box[1], s_box[0] - m.xmax));
-            const double gz = fmax(0.0, fmax(m.zmin - s_box[3], s_box[2] - m.zmax));
-            const bool far = gx * gx + gz * gz > m.thr * 1.001 + 1e-30;
-            const uint32_t j = s0 + tid;
-            if (j < j1) {
-                const double4 p = P[j];
+            const double gx = fmax(0.0, fmax(m.xmin - tm.xmax, tm.xmin - m.xmax));
+            const double gz = fmax(0.0, fmax(m.zmin - tm.zmax, tm.zmin - m.zmax));
+            const double ex = fmax(m.xmax, tm.xmax) - fmin(m.xmin, tm.xmin);
+            const double ez = fmax(m.zmax, tm.zmax) - fmin(m.zmin, tm.zmin);
+            // (the last: every r^2 of the stage is in rcp_newton's range)
+            const bool far = gx * gx + gz * gz > m.thr * 1.001 + 1e-30 && ex * ex + ez * ez < 1e290;
+            __syncthreads();
+            for (int q = tid; q < cnt; q += kF64Threads) {
+                const double4 p = P[s0 + q];
                 const double s2 = dmul(p.w, p.w);
-                s_src[tid] = make_double4(p.x, p.y, p.z, dmul(10.0, s2));
-                if (!far) s_rs[tid] = ddiv(1.0, s2);
+                s_src[q] = make_double4(p.x, p.y, p.z, dmul(10.0, s2));
+                if (!far) s_rs[q] = ddiv(1.0, s2);
             }
             __syncthreads();
-            const int cnt = (int)min((uint32_t)kBsST, j1 - s0);
             if (far) {
+#pragma unroll 4
                 for (int jj = 0; jj < cnt; ++jj) {
                     const double4 sj = s_src[jj];
 #pragma unroll
-                    for (int r = 0; r < kBsR; ++r) {
-                        const double dx = dsub(tx[r], sj.x);
-                        const double dz = dsub(tz[r], sj.y);
-                        const double K = __drcp_rn(dadd(dmul(dx, dx), dmul(dz, dz)));
-                        uu[r] = dsub(uu[r], dmul(dmul(K, dz), sj.z));
-                        ww[r] = dadd(ww[r], dmul(dmul(K, dx), sj.z));
+                    for (int r = 0; r < 2; ++r) {
+                        const double dx = dsub(tx[r], sj.x), dz = dsub(tz[r], sj.y);
+                        const double g = dmul(rcp_newton(fma(dx, dx, dmul(dz, dz))), sj.z);
+                        uu[r] = fma(-g, dz, uu[r]);
+                        ww[r] = fma(g, dx, ww[r]);
                     }
                 }
-                continue;
-            }
-            for (int jj = 0; jj < cnt; ++jj) {
-                const double4 s = s_src[jj];
+            } else {
+                for (int jj = 0; jj < cnt; ++jj) {
+                    const double4 sj = s_src[jj];
 #pragma unroll
-                for (int r = 0; r < kBsR; ++r) {
-                    if (tb + r == s0 + jj) continue;  // i != j (src/VelocityKernel.cpp:43)
-                    const double dx = dsub(tx[r], s.x);
-                    const double dz = dsub(tz[r], s.y);
-                    const double r2 = dadd(dmul(dx, dx), dmul(dz, dz));
-                    double K;
-                    if (r2 < s.w) K = ddiv(dsub(1.0, exp(dmul(-r2, s_rs[jj]))), r2);
-                    else K = __drcp_rn(r2);  // correctly rounded: the same value as 1.0 / r2
-                    uu[r] = dsub(uu[r], dmul(dmul(K, dz), s.z));
-                    ww[r] = dadd(ww[r], dmul(dmul(K, dx), s.z));
+                    for (int r = 0; r < 2; ++r) {
+                        if (tb + r * kF64Threads == s0 + jj) continue;  // i != j (src/VelocityKernel.cpp:43)
+                        const double dx = dsub(tx[r], sj.x), dz = dsub(tz[r], sj.y);
+                        const double K = kernel_f64(fma(dx, dx, dmul(dz, dz)), sj.w, s_rs[jj]);
+                        const double g = dmul(K, sj.z);
+                        uu[r] = fma(-g, dz, uu[r]);
+                        ww[r] = fma(g, dx, ww[r]);
+                    }
                 }
             }
+            s0 += cnt;
         }
         double2* __restrict__ out = part + e.poff + (uint64_t)c * e.cap;
 #pragma unroll
-        for (int r = 0; r < kBsR; ++r)
-            if (tb + r < n) out[tb + r] = make_double2(uu[r], ww[r]);
+        for (int r = 0; r < 2; ++r)
+            if (tb + r * kF64Threads < n) out[tb + r * kF64Threads] = make_double2(uu[r], ww[r]);
     }
 }
 
@@ -1065,7 +1087,9 @@ __global__ void k_self_combine(const InstDesc* __restrict__ table,
         const uint32_t t = (item - s_pre[k]) * blockDim.x + threadIdx.x;
         if (t >= n) continue;
         double su = 0.0, sw = 0.0;
-        for (int c = 0; c < e.chunks; ++c) {
+        const uint32_t chunks = chunk_count(n, e.chunks);
+#pragma unroll 4
+        for (uint32_t c = 0; c < chunks; ++c) {
             const double2 v = part[e.poff + (uint64_t)c * e.cap + t];
             su += v.x;
             sw += v.y;
@@ -1429,8 +1453,6 @@ void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* 
                          int precision, const Workspace& ws, int sms, cudaStream_t s,
                          const PairConfig& cfg, bool dry) {
     if (precision == kF32) {
-        // cfg.ctas = 1 .. 4 quarters of full occupancy
-        const int g = std::max(1, sms * kNearBlocks * std::max(1, std::min(cfg.ctas, 4)) / 4);
         const double2* pxz = reinterpret_cast<const double2*>(ws.packed);
         cudaMemsetAsync(ws.work, 0, 2 * sizeof(unsigned), s);
         constexpr size_t far_smem = sizeof(FarShared) * kFarWarps;
@@ -1438,14 +1460,21 @@ void biot_savart_compute(const InstDesc* table, InstState* st, const ListEntry* 
         k_far<<<sms * kFarBlocks, 32 * kFarWarps, far_smem, s>>>(st, list, nlist, pxz, ws.nodes,
                                                                  ws.mom, ws.loc, ws.near,
                                                                  ws.work + 1);
-        k_self_f32<kNearBlocks><<<g, 32 * kNearWarps, 0, s>>>(
-            table, st, list, nlist, pxz,
-            reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.perm, ws.nodes,
-            ws.mom, ws.loc, ws.near, dry ? reinterpret_cast<double*>(ws.keys_in) : nullptr,
-            dry ? reinterpret_cast<double*>(ws.keys_out) : nullptr, ws.work);
+        auto near = [&](auto kernel, int warps) {
+            // cfg.ctas = 1 .. 4 quarters of full occupancy
+            const int full = sms * (kNearThreads / (32 * warps));
+            const int g = std::max(1, full * std::max(1, std::min(cfg.ctas, 4)) / 4);
+            kernel<<<g, 32 * warps, 0, s>>>(
+                table, st, list, nlist, pxz,
+                reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.perm, ws.nodes,
+                ws.mom, ws.loc, ws.near, dry ? reinterpret_cast<double*>(ws.keys_in) : nullptr,
+                dry ? reinterpret_cast<double*>(ws.keys_out) : nullptr, ws.work);
+        };
+        if (ws.total_cap / kLeaf <= (uint64_t)sms * 4) near(k_self_f32<8>, 8);
+        else near(k_self_f32<4>, 4);
     } else {
         cudaMemsetAsync(ws.work, 0, sizeof(unsigned), s);
-        k_self_f64<<<sms * kF64Ctas, kBsThreads, 0, s>>>(st, list, nlist, ws.packed, ws.meta,
+        k_self_f64<<<sms * kF64Ctas, kF64Threads, 0, s>>>(st, list, nlist, ws.packed, ws.meta,
                                                              ws.part, ws.work);
     }
 }

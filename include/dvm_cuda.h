@@ -58,7 +58,7 @@ extern "C" {
 #define DVM_ERR_NO_DEVICE 9  /* no CUDA device / library built for another GPU */
 
 /* arithmetic of the pair interactions */
-#define DVM_F64 0 /* FP64, reference operation order */
+#define DVM_F64 0 /* FP64, the reference's formulas */
 #define DVM_F32 1 /* FP32 pair terms with compensated / FP64 sums; FP64 state, QR,
                      refinement residual and Kelvin row */
 
