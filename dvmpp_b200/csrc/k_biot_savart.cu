@@ -1102,11 +1102,8 @@ __global__ void k_self_combine(const InstDesc* __restrict__ table,
 }
 
 // ---- arbitrary targets --------------------------------------------------------
-// One item = (job, a tile of targets, a chunk of `chunk` sources: kAtChunk for
-// at-target calls, rhs_chunk_for(...) for a simulation's right-hand side).
-// Sources are staged with FP64 positions; each pair forms dx, dz in FP64
-// (exact for close pairs) and, in FP32 mode, evaluates the kernel in FP32 with
-// Kahan-compensated sums.
+// One item = (job, a tile of 256 targets, a chunk of `chunk` sources: at_chunk(...)
+// for at-target calls, rhs_chunk_for(...) for a simulation's right-hand side).
 struct AtJob {
     const double* tx;
     const double* tz;
@@ -1137,20 +1134,25 @@ __device__ __forceinline__ void kahan2_fma(uint64_t& s, uint64_t& e, uint64_t a,
 // Velocity at targets from a chunk of J.chunk sources per work item, 256
 // targets per item, one per thread.
 //
-// FP32 jobs without the close-pair skip (the blob-on-collocation right-hand
-// side) pack two SOURCES per FP32x2 instruction, so no lane idles however few
-// targets a body has.  Offsets are formed without per-pair conversions: every
-// position is taken relative to the job's first target in FP64 and split
-// exactly into an FP32 pair (hi, lo = the FP64 remainder); dx = (t_hi - s_hi)
-// + (t_lo - s_lo), exact before its final rounding for close pairs (Sterbenz)
-// and within an ulp otherwise.  Each pair keeps its compensated update (the
+// FP32 jobs pack two SOURCES per FP32x2 instruction, so no lane idles however few
+// targets a job has.  Offsets are formed without per-pair conversions: every
+// position is taken relative to the tile's first target in FP64 and split into an
+// FP32 pair, hi of 16 bits and lo = the remainder (40 bits together); dx = (t_hi -
+// s_hi) + (t_lo - s_lo), where the first difference is exact unless one
+// position is 2^8 times farther out than the other, so dx is rounded once (hi of
+// 24 bits rounds it twice: error against 64 bits 4 % up, this 7 % down against
+// FP64 differences rounded once).  Each pair keeps its compensated update (the
 // right-hand side is the small residual normal velocity, so its rounding must
 // stay relative to the few large near-blob terms, not compound): one Kahan
 // sum per half, the halves added at the end.  The core kernel runs for both
 // halves when any lane of the warp has a pair inside a core.  Sources are
 // staged as packed pairs (two 16-byte loads bring positions, two more the
-// circulations and core constants).  Skip jobs (at-target plugin calls,
-// probes) and FP64 jobs run the scalar loops.
+// circulations and core constants).  Where close pairs are skipped, a pair with
+// not r2 > 1e-15 (NaN included) adds nothing.
+__device__ __forceinline__ void split_16(double v, float& hi, float& lo) {
+    hi = __int_as_float((__float_as_int((float)v) + 0x80) & ~0xFF);
+    lo = (float)(v - (double)hi);
+}
 struct AtStage {
     float4 pos_hi[128];  // (x_hi a, x_hi b, z_hi a, z_hi b) of sources 2i, 2i+1
     float4 pos_lo[128];  // (x_lo a, x_lo b, z_lo a, z_lo b)
@@ -1161,64 +1163,63 @@ struct AtStage {
 template <bool F32>
 __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int njobs) {
     __shared__ unsigned s_pre[kMaxList + 1];
-    __shared__ double s_x[256], s_z[256], s_c[256], s_thr[256], s_rs[256];
-    __shared__ float s_cf[256], s_thrf[256], s_rsf[256];  // FP32 copies (scalar FP32 path)
-    __shared__ AtStage s_pk;                               // packed pairs (fast FP32 path)
+    // FP64: x, z, circ, 10 sigma^2 and 1 / sigma^2; FP32: packed pairs
+    __shared__ union Stage {
+        struct {
+            double4 src[256];
+            double rs[256];
+        } d;
+        AtStage f;
+        __device__ Stage() {}
+    } S;
     __shared__ double s_red[8];
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < njobs; ++k) {
-            s_pre[k] = acc;
-            const uint32_t ns = jobs[k].pns ? *jobs[k].pns : jobs[k].ns;
-            acc += ((jobs[k].nt + 255) / 256) * ((ns + jobs[k].chunk - 1) / jobs[k].chunk);
-        }
-        s_pre[njobs] = acc;
-    }
-    __syncthreads();
+    list_prefix(s_pre, njobs, [&](int k) {
+        const uint32_t ns = jobs[k].pns ? *jobs[k].pns : jobs[k].ns;
+        return ((jobs[k].nt + 255) / 256) * ((ns + jobs[k].chunk - 1) / jobs[k].chunk);
+    });
     const unsigned total = s_pre[njobs];
     for (unsigned item = blockIdx.x; item < total; item += gridDim.x) {
         const int k = locate(s_pre, njobs, item);
         const AtJob J = jobs[k];
-        const bool packed = F32 && !J.skip_close;
+        const bool skip = J.skip_close != 0;
         const uint32_t ns = J.pns ? *J.pns : J.ns;
         const uint32_t nchunk = (ns + J.chunk - 1) / J.chunk;
         const unsigned local = item - s_pre[k];
         const uint32_t ttile = local / nchunk, c = local % nchunk;
         const uint32_t t = ttile * 256 + threadIdx.x;
         const double tx = t < J.nt ? J.tx[t] : 0.0, tz = t < J.nt ? J.tz[t] : 0.0;
-        const double ox = J.tx[0], oz = J.tz[0];  // the job's origin: its first target
+        const double ox = J.tx[ttile * 256], oz = J.tz[ttile * 256];  // the tile's origin
         float txh, txl, tzh, tzl;
-        split_hi_lo(tx - ox, txh, txl);
-        split_hi_lo(tz - oz, tzh, tzl);
+        split_16(tx - ox, txh, txl);
+        split_16(tz - oz, tzh, tzl);
         const uint64_t TXH = f2pack(txh, txh), TXL = f2pack(txl, txl);
         const uint64_t TZH = f2pack(tzh, tzh), TZL = f2pack(tzl, tzl);
         const uint32_t j0 = c * J.chunk, j1 = min(ns, j0 + J.chunk);
         double uu = 0.0, ww = 0.0, csum = 0.0;
         const uint64_t zero2 = f2pack(0.0f, 0.0f);
         uint64_t snu = zero2, enu = zero2, sw = zero2, ew = zero2;  // -u and w, packed Kahan
-        float su = 0.f, cu = 0.f, sws = 0.f, cws = 0.f;
         for (uint32_t s0 = j0; s0 < j1; s0 += 256) {
             __syncthreads();
             const uint32_t j = s0 + threadIdx.x;
-            if (packed) {
+            if (F32) {
                 // slot (pair i = tid / 2, half h = tid % 2); a slot past the
                 // chunk holds a far, circulation-free source (it adds 0)
                 float xh = 1.0e18f, xl = 0.f, zh = 0.f, zl = 0.f, cf = 0.f, thr = 0.f, rsf = 0.f;
                 if (j < j1) {
                     const double sg = J.ss[j];
                     const double s2 = dmul(sg, sg);
-                    split_hi_lo(J.sx[j] - ox, xh, xl);
-                    split_hi_lo(J.sz[j] - oz, zh, zl);
+                    split_16(J.sx[j] - ox, xh, xl);
+                    split_16(J.sz[j] - oz, zh, zl);
                     cf = (float)J.sc[j];
                     thr = (float)dmul(10.0, s2);
                     rsf = (float)ddiv(1.0, s2);
                     if (ttile == 0) csum += J.sc[j];
                 }
                 const int i = threadIdx.x >> 1, h = threadIdx.x & 1;
-                float* ph = reinterpret_cast<float*>(&s_pk.pos_hi[i]);
-                float* pl = reinterpret_cast<float*>(&s_pk.pos_lo[i]);
-                float* pc = reinterpret_cast<float*>(&s_pk.cst[i]);
-                float* pr = reinterpret_cast<float*>(&s_pk.rs[i]);
+                float* ph = reinterpret_cast<float*>(&S.f.pos_hi[i]);
+                float* pl = reinterpret_cast<float*>(&S.f.pos_lo[i]);
+                float* pc = reinterpret_cast<float*>(&S.f.cst[i]);
+                float* pr = reinterpret_cast<float*>(&S.f.rs[i]);
                 ph[h] = xh;
                 ph[2 + h] = zh;
                 pl[h] = xl;
@@ -1229,74 +1230,55 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
             } else if (j < j1) {
                 const double sg = J.ss[j];
                 const double s2 = dmul(sg, sg);
-                s_x[threadIdx.x] = J.sx[j];
-                s_z[threadIdx.x] = J.sz[j];
-                s_c[threadIdx.x] = J.sc[j];
-                s_thr[threadIdx.x] = dmul(10.0, s2);
-                s_rs[threadIdx.x] = ddiv(1.0, s2);
-                if (F32) {  // converted once per source instead of once per pair
-                    s_cf[threadIdx.x] = (float)s_c[threadIdx.x];
-                    s_thrf[threadIdx.x] = (float)s_thr[threadIdx.x];
-                    s_rsf[threadIdx.x] = (float)s_rs[threadIdx.x];
-                }
+                S.d.src[threadIdx.x] = make_double4(J.sx[j], J.sz[j], J.sc[j], dmul(10.0, s2));
+                S.d.rs[threadIdx.x] = ddiv(1.0, s2);
                 if (ttile == 0) csum += J.sc[j];
             }
             __syncthreads();
             const int cnt = (int)min(256u, j1 - s0);
-            if (packed) {
+            if (F32) {
+#pragma unroll 4
                 for (int i = 0; i < (cnt + 1) / 2; ++i) {
-                    const float4 H = s_pk.pos_hi[i], L = s_pk.pos_lo[i], Cs = s_pk.cst[i];
-                    const uint64_t DX = f2add(f2sub(TXH, f2pack(H.x, H.y)),
-                                              f2sub(TXL, f2pack(L.x, L.y)));
-                    const uint64_t DZ = f2add(f2sub(TZH, f2pack(H.z, H.w)),
-                                              f2sub(TZL, f2pack(L.z, L.w)));
+                    const float4 H = S.f.pos_hi[i], L = S.f.pos_lo[i], Cs = S.f.cst[i];
+                    uint64_t DX = f2add(f2sub(TXH, f2pack(H.x, H.y)), f2sub(TXL, f2pack(L.x, L.y)));
+                    uint64_t DZ = f2add(f2sub(TZH, f2pack(H.z, H.w)), f2sub(TZL, f2pack(L.z, L.w)));
                     const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
                     const float ra = f2lo(R2), rb = f2hi(R2);
                     float ka = rcp_approx(ra), kb = rcp_approx(rb);
                     const bool ca = ra < Cs.z, cb = rb < Cs.w;
                     if (__any_sync(0xffffffffu, ca || cb)) {
-                        const float2 R = s_pk.rs[i];
+                        const float2 R = S.f.rs[i];
                         const float qa = core_kernel_expm1(ra, R.x, ka);
                         const float qb = core_kernel_expm1(rb, R.y, kb);
                         ka = ca ? qa : ka;
                         kb = cb ? qb : kb;
                     }
+                    if (skip) {  // computeInducedAt (src/VelocityKernel.cpp:89)
+                        const bool oa = ra > 1e-15f, ob = rb > 1e-15f;
+                        ka = oa ? ka : 0.f;
+                        kb = ob ? kb : 0.f;
+                        DX = f2pack(oa ? f2lo(DX) : 0.f, ob ? f2hi(DX) : 0.f);
+                        DZ = f2pack(oa ? f2lo(DZ) : 0.f, ob ? f2hi(DZ) : 0.f);
+                    }
                     const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
                     kahan2_fma(snu, enu, G, DZ);
                     kahan2_fma(sw, ew, G, DX);
                 }
-            } else if (F32) {
-                for (int jj = 0; jj < cnt; ++jj) {
-                    const float dx = (float)(tx - s_x[jj]);
-                    const float dz = (float)(tz - s_z[jj]);
-                    const float r2 = fmaf(dx, dx, dz * dz);
-                    if (!(r2 > 1e-15f)) continue;  // skip_close (computeInducedAt :89)
-                    float K = rcp_approx(r2);
-                    if (r2 < s_thrf[jj]) K = core_kernel_expm1(r2, s_rsf[jj], K);
-                    const float g = K * s_cf[jj];
-                    kahan(su, cu, -g * dz);
-                    kahan(sws, cws, g * dx);
-                }
             } else {
                 for (int jj = 0; jj < cnt; ++jj) {
-                    const double dx = dsub(tx, s_x[jj]);
-                    const double dz = dsub(tz, s_z[jj]);
-                    const double r2 = dadd(dmul(dx, dx), dmul(dz, dz));
-                    if (J.skip_close && !(r2 > 1e-15)) continue;
-                    double K;
-                    if (r2 < s_thr[jj]) K = ddiv(dsub(1.0, exp(dmul(-r2, s_rs[jj]))), r2);
-                    else K = __drcp_rn(r2);  // correctly rounded: the same value as 1.0 / r2
-                    uu = dsub(uu, dmul(dmul(K, dz), s_c[jj]));
-                    ww = dadd(ww, dmul(dmul(K, dx), s_c[jj]));
+                    const double4 sj = S.d.src[jj];
+                    const double dx = dsub(tx, sj.x), dz = dsub(tz, sj.y);
+                    const double r2 = fma(dx, dx, dmul(dz, dz));
+                    if (skip && !(r2 > 1e-15)) continue;
+                    const double g = dmul(kernel_f64(r2, sj.w, S.d.rs[jj]), sj.z);
+                    uu = fma(-g, dz, uu);
+                    ww = fma(g, dx, ww);
                 }
             }
         }
-        if (packed) {
+        if (F32) {
             uu = -(((double)f2lo(snu) + (double)f2lo(enu)) + ((double)f2hi(snu) + (double)f2hi(enu)));
             ww = ((double)f2lo(sw) + (double)f2lo(ew)) + ((double)f2hi(sw) + (double)f2hi(ew));
-        } else if (F32) {
-            uu = (double)su - (double)cu;
-            ww = (double)sws - (double)cws;
         }
         if (t < J.nt) J.part[(uint64_t)c * J.npad + t] = make_double2(uu, ww);
         if (ttile == 0 && J.circ_part) {
@@ -1312,20 +1294,38 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
     }
 }
 
-__global__ void k_at_combine(const AtJob* __restrict__ jobs, double* __restrict__ u,
-                             double* __restrict__ w) {
+// Sums a job's chunk partials: a block finishes 32 targets, warp w adding chunks
+// w, w + W, ... for its lane's target and the W warp sums added in warp order.
+__global__ void __launch_bounds__(1024) k_at_combine(const AtJob* __restrict__ jobs,
+                                                     double* __restrict__ u,
+                                                     double* __restrict__ w) {
+    __shared__ double2 s_sum[32][32];
     const AtJob J = jobs[0];
     const uint32_t ns = J.pns ? *J.pns : J.ns;
     const uint32_t nchunk = (ns + J.chunk - 1) / J.chunk;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < J.nt; t += gridDim.x * blockDim.x) {
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (uint32_t t0 = blockIdx.x * 32; t0 < J.nt; t0 += gridDim.x * 32) {
+        const uint32_t t = t0 + lane;
         double su = 0.0, sw = 0.0;
-        for (uint32_t c = 0; c < nchunk; ++c) {
-            const double2 v = J.part[(uint64_t)c * J.npad + t];
-            su += v.x;
-            sw += v.y;
+        if (t < J.nt) {
+#pragma unroll 4
+            for (uint32_t c = wid; c < nchunk; c += warps) {
+                const double2 v = J.part[(uint64_t)c * J.npad + t];
+                su += v.x;
+                sw += v.y;
+            }
         }
-        u[t] = su * kRpi2;
-        w[t] = sw * kRpi2;
+        s_sum[wid][lane] = make_double2(su, sw);
+        __syncthreads();
+        if (wid == 0 && t < J.nt) {
+            for (uint32_t q = 1; q < warps; ++q) {
+                su += s_sum[q][lane].x;
+                sw += s_sum[q][lane].y;
+            }
+            u[t] = su * kRpi2;
+            w[t] = sw * kRpi2;
+        }
+        __syncthreads();
     }
 }
 
@@ -1504,10 +1504,36 @@ void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int 
     k_rhs_combine<<<dim3((max_np + 31) / 32, nlist), 256, 0, s>>>(table, st, list, jobs);
 }
 
+// Sources per work item of an at-target call: a multiple of 256, at most kAtChunk,
+// that leaves about 1184 items, two to three rounds of the resident blocks (256
+// targets against 2^20 sources: 256 items of 4096 left half of the blocks idle, the
+// call 685 us; 303 now; chunks in multiples of 64, 348).
+static uint32_t at_chunk(uint64_t ns, uint64_t nt) {
+    const uint64_t want = (ns * ((nt + 255) / 256) + 1183) / 1184;
+    return (uint32_t)std::max<uint64_t>(256, std::min<uint64_t>(kAtChunk, (want + 255) / 256 * 256));
+}
+
+// Warps per block of k_at_combine: about four chunks each.
+static unsigned combine_threads(uint64_t nchunk) {
+    unsigned w = 1;
+    while (w < 32 && 4ull * w < nchunk) w *= 2;
+    return 32 * w;
+}
+
 size_t direct_at_part_elems(uint32_t ns, uint32_t nt) {
-    const size_t nchunk = (ns + kAtChunk - 1) / kAtChunk;
+    const size_t chunk = at_chunk(ns, nt);
+    const size_t nchunk = (ns + chunk - 1) / chunk;
     const size_t npad = (nt + 255) / 256 * 256;
     return std::max<size_t>(1, nchunk) * std::max<size_t>(npad, 256) + 64;
+}
+
+static void launch_at(const AtJob* job, const AtJob& J, int precision, double* u, double* w, int sms,
+                      cudaStream_t s) {
+    if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(job, 1);
+    else k_at<false><<<sms * 4, 256, 0, s>>>(job, 1);
+    const unsigned blocks = (unsigned)std::min<uint64_t>(((uint64_t)J.nt + 31) / 32, (uint64_t)sms * 16);
+    k_at_combine<<<std::max(1u, blocks), combine_threads((J.ns + J.chunk - 1) / J.chunk), 0, s>>>(
+        job, u, w);
 }
 
 void direct_at_raw(const double* x, const double* z, const double* circ, const double* sigma,
@@ -1529,15 +1555,12 @@ void direct_at_raw(const double* x, const double* z, const double* circ, const d
     J.pns = nullptr;
     J.ns = ns;
     J.npad = (int)std::max<size_t>((nt + 255) / 256 * 256, 256);
-    J.chunk = kAtChunk;
+    J.chunk = at_chunk(ns, nt);
     J.part = part;
     J.circ_part = nullptr;
     cudaMemcpyAsync(job, &J, sizeof(AtJob), cudaMemcpyHostToDevice, s);
     if (ns > 0) {
-        if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(job, 1);
-        else k_at<false><<<sms * 4, 256, 0, s>>>(job, 1);
-        k_at_combine<<<std::max<uint32_t>(1, std::min<uint32_t>((nt + 255) / 256, sms * 8)), 256, 0,
-                       s>>>(job, u, w);
+        launch_at(job, J, precision, u, w, sms, s);
     } else {
         cudaMemsetAsync(u, 0, sizeof(double) * nt, s);
         cudaMemsetAsync(w, 0, sizeof(double) * nt, s);
@@ -1614,15 +1637,15 @@ extern "C" int dvm_biot_savart_at_noalloc(const double* x, const double* z, cons
     J.pns = nullptr;
     J.ns = (uint32_t)ns;
     J.npad = (int)npad;
-    J.chunk = kAtChunk;
+    // (kAtChunk fits, by the check above; shorter chunks as far as the scratch holds them)
+    const uint64_t most = (kNoAllocElems - kNoAllocJobElems) / npad;
+    J.chunk = std::max<uint32_t>(at_chunk(ns, nt),
+                                 (uint32_t)std::min<uint64_t>(kAtChunk, ((ns + most - 1) / most + 255) / 256 * 256));
     J.part = scratch;  // every entry read by k_at_combine is written by k_at first
     J.circ_part = nullptr;
     AtJob* job = reinterpret_cast<AtJob*>(scratch + (kNoAllocElems - kNoAllocJobElems));
     k_write_job<<<1, 1, 0, s>>>(job, J);
-    if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(job, 1);
-    else k_at<false><<<sms * 4, 256, 0, s>>>(job, 1);
-    const unsigned cb = (unsigned)std::min<uint64_t>((nt + 255) / 256, (uint64_t)sms * 8);
-    k_at_combine<<<std::max(1u, cb), 256, 0, s>>>(job, u, w);
+    launch_at(job, J, precision, u, w, sms, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return report_error(3, (std::string("dvm_biot_savart_at_noalloc launch: ") +
