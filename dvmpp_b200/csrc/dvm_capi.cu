@@ -78,7 +78,8 @@ struct SubList {
     ListEntry* d_list = nullptr;
     int n = 0;
     int max_np = 0;
-    uint64_t total = 0;  // sum of capacities
+    uint64_t total = 0;   // sum of capacities
+    uint64_t pnodes = 0;  // nodes of the panels' trees
     std::vector<ListEntry> host;  // the entries as uploaded
     // FP32 pair-kernel launch shape (from the context's tuning table) and, for
     // order 1, the same entries costliest-first (the pair kernel's list only)
@@ -115,9 +116,9 @@ bool valid_pair_config(const dvm_pair_config& p) {
 
 struct Plan {
     std::vector<int> slots;            // the batch, in launch order
-    SubList all, euler, rk3, rk3_f32, rk3_f64, eul_f32, eul_f64, refl, del;
+    SubList all, rk3_f32, rk3_f64, eul_f32, eul_f64, refl, del;
     uint64_t ws_need_cap = 0;          // sizing inputs
-    uint64_t part_elems = 0, rhs_elems = 0, circ_elems = 0;
+    uint64_t part_elems = 0, rhs_elems = 0, circ_elems = 0, pan_elems = 0;
     bool need_delete = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -141,7 +142,7 @@ struct dvm_ctx {
     uint32_t next_uid = 1;
     // shared workspace
     Workspace ws;
-    uint64_t ws_cap = 0, ws_part = 0, ws_rhs = 0, ws_circ = 0, ws_lists = 0;
+    uint64_t ws_cap = 0, ws_part = 0, ws_rhs = 0, ws_circ = 0, ws_panels = 0, ws_lists = 0;
     bool ws_delete = false;
     void* ws_block = nullptr;
     uint64_t ws_generation = 0;
@@ -265,13 +266,20 @@ void pool_free(dvm_ctx* c, void* p) {
     if (p) cudaFreeAsync(p, c->stream);
 }
 
+// Nodes of a simulation's panel tree, and an upper bound of those of `lists`
+// simulations with `panels` panels together.
+uint64_t panel_nodes(int np) { return 2ull * panel_leaves(np) + kNodeSlack; }
+uint64_t panel_nodes_bound(uint64_t panels, uint64_t lists) {
+    return 2 * (panels / kPanelLeaf + lists) + kNodeSlack * lists;
+}
+
 int build_sublist(dvm_ctx* c, SubList& sl, Plan& pl, bool f32_pairs = false) {
     sl.n = (int)sl.slots.size();
     if (sl.n == 0) return DVM_OK;
     if (pl.pool_used + (size_t)sl.n * (f32_pairs ? 2 : 1) > kPoolPerPlan)
         return fail(DVM_ERR_STATE, "plan list pool exhausted");
     std::vector<ListEntry> h(sl.n);
-    uint64_t coff = 0, poff = 0, roff = 0, cofs = 0;
+    uint64_t coff = 0, poff = 0, roff = 0, cofs = 0, panoff = 0;
     for (int k = 0; k < sl.n; ++k) {
         const dvm_sim* s = c->slots[sl.slots[k]];
         ListEntry& e = h[k];
@@ -287,6 +295,10 @@ int build_sublist(dvm_ctx* c, SubList& sl, Plan& pl, bool f32_pairs = false) {
         e.roff = roff;
         e.cofs = cofs;
         e.noff = 2 * coff / kLeaf + (uint64_t)kNodeSlack * k;
+        e.pnoff = sl.pnodes;
+        e.panoff = panoff;
+        sl.pnodes += panel_nodes(s->h.np);
+        panoff += (uint64_t)s->h.np;
         coff += e.cap;  // caps are multiples of kCapAlign
         if (s->h.precision != kF32)  // the FP32 path has no chunk partials
             poff += (uint64_t)e.chunks * e.cap;
@@ -299,6 +311,7 @@ int build_sublist(dvm_ctx* c, SubList& sl, Plan& pl, bool f32_pairs = false) {
     pl.part_elems = std::max(pl.part_elems, poff);
     pl.rhs_elems = std::max(pl.rhs_elems, roff);
     pl.circ_elems = std::max(pl.circ_elems, cofs);
+    pl.pan_elems = std::max(pl.pan_elems, panoff);
     // The plan's lists live in its slot of the context's list pool; the copy is
     // ordered on the stream after every kernel that read the slot before.
     sl.d_list = c->list_pool + (size_t)pl.pool_slot * kPoolPerPlan + pl.pool_used;
@@ -322,14 +335,15 @@ int build_sublist(dvm_ctx* c, SubList& sl, Plan& pl, bool f32_pairs = false) {
 }
 
 int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint64_t circ,
-                     int nlist, bool need_delete) {
-    if (cap <= c->ws_cap && part <= c->ws_part && rhs <= c->ws_rhs && circ <= c->ws_circ &&
+                     uint64_t panels, int nlist, bool need_delete) {
+    if (panels <= c->ws_panels && cap <= c->ws_cap && part <= c->ws_part && rhs <= c->ws_rhs && circ <= c->ws_circ &&
         (uint64_t)nlist <= c->ws_lists && (!need_delete || c->ws_delete))
         return DVM_OK;
     cap = std::max<uint64_t>({cap, c->ws_cap, kCapAlign});
     part = std::max(part, c->ws_part);
     rhs = std::max(rhs, c->ws_rhs);
     circ = std::max(circ, c->ws_circ);
+    panels = std::max(panels, c->ws_panels);
     const uint64_t lists = std::max<uint64_t>({(uint64_t)nlist, c->ws_lists, 64});
     need_delete = need_delete || c->ws_delete;
     CK(cudaStreamSynchronize(c->stream));
@@ -340,6 +354,7 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     }
     const size_t cub = cub_sort_bytes(cap);
     const uint64_t nodes = 2 * cap / kLeaf + (uint64_t)kNodeSlack * lists;
+    const uint64_t pnodes = panel_nodes_bound(panels, lists);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -352,6 +367,8 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
                  o_nodes = take(sizeof(TreeNode) * nodes), o_mom = take(16 * kTerms * nodes),
                  o_loc = take(16 * kTerms * nodes), o_arr = take(4 * nodes),
                  o_near = take(sizeof(NearRow) * (cap / kLeaf + 1)),
+                 o_pnodes = take(sizeof(TreeNode) * pnodes), o_pmom = take(16 * kTerms * pnodes),
+                 o_parr = take(4 * pnodes), o_pan = take(sizeof(PanelRec) * panels),
                  o_rhs = take(16 * rhs), o_circ = take(8 * circ + 8), o_cub = take(cub + 256),
                  o_work = take(64 * sizeof(unsigned)), o_flags = take(cap),
                  o_tiles = take(4 * (cap / 1024 + 1)),
@@ -382,6 +399,10 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     w.mom = reinterpret_cast<double2*>(b + o_mom);
     w.loc = reinterpret_cast<double2*>(b + o_loc);
     w.near = reinterpret_cast<NearRow*>(b + o_near);
+    w.pnodes = reinterpret_cast<TreeNode*>(b + o_pnodes);
+    w.pmom = reinterpret_cast<double2*>(b + o_pmom);
+    w.parrived = reinterpret_cast<unsigned*>(b + o_parr);
+    w.pan = reinterpret_cast<PanelRec*>(b + o_pan);
     w.arrived = reinterpret_cast<unsigned*>(b + o_arr);
     w.rhs_part = reinterpret_cast<double2*>(b + o_rhs);
     w.circ_part = reinterpret_cast<double*>(b + o_circ);
@@ -398,6 +419,7 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     c->ws_part = part;
     c->ws_rhs = rhs;
     c->ws_circ = circ;
+    c->ws_panels = panels;
     c->ws_lists = lists;
     c->ws_delete = need_delete;
     c->ws_generation++;
@@ -467,9 +489,12 @@ void issue_step(dvm_ctx* c, Plan& pl) {
     auto on = [&](const SubList& sl) {
         ws.total_cap = sl.total;
         ws.key_bits = key_bits_for(sl.n);
+        ws.pnodes_used = sl.pnodes;
         return ws;
     };
-    auto nbody = [&](SubList& sl, int prec) {
+    // velocities, right-hand side, solve and sheet velocity of one stage for the
+    // simulations of one precision (the FP32 kernels share one tree of the blobs)
+    auto stage = [&](SubList& sl, int prec, int mode) {
         if (!sl.n) return;
         on(sl);
         int p = prof_begin(c, DVM_PROF_SORT);
@@ -484,38 +509,29 @@ void issue_step(dvm_ctx* c, Plan& pl) {
         p = prof_begin(c, DVM_PROF_SORT);
         biot_savart_finish(T, S, sl.d_list, sl.n, prec, ws, sms, s);
         prof_end(c, p);
-        L += 4;  // keys, pack, pair kernel, combine
         p = prof_begin(c, DVM_PROF_RHS);
         sheet_rhs(T, S, sl.d_list, sl.n, sl.max_np, prec, ws, sms, s);
         prof_end(c, p);
-        L += 3;
-    };
-    auto stage = [&](SubList& g, int mode) {
-        on(g);
-        int p = prof_begin(c, DVM_PROF_SOLVE);
-        sheet_solve(T, S, g.d_list, g.n, g.max_np, s);
+        p = prof_begin(c, DVM_PROF_SOLVE);
+        sheet_solve(T, S, sl.d_list, sl.n, sl.max_np, s);
         prof_end(c, p);
         p = prof_begin(c, DVM_PROF_SHEETVEL);
-        sheet_velocity(T, S, g.d_list, g.n, mode, g.max_np, ws, sms, s);
+        sheet_velocity(T, S, sl.d_list, sl.n, mode, sl.max_np, prec, ws, sms, s);
         prof_end(c, p);
-        L += 4;
+        // FP32: keys, tree, far, pairs, right-hand side, solve 3, panels' tree, sheet;
+        // FP64: keys, pack, pairs, combine, right-hand side 3, solve 3, sheet
+        L += prec == kF32 ? 10 : 11;
     };
     const int pstep = prof_begin(c, DVM_PROF_STEP);
     int p = prof_begin(c, DVM_PROF_LOADS);
     step_counter(S, pl.all.d_list, pl.all.n, s);
     prof_end(c, p);
     L += 1;
-    if (pl.euler.n) {
-        nbody(pl.eul_f32, kF32);
-        nbody(pl.eul_f64, kF64);
-        stage(pl.euler, 1);
-    }
-    if (pl.rk3.n) {
-        for (int st = 0; st < 3; ++st) {
-            nbody(pl.rk3_f32, kF32);
-            nbody(pl.rk3_f64, kF64);
-            stage(pl.rk3, 2 + st);
-        }
+    stage(pl.eul_f32, kF32, 1);
+    stage(pl.eul_f64, kF64, 1);
+    for (int st = 0; st < 3; ++st) {
+        stage(pl.rk3_f32, kF32, 2 + st);
+        stage(pl.rk3_f64, kF64, 2 + st);
     }
     on(pl.all);
     p = prof_begin(c, DVM_PROF_DIFFREL);
@@ -569,7 +585,6 @@ int get_plan(dvm_ctx* c, const std::vector<int>& slots, Plan** out) {
         const dvm_sim* s = c->slots[sl];
         pl->all.slots.push_back(sl);
         const bool rk3 = s->h.scheme == kRK3, f32 = s->h.precision == kF32;
-        (rk3 ? pl->rk3 : pl->euler).slots.push_back(sl);
         if (rk3) (f32 ? pl->rk3_f32 : pl->rk3_f64).slots.push_back(sl);
         else (f32 ? pl->eul_f32 : pl->eul_f64).slots.push_back(sl);
         if (s->h.cross == kDelete) {
@@ -579,7 +594,7 @@ int get_plan(dvm_ctx* c, const std::vector<int>& slots, Plan** out) {
             pl->refl.slots.push_back(sl);
         }
     }
-    SubList* subs[] = {&pl->all, &pl->euler, &pl->rk3, &pl->rk3_f32, &pl->rk3_f64,
+    SubList* subs[] = {&pl->all, &pl->rk3_f32, &pl->rk3_f64,
                        &pl->eul_f32, &pl->eul_f64, &pl->refl, &pl->del};
     for (SubList* s : subs) {
         const int rc = build_sublist(c, *s, *pl, s == &pl->rk3_f32 || s == &pl->eul_f32);
@@ -611,7 +626,7 @@ int run_steps(dvm_ctx* c, const std::vector<int>& slots, int nsteps, bool use_gr
     Plan* pl = nullptr;
     int rc = get_plan(c, slots, &pl);
     if (rc) return rc;
-    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems,
+    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems, pl->pan_elems,
                           (int)slots.size(), pl->need_delete);
     if (rc) return rc;
     if (pl->exec && pl->ws_generation != c->ws_generation) {
@@ -874,7 +889,7 @@ int dvm_ctx_reserve(dvm_ctx* c, uint64_t total_capacity, int max_sims, int max_p
     const uint64_t part = 16 * T + S * (2u << 20);
     const uint64_t rchunks = T / kAtChunk + S * 602;
     return ensure_workspace(c, T, part, rchunks * align_up((size_t)max_panels, 256), rchunks,
-                            max_sims, with_delete != 0);
+                            S * (uint64_t)max_panels, max_sims, with_delete != 0);
 }
 
 int dvm_ctx_pool_reserve(dvm_ctx* c, uint64_t bytes) {
@@ -1963,7 +1978,7 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
     Plan* pl = nullptr;
     int rc = get_plan(c, one, &pl);
     if (rc) return rc;
-    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems, 1,
+    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems, pl->pan_elems, 1,
                           pl->need_delete || phase == DVM_PHASE_DELETE);
     if (rc) return rc;
     InstDesc* T = c->d_table;
@@ -1971,6 +1986,7 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
     Workspace ws = c->ws;
     ws.key_bits = key_bits_for(1);
     ws.total_cap = pl->all.total;
+    ws.pnodes_used = pl->all.pnodes;
     cudaStream_t st = c->stream;
     const ListEntry* L = pl->all.d_list;
     const int np = s->h.np, prec = s->h.precision;
@@ -1989,17 +2005,21 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
             break;
         }
         case DVM_PHASE_SOLVE:
+            if (prec == kF32) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
             sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st);
             sheet_solve(T, S, L, 1, np, st);
             break;
-        case DVM_PHASE_SHEETBC: sheet_velocity(T, S, L, 1, 0, np, ws, c->sms, st); break;
+        case DVM_PHASE_SHEETBC:
+            if (prec == kF32) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            sheet_velocity(T, S, L, 1, 0, np, prec, ws, c->sms, st);
+            break;
         case DVM_PHASE_CONVECT:
             for (int k = 0; k < (s->h.scheme == kRK3 ? 3 : 1); ++k) {
                 biot_savart_self(T, S, L, 1, prec, ws, c->sms, st,
                                  tuned_config(c, shape_class(s->h.cap, 1)));
                 sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st);
                 sheet_solve(T, S, L, 1, np, st);
-                sheet_velocity(T, S, L, 1, s->h.scheme == kRK3 ? 2 + k : 1, np, ws, c->sms, st);
+                sheet_velocity(T, S, L, 1, s->h.scheme == kRK3 ? 2 + k : 1, np, prec, ws, c->sms, st);
             }
             break;
         case DVM_PHASE_DIFFUSE: diffuse(T, S, L, 1, ws, c->sms, st); break;
@@ -2145,7 +2165,7 @@ int dvm_ctx_autotune(dvm_ctx* c, dvm_sim* const* sims, int nsims, int reps, dvm_
     Plan* pl = nullptr;
     rc = get_plan(c, slots, &pl);  // its `all` list is exactly the FP32 members
     if (rc) return rc;
-    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems,
+    rc = ensure_workspace(c, pl->ws_need_cap, pl->part_elems, pl->rhs_elems, pl->circ_elems, pl->pan_elems,
                           (int)slots.size(), pl->need_delete);
     if (rc) return rc;
     if (!c->d_tune_list) CK(cudaMalloc(&c->d_tune_list, sizeof(ListEntry) * 1024));
@@ -2254,7 +2274,7 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     e.rhs_chunk = kAtChunk;
     e.npad = 256;
     const uint64_t part = precision == kF32 ? 1 : (uint64_t)e.chunks * cap;  // FP64 partials
-    int rc = ensure_workspace(c, cap, part, 256, 1, 1, false);
+    int rc = ensure_workspace(c, cap, part, 256, 1, 1, 1, false);
     if (rc) return rc;
     ListEntry* d_list = reinterpret_cast<ListEntry*>(c->ws.jobs);
     InstState st0;

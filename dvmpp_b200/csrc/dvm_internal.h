@@ -62,6 +62,24 @@ struct __align__(16) TreeNode {
     double pad2;
 };
 
+// The sheet as a source: kPanelPoints vortices per panel (Gauss points), a leaf of
+// the panels' tree holds kPanelLeaf panels.
+constexpr int kPanelPoints = 4;
+constexpr int kPanelLeaf = kLeaf / kPanelPoints;
+__host__ __device__ inline uint32_t panel_leaves(int np) {
+    return ((uint32_t)np + kPanelLeaf - 1) / kPanelLeaf;
+}
+// FP32 panel constants, each duplicated into both halves of a packed pair, so
+// that one 16-byte shared load brings two of them for both blobs of a thread
+// (.x and .y of each field are (v, v) pairs), and the FP64 panel origin and end.
+struct __align__(16) PanelRec {
+    ulonglong2 cs;  // (cos th, cos th), (sin th, sin th)
+    ulonglong2 dd;  // (ds, ds), (1/ds, 1/ds)
+    ulonglong2 cc;  // (cos -2th, ...), (sin -2th, ...)
+    ulonglong2 gd;  // (gamma_j, ...), (gamma_{j+1} - gamma_j, ...)
+    double xc, zc, ex, ez;
+};
+
 // What a leaf of targets sums itself: leaves pair by pair (from the front) and
 // nodes whose moments it evaluates at every target (from the back).
 constexpr uint32_t kNearRow = 126;
@@ -72,7 +90,7 @@ struct __align__(16) NearRow {
 };
 
 // Sources per work item of a simulation's blob-on-collocation right-hand side:
-// a power of two in [512, kAtChunk], the smallest that still leaves about 600
+// a power of two in [64, kAtChunk], the smallest that still leaves about 600
 // items (four per SM) when the simulation is evaluated alone, so a single
 // simulation fills the GPU.  It depends only on the capacity and the panel
 // count, so the sum is grouped the same way alone and in any batch; a
@@ -80,7 +98,7 @@ struct __align__(16) NearRow {
 inline uint32_t rhs_chunk_for(uint32_t cap, int np) {
     const uint64_t tiles = ((uint64_t)np + 511) / 512;
     const uint64_t want = ((uint64_t)cap * tiles + 599) / 600;
-    uint32_t c = 512;
+    uint32_t c = 64;
     while (c < (uint32_t)kAtChunk && c < want) c <<= 1;
     return c;
 }
@@ -160,6 +178,8 @@ struct ListEntry {
     uint64_t roff;     // at-target partials offset (double2): sum rhs_chunks * npad
     uint64_t cofs;     // circulation partials offset (double): sum rhs_chunks
     uint64_t noff;     // first node of the far-field tree: sum 2 cap / kLeaf + kNodeSlack
+    uint64_t pnoff;    // first node of the panels' tree: sum 2 panel_leaves(np) + kNodeSlack
+    uint64_t panoff;   // first panel record: sum np
 };
 
 // Per-tile bounds of a 256-blob tile of the spatially sorted sources.
@@ -185,6 +205,12 @@ struct Workspace {
     double2* loc = nullptr;        // kTerms local coefficients per node that is a target group
     unsigned* arrived = nullptr;   // children done, per node
     NearRow* near = nullptr;       // per leaf
+    // FP32 sheet velocity: the panels' tree and records
+    TreeNode* pnodes = nullptr;
+    double2* pmom = nullptr;
+    unsigned* parrived = nullptr;
+    uint64_t pnodes_used = 0;      // of the present list
+    PanelRec* pan = nullptr;
     uint64_t nodes_cap = 0;
     double2* rhs_part = nullptr;   // at-target partials
     double* circ_part = nullptr;
@@ -233,7 +259,8 @@ void biot_savart_finish(const InstDesc* table, InstState* st, const ListEntry* l
 // The sort domain of descriptor d (device) from the box of n device points.
 void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const Workspace& ws,
                 int sms, cudaStream_t s);
-// Blob-on-collocation right-hand side b (src/VortexSheet.cpp:171-210).
+// Blob-on-collocation right-hand side b (src/VortexSheet.cpp:171-210).  FP32: from
+// the tree that biot_savart_prepare has built of the same positions.
 void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s);
 // Velocity at arbitrary targets from one blob set (src/VelocityKernel.cpp:69-109).
@@ -279,10 +306,16 @@ void sheet_at(const InstDesc& d, const double* px, const double* pz, uint32_t n,
 void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                  int max_np, cudaStream_t s);
 // Sheet-on-blob velocity (src/VortexSheet.cpp:217-273), optionally fused with
-// the convection update of the Euler / RK3 stage (src/DVMBase.cpp:167-209).
+// the convection update of the Euler / RK3 stage (src/DVMBase.cpp:167-209), for
+// sims of one precision.  FP32: over the tree that biot_savart_prepare has built
+// of the same positions.
 //   mode 0: uvs/wvs only; 1: Euler update; 2+k: RK3 stage k (k = 0,1,2)
 void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
-                    int mode, int max_np, const Workspace& ws, int sms, cudaStream_t s);
+                    int mode, int max_np, int precision, const Workspace& ws, int sms,
+                    cudaStream_t s);
+// The FP32 panels' tree and records from gamma (k_biot_savart.cu).
+void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
+                int max_np, const Workspace& ws, int sms, cudaStream_t s);
 // x += (u + uvs + Ux) dt without recomputing uvs (used by the phase API).
 void convect_update(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, const Workspace& ws, int sms, cudaStream_t s);

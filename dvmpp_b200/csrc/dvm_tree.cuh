@@ -194,6 +194,24 @@ __device__ __forceinline__ int walk_begin(TreeWalk& W, const TreeNode* __restric
     return top;
 }
 
+// Starts a walk for one group alone, given its box: the nodes first, first + step, ...
+// of the lowest level with at most `most` nodes.
+__device__ __forceinline__ int walk_begin(TreeWalk& W, uint32_t nleaves, const TargetBox& t,
+                                          uint32_t most, uint32_t first, uint32_t step, int lane) {
+    int l0 = 0;
+    while (level_count(nleaves, l0) > most) ++l0;
+    const uint32_t top = level_count(nleaves, l0);
+    const uint32_t have = first < top ? (top - first + step - 1) / step : 0u;
+    __syncwarp();
+    for (uint32_t i = lane; i < have; i += 32) {
+        W.stack[i] = ((uint32_t)l0 << 27) | (first + i * step);
+        W.place[i] = 0;
+    }
+    if (lane == 0) W.chain[0] = t;
+    __syncwarp();
+    return (int)have;
+}
+
 // What the walk's own group (chain[0]) makes of the lane's node: translate (far),
 // sum its pairs (near, a leaf), evaluate its moments at every target (mid); none:
 // another group's, or no node.

@@ -317,17 +317,31 @@ __device__ __forceinline__ void parent_node(const TreeNode& a, const TreeNode& b
     acc.y = ((sum[0].y + sum[1].y) + (sum[2].y + sum[3].y)) * fact;
 }
 
+// Gauss points and weights of four-point quadrature on [0, 1].  A leaf spans many
+// panels, so a panel's moments to order kTerms are as good as exact.
+__device__ __constant__ const double kGaussT[kPanelPoints] = {
+    0.06943184420297371, 0.33000947820757187, 0.66999052179242813, 0.93056815579702629};
+__device__ __constant__ const double kGaussW[kPanelPoints] = {
+    0.17392742256872693, 0.32607257743127307, 0.32607257743127307, 0.17392742256872693};
+
+// PANELS: the same over the sheet's Gauss points (panel order; circulation -gamma ds
+// dt each, which gives the sheet's velocity the blobs' convention), and the
+// panels' records for the near sums.
 constexpr int kTreeWarps = 8;
+template <bool PANELS>
 __global__ void __launch_bounds__(32 * kTreeWarps, 2)
     k_tree(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
            const ListEntry* __restrict__ list, int nlist, const uint32_t* __restrict__ perm,
            double2* __restrict__ pxz, float4* __restrict__ pf, TreeNode* __restrict__ nodes,
-           double2* __restrict__ mom, unsigned* __restrict__ arrived) {
+           double2* __restrict__ mom, unsigned* __restrict__ arrived,
+           PanelRec* __restrict__ pan) {
     __shared__ unsigned s_pre[kMaxList + 1];
     __shared__ TreeShared S;
     __shared__ unsigned s_last;
     list_prefix(s_pre, nlist, [&](int k) {
-        return (st[list[k].inst].n + kLeaf * kFan - 1) / (kLeaf * kFan);
+        const uint32_t n = PANELS ? (uint32_t)(kPanelPoints * table[list[k].inst].np)
+                                  : st[list[k].inst].n;
+        return (n + kLeaf * kFan - 1) / (kLeaf * kFan);
     });
     const unsigned total = s_pre[nlist], all = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -338,16 +352,40 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
         const InstDesc& d = table[e.inst];
-        const uint32_t n = st[e.inst].n, C = e.cap / kLeaf;
+        const uint32_t n = PANELS ? (uint32_t)(kPanelPoints * d.np) : st[e.inst].n;
+        const uint32_t C = PANELS ? panel_leaves(d.np) : e.cap / kLeaf;
         const uint32_t nl = (n + kLeaf - 1) / kLeaf;
-        TreeNode* __restrict__ N = nodes + e.noff;
-        double2* __restrict__ A = mom + e.noff * kTerms;
+        const uint64_t noff = PANELS ? e.pnoff : e.noff;
+        TreeNode* __restrict__ N = nodes + noff;
+        double2* __restrict__ A = mom + noff * kTerms;
         uint32_t g = item - s_pre[k];  // the block's share: nodes kFan g .. of its lowest level
+        if (PANELS) {
+            auto dup = [](double v) {
+                const float f = (float)v;
+                return f2pack(f, f);
+            };
+            const uint32_t p = g * (kFan * kPanelLeaf) + threadIdx.x;
+            static_assert(kFan * kPanelLeaf == 32 * kTreeWarps, "a record per thread");
+            if (p < (uint32_t)d.np) {
+                const double dsp = d.ds[p], g0 = d.gamma[p];
+                const double g1 = d.gamma[p + 1 == (uint32_t)d.np ? 0 : p + 1];
+                PanelRec r;
+                r.cs = make_ulonglong2(dup(d.cth[p]), dup(d.sth[p]));
+                r.dd = make_ulonglong2(dup(dsp), dup(1.0 / dsp));
+                r.cc = make_ulonglong2(dup(d.c2th[p]), dup(d.s2th[p]));
+                r.gd = make_ulonglong2(dup(g0), dup(g1 - g0));
+                r.xc = d.xc[p];
+                r.zc = d.zc[p];
+                r.ex = d.xc[p] + dsp * d.cth[p];
+                r.ez = d.zc[p] + dsp * d.sth[p];
+                pan[e.panoff + p] = r;
+            }
+        }
         uint32_t next[2];  // the next leaf's blobs, ahead of its gather
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t i = (g * kFan + wid) * kLeaf + h * 32 + lane;
-            next[h] = i < n ? perm[e.coff + i] : 0u;
+            next[h] = !PANELS && i < n ? perm[e.coff + i] : 0u;
         }
         for (int w = wid; w < kFan && g * kFan + w < nl; w += kTreeWarps) {
             const uint32_t idx = g * kFan + w;
@@ -355,7 +393,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t i = (idx + kTreeWarps) * kLeaf + h * 32 + lane;
-                next[h] = i < n ? perm[e.coff + i] : 0u;
+                next[h] = !PANELS && i < n ? perm[e.coff + i] : 0u;
             }
             double px[2], pz[2], gc[2];
             double x0 = DBL_MAX, x1 = -DBL_MAX, z0 = DBL_MAX, z1 = -DBL_MAX, thr = 0.0;
@@ -364,19 +402,29 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                 const uint32_t i = idx * kLeaf + h * 32 + lane;
                 px[h] = pz[h] = gc[h] = 0.0;
                 if (i < n) {
-                    const uint32_t p = here[h];
-                    const double sg = d.sigma[p], s2 = sg * sg;
-                    px[h] = d.x[p];
-                    pz[h] = d.z[p];
-                    gc[h] = d.circ[p];
-                    pxz[e.coff + i] = make_double2(px[h], pz[h]);
-                    pf[e.coff + i] =
-                        make_float4((float)gc[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
+                    if (PANELS) {
+                        const uint32_t p = i / kPanelPoints;
+                        const double t = kGaussT[i % kPanelPoints], w = kGaussW[i % kPanelPoints];
+                        const double dsp = d.ds[p], g0 = d.gamma[p];
+                        const double g1 = d.gamma[p + 1 == (uint32_t)d.np ? 0 : p + 1];
+                        px[h] = fma(dsp * t, d.cth[p], d.xc[p]);
+                        pz[h] = fma(dsp * t, d.sth[p], d.zc[p]);
+                        gc[h] = -(w * dsp) * fma(g1 - g0, t, g0);
+                    } else {
+                        const uint32_t p = here[h];
+                        const double sg = d.sigma[p], s2 = sg * sg;
+                        px[h] = d.x[p];
+                        pz[h] = d.z[p];
+                        gc[h] = d.circ[p];
+                        pxz[e.coff + i] = make_double2(px[h], pz[h]);
+                        pf[e.coff + i] =
+                            make_float4((float)gc[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
+                        thr = fmax(thr, 10.0 * s2);
+                    }
                     x0 = fmin(x0, px[h]);
                     x1 = fmax(x1, px[h]);
                     z0 = fmin(z0, pz[h]);
                     z1 = fmax(z1, pz[h]);
-                    thr = fmax(thr, 10.0 * s2);
                 }
             }
 #pragma unroll
@@ -445,7 +493,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
             __syncthreads();
             if (threadIdx.x == 0) {
                 const uint32_t up = g / kFan, want = min((uint32_t)kFan, tops - up * kFan);
-                s_last = atomicAdd(&arrived[e.noff + node_level(C, l + kFanLevels) + up], 1u) + 1 == want;
+                s_last = atomicAdd(&arrived[noff + node_level(C, l + kFanLevels) + up], 1u) + 1 == want;
             }
             __syncthreads();
             if (!s_last) break;
@@ -1386,6 +1434,189 @@ __global__ void __launch_bounds__(256) k_rhs_combine(const InstDesc* __restrict_
     }
 }
 
+// The same right-hand side for FP32 simulations, over the tree of the blobs: one
+// block per group of 32 collocation points, lane t of every warp at point t.
+// The tree's top nodes are dealt out to the warps, and each walks its own: far
+// nodes are translated, near leaves summed pair by pair as in k_at (offsets in
+// two parts, one compensated sum per half), their sums added in FP64; the
+// warps' results are added in order.  The circulations' sum is the root's first
+// moment.  Depends only on the simulation, never on the batch.
+//
+// Measured (B200, 250 k blobs, 1024 panels): 46 us for 240 us of all pairs
+// (and 12 us to combine their chunks); 2^17 blobs 38 for 122.
+constexpr int kRhsWarps = 8;
+constexpr int kRhsGroup = 32;
+struct RhsWarp {
+    TreeWalk walk;
+    TransBuf buf;
+    uint32_t far[kFarList];
+    float4 pos_hi[kLeaf / 2], pos_lo[kLeaf / 2];  // (x a, x b, z a, z b) of sources 2i, 2i + 1
+    float4 cst[kLeaf / 2];                        // (circ a, circ b, 10 sigma^2 a, b)
+    float2 rs[kLeaf / 2];
+    double2 sum[kRhsGroup];
+};
+struct RhsShared {
+    RhsWarp w[kRhsWarps];
+    double2 at[kRhsGroup];
+};
+__global__ void __launch_bounds__(32 * kRhsWarps, 2)
+    k_rhs_tree(const InstDesc* __restrict__ table, InstState* __restrict__ st,
+               const ListEntry* __restrict__ list, const double2* __restrict__ pxz,
+               const float4* __restrict__ pf, const TreeNode* __restrict__ nodes,
+               const double2* __restrict__ mom) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    RhsShared& S = *reinterpret_cast<RhsShared*>(s_raw);
+    const ListEntry e = list[blockIdx.y];
+    const InstDesc& d = table[e.inst];
+    const int i0 = (int)blockIdx.x * kRhsGroup;
+    if (i0 >= d.np) return;  // block-uniform
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned all = 0xffffffffu;
+    RhsWarp& W = S.w[wid];
+    const uint32_t n = st[e.inst].n, C = e.cap / kLeaf, nl = (n + kLeaf - 1) / kLeaf;
+    const TreeNode* __restrict__ N = nodes + e.noff;
+    const double2* __restrict__ A = mom + e.noff * kTerms;
+    const double2* __restrict__ X = pxz + e.coff;
+    const float4* __restrict__ F = pf + e.coff;
+    const int i = min(i0 + lane, d.np - 1);
+    const double tx = d.xc[i], tz = d.zc[i];
+    if (wid == 0) S.at[lane] = make_double2(tx, tz);
+    double x0 = tx, x1 = tx, z0 = tz, z1 = tz;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x0 = fmin(x0, __shfl_xor_sync(all, x0, o));
+        x1 = fmax(x1, __shfl_xor_sync(all, x1, o));
+        z0 = fmin(z0, __shfl_xor_sync(all, z0, o));
+        z1 = fmax(z1, __shfl_xor_sync(all, z1, o));
+    }
+    TargetBox tb;
+    tb.cx = 0.5 * (x0 + x1);
+    tb.cz = 0.5 * (z0 + z1);
+    tb.hx = 0.5 * (x1 - x0);
+    tb.hz = 0.5 * (z1 - z0);
+    tb.R = sqrt(tb.hx * tb.hx + tb.hz * tb.hz) * (1.0 + 1e-12);
+    tb.e = scale_exp(tb.R);
+    tb.n = kRhsGroup;
+    tb.at = S.at;
+    const double ox = __shfl_sync(all, tx, 0), oz = __shfl_sync(all, tz, 0);  // the group's origin
+    float txh, txl, tzh, tzl;
+    split_16(tx - ox, txh, txl);
+    split_16(tz - oz, tzh, tzl);
+    const uint64_t TXH = f2pack(txh, txh), TXL = f2pack(txl, txl);
+    const uint64_t TZH = f2pack(tzh, tzh), TZL = f2pack(tzl, tzl);
+    __syncthreads();
+    double row[kTerms];
+    binomial_row(row, lane);
+    Cplx b{0.0, 0.0};            // lane l: local coefficient l, this warp's share
+    double nu = 0.0, sw = 0.0;   // -u and w at the lane's point, near and mid
+    int sp = nl ? walk_begin(W.walk, nl, tb, kWalkTop, (uint32_t)wid, kRhsWarps, lane) : 0;
+    int nfar = 0;
+    while (sp > 0) {
+        uint32_t id;
+        const int kind = walk_step(W.walk, N, C, nl, sp, id, lane);
+        int cnt;
+        const int at = warp_place(kind == kWalkFar, lane, cnt);
+        if (kind == kWalkFar) W.far[nfar + at] = id;
+        nfar += cnt;
+        __syncwarp();
+        while (nfar >= kBatch || (sp == 0 && nfar > 0)) {
+            const int m = min(kBatch, nfar);
+            nfar -= m;
+            translate(N, A, C, W.far + nfar, m, tb, row, W.buf, lane, b);
+        }
+        for (unsigned todo = __ballot_sync(all, kind == kWalkMid); todo; todo &= todo - 1) {
+            const uint32_t q = __shfl_sync(all, id, __ffs(todo) - 1);
+            const uint64_t at = node_level(C, (int)(q >> 27)) + (q & ((1u << 27) - 1));
+            __syncwarp();
+            if (lane < kTerms) W.buf.c[0][lane] = Cplx{A[at * kTerms + lane].x, A[at * kTerms + lane].y};
+            __syncwarp();
+            const Cplx f = moment_value(W.buf.c[0], exp2_int(N[at].e), tx - N[at].cx, tz - N[at].cz);
+            nu -= f.y;
+            sw += f.x;
+        }
+        for (unsigned todo = __ballot_sync(all, kind == kWalkNear); todo; todo &= todo - 1) {
+            const uint32_t j0 = __shfl_sync(all, id, __ffs(todo) - 1) * kLeaf;
+            // (padding: far away, no circulation)
+            float xh[2] = {1e18f, 1e18f}, xl[2] = {0.f, 0.f}, zh[2] = {0.f, 0.f}, zl[2] = {0.f, 0.f};
+            float g[2] = {0.f, 0.f}, thr[2] = {0.f, 0.f}, rs[2] = {0.f, 0.f};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t j = j0 + 2 * lane + h;
+                if (j < n) {
+                    const double2 p = X[j];
+                    const float4 f = F[j];
+                    split_16(p.x - ox, xh[h], xl[h]);
+                    split_16(p.y - oz, zh[h], zl[h]);
+                    g[h] = f.x;
+                    thr[h] = f.y;
+                    rs[h] = f.z;
+                }
+            }
+            __syncwarp();
+            W.pos_hi[lane] = make_float4(xh[0], xh[1], zh[0], zh[1]);
+            W.pos_lo[lane] = make_float4(xl[0], xl[1], zl[0], zl[1]);
+            W.cst[lane] = make_float4(g[0], g[1], thr[0], thr[1]);
+            W.rs[lane] = make_float2(rs[0], rs[1]);
+            __syncwarp();
+            const uint64_t zero2 = f2pack(0.0f, 0.0f);
+            uint64_t snu = zero2, enu = zero2, s2 = zero2, e2 = zero2;
+#pragma unroll 4
+            for (int q = 0; q < kLeaf / 2; ++q) {
+                const float4 H = W.pos_hi[q], L = W.pos_lo[q], Cs = W.cst[q];
+                const uint64_t DX = f2add(f2sub(TXH, f2pack(H.x, H.y)), f2sub(TXL, f2pack(L.x, L.y)));
+                const uint64_t DZ = f2add(f2sub(TZH, f2pack(H.z, H.w)), f2sub(TZL, f2pack(L.z, L.w)));
+                const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
+                const float ra = f2lo(R2), rb = f2hi(R2);
+                float ka = rcp_approx(ra), kb = rcp_approx(rb);
+                const bool ca = ra < Cs.z, cb = rb < Cs.w;
+                if (__any_sync(all, ca || cb)) {
+                    const float2 R = W.rs[q];
+                    const float qa = core_kernel_expm1(ra, R.x, ka);
+                    const float qb = core_kernel_expm1(rb, R.y, kb);
+                    ka = ca ? qa : ka;
+                    kb = cb ? qb : kb;
+                }
+                const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
+                kahan2_fma(snu, enu, G, DZ);
+                kahan2_fma(s2, e2, G, DX);
+            }
+            nu += ((double)f2lo(snu) + (double)f2lo(enu)) + ((double)f2hi(snu) + (double)f2hi(enu));
+            sw += ((double)f2lo(s2) + (double)f2lo(e2)) + ((double)f2hi(s2) + (double)f2hi(e2));
+        }
+    }
+    __syncwarp();
+    W.sum[lane] = make_double2(nu, sw);
+    if (lane < kTerms) W.buf.c[0][lane] = b;
+    __syncthreads();
+    if (wid != 0) return;
+    if (lane < kTerms) {
+        for (int q = 1; q < kRhsWarps; ++q) {
+            b.x += S.w[q].buf.c[0][lane].x;
+            b.y += S.w[q].buf.c[0][lane].y;
+        }
+        W.buf.c[0][lane] = b;
+    }
+    __syncwarp();
+    const Cplx f = local_value(W.buf.c[0], tx - tb.cx, tz - tb.cz, tb.e);
+    nu -= f.y;
+    sw += f.x;
+    for (int q = 1; q < kRhsWarps; ++q) {
+        nu += S.w[q].sum[lane].x;
+        sw += S.w[q].sum[lane].y;
+    }
+    if (i0 + lane < d.np) {
+        const double ui = dmul(-nu, kRpi2), wi = dmul(sw, kRpi2);
+        d.b[i] = dadd(dmul(dadd(d.ux, ui), d.enx[i]), dmul(dadd(d.uz, wi), d.enz[i]));
+    }
+    if (i0 == 0 && lane == 0) {
+        int l = 0;
+        while (level_count(nl, l) > 1u) ++l;
+        const double a = nl ? A[node_level(C, l) * kTerms].x : 0.0;
+        d.b[d.np] = -a;
+        st[e.inst].totalcirc = a;
+    }
+}
+
 __global__ void k_build_rhs_jobs(const InstDesc* __restrict__ table, InstState* __restrict__ st,
                                  const ListEntry* __restrict__ list, int nlist,
                                  double2* rhs_part, double* circ_part, AtJob* jobs) {
@@ -1440,10 +1671,10 @@ void biot_savart_prepare(const InstDesc* table, InstState* st, const ListEntry* 
     }
     if (precision == kF32) {
         cudaMemsetAsync(ws.arrived, 0, sizeof(unsigned) * (2 * ws.total_cap / kLeaf + (uint64_t)kNodeSlack * nlist), s);
-        k_tree<<<sms * 2, 32 * kTreeWarps, 0, s>>>(table, st, list, nlist, ws.perm,
-                                       reinterpret_cast<double2*>(ws.packed),
-                                       reinterpret_cast<float4*>(ws.packed + ws.packed_cap / 2),
-                                       ws.nodes, ws.mom, ws.arrived);
+        k_tree<false><<<sms * 2, 32 * kTreeWarps, 0, s>>>(
+            table, st, list, nlist, ws.perm, reinterpret_cast<double2*>(ws.packed),
+            reinterpret_cast<float4*>(ws.packed + ws.packed_cap / 2), ws.nodes, ws.mom, ws.arrived,
+            nullptr);
     } else {
         k_pack<<<sms * 8, kBsST, 0, s>>>(table, st, list, nlist, ws.perm, ws.packed, ws.meta);
     }
@@ -1495,12 +1726,20 @@ void biot_savart_self(const InstDesc* table, InstState* st, const ListEntry* lis
 
 void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s) {
+    if (precision == kF32) {
+        cudaFuncSetAttribute(k_rhs_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(RhsShared));
+        k_rhs_tree<<<dim3((max_np + kRhsGroup - 1) / kRhsGroup, nlist), 32 * kRhsWarps,
+                     sizeof(RhsShared), s>>>(
+            table, st, list, reinterpret_cast<const double2*>(ws.packed),
+            reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.nodes, ws.mom);
+        return;
+    }
     static_assert(sizeof(AtJob) <= 256, "job record size");
     AtJob* jobs = reinterpret_cast<AtJob*>(ws.jobs);
     k_build_rhs_jobs<<<(nlist + 127) / 128, 128, 0, s>>>(table, st, list, nlist, ws.rhs_part,
                                                          ws.circ_part, jobs);
-    if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(jobs, nlist);
-    else k_at<false><<<sms * 4, 256, 0, s>>>(jobs, nlist);
+    k_at<false><<<sms * 4, 256, 0, s>>>(jobs, nlist);
     k_rhs_combine<<<dim3((max_np + 31) / 32, nlist), 256, 0, s>>>(table, st, list, jobs);
 }
 
@@ -1518,6 +1757,14 @@ static unsigned combine_threads(uint64_t nchunk) {
     unsigned w = 1;
     while (w < 32 && 4ull * w < nchunk) w *= 2;
     return 32 * w;
+}
+
+void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
+                int max_np, const Workspace& ws, int sms, cudaStream_t s) {
+    const int shares = ((int)panel_leaves(max_np) + kFan - 1) / kFan;
+    cudaMemsetAsync(ws.parrived, 0, sizeof(unsigned) * ws.pnodes_used, s);
+    k_tree<true><<<std::min(sms * 2, nlist * shares), 32 * kTreeWarps, 0, s>>>(
+        table, st, list, nlist, nullptr, nullptr, nullptr, ws.pnodes, ws.pmom, ws.parrived, ws.pan);
 }
 
 size_t direct_at_part_elems(uint32_t ns, uint32_t nt) {

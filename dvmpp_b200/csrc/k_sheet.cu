@@ -5,9 +5,10 @@
 //
 // FP64 instances: pair formulas keep the reference's operation order with one
 // rounding per operation (dadd/dmul/...), so they round like the reference
-// compiled without FP contraction.  FP32 instances evaluate the sheet-on-blob
-// panel terms in single precision (accumulated in FP64); the influence matrix,
-// QR, solve, refinement and loads are FP64 for both.
+// compiled without FP contraction.  FP32 instances evaluate the near sheet-on-blob
+// panel terms in single precision (accumulated in FP64) and the far ones by FP64
+// expansions; the influence matrix, QR, solve, refinement and loads are FP64 for
+// both.
 //
 // The solve: the reference forms A^T A and A^T b and solves with LAPACK every
 // call.  Here A ((np+1) x np) is factorised ONCE per body by Householder QR on
@@ -23,6 +24,7 @@
 
 #include "dvm_device.cuh"
 #include "dvm_internal.h"
+#include "dvm_tree.cuh"
 
 namespace dvmk {
 namespace {
@@ -513,16 +515,6 @@ __device__ __forceinline__ uint64_t f2atan_quarter(uint64_t t) {
     return f2mul(t, p);
 }
 
-// FP32 panel constants, each duplicated into both halves of a packed pair so
-// that one 16-byte shared load brings two of them for both blobs of a thread:
-// .x and .y of each field are (v, v) pairs.
-struct PanelX2 {
-    ulonglong2 cs;  // (cos th, cos th), (sin th, sin th)
-    ulonglong2 dd;  // (ds, ds), (1/ds, 1/ds)
-    ulonglong2 cc;  // (cos -2th, ...), (sin -2th, ...)
-    ulonglong2 gd;  // (gamma_j, ...), (gamma_{j+1} - gamma_j, ...)
-};
-
 // The near-regime values of one blob (see above): c6 by log_pos from the
 // FP64-formed end offsets when |x| > 1/4, c7 by atan2_any when the angle is
 // wide; other values are left as the far evaluations gave them.
@@ -541,12 +533,8 @@ __device__ __forceinline__ void near_values(double xi, double zi, double ex, dou
 // high half of every packed value) over the np panels staged in shared
 // memory.  Every lane of the warp must call it: the regime is voted.
 __device__ __forceinline__ void sheet_sum_f32x2(double xa, double za, double xb, double zb,
-                                                int np, const double* __restrict__ sxc,
-                                                const double* __restrict__ szc,
-                                                const double* __restrict__ sex,
-                                                const double* __restrict__ sez,
-                                                const PanelX2* __restrict__ pan, double& ua,
-                                                double& wa, double& ub, double& wb) {
+                                                int np, const PanelRec* __restrict__ pan,
+                                                double& ua, double& wa, double& ub, double& wb) {
     const uint64_t two = f2pack(2.0f, 2.0f), half = f2pack(0.5f, 0.5f);
     // Panel terms are summed in FP32 over blocks of eight panels, each block
     // then added in FP64 (a quarter of the conversions and FP64 adds; the
@@ -557,10 +545,10 @@ __device__ __forceinline__ void sheet_sum_f32x2(double xa, double za, double xb,
         const int jn = min(np, j0 + 8);
 #pragma unroll 2
         for (int j = j0; j < jn; ++j) {
-            const PanelX2 P = pan[j];
+            const PanelRec& P = pan[j];
             const uint64_t CT = P.cs.x, ST = P.cs.y, DS = P.dd.x, IDS = P.dd.y;
             const uint64_t C2T = P.cc.x, S2T = P.cc.y, G0 = P.gd.x, DG = P.gd.y;
-            const double xc = sxc[j], zc = szc[j];
+            const double xc = P.xc, zc = P.zc;
             const uint64_t DX = f2pack((float)(xa - xc), (float)(xb - xc));
             const uint64_t DZ = f2pack((float)(za - zc), (float)(zb - zc));
             const uint64_t C1 = f2sub(f2pack(0.0f, 0.0f), f2fma(DX, CT, f2mul(DZ, ST)));
@@ -580,7 +568,7 @@ __device__ __forceinline__ void sheet_sum_f32x2(double xa, double za, double xb,
             uint64_t C7 = f2atan_quarter(T);
             if (__any_sync(0xffffffffu, nla || nlb || wa_ || wb_)) {
                 float c6a = f2lo(C6), c6b = f2hi(C6), c7a = f2lo(C7), c7b = f2hi(C7);
-                const double ex = sex[j], ez = sez[j];
+                const double ex = P.ex, ez = P.ez;
                 near_values(xa, za, ex, ez, xxa, r2a, f2lo(Y), Xa, nla, wa_, c6a, c7a);
                 near_values(xb, zb, ex, ez, xxb, r2b, f2hi(Y), Xb, nlb, wb_, c6b, c7b);
                 C6 = f2pack(c6a, c6b);
@@ -608,12 +596,11 @@ __device__ __forceinline__ void sheet_sum_f32x2(double xa, double za, double xb,
     }
 }
 
-// One panel term of src/VortexSheet.cpp:235-249, 261-268 in FP64 with the
-// reference's operation order (one rounding per operation); dx, dz are the
-// point's offsets from the panel's collocation point.
-__device__ __forceinline__ void sheet_pair_f64(double dx, double dz, double dsj, double ct,
-                                               double stt, double c2t, double s2t, double g0,
-                                               double g1, double& us, double& ws) {
+// One panel term of src/VortexSheet.cpp:235-249, 261-268 in FP64; dx, dz are the
+// point's offsets from the panel's collocation point, ids = 1 / ds.
+__device__ __forceinline__ void sheet_pair_f64(double dx, double dz, double dsj, double ids,
+                                               double ct, double stt, double c2t, double s2t,
+                                               double g0, double g1, double& us, double& ws) {
     const double c1 = dsub(dmul(-dx, ct), dmul(dz, stt));
     const double c2 = dadd(dmul(dx, dx), dmul(dz, dz));
     const double c5 = dsub(dmul(dx, stt), dmul(dz, ct));
@@ -621,11 +608,11 @@ __device__ __forceinline__ void sheet_pair_f64(double dx, double dz, double dsj,
     const double c7 = atan2(dmul(c5, dsj), dadd(c2, dmul(c1, dsj)));
     const double c8 = dadd(dmul(dx, s2t), dmul(dz, c2t));
     const double c9 = dsub(dmul(dx, c2t), dmul(dz, s2t));
-    const double qx = dadd(dadd(-stt, ddiv(dmul(dmul(0.5, c8), c6), dsj)),
-                           ddiv(dmul(dadd(dmul(c1, ct), dmul(c5, stt)), c7), dsj));
+    const double qx = dadd(dadd(-stt, dmul(dmul(dmul(0.5, c8), c6), ids)),
+                           dmul(dmul(dadd(dmul(c1, ct), dmul(c5, stt)), c7), ids));
     const double px = dsub(dsub(dmul(dmul(-0.5, c6), stt), dmul(c7, ct)), qx);
-    const double qy = dadd(dadd(ct, ddiv(dmul(dmul(0.5, c9), c6), dsj)),
-                           ddiv(dmul(dsub(dmul(c1, stt), dmul(c5, ct)), c7), dsj));
+    const double qy = dadd(dadd(ct, dmul(dmul(dmul(0.5, c9), c6), ids)),
+                           dmul(dmul(dsub(dmul(c1, stt), dmul(c5, ct)), c7), ids));
     const double py = dsub(dsub(dmul(dmul(0.5, c6), ct), dmul(c7, stt)), qy);
     us = dadd(us, dadd(dmul(px, g0), dmul(qx, g1)));
     ws = dadd(ws, dadd(dmul(py, g0), dmul(qy, g1)));
@@ -650,8 +637,8 @@ __global__ void __launch_bounds__(128) k_sheet_at(const double* __restrict__ xc,
     const double xi = px[i], zi = pz[i];
     double us = 0.0, ws = 0.0;
     for (int j = 0; j < np; ++j)
-        sheet_pair_f64(dsub(xi, xc[j]), dsub(zi, zc[j]), ds[j], cth[j], sth[j], c2th[j], s2th[j],
-                       gamma[j], gamma[j == np - 1 ? 0 : j + 1], us, ws);
+        sheet_pair_f64(dsub(xi, xc[j]), dsub(zi, zc[j]), ds[j], ddiv(1.0, ds[j]), cth[j], sth[j],
+                       c2th[j], s2th[j], gamma[j], gamma[j == np - 1 ? 0 : j + 1], us, ws);
     uvs[i] = dmul(us, kRpi2);
     wvs[i] = dmul(ws, kRpi2);
 }
@@ -686,8 +673,13 @@ __device__ __forceinline__ void sheet_store(const InstDesc& d, uint32_t i, doubl
     }
 }
 
-constexpr uint32_t kSheetItem = 512;  // blobs per work item: two per thread
-constexpr size_t kSheetSmemPerPanel = 96;  // FP32: 4 FP64 + one PanelX2; FP64: 8 FP64 arrays
+// FP64 simulations: every panel term.  A work item is 64 blobs, four threads per
+// blob with a quarter of the panels each (their sums added in order): with two
+// blobs per thread and all panels in turn, a simulation of 2000 blobs was four
+// blocks' work (222 us a call at 128 panels; 49 now).
+constexpr uint32_t kSheetItem = 64;
+constexpr int kSheetParts = 4;
+constexpr size_t kSheetSmemPerPanel = 72;  // nine FP64 arrays
 
 __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restrict__ table,
                                                         const InstState* __restrict__ st,
@@ -696,19 +688,13 @@ __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restri
                                                         unsigned* __restrict__ work) {
     extern __shared__ double s_pan[];  // kSheetSmemPerPanel bytes per panel of max_np
     __shared__ unsigned s_pre[1025];
+    __shared__ double2 s_sum[kSheetParts][kSheetItem];
     __shared__ unsigned s_item;
-    __shared__ int s_loaded;
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += (st[list[k].inst].n + kSheetItem - 1) / kSheetItem;
-        }
-        s_pre[nlist] = acc;
-        s_loaded = -1;
-    }
-    __syncthreads();
+    list_prefix(s_pre, nlist,
+                [&](int k) { return (st[list[k].inst].n + kSheetItem - 1) / kSheetItem; });
     const unsigned total = s_pre[nlist];
+    const uint32_t part = threadIdx.x / kSheetItem, at = threadIdx.x % kSheetItem;
+    int loaded = -1;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(work, 1u);
         __syncthreads();
@@ -718,78 +704,157 @@ __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restri
         const ListEntry e = list[k];
         const InstDesc& d = table[e.inst];
         const int np = d.np;
-        const bool f32 = d.precision == kF32;
         double* sxc = s_pan;
         double* szc = sxc + np;
-        // FP64 layout after xc, zc: ds, cos, sin, cos -2th, sin -2th, gamma
         double* sds = szc + np;
-        double* sct = sds + np;
+        double* sid = sds + np;
+        double* sct = sid + np;
         double* sst = sct + np;
         double* sc2 = sst + np;
         double* ss2 = sc2 + np;
         double* sg = ss2 + np;
-        // FP32 layout after xc, zc: the panel ends (FP64), then np PanelX2
-        double* sex = szc + np;
-        double* sez = sex + np;
-        PanelX2* pan = reinterpret_cast<PanelX2*>(sez + np);
-        if (s_loaded != k) {
+        if (loaded != k) {
             for (int j = threadIdx.x; j < np; j += blockDim.x) {
                 sxc[j] = d.xc[j];
                 szc[j] = d.zc[j];
-                if (f32) {
-                    const double dsj = d.ds[j];
-                    sex[j] = d.xc[j] + dsj * d.cth[j];
-                    sez[j] = d.zc[j] + dsj * d.sth[j];
-                    const double g0 = d.gamma[j], g1 = d.gamma[j == np - 1 ? 0 : j + 1];
-                    auto dup = [](double v) {
-                        const float f = (float)v;
-                        return f2pack(f, f);
-                    };
-                    PanelX2 P;
-                    P.cs = make_ulonglong2(dup(d.cth[j]), dup(d.sth[j]));
-                    P.dd = make_ulonglong2(dup(dsj), dup(1.0 / dsj));
-                    P.cc = make_ulonglong2(dup(d.c2th[j]), dup(d.s2th[j]));
-                    P.gd = make_ulonglong2(dup(g0), dup(g1 - g0));
-                    pan[j] = P;
-                } else {
-                    sds[j] = d.ds[j];
-                    sct[j] = d.cth[j];
-                    sst[j] = d.sth[j];
-                    sc2[j] = d.c2th[j];
-                    ss2[j] = d.s2th[j];
-                    sg[j] = d.gamma[j];
-                }
+                sds[j] = d.ds[j];
+                sid[j] = ddiv(1.0, d.ds[j]);
+                sct[j] = d.cth[j];
+                sst[j] = d.sth[j];
+                sc2[j] = d.c2th[j];
+                ss2[j] = d.s2th[j];
+                sg[j] = d.gamma[j];
             }
+            loaded = k;
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_loaded = k;
-        const uint32_t n = st[e.inst].n;
-        const uint32_t ia = (item - s_pre[k]) * kSheetItem + threadIdx.x, ib = ia + 256;
-        const bool acta = ia < n, actb = ib < n;
-        if (f32) {
-            // every lane runs the panel loop (its warp votes on the regime); a
-            // blob slot past the count evaluates a point far from the body
-            const double far_x = sxc[0] + 1.0e3, far_z = szc[0] + 1.0e3;
-            double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
-            sheet_sum_f32x2(acta ? d.x[ia] : far_x, acta ? d.z[ia] : far_z,
-                            actb ? d.x[ib] : far_x, actb ? d.z[ib] : far_z, np, sxc, szc, sex,
-                            sez, pan, ua, wa, ub, wb);
-            if (acta) sheet_store(d, ia, ua, wa, mode);
-            if (actb) sheet_store(d, ib, ub, wb, mode);
-        } else {
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t i = h ? ib : ia;
-                if (i >= n) continue;
-                const double xi = d.x[i], zi = d.z[i];
-                double us = 0.0, ws = 0.0;
-                for (int j = 0; j < np; ++j)
-                    sheet_pair_f64(dsub(xi, sxc[j]), dsub(zi, szc[j]), sds[j], sct[j], sst[j],
-                                   sc2[j], ss2[j], sg[j], (j == np - 1) ? sg[0] : sg[j + 1], us,
-                                   ws);
-                sheet_store(d, i, us, ws, mode);
+        const uint32_t n = st[e.inst].n, i = (item - s_pre[k]) * kSheetItem + at;
+        double us = 0.0, ws = 0.0;
+        if (i < n) {
+            const double xi = d.x[i], zi = d.z[i];
+            const int j0 = (int)part * np / kSheetParts, j1 = (int)(part + 1) * np / kSheetParts;
+            for (int j = j0; j < j1; ++j)
+                sheet_pair_f64(dsub(xi, sxc[j]), dsub(zi, szc[j]), sds[j], sid[j], sct[j], sst[j],
+                               sc2[j], ss2[j], sg[j], (j == np - 1) ? sg[0] : sg[j + 1], us, ws);
+        }
+        s_sum[part][at] = make_double2(us, ws);
+        __syncthreads();
+        if (part == 0 && i < n) {
+            for (int q = 1; q < kSheetParts; ++q) {
+                us = dadd(us, s_sum[q][at].x);
+                ws = dadd(ws, s_sum[q][at].y);
             }
+            sheet_store(d, i, us, ws, mode);
         }
         __syncthreads();
+    }
+}
+
+// FP32 simulations: one warp per leaf of 64 blobs (two per lane) walks the panels'
+// tree: nodes far enough are translated into a local expansion about the leaf
+// (or evaluated at every blob of a spread leaf), and only the near panels'
+// terms are evaluated, kPanelLeaf at a time.  All panels for all blobs took
+// 716 us for 250 k blobs and 1024 panels (FMA pipe and issue); 70 to 90 now, the
+// panels' tree included.
+constexpr int kSheetWarps = 4;
+struct SheetWarp {
+    TreeWalk walk;
+    TransBuf buf;
+    double2 at[kLeaf];
+    uint32_t far[kBatch + 32];
+    PanelRec pan[kPanelLeaf];
+};
+
+__global__ void __launch_bounds__(32 * kSheetWarps, 3)
+    k_sheet_f32(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
+                const ListEntry* __restrict__ list, int nlist, int mode,
+                const uint32_t* __restrict__ perm, const double2* __restrict__ pxz,
+                const TreeNode* __restrict__ nodes, const TreeNode* __restrict__ pnodes,
+                const double2* __restrict__ pmom, const PanelRec* __restrict__ pan,
+                unsigned* __restrict__ work) {
+    __shared__ unsigned s_pre[1025];
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
+    const unsigned total = s_pre[nlist], all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[threadIdx.x >> 5];
+    double row[kTerms];
+    binomial_row(row, lane);
+    for (;;) {
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(work, 1u);
+        item = __shfl_sync(all, item, 0);
+        if (item >= total) break;
+        const int k = locate(s_pre, nlist, item);
+        const ListEntry e = list[k];
+        const InstDesc& d = table[e.inst];
+        const uint32_t n = st[e.inst].n, leaf = item - s_pre[k], t0 = leaf * kLeaf;
+        const uint32_t C = panel_leaves(d.np), nl = C;
+        const TreeNode* __restrict__ N = pnodes + e.pnoff;
+        const double2* __restrict__ A = pmom + e.pnoff * kTerms;
+        __syncwarp();
+        for (int q = lane; q < kLeaf; q += 32) S.at[q] = pxz[e.coff + min(t0 + q, n - 1)];
+        __syncwarp();
+        TargetBox tb = target_box(nodes[e.noff + leaf]);
+        tb.n = (int)min((uint32_t)kLeaf, n - t0);
+        tb.at = S.at;
+        const double2 pa = S.at[lane], pb = S.at[lane + 32];
+        Cplx b{0.0, 0.0};
+        double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
+        int sp = walk_begin(S.walk, nl, tb, 1u, 0u, 1u, lane), nfar = 0;
+        bool any_far = false;
+        while (sp > 0) {
+            uint32_t id;
+            const int kind = walk_step(S.walk, N, C, nl, sp, id, lane);
+            int cnt;
+            const int at = warp_place(kind == kWalkFar, lane, cnt);
+            if (kind == kWalkFar) S.far[nfar + at] = id;
+            nfar += cnt;
+            any_far = any_far || cnt > 0;
+            __syncwarp();
+            while (nfar >= kBatch || (sp == 0 && nfar > 0)) {
+                const int m = min(kBatch, nfar);
+                nfar -= m;
+                translate(N, A, C, S.far + nfar, m, tb, row, S.buf, lane, b);
+            }
+            for (unsigned todo = __ballot_sync(all, kind == kWalkMid); todo; todo &= todo - 1) {
+                const uint32_t q = __shfl_sync(all, id, __ffs(todo) - 1);
+                const uint64_t to = node_level(C, (int)(q >> 27)) + (q & ((1u << 27) - 1));
+                __syncwarp();
+                if (lane < kTerms) S.buf.c[0][lane] = Cplx{A[to * kTerms + lane].x, A[to * kTerms + lane].y};
+                __syncwarp();
+                const double s = exp2_int(N[to].e);
+                const Cplx fa = moment_value(S.buf.c[0], s, pa.x - N[to].cx, pa.y - N[to].cz);
+                const Cplx fb = moment_value(S.buf.c[0], s, pb.x - N[to].cx, pb.y - N[to].cz);
+                ua += fa.y;
+                wa += fa.x;
+                ub += fb.y;
+                wb += fb.x;
+            }
+            for (unsigned todo = __ballot_sync(all, kind == kWalkNear); todo; todo &= todo - 1) {
+                const int j0 = (int)__shfl_sync(all, id, __ffs(todo) - 1) * kPanelLeaf;
+                const int m = min(kPanelLeaf, d.np - j0);
+                __syncwarp();
+                const double2* from = reinterpret_cast<const double2*>(pan + e.panoff + j0);
+                for (int q = lane; q < m * (int)(sizeof(PanelRec) / 16); q += 32)
+                    reinterpret_cast<double2*>(S.pan)[q] = from[q];
+                __syncwarp();
+                sheet_sum_f32x2(pa.x, pa.y, pb.x, pb.y, m, S.pan, ua, wa, ub, wb);
+            }
+        }
+        if (any_far) {  // warp-uniform
+            __syncwarp();
+            if (lane < kTerms) S.buf.c[0][lane] = b;
+            __syncwarp();
+            const Cplx fa = local_value(S.buf.c[0], pa.x - tb.cx, pa.y - tb.cz, tb.e);
+            const Cplx fb = local_value(S.buf.c[0], pb.x - tb.cx, pb.y - tb.cz, tb.e);
+            ua += fa.y;
+            wa += fa.x;
+            ub += fb.y;
+            wb += fb.x;
+        }
+        if (t0 + lane < n) sheet_store(d, perm[e.coff + t0 + lane], ua, wa, mode);
+        if (t0 + 32 + lane < n) sheet_store(d, perm[e.coff + t0 + 32 + lane], ub, wb, mode);
     }
 }
 
@@ -820,30 +885,69 @@ __global__ void k_convect_update(const InstDesc* __restrict__ table,
 }
 
 // ---- loads (src/VortexSheet.cpp:489-513), one block per simulation ---------------
-__global__ void k_loads(const InstDesc* __restrict__ table, InstState* __restrict__ st,
-                        const ListEntry* __restrict__ list) {
-    extern __shared__ double s_P[];
+// The pressure along the panels is a running sum; each thread takes consecutive
+// panels and the block scans (one thread going through the panels twice took 18 us
+// at 128 panels and 129 at 1024; 4 and 5 now).
+constexpr int kLoadThreads = 256;
+__device__ __forceinline__ double block_total(double v, double* s_red, bool max) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = max ? fmax(v, t) : dadd(v, t);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = s_red[0];
+    for (int q = 1; q < kLoadThreads / 32; ++q) v = max ? fmax(v, s_red[q]) : dadd(v, s_red[q]);
+    return v;
+}
+__global__ void __launch_bounds__(kLoadThreads) k_loads(const InstDesc* __restrict__ table,
+                                                        InstState* __restrict__ st,
+                                                        const ListEntry* __restrict__ list) {
+    extern __shared__ double s_P[];  // np + 1 running sums
+    __shared__ double s_red[kLoadThreads / 32];
     const ListEntry e = list[blockIdx.x];
     const InstDesc& d = table[e.inst];
-    const int np = d.np;
-    if (threadIdx.x != 0) return;
+    const int np = d.np, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const double c = ddiv(-d.rho, d.dt);
-    s_P[0] = 0.0;
-    for (int i = 0; i < np - 1; ++i) s_P[i + 1] = dadd(s_P[i], dmul(c, dmul(d.gamma[i], d.ds[i])));
-    for (int i = 0; i < np - 1; ++i) s_P[i] = dmul(0.5, dadd(s_P[i], s_P[i + 1]));
-    s_P[np - 1] = dmul(0.5, dadd(s_P[np - 1], s_P[0]));
-    double pmax = s_P[0];
-    for (int i = 1; i < np; ++i)
-        if (s_P[i] > pmax) pmax = s_P[i];
+    const int per = (np + kLoadThreads - 1) / kLoadThreads, j0 = min(np, tid * per),
+              j1 = min(np, j0 + per);
+    double mine = 0.0;
+    for (int j = j0; j < j1; ++j) mine = dadd(mine, dmul(c, dmul(d.gamma[j], d.ds[j])));
+    double before = mine;  // inclusive scan over the block, then exclusive
+    for (int o = 1; o < 32; o <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before = dadd(t, before);
+    }
+    if (lane == 31) s_red[wid] = before;
+    __syncthreads();
+    double run = 0.0;
+    for (int q = 0; q < wid; ++q) run = dadd(run, s_red[q]);
+    const double left = __shfl_up_sync(0xffffffffu, before, 1);
+    if (lane > 0) run = dadd(run, left);
+    for (int j = j0; j < j1; ++j) {
+        s_P[j] = run;
+        run = dadd(run, dmul(c, dmul(d.gamma[j], d.ds[j])));
+    }
+    __syncthreads();
+    // panel pressures: means of neighbours; the last with the first panel's mean
+    const double first = dmul(0.5, dadd(s_P[0], np > 1 ? s_P[1] : s_P[0]));
+    auto pressure = [&](int j) {
+        return j < np - 1 ? dmul(0.5, dadd(s_P[j], s_P[j + 1])) : dmul(0.5, dadd(s_P[j], first));
+    };
+    double pmax = -DBL_MAX;
+    for (int j = j0; j < j1; ++j) pmax = fmax(pmax, pressure(j));
+    pmax = block_total(pmax, s_red, true);
     const double pref = dmul(dmul(dmul(0.5, d.rho), d.Ur), d.Ur);
     const double shift = dmul(dsub(pref, pmax), 1.0);
     double sx = 0.0, sz = 0.0;
-    for (int i = 0; i < np; ++i) {
-        const double Pi = dadd(s_P[i], shift);
-        sx = dadd(sx, dmul(dmul(Pi, d.enx[i]), d.ds[i]));
-        sz = dadd(sz, dmul(dmul(Pi, d.enz[i]), d.ds[i]));
+    for (int j = j0; j < j1; ++j) {
+        const double Pj = dadd(pressure(j), shift);
+        sx = dadd(sx, dmul(dmul(Pj, d.enx[j]), d.ds[j]));
+        sz = dadd(sz, dmul(dmul(Pj, d.enz[j]), d.ds[j]));
     }
-    const double fx = -sx, fz = -sz;
+    const double fx = -block_total(sx, s_red, false), fz = -block_total(sz, s_red, false);
+    if (tid != 0) return;
     const double den = dmul(dmul(dmul(dmul(0.5, d.rho), d.area), d.Ur), d.Ur);
     InstState& s = st[e.inst];
     s.fx = fx;
@@ -1006,15 +1110,20 @@ void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, in
 }
 
 void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
-                    int mode, int max_np, const Workspace& ws, int sms, cudaStream_t s) {
-    const size_t smem = kSheetSmemPerPanel * (size_t)max_np;
-    static bool attr = false;  // set once, before any graph capture (first call is eager)
-    if (!attr) {
-        cudaFuncSetAttribute(k_sheet_velocity, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
-        attr = true;
-    }
+                    int mode, int max_np, int precision, const Workspace& ws, int sms,
+                    cudaStream_t s) {
     cudaMemsetAsync(ws.work + 1, 0, sizeof(unsigned), s);
+    if (precision == kF32) {
+        panel_tree(table, st, list, nlist, max_np, ws, sms, s);
+        constexpr size_t smem = sizeof(SheetWarp) * kSheetWarps;
+        cudaFuncSetAttribute(k_sheet_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_sheet_f32<<<sms * 3, 32 * kSheetWarps, smem, s>>>(
+            table, st, list, nlist, mode, ws.perm, reinterpret_cast<const double2*>(ws.packed),
+            ws.nodes, ws.pnodes, ws.pmom, ws.pan, ws.work + 1);
+        return;
+    }
+    const size_t smem = kSheetSmemPerPanel * (size_t)max_np;
+    cudaFuncSetAttribute(k_sheet_velocity, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     k_sheet_velocity<<<sms * 4, 256, smem, s>>>(table, st, list, nlist, mode, ws.work + 1);
 }
 
@@ -1034,7 +1143,7 @@ void convect_update(const InstDesc* table, InstState* st, const ListEntry* list,
 
 void loads(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, int max_np,
            cudaStream_t s) {
-    k_loads<<<nlist, 32, sizeof(double) * max_np, s>>>(table, st, list);
+    k_loads<<<nlist, kLoadThreads, sizeof(double) * (max_np + 1), s>>>(table, st, list);
 }
 
 void step_counter(InstState* st, const ListEntry* list, int nlist, cudaStream_t s) {
