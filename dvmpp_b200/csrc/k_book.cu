@@ -13,6 +13,7 @@
 
 #include "dvm_device.cuh"
 #include "dvm_internal.h"
+#include "dvm_tree.cuh"
 
 namespace dvmk {
 namespace {
@@ -249,6 +250,38 @@ __device__ __forceinline__ void load_contour(const InstDesc& d, double* sx, doub
     }
 }
 
+// Crossing work comes in items of 64 blobs.  Most are settled by the bounding box;
+// the rest queue up in shared memory and the block's eight warps take them in turn.
+// Freshly released blobs are candidates all, and neighbours in the arrays: with
+// items of 256 or 1024, each warp going through its own 32, they were one or a few
+// blocks' work (1024 panels, RK3, DELETE: 231 us, 31 now; 128 panels, 2 k blobs,
+// REFLECT: 22-43 us, 12-29 now).
+constexpr uint32_t kCrossItem = 64;
+struct CrossQueue {
+    double2 at[kCrossItem];
+    uint32_t slot[kCrossItem];
+    uint32_t count;
+};
+
+// Fills the queue from blobs i0 .. i0 + 63 (every thread calls it; ends with a
+// barrier).
+__device__ __forceinline__ void cross_candidates(CrossQueue& Q, const InstDesc& d, uint32_t i0,
+                                                 uint32_t n) {
+    if (threadIdx.x == 0) Q.count = 0;
+    __syncthreads();
+    if (threadIdx.x < kCrossItem) {
+        const uint32_t i = i0 + threadIdx.x;
+        const bool valid = i < n;
+        const double px = valid ? d.x[i] : 0.0, pz = valid ? d.z[i] : 0.0;
+        if (valid && in_bbox(d, px, pz)) {
+            const uint32_t q = atomicAdd(&Q.count, 1u);  // (their order does not matter)
+            Q.at[q] = make_double2(px, pz);
+            Q.slot[q] = threadIdx.x;
+        }
+    }
+    __syncthreads();
+}
+
 // REFLECT / ABSORB (src/VortexSheet.cpp:345-405): each blob moves independently.
 __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ table,
                                                  const InstState* __restrict__ st,
@@ -256,19 +289,14 @@ __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ ta
                                                  unsigned* __restrict__ work) {
     extern __shared__ double s_c[];
     __shared__ unsigned s_pre[1025];
+    __shared__ CrossQueue Q;
     __shared__ unsigned s_item;
-    __shared__ int s_loaded;
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int k = 0; k < nlist; ++k) {
-            s_pre[k] = acc;
-            acc += st[list[k].inst].status ? 0u : (st[list[k].inst].n + 255) / 256;
-        }
-        s_pre[nlist] = acc;
-        s_loaded = -1;
-    }
-    __syncthreads();
+    list_prefix(s_pre, nlist, [&](int k) {
+        const InstState& S = st[list[k].inst];
+        return S.status ? 0u : (S.n + kCrossItem - 1) / kCrossItem;
+    });
     const unsigned total = s_pre[nlist];
+    int loaded = -1;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(work, 1u);
         __syncthreads();
@@ -282,22 +310,17 @@ __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ ta
         double* sz = sx + (np + 1);
         double* snx = sz + (np + 1);
         double* snz = snx + np;
-        if (s_loaded != k) load_contour(d, sx, sz, snx, snz);
-        __syncthreads();
-        if (threadIdx.x == 0) s_loaded = k;
-        const uint32_t n = st[e.inst].n;
-        const uint32_t i = (item - s_pre[k]) * 256 + threadIdx.x;
-        const bool valid = i < n;
-        const double px = valid ? d.x[i] : 0.0, pz = valid ? d.z[i] : 0.0;
-        // blobs in the contour's bounding box, handled one at a time by the
-        // whole warp (edges and panels split over the lanes)
-        unsigned cand = __ballot_sync(0xffffffffu, valid && in_bbox(d, px, pz));
+        const uint32_t i0 = (item - s_pre[k]) * kCrossItem;
+        cross_candidates(Q, d, i0, st[e.inst].n);
+        const uint32_t count = Q.count;
+        if (count && loaded != k) {  // block-uniform
+            load_contour(d, sx, sz, snx, snz);
+            loaded = k;
+            __syncthreads();
+        }
         const int lane = threadIdx.x & 31;
-        while (cand) {
-            const int src = __ffs(cand) - 1;
-            cand &= cand - 1;
-            const double qx = __shfl_sync(0xffffffffu, px, src);
-            const double qz = __shfl_sync(0xffffffffu, pz, src);
+        for (uint32_t c = threadIdx.x >> 5; c < count; c += 8) {
+            const double qx = Q.at[c].x, qz = Q.at[c].y;
             if (!inside_body_warp(sx, sz, np, qx, qz)) continue;
             // nearest panel: the first minimum of the clamped point-segment
             // distance (src/VortexSheet.cpp:378-390), per lane over its
@@ -335,65 +358,71 @@ __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ ta
                 nx = dadd(qx, dmul(dmul(3.0, off), snx[cp]));
                 nz = dadd(qz, dmul(dmul(3.0, off), snz[cp]));
             }
-            if (lane == src) {
-                d.x[i] = nx;
-                d.z[i] = nz;
+            if (lane == 0) {
+                d.x[i0 + Q.slot[c]] = nx;
+                d.z[i0 + Q.slot[c]] = nz;
             }
         }
         __syncthreads();
     }
 }
 
-// DELETE (src/VortexSheet.cpp:407-445): keep flags and kept count per 1024-tile.
+// DELETE (src/VortexSheet.cpp:407-445): keep flags and kept count per 1024-tile
+// (tile_counts starts at zero).
 constexpr int kDelTile = 1024;
 
 __global__ void __launch_bounds__(256) k_del_flags(const InstDesc* __restrict__ table,
                                                    const InstState* __restrict__ st,
-                                                   const ListEntry* __restrict__ list,
+                                                   const ListEntry* __restrict__ list, int nlist,
                                                    uint8_t* __restrict__ flags,
-                                                   uint32_t* __restrict__ tile_counts) {
+                                                   uint32_t* __restrict__ tile_counts,
+                                                   unsigned* __restrict__ work) {
     extern __shared__ double s_c[];
-    __shared__ uint32_t s_cnt;
-    const ListEntry e = list[blockIdx.y];
-    const InstDesc& d = table[e.inst];
-    const InstState& S = st[e.inst];
-    const uint32_t n = S.n;
-    const uint32_t ntiles = (n + kDelTile - 1) / kDelTile;
-    if (S.status) return;
-    double* sx = s_c;
-    double* sz = sx + (d.np + 1);
-    double* snx = sz + (d.np + 1);
-    double* snz = snx + d.np;
-    load_contour(d, sx, sz, snx, snz);
-    __syncthreads();
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        if (threadIdx.x == 0) s_cnt = 0;
+    __shared__ unsigned s_pre[1025];
+    __shared__ CrossQueue Q;
+    __shared__ uint8_t s_in[kCrossItem];
+    __shared__ unsigned s_item;
+    list_prefix(s_pre, nlist, [&](int k) {
+        const InstState& S = st[list[k].inst];
+        return S.status ? 0u : (S.n + kCrossItem - 1) / kCrossItem;
+    });
+    const unsigned total = s_pre[nlist];
+    int loaded = -1;
+    for (;;) {
+        if (threadIdx.x == 0) s_item = atomicAdd(work, 1u);
         __syncthreads();
-        uint32_t mine = 0;
-        for (uint32_t q = threadIdx.x; q < kDelTile; q += blockDim.x) {  // uniform trip count
-            const uint32_t i = t * kDelTile + q;
-            const bool valid = i < n;
-            const double px = valid ? d.x[i] : 0.0, pz = valid ? d.z[i] : 0.0;
-            // bounding-box candidates, tested by the whole warp one at a time
-            unsigned cand = __ballot_sync(0xffffffffu, valid && in_bbox(d, px, pz));
-            bool inside = false;
-            while (cand) {
-                const int src = __ffs(cand) - 1;
-                cand &= cand - 1;
-                const bool in = inside_body_warp(sx, sz, d.np, __shfl_sync(0xffffffffu, px, src),
-                                                 __shfl_sync(0xffffffffu, pz, src));
-                if ((threadIdx.x & 31) == src) inside = in;
+        const unsigned item = s_item;
+        if (item >= total) break;
+        const int k = locate(s_pre, nlist, item);
+        const ListEntry e = list[k];
+        const InstDesc& d = table[e.inst];
+        const uint32_t n = st[e.inst].n, i0 = (item - s_pre[k]) * kCrossItem;
+        double* sx = s_c;
+        double* sz = sx + (d.np + 1);
+        if (threadIdx.x < kCrossItem) s_in[threadIdx.x] = 0;
+        cross_candidates(Q, d, i0, n);
+        const uint32_t count = Q.count;
+        if (count && loaded != k) {  // block-uniform
+            for (int j = threadIdx.x; j <= d.np; j += blockDim.x) {
+                sx[j] = d.xp[j];
+                sz[j] = d.zp[j];
             }
-            if (valid) {
-                const uint8_t keep = inside ? 0 : 1;
-                flags[e.coff + i] = keep;
-                mine += keep;
-            }
+            loaded = k;
+            __syncthreads();
         }
-        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&s_cnt, mine);
+        for (uint32_t c = threadIdx.x >> 5; c < count; c += 8) {
+            const bool in = inside_body_warp(sx, sz, d.np, Q.at[c].x, Q.at[c].y);
+            if ((threadIdx.x & 31) == 0 && in) s_in[Q.slot[c]] = 1;
+        }
         __syncthreads();
-        if (threadIdx.x == 0) tile_counts[e.coff / kDelTile + t] = s_cnt;
+        if (threadIdx.x < kCrossItem) {  // two warps
+            const uint32_t i = i0 + threadIdx.x;
+            const bool keep = i < n && !s_in[threadIdx.x];
+            if (i < n) flags[e.coff + i] = keep ? 1 : 0;
+            const unsigned b = __ballot_sync(0xffffffffu, keep);
+            if ((threadIdx.x & 31) == 0 && b)
+                atomicAdd(&tile_counts[e.coff / kDelTile + i0 / kDelTile], (uint32_t)__popc(b));
+        }
         __syncthreads();
     }
 }
@@ -592,28 +621,20 @@ void release(const InstDesc* table, InstState* st, const ListEntry* list, int nl
 void reflect(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, int max_np,
              const Workspace& ws, int sms, cudaStream_t s) {
     const size_t smem = contour_smem(max_np);
-    static bool attr = false;  // set once, before any graph capture (first call is eager)
-    if (!attr) {
-        cudaFuncSetAttribute(k_reflect, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr = true;
-    }
+    cudaFuncSetAttribute(k_reflect, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaMemsetAsync(ws.work + 2, 0, sizeof(unsigned), s);
     k_reflect<<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.work + 2);
 }
 
 void delete_inside(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                    int max_np, const Workspace& ws, int sms, cudaStream_t s) {
-    const size_t smem = contour_smem(max_np);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_del_flags, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr = true;
-    }
-    const int gx = std::max(1, sms * 4 / std::max(1, nlist));
-    k_del_flags<<<dim3(gx, nlist), 256, smem, s>>>(table, st, list, ws.flags, ws.tile_counts);
+    const size_t smem = sizeof(double) * (2 * (size_t)max_np + 2);
+    cudaMemsetAsync(ws.tile_counts, 0, sizeof(uint32_t) * (ws.total_cap / kDelTile + 1), s);
+    cudaMemsetAsync(ws.work + 3, 0, 2 * sizeof(unsigned), s);
+    k_del_flags<<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.flags, ws.tile_counts,
+                                           ws.work + 4);
     k_del_scan<<<nlist, 1024, 0, s>>>(st, list, ws.tile_counts, ws.tile_base, ws.del_kept);
     cudaMemsetAsync(ws.del_ready, 0, sizeof(uint32_t) * (ws.total_cap / kDelTile + 1), s);
-    cudaMemsetAsync(ws.work + 3, 0, sizeof(unsigned), s);
     k_del_move<<<sms * 2, kDelTile, 0, s>>>(table, st, list, nlist, ws.flags, ws.tile_base,
                                             ws.del_kept, ws.del_ready, ws.work + 3);
     k_del_finish<<<(nlist + 127) / 128, 128, 0, s>>>(st, list, nlist, ws.del_kept);
