@@ -1279,30 +1279,34 @@ int dvm_sim_set_blobs(dvm_sim* s, uint64_t n, const double* x, const double* z, 
     if (!s) return fail(DVM_ERR_ARG, "sim is null");
     if (n > s->h.cap) return fail(DVM_ERR_CAPACITY, "more blobs than the simulation's capacity");
     if (n && (!x || !z || !circ || !sigma)) return fail(DVM_ERR_ARG, "null blob array");
-    for (uint64_t i = 0; i < n; ++i)
-        if (!std::isfinite(x[i]) || !std::isfinite(z[i]) || !std::isfinite(circ[i]) ||
-            !std::isfinite(sigma[i]))
-            return fail(DVM_ERR_ARG, "blob " + std::to_string(i) + " has a non-finite value");
     SIM_LOCK(s);
-    cudaStream_t st = s->ctx->stream;
-    CK(cudaStreamSynchronize(st));
-    if (n) {
-        CK(cudaMemcpyAsync(s->h.x, x, 8 * n, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(s->h.z, z, 8 * n, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(s->h.circ, circ, 8 * n, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(s->h.sigma, sigma, 8 * n, cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(s->h.u, 0, 8 * n, st));
-        CK(cudaMemsetAsync(s->h.w, 0, 8 * n, st));
-        CK(cudaMemsetAsync(s->h.uvs, 0, 8 * n, st));
-        CK(cudaMemsetAsync(s->h.wvs, 0, 8 * n, st));
-        std::vector<uint32_t> ids(n);
-        for (uint64_t i = 0; i < n; ++i) ids[i] = (uint32_t)i;
-        CK(cudaMemcpyAsync(s->h.id, ids.data(), 4 * n, cudaMemcpyHostToDevice, st));
-        CK(cudaStreamSynchronize(st));
-    }
-    const uint32_t n32 = (uint32_t)n;
-    CK(cudaMemcpyAsync(&s->ctx->d_state[s->slot].n, &n32, 4, cudaMemcpyHostToDevice, st));
-    CK(cudaStreamSynchronize(st));
+    dvm_ctx* c = s->ctx;
+    cudaStream_t st = c->stream;
+    // Uploaded to scratch, checked and taken over on the device: a set with a
+    // non-finite value leaves the simulation as it was.
+    double* v = nullptr;
+    const cudaError_t e = pool_alloc(c, reinterpret_cast<void**>(&v), 32 * n + 16);
+    if (e != cudaSuccess) return fail(DVM_ERR_OOM, std::string("blob upload: ") + cudaGetErrorString(e));
+    uint32_t* d_bad = reinterpret_cast<uint32_t*>(v + 4 * n);
+    const double* src[4] = {x, z, circ, sigma};
+    cudaError_t up = cudaSuccess;
+    for (int k = 0; k < 4 && n && up == cudaSuccess; ++k)
+        up = cudaMemcpyAsync(v + k * n, src[k], 8 * n, cudaMemcpyHostToDevice, st);
+    const InstDesc& h = s->h;
+    if (up == cudaSuccess)
+        take_blobs(v, (uint32_t)n, d_bad,
+                   BlobArrays{h.x, h.z, h.circ, h.sigma, h.u, h.w, h.uvs, h.wvs, h.id},
+                   &c->d_state[s->slot].n, st);
+    g_launches += 2;
+    uint32_t bad = UINT32_MAX;
+    if (up == cudaSuccess)
+        up = cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, st);
+    pool_free(c, v);
+    const cudaError_t end = cudaStreamSynchronize(st);
+    if (up == cudaSuccess) up = end;
+    if (up != cudaSuccess) return fail(DVM_ERR_CUDA, std::string("blob upload: ") + cudaGetErrorString(up));
+    if (bad != UINT32_MAX)
+        return fail(DVM_ERR_ARG, "blob " + std::to_string(bad) + " has a non-finite value");
     return DVM_OK;
 }
 
@@ -2280,9 +2284,7 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     InstState st0;
     std::memset(&st0, 0, sizeof(st0));
     st0.n = (uint32_t)n;
-    CK(cudaMemcpyAsync(c->d_table, &h, sizeof(h), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->d_state, &st0, sizeof(st0), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_list, &e, sizeof(e), cudaMemcpyHostToDevice, c->stream));
+    setup_slot(c->d_table, h, c->d_state, st0, d_list, e, c->stream);
     Workspace ws = c->ws;
     ws.key_bits = key_bits_for(1);
     ws.total_cap = cap;
@@ -2309,36 +2311,23 @@ int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velo
     if (!c || (n && (!p || !out))) return fail(DVM_ERR_ARG, "null argument");
     if (precision != DVM_F64 && precision != DVM_F32) return fail(DVM_ERR_ARG, "bad precision");
     if (n == 0) return DVM_OK;
+    if (n > 0xF0000000ull) return fail(DVM_ERR_ARG, "too many particles");
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    // AoS -> SoA on the host while computing the Morton domain.
-    std::vector<double> h(6 * n);
-    double xmn = p[0].x, xmx = p[0].x, zmn = p[0].z, zmx = p[0].z;
-    for (uint64_t i = 0; i < n; ++i) {
-        h[i] = p[i].x;
-        h[n + i] = p[i].z;
-        h[2 * n + i] = p[i].circ;
-        h[3 * n + i] = p[i].sigma;
-        xmn = std::min(xmn, p[i].x);
-        xmx = std::max(xmx, p[i].x);
-        zmn = std::min(zmn, p[i].z);
-        zmx = std::max(zmx, p[i].z);
-    }
-    int rc = raw_reserve(c, 8 * 6 * n);
+    int rc = raw_reserve(c, 8 * 8 * n);
     if (rc) return rc;
+    // x z circ sigma | particles, then u w and the velocity pairs in their place
     double* d = static_cast<double*>(c->raw_block);
-    CK(cudaMemcpyAsync(d, h.data(), 8 * 4 * n, cudaMemcpyHostToDevice, c->stream));
-    double L = std::max(xmx - xmn, zmx - zmn);
-    if (!(L > 0)) L = 1.0;
-    rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, d + 4 * n, d + 5 * n, precision, xmn, zmn,
-                  65535.0 / L);
+    double* aos = d + 4 * n;
+    double* pairs = aos + 2 * n;
+    CK(cudaMemcpyAsync(aos, p, sizeof(dvm_particle) * n, cudaMemcpyHostToDevice, c->stream));
+    aos_to_soa(aos, (uint32_t)n, d, c->stream);
+    rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, aos, aos + n, precision, 0.0, 0.0, 0.0);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(h.data() + 4 * n, d + 4 * n, 8 * 2 * n, cudaMemcpyDeviceToHost, c->stream));
+    velocity_pairs(aos, aos + n, (uint32_t)n, pairs, c->stream);
+    g_launches += 2;
+    CK(cudaMemcpyAsync(out, pairs, sizeof(dvm_velocity) * n, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    for (uint64_t i = 0; i < n; ++i) {
-        out[i].u = h[4 * n + i];
-        out[i].w = h[5 * n + i];
-    }
     return DVM_OK;
 }
 
@@ -2530,21 +2519,18 @@ int dvm_remesh(dvm_ctx* c, const dvm_particle* in, uint64_t n, const dvm_remesh_
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    const size_t data = align_up(8 * 4 * (size_t)n, 256) + align_up(8 * 4 * (size_t)out_cap, 256) + 256;
+    // particles in, x z circ sigma | x z circ sigma out, particles out | count
+    const size_t in_b = align_up(8 * 4 * (size_t)n, 256), out_b = align_up(8 * 4 * (size_t)out_cap, 256);
+    const size_t data = 2 * in_b + 2 * out_b + 256;
     rc = raw_reserve(c, data);
     if (rc) return rc;
     char* base = static_cast<char*>(c->raw_block);
-    double* din = reinterpret_cast<double*>(base);
-    double* dout = reinterpret_cast<double*>(base + align_up(8 * 4 * (size_t)n, 256));
+    double* din = reinterpret_cast<double*>(base + in_b);
+    double* dout = reinterpret_cast<double*>(base + 2 * in_b);
+    char* aos_out = base + 2 * in_b + out_b;
     uint32_t* dneed = reinterpret_cast<uint32_t*>(base + data - 256);
-    std::vector<double> h(4 * n);
-    for (uint64_t i = 0; i < n; ++i) {
-        h[i] = in[i].x;
-        h[n + i] = in[i].z;
-        h[2 * n + i] = in[i].circ;
-        h[3 * n + i] = in[i].sigma;
-    }
-    if (n) CK(cudaMemcpyAsync(din, h.data(), 8 * 4 * n, cudaMemcpyHostToDevice, c->stream));
+    if (n) CK(cudaMemcpyAsync(base, in, sizeof(dvm_particle) * n, cudaMemcpyHostToDevice, c->stream));
+    aos_to_soa(base, (uint32_t)n, din, c->stream);
     void* scratch = nullptr;
     const cudaError_t e = pool_alloc(c, &scratch, remesh_scratch_bytes(g, (uint32_t)n, (uint32_t)out_cap));
     if (e != cudaSuccess) return fail(DVM_ERR_OOM, std::string("remesh scratch: ") + cudaGetErrorString(e));
@@ -2553,17 +2539,19 @@ int dvm_remesh(dvm_ctx* c, const dvm_particle* in, uint64_t n, const dvm_remesh_
     remesh_run(g, din, din + n, din + 2 * n, din + 3 * n, (uint32_t)n, (uint32_t)out_cap, d,
                nullptr, scratch, c->sms, c->stream);
     pool_free(c, scratch);
-    g_launches += 7;
+    soa_to_aos(dout, dout + out_cap, dout + 2 * out_cap, dout + 3 * out_cap, dneed,
+               (uint32_t)out_cap, aos_out, c->stream);
+    g_launches += 9;
     uint32_t need = 0;
     CK(cudaMemcpyAsync(&need, dneed, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     *n_out = need;
     if (need > out_cap)
         return fail(DVM_ERR_CAPACITY, "remesh: " + std::to_string(need) + " blobs do not fit out_cap");
-    std::vector<double> r(4 * (size_t)out_cap);
-    if (need) CK(cudaMemcpy(r.data(), dout, 8 * 4 * (size_t)out_cap, cudaMemcpyDeviceToHost));
-    for (uint32_t i = 0; i < need; ++i)
-        out[i] = dvm_particle{r[i], r[out_cap + i], r[2 * out_cap + i], r[3 * out_cap + i]};
+    if (need) {
+        CK(cudaMemcpyAsync(out, aos_out, sizeof(dvm_particle) * need, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
     return DVM_OK;
 }
 
@@ -2593,16 +2581,13 @@ int dvm_sim_probe(dvm_sim* s, const double* px, const double* pz, uint64_t n, do
     direct_at_raw(s->h.x, s->h.z, s->h.circ, s->h.sigma, ns, dx, dz, nt, dres, dres + n,
                   s->h.precision, 1, static_cast<double2*>(c->raw_block), c->sms, c->stream);
     sheet_at(s->h, dx, dz, nt, dres + 2 * n, dres + 3 * n, c->stream);
-    g_launches += ns ? 3 : 1;
-    std::vector<double> h(4 * n);
-    CK(cudaMemcpyAsync(h.data(), dres, 8 * 4 * n, cudaMemcpyDeviceToHost, c->stream));
+    probe_total(dres, nt, s->h.ux, s->h.uz, c->stream);
+    g_launches += ns ? 4 : 2;
+    double* const out[4] = {u, w, uvs, wvs};
+    for (int k = 0; k < 4; ++k)
+        if (out[k])
+            CK(cudaMemcpyAsync(out[k], dres + k * n, 8 * n, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    for (uint64_t i = 0; i < n; ++i) {
-        u[i] = (h[i] + h[2 * n + i]) + s->h.ux;
-        w[i] = (h[n + i] + h[3 * n + i]) + s->h.uz;
-        if (uvs) uvs[i] = h[2 * n + i];
-        if (wvs) wvs[i] = h[3 * n + i];
-    }
     return DVM_OK;
 }
 
@@ -2615,34 +2600,27 @@ int dvm_biot_savart_at(dvm_ctx* c, const dvm_particle* p, uint64_t ns, const dou
     CK(cudaSetDevice(c->device));
     const size_t elems = direct_at_part_elems((uint32_t)ns, (uint32_t)nt);
     const size_t part_bytes = align_up(16 * elems, 256);
-    const size_t data_bytes = 8 * (4 * ns + 4 * nt);
+    // x z circ sigma | tx tz | u w | particles, later velocities
+    const size_t aos = std::max<size_t>(sizeof(dvm_particle) * ns, sizeof(dvm_velocity) * nt);
+    const size_t data_bytes = align_up(8 * (4 * ns + 4 * nt), 256) + aos;
     int rc = raw_reserve(c, part_bytes + data_bytes);
     if (rc) return rc;
     char* base = static_cast<char*>(c->raw_block);
     double* d = reinterpret_cast<double*>(base + part_bytes);
-    std::vector<double> h(4 * ns + 2 * nt);
-    for (uint64_t i = 0; i < ns; ++i) {
-        h[i] = p[i].x;
-        h[ns + i] = p[i].z;
-        h[2 * ns + i] = p[i].circ;
-        h[3 * ns + i] = p[i].sigma;
-    }
-    std::memcpy(h.data() + 4 * ns, tx, 8 * nt);
-    std::memcpy(h.data() + 4 * ns + nt, tz, 8 * nt);
-    CK(cudaMemcpyAsync(d, h.data(), 8 * h.size(), cudaMemcpyHostToDevice, c->stream));
-    double* du = d + 4 * ns + 2 * nt;
+    void* d_aos = base + part_bytes + align_up(8 * (4 * ns + 4 * nt), 256);
+    double* dt = d + 4 * ns;
+    if (ns) CK(cudaMemcpyAsync(d_aos, p, sizeof(dvm_particle) * ns, cudaMemcpyHostToDevice, c->stream));
+    aos_to_soa(d_aos, (uint32_t)ns, d, c->stream);
+    CK(cudaMemcpyAsync(dt, tx, 8 * nt, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(dt + nt, tz, 8 * nt, cudaMemcpyHostToDevice, c->stream));
+    double* du = dt + 2 * nt;
     double* dw = du + nt;
-    direct_at_raw(d, d + ns, d + 2 * ns, d + 3 * ns, (uint32_t)ns, d + 4 * ns, d + 4 * ns + nt,
-                  (uint32_t)nt, du, dw, precision, 1, reinterpret_cast<double2*>(base), c->sms,
-                  c->stream);
-    g_launches += 2;
-    std::vector<double> r(2 * nt);
-    CK(cudaMemcpyAsync(r.data(), du, 8 * 2 * nt, cudaMemcpyDeviceToHost, c->stream));
+    direct_at_raw(d, d + ns, d + 2 * ns, d + 3 * ns, (uint32_t)ns, dt, dt + nt, (uint32_t)nt, du, dw,
+                  precision, 1, reinterpret_cast<double2*>(base), c->sms, c->stream);
+    velocity_pairs(du, dw, (uint32_t)nt, d_aos, c->stream);
+    g_launches += 4;
+    CK(cudaMemcpyAsync(out, d_aos, sizeof(dvm_velocity) * nt, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    for (uint64_t i = 0; i < nt; ++i) {
-        out[i].u = r[i];
-        out[i].w = r[nt + i];
-    }
     return DVM_OK;
 }
 

@@ -297,6 +297,29 @@ size_t merge_count_offset(uint32_t n);
 void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
                uint32_t* n_dev, uint32_t* count_dev, void* scratch, int sms, cudaStream_t s);
 
+// Conversions between host and device layouts (k_convert.cu).  Arrays "of four" are
+// n values each, one after another.
+struct BlobArrays {
+    double *x, *z, *circ, *sigma, *u, *w, *uvs, *wvs;
+    uint32_t* id;
+};
+// n particles (x, z, circ, sigma) to four arrays.
+void aos_to_soa(const void* in, uint32_t n, double* out, cudaStream_t s);
+// n pairs (u, w).
+void velocity_pairs(const double* u, const double* w, uint32_t n, void* out, cudaStream_t s);
+// min(*n, cap) particles.
+void soa_to_aos(const double* x, const double* z, const double* c, const double* sg,
+                const uint32_t* n, uint32_t cap, void* out, cudaStream_t s);
+// Blob set v (x, z, circ, sigma) into a simulation's arrays and count, unless a
+// value is not finite: *bad is then the first such blob, else the largest value.
+void take_blobs(const double* v, uint32_t n, uint32_t* bad, const BlobArrays& a, uint32_t* count,
+                cudaStream_t s);
+// u += uvs + ux, w += wvs + uz for v = u, w, uvs, wvs.
+void probe_total(double* v, uint32_t n, double ux, double uz, cudaStream_t s);
+// One descriptor, state and list entry, by value.
+void setup_slot(InstDesc* d, const InstDesc& dv, InstState* st, const InstState& sv, ListEntry* e,
+                const ListEntry& ev, cudaStream_t s);
+
 // Sheet velocity at arbitrary points from one simulation's panels and gamma
 // (the sheet-on-blob sum of src/VortexSheet.cpp:217-273, FP64), for probes.
 void sheet_at(const InstDesc& d, const double* px, const double* pz, uint32_t n, double* uvs,

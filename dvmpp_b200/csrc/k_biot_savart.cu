@@ -1774,6 +1774,10 @@ size_t direct_at_part_elems(uint32_t ns, uint32_t nt) {
     return std::max<size_t>(1, nchunk) * std::max<size_t>(npad, 256) + 64;
 }
 
+namespace {
+__global__ void k_write_job(AtJob* dst, AtJob job) { *dst = job; }
+}  // namespace
+
 static void launch_at(const AtJob* job, const AtJob& J, int precision, double* u, double* w, int sms,
                       cudaStream_t s) {
     if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(job, 1);
@@ -1805,8 +1809,8 @@ void direct_at_raw(const double* x, const double* z, const double* circ, const d
     J.chunk = at_chunk(ns, nt);
     J.part = part;
     J.circ_part = nullptr;
-    cudaMemcpyAsync(job, &J, sizeof(AtJob), cudaMemcpyHostToDevice, s);
     if (ns > 0) {
+        k_write_job<<<1, 1, 0, s>>>(job, J);
         launch_at(job, J, precision, u, w, sms, s);
     } else {
         cudaMemsetAsync(u, 0, sizeof(double) * nt, s);
@@ -1824,8 +1828,6 @@ namespace {
 constexpr size_t kNoAllocElems = 262144;  // double2 entries: 4 MiB per device
 constexpr size_t kNoAllocJobElems = 64;   // tail entries that hold the job record
 static __device__ __align__(256) double2 g_noalloc_scratch[kNoAllocElems];
-
-__global__ void k_write_job(AtJob* dst, AtJob job) { *dst = job; }
 
 }  // namespace
 
