@@ -11,15 +11,15 @@
 // both.
 //
 // The solve: the reference forms A^T A and A^T b and solves with LAPACK every
-// call.  Here A ((np+1) x np) is factorised ONCE per body by Householder QR on
-// the GPU and the pseudo-inverse P = R^-1 Q^T is kept in HBM; each step is then
-// gamma = P b (a batched GEMV) plus one iterative-refinement step with the FP64
-// residual r = b - A gamma (gamma += P r).  Same least-squares solution, no
-// O(np^3) work per step.
+// call.  Here the pseudo-inverse P of A ((np+1) x np) is formed ONCE per body and
+// kept in HBM; each step is then gamma = P b (a batched GEMV) plus one
+// iterative-refinement step with the FP64 residual r = b - A gamma (gamma += P r).
+// Same least-squares solution, no O(np^3) work per step.
 #include <algorithm>
 #include <cfloat>
 
 #include <cooperative_groups.h>
+#include <cstring>
 #include <vector>
 
 #include "dvm_device.cuh"
@@ -77,7 +77,313 @@ __global__ void k_assemble_A(const double* __restrict__ p, const double* __restr
     A[(size_t)i * np + j] = dmul(-kRpi2, dadd(p[(size_t)i * np + j], q[(size_t)i * np + jm]));
 }
 
-// ---- Householder QR of A (column-major, m = np+1 rows) ------------------------
+// ---- pseudo-inverse ------------------------------------------------------------
+// P0 = (A^T A)^-1 A^T by a blocked Gauss-Jordan inversion, then P = P0 + (I - P0 A) P0,
+// a step of the Newton-Schulz iteration for inverses (Schulz, ZAMM 13 (1933) 57;
+// Ben-Israel and Cohen, SIAM J. Numer. Anal. 3 (1966) 410), which squares the
+// error: forming A^T A loses cond(A)^2 ulps, and the step, with the residual formed
+// from A itself, brings that back to about cond(A).  The residual's largest entry E
+// is looked at.  Up to kSchulzExact (condition numbers to about 60: circles,
+// ellipses, blunt airfoils) one step is all.  Up to kSchulzDone it is followed by
+// P <- P (A P)^T, which takes out what rounding in (A^T A)^-1 A^T left outside A's
+// column space (the step cannot); up to kSchulzStart the step is repeated before
+// that; above it (condition about 1e5: plates thinner than 0.05 % of their chord) a
+// Householder factorisation takes the place of all this.  Error of gamma against
+// extended precision over 126 Joukowski airfoils 0.1 to 12 % thick (condition 100 to
+// 2e4), as a ratio to the Householder factorisation's: geometric mean 0.82 to 1.34
+// per decade of E, 1.0 over all; ellipses and circles 0.98.
+//
+// All of it is matrix products in 32 x 32 tiles and np / 32 dependent steps of the
+// inversion, where a Householder factorisation is np dependent steps with a grid
+// barrier each: dvm_sim_create at 64, 512, 1024 and 2048 panels 0.25, 1.9, 10.0 and
+// 98 ms -> 0.19, 0.99, 2.8 and 13 ms; eight bodies of 512 8.6 -> 2.6 ms.
+constexpr int kTile = 32;
+constexpr int kTileThreads = 64;  // 8 x 8 threads with 4 x 4 outputs each
+constexpr int kTileDepth = 16;
+constexpr double kSchulzExact = 1e-12, kSchulzDone = 1e-8, kSchulzStart = 1e-5;
+// Bodies that would end in the Householder factorisation anyway, or whose extra
+// launches and waits outweigh the products (0.28 ms against 0.24 at 64 panels), go
+// there at once.
+constexpr double kThinCond = 1e5, kThinCondSmall = 5e3;
+constexpr int kThinSmall = 100;
+
+struct PinvBody {
+    const double* A;  // m x np
+    double* P;        // np x m: the result
+    double* G[2];     // np x np: A^T A and its inverse, the residual; W
+    double* T;        // np x m: every other P
+    int in_p;         // the latest P is in P (else in T)
+    unsigned long long* err;  // largest |I - P A|, as bits
+    int np, steps;            // steps of the inversion: it ends in G[steps & 1]
+    int block0, blocks;  // of the inversion's launch
+};
+constexpr int kPinvMaxBodies = 8;
+struct PinvGroup {
+    PinvBody b[kPinvMaxBodies];
+    int nb, steps;
+};
+
+struct TileShared {
+    double a[kTileDepth][kTile + 1], b[kTileDepth][kTile + 1];
+};
+
+// acc += sum over k < K of la(row, k) lb(k, col) for the block's 32 x 32 tile (rows
+// and columns relative to it).  AK, BK: the operand is contiguous along k (its
+// loads run that way).  The next slice is fetched while this one is multiplied.
+template <bool AK, bool BK, typename LA, typename LB>
+__device__ __forceinline__ void tile_product(TileShared& S, int K, LA la, LB lb, double (&acc)[4][4]) {
+    const int t = threadIdx.x, r0 = (t >> 3) * 4, c0 = (t & 7) * 4;
+    constexpr int N = kTileDepth * kTile / kTileThreads;
+    double fa[N], fb[N];
+    auto place = [&](int q, bool along_k, int& k, int& x) {
+        const int i = q * kTileThreads + t;
+        k = along_k ? i % kTileDepth : i / kTile;
+        x = along_k ? i / kTileDepth : i % kTile;
+    };
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            int k, x;
+            place(q, AK, k, x);
+            fa[q] = k0 + k < K ? la(x, k0 + k) : 0.0;
+            place(q, BK, k, x);
+            fb[q] = k0 + k < K ? lb(k0 + k, x) : 0.0;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += kTileDepth) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            int k, x;
+            place(q, AK, k, x);
+            S.a[k][x] = fa[q];
+            place(q, BK, k, x);
+            S.b[k][x] = fb[q];
+        }
+        __syncthreads();
+        if (k0 + kTileDepth < K) fetch(k0 + kTileDepth);
+#pragma unroll
+        for (int k = 0; k < kTileDepth; ++k) {
+            double x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                x[i] = S.a[k][r0 + i];
+                y[i] = S.b[k][c0 + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma(x[i], y[j], acc[i][j]);
+        }
+    }
+}
+
+// One 32 x 32 tile per block of 64 threads, blockIdx.y the body.
+//   G: G[0] = A^T A;  P0: T = M A^T, M the inverse;
+//   E: E = I - P A (over the other G) and its largest entry;  P1: P + E P;
+//   W: W = A P (m x m, over both G);  P2: P W^T.
+enum PinvProduct : int { kProdG = 0, kProdP0 = 1, kProdE = 2, kProdP1 = 3, kProdW = 4, kProdP2 = 5 };
+template <int WHAT>
+__global__ void __launch_bounds__(kTileThreads) k_pinv_product(const __grid_constant__ PinvGroup Q) {
+    __shared__ TileShared S;
+    const PinvBody& B = Q.b[blockIdx.y];
+    const int np = B.np, m = np + 1;
+    const int cols = WHAT == kProdG || WHAT == kProdE ? np : m, rows = WHAT == kProdW ? m : np;
+    const int tc = (cols + kTile - 1) / kTile, tiles = tc * ((rows + kTile - 1) / kTile);
+    if ((int)blockIdx.x >= tiles) return;
+    const int i0 = (int)blockIdx.x / tc * kTile, j0 = (int)blockIdx.x % tc * kTile;
+    const double* __restrict__ A = B.A;
+    const double* M = B.G[B.steps & 1];
+    double* E = B.G[(B.steps & 1) ^ 1];
+    const double* P = B.in_p ? B.P : B.T;
+    double* next = B.in_p ? B.T : B.P;
+    double acc[4][4] = {};
+    if (WHAT == kProdG) {
+        tile_product<false, false>(
+            S, m, [&](int r, int k) { return i0 + r < np ? A[(size_t)k * np + i0 + r] : 0.0; },
+            [&](int k, int c) { return j0 + c < np ? A[(size_t)k * np + j0 + c] : 0.0; }, acc);
+    } else if (WHAT == kProdP0) {
+        tile_product<true, true>(
+            S, np, [&](int r, int k) { return i0 + r < np ? M[(size_t)(i0 + r) * np + k] : 0.0; },
+            [&](int k, int c) { return j0 + c < m ? A[(size_t)(j0 + c) * np + k] : 0.0; }, acc);
+    } else if (WHAT == kProdE) {
+        tile_product<true, false>(
+            S, m, [&](int r, int k) { return i0 + r < np ? P[(size_t)(i0 + r) * m + k] : 0.0; },
+            [&](int k, int c) { return j0 + c < np ? A[(size_t)k * np + j0 + c] : 0.0; }, acc);
+    } else if (WHAT == kProdW) {
+        tile_product<true, false>(
+            S, np, [&](int r, int k) { return i0 + r < m ? A[(size_t)(i0 + r) * np + k] : 0.0; },
+            [&](int k, int c) { return j0 + c < m ? P[(size_t)k * m + j0 + c] : 0.0; }, acc);
+    } else if (WHAT == kProdP2) {
+        tile_product<true, true>(
+            S, m, [&](int r, int k) { return i0 + r < np ? P[(size_t)(i0 + r) * m + k] : 0.0; },
+            [&](int k, int c) { return j0 + c < m ? B.G[0][(size_t)(j0 + c) * m + k] : 0.0; }, acc);
+    } else {
+        tile_product<true, false>(
+            S, np, [&](int r, int k) { return i0 + r < np ? E[(size_t)(i0 + r) * np + k] : 0.0; },
+            [&](int k, int c) { return j0 + c < m ? P[(size_t)k * m + j0 + c] : 0.0; }, acc);
+    }
+    const int t = threadIdx.x, r0 = i0 + (t >> 3) * 4, c0 = j0 + (t & 7) * 4;
+    unsigned long long worst = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = r0 + i, c = c0 + j;
+            if (r >= rows || c >= cols) continue;
+            const double v = acc[i][j];
+            if (WHAT == kProdG) {
+                B.G[0][(size_t)r * np + c] = v;
+            } else if (WHAT == kProdP0) {
+                B.T[(size_t)r * m + c] = v;
+            } else if (WHAT == kProdE) {
+                const double e = (r == c ? 1.0 : 0.0) - v;
+                E[(size_t)r * np + c] = e;
+                const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(e));
+                worst = worst > bits ? worst : bits;  // (a NaN's bits are above all)
+            } else if (WHAT == kProdW) {
+                B.G[0][(size_t)r * m + c] = v;
+            } else if (WHAT == kProdP2) {
+                next[(size_t)r * m + c] = v;
+            } else {
+                next[(size_t)r * m + c] = P[(size_t)r * m + c] + v;
+            }
+        }
+    if (WHAT == kProdE) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, worst, o);
+            worst = worst > v ? worst : v;
+        }
+        if ((t & 31) == 0) atomicMax(B.err, worst);
+    }
+}
+
+// Blocked Gauss-Jordan inversion of each body's G (positive definite: no pivoting),
+// one 32-column block per step and grid barrier, from G[step & 1] to the other:
+// with D the inverse of the diagonal block (every block of threads forms it, a
+// barrier less), tile (i, j) -> G_ij - (G_ik D) G_kj, row k -> D G_kj, column k ->
+// -G_ik D, the diagonal block -> D.  Beyond np the matrix is the identity.  Four
+// groups of 64 threads take a tile each.
+constexpr int kGjGroups = 4;
+struct GjTile {
+    double u[kTile][kTile + 1], v[kTile][kTile + 1];
+};
+struct GjShared {
+    double d[kTile][kTile + 1];
+    GjTile t[kGjGroups];
+};
+__device__ __forceinline__ void gj_barrier(int group) {  // the group's 64 threads
+    asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory");
+}
+__device__ __forceinline__ void gj_product(const double (*x)[kTile + 1], const double (*y)[kTile + 1],
+                                           int r0, int c0, double (&acc)[4][4]) {
+#pragma unroll 4
+    for (int k = 0; k < kTile; ++k) {
+        double a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            a[i] = x[r0 + i][k];
+            b[i] = y[k][c0 + i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+    }
+}
+__global__ void __launch_bounds__(kTileThreads * kGjGroups) k_pinv_invert(const __grid_constant__ PinvGroup Q) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    GjShared& S = *reinterpret_cast<GjShared*>(s_raw);
+    cg::grid_group grid = cg::this_grid();
+    int which = 0;
+    while (which + 1 < Q.nb && (int)blockIdx.x >= Q.b[which + 1].block0) ++which;
+    const PinvBody& B = Q.b[which];
+    const int np = B.np, nt = B.steps;
+    const int tid = threadIdx.x, group = tid / kTileThreads, t = tid % kTileThreads;
+    const int first = ((int)blockIdx.x - B.block0) * kGjGroups + group, stride = B.blocks * kGjGroups;
+    GjTile& W = S.t[group];
+    const int r0 = (t >> 3) * 4, c0 = (t & 7) * 4;
+    for (int step = 0; step < Q.steps; ++step) {
+        if (step < nt) {
+            // (__ldcg: written by other SMs during this launch)
+            const double* G = B.G[step & 1];
+            auto from = [&](int r, int c) {
+                return r < np && c < np ? __ldcg(&G[(size_t)r * np + c]) : (r == c ? 1.0 : 0.0);
+            };
+            double* to = B.G[(step + 1) & 1];
+            const int k0 = step * kTile;
+            if (tid < 32) {  // lane: column of the diagonal block
+                double d[kTile];
+#pragma unroll
+                for (int i = 0; i < kTile; ++i) d[i] = from(k0 + i, k0 + tid);
+#pragma unroll
+                for (int k = 0; k < kTile; ++k) {
+                    const double p = 1.0 / __shfl_sync(0xffffffffu, d[k], k);
+                    const double row = tid == k ? p : d[k] * p;
+#pragma unroll
+                    for (int i = 0; i < kTile; ++i) {
+                        if (i == k) continue;
+                        const double f = __shfl_sync(0xffffffffu, d[i], k);
+                        d[i] = tid == k ? -f * p : fma(-f, row, d[i]);
+                    }
+                    d[k] = row;
+                }
+#pragma unroll
+                for (int i = 0; i < kTile; ++i) S.d[i][tid] = d[i];
+            }
+            __syncthreads();
+            for (int q = first; q < nt * nt; q += stride) {
+                const int ti = q / nt, tj = q % nt;
+                const int i0 = ti * kTile, j0 = tj * kTile;
+                gj_barrier(group);
+                for (int e = t; e < kTile * kTile; e += kTileThreads) {
+                    const int r = e / kTile, c = e % kTile;
+                    W.u[r][c] = from(i0 + r, k0 + c);
+                    W.v[r][c] = from(k0 + r, j0 + c);
+                }
+                gj_barrier(group);
+                double acc[4][4] = {};
+                if (ti == step && tj == step) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[i][j] = S.d[r0 + i][c0 + j];
+                } else if (ti == step) {
+                    gj_product(S.d, W.v, r0, c0, acc);
+                } else {
+                    gj_product(W.u, S.d, r0, c0, acc);  // G_ik D
+                    if (tj == step) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) acc[i][j] = -acc[i][j];
+                    } else {
+                        gj_barrier(group);  // every thread has read u
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                W.u[r0 + i][c0 + j] = -acc[i][j];
+                                acc[i][j] = from(i0 + r0 + i, j0 + c0 + j);
+                            }
+                        gj_barrier(group);
+                        gj_product(W.u, W.v, r0, c0, acc);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (i0 + r0 + i < np && j0 + c0 + j < np)
+                            to[(size_t)(i0 + r0 + i) * np + j0 + c0 + j] = acc[i][j];
+            }
+        }
+        if (step + 1 < Q.steps) grid.sync();
+    }
+}
+
+// ---- Householder QR of A (column-major, m = np+1 rows), for nearly singular A ------------------------
 // M holds [A | Q^T]: columns 0..np-1 are A (overwritten by R on and above the
 // diagonal), columns np..np+m-1 receive Q^T.  Both paths are one cooperative
 // launch with one grid barrier per Householder step (a chain of np dependent
@@ -977,7 +1283,8 @@ void influence_matrix(const double* xp, const double* zp, const double* xc, cons
 
 size_t pseudo_inverse_work_doubles(int np) {
     const size_t m = (size_t)np + 1;
-    return m * (np + m) + 2 * m + 2 * (size_t)np + 8;
+    // Householder: [A | Q^T] and reflectors; else two G, T and the errors
+    return 2 * (size_t)np * np + m * (np + m) + 2 * m + 2 * (size_t)np + 8;
 }
 
 namespace {
@@ -1041,11 +1348,10 @@ cudaError_t qr_general(const QrBody& b, int sms, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-}  // namespace
-
-cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, double* const* P,
-                                double* const* work, cudaStream_t s, int* launches) {
-    int nl = 0;  // QR-stage launches (the loads of [A | I] are counted by the caller)
+// P = R^-1 Q^T for n bodies; *launches grows by the number of kernels.
+cudaError_t householder_many(int n, const double* const* A, const int* np, double* const* P,
+                             double* const* work, cudaStream_t s, int* launches) {
+    int nl = n;  // the loads of [A | I]
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1094,8 +1400,131 @@ cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, do
         if (e != cudaSuccess) return e;
         nl += 3;
     }
-    if (launches) *launches = nl;
+    *launches += nl;
     return cudaGetLastError();
+}
+
+template <int WHAT>
+void pinv_product(const PinvGroup& Q, int max_np, cudaStream_t s) {
+    const int t = max_np / kTile + 1;  // tiles of np, and of m = np + 1
+    k_pinv_product<WHAT><<<dim3(t * t, Q.nb), kTileThreads, 0, s>>>(Q);
+}
+
+}  // namespace
+
+cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, double* const* P,
+                                double* const* work, const double* cond, cudaStream_t s,
+                                int* launches) {
+    int nl = 0;
+    std::vector<const double*> hA, gA;  // Householder, Gauss-Jordan
+    std::vector<double*> hP, hw, gP, gw;
+    std::vector<int> hn, gn;
+    auto householder = [&](const double* a, int m, double* p, double* w) {
+        hA.push_back(a);
+        hn.push_back(m);
+        hP.push_back(p);
+        hw.push_back(w);
+    };
+    for (int i = 0; i < n; ++i) {
+        if (cond[i] > (np[i] < kThinSmall ? kThinCondSmall : kThinCond)) {
+            householder(A[i], np[i], P[i], work[i]);
+            continue;
+        }
+        gA.push_back(A[i]);
+        gn.push_back(np[i]);
+        gP.push_back(P[i]);
+        gw.push_back(work[i]);
+    }
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(k_pinv_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GjShared));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pinv_invert, kTileThreads * kGjGroups,
+                                                  sizeof(GjShared));
+    if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+    const int most = sms;  // blocks of the inversion, all resident, one per SM
+    const int ng = (int)gA.size();
+    for (int first = 0; first < ng; first += kPinvMaxBodies) {
+        PinvGroup Q{};
+        Q.nb = std::min(kPinvMaxBodies, ng - first);
+        const size_t np_m0 = (size_t)gn[first] * (gn[first] + 1);
+        int max_np = 0, wanted = 0, want[kPinvMaxBodies];
+        for (int i = 0; i < Q.nb; ++i) {
+            PinvBody& b = Q.b[i];
+            b.np = gn[first + i];
+            const int nt = b.steps = (b.np + kTile - 1) / kTile;
+            b.A = gA[first + i];
+            b.P = gP[first + i];
+            const size_t np_m = (size_t)b.np * (b.np + 1);
+            b.G[0] = gw[first + i];
+            b.G[1] = b.G[0] + np_m;
+            b.T = b.G[1] + np_m + b.np + 1;  // (W is m x m)
+            b.err = reinterpret_cast<unsigned long long*>(Q.b[0].T + np_m0) + i;
+            max_np = std::max(max_np, b.np);
+            Q.steps = std::max(Q.steps, nt);
+            want[i] = std::max(1, (nt * nt + kGjGroups - 1) / kGjGroups);
+            wanted += want[i];
+        }
+        cudaMemsetAsync(Q.b[0].err, 0, 8 * Q.nb, s);
+        int blocks = 0;  // shared out by tiles; a body's arithmetic does not depend on its share
+        for (int i = 0; i < Q.nb; ++i) {
+            PinvBody& b = Q.b[i];
+            b.block0 = blocks;
+            b.blocks = wanted <= most ? want[i]
+                                      : std::max(1, (int)((int64_t)want[i] * (most - Q.nb) / wanted));
+            blocks += b.blocks;
+        }
+        pinv_product<kProdG>(Q, max_np, s);
+        void* args[] = {&Q};
+        cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_pinv_invert), dim3(blocks),
+                                                    dim3(kTileThreads * kGjGroups), args, sizeof(GjShared), s);
+        if (e != cudaSuccess) return e;
+        pinv_product<kProdP0>(Q, max_np, s);
+        nl += 3;
+        // Newton-Schulz steps until every body's residual was small enough before one;
+        // a body that is done, or lost, drops out.
+        PinvGroup R = Q, polish{};
+        for (int it = 0; R.nb > 0; ++it) {
+            pinv_product<kProdE>(R, max_np, s);
+            pinv_product<kProdP1>(R, max_np, s);
+            nl += 2;
+            unsigned long long bits[kPinvMaxBodies];
+            cudaMemcpyAsync(bits, Q.b[0].err, 8 * Q.nb, cudaMemcpyDeviceToHost, s);
+            e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return e;
+            cudaMemsetAsync(Q.b[0].err, 0, 8 * Q.nb, s);
+            PinvGroup next{};
+            next.steps = R.steps;
+            for (int i = 0; i < R.nb; ++i) {
+                PinvBody& b = R.b[i];
+                b.in_p ^= 1;
+                double worst;
+                std::memcpy(&worst, &bits[b.err - Q.b[0].err], 8);
+                if (worst <= kSchulzDone) {
+                    if (it > 0 || worst > kSchulzExact) polish.b[polish.nb++] = b;
+                } else if (worst <= kSchulzStart && it < 6) {
+                    next.b[next.nb++] = b;
+                } else {
+                    householder(b.A, b.np, b.P, b.G[0]);
+                }
+            }
+            R = next;
+        }
+        if (polish.nb > 0) {
+            pinv_product<kProdW>(polish, max_np, s);
+            pinv_product<kProdP2>(polish, max_np, s);
+            nl += 2;
+            for (int i = 0; i < polish.nb; ++i) {
+                const PinvBody& b = polish.b[i];
+                if (b.in_p)  // the last one is in T
+                    cudaMemcpyAsync(b.P, b.T, sizeof(double) * b.np * (size_t)(b.np + 1),
+                                    cudaMemcpyDeviceToDevice, s);
+            }
+        }
+    }
+    const cudaError_t e = householder_many((int)hA.size(), hA.data(), hn.data(), hP.data(), hw.data(), s, &nl);
+    if (launches) *launches = nl;
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
