@@ -96,7 +96,7 @@ __global__ void k_assemble_A(const double* __restrict__ p, const double* __restr
 // All of it is matrix products in 32 x 32 tiles and np / 32 dependent steps of the
 // inversion, where a Householder factorisation is np dependent steps with a grid
 // barrier each: dvm_sim_create at 64, 512, 1024 and 2048 panels 0.25, 1.9, 10.0 and
-// 98 ms -> 0.19, 0.99, 2.8 and 13 ms; eight bodies of 512 8.6 -> 2.6 ms.
+// 98 ms -> 0.15, 0.62, 1.9 and 9.8 ms; eight bodies of 512 8.6 -> 2.1 ms.
 constexpr int kTile = 32;
 constexpr int kTileThreads = 64;  // 8 x 8 threads with 4 x 4 outputs each
 constexpr int kTileDepth = 16;
@@ -264,13 +264,17 @@ __global__ void __launch_bounds__(kTileThreads) k_pinv_product(const __grid_cons
 // with D the inverse of the diagonal block (every block of threads forms it, a
 // barrier less), tile (i, j) -> G_ij - (G_ik D) G_kj, row k -> D G_kj, column k ->
 // -G_ik D, the diagonal block -> D.  Beyond np the matrix is the identity.  Four
-// groups of 64 threads take a tile each.
+// groups of 64 threads take tiles that follow one another, so G_ik D is formed once a
+// row.  The diagonal block's chain of 32 pivots bounds a step: by one warp with its
+// columns in registers (straight code too long for the instruction cache) 43 us a
+// step, by the whole block through shared memory 20 us (4 bodies of 512 panels).
 constexpr int kGjGroups = 4;
 struct GjTile {
     double u[kTile][kTile + 1], v[kTile][kTile + 1];
 };
 struct GjShared {
     double d[kTile][kTile + 1];
+    double row[2][kTile], col[2][kTile];
     GjTile t[kGjGroups];
 };
 __device__ __forceinline__ void gj_barrier(int group) {  // the group's 64 threads
@@ -301,7 +305,9 @@ __global__ void __launch_bounds__(kTileThreads * kGjGroups) k_pinv_invert(const 
     const PinvBody& B = Q.b[which];
     const int np = B.np, nt = B.steps;
     const int tid = threadIdx.x, group = tid / kTileThreads, t = tid % kTileThreads;
-    const int first = ((int)blockIdx.x - B.block0) * kGjGroups + group, stride = B.blocks * kGjGroups;
+    // a group's tiles follow one another, mostly in one row
+    const int g = ((int)blockIdx.x - B.block0) * kGjGroups + group, ng = B.blocks * kGjGroups;
+    const int q0 = nt * nt * g / ng, q1 = nt * nt * (g + 1) / ng;
     GjTile& W = S.t[group];
     const int r0 = (t >> 3) * 4, c0 = (t & 7) * 4;
     for (int step = 0; step < Q.steps; ++step) {
@@ -313,63 +319,66 @@ __global__ void __launch_bounds__(kTileThreads * kGjGroups) k_pinv_invert(const 
             };
             double* to = B.G[(step + 1) & 1];
             const int k0 = step * kTile;
-            if (tid < 32) {  // lane: column of the diagonal block
-                double d[kTile];
+            {  // Gauss-Jordan on the diagonal block: a thread holds four of a row
+                const int r = tid >> 3, c = (tid & 7) * 4;
+                double d[4];
 #pragma unroll
-                for (int i = 0; i < kTile; ++i) d[i] = from(k0 + i, k0 + tid);
-#pragma unroll
+                for (int j = 0; j < 4; ++j) d[j] = from(k0 + r, k0 + c + j);
+#pragma unroll 1
                 for (int k = 0; k < kTile; ++k) {
-                    const double p = 1.0 / __shfl_sync(0xffffffffu, d[k], k);
-                    const double row = tid == k ? p : d[k] * p;
+                    double* row = S.row[k & 1];
+                    double* col = S.col[k & 1];
 #pragma unroll
-                    for (int i = 0; i < kTile; ++i) {
-                        if (i == k) continue;
-                        const double f = __shfl_sync(0xffffffffu, d[i], k);
-                        d[i] = tid == k ? -f * p : fma(-f, row, d[i]);
+                    for (int j = 0; j < 4; ++j) {
+                        if (r == k) row[c + j] = d[j];
+                        if (c + j == k) col[r] = d[j];
                     }
-                    d[k] = row;
+                    __syncthreads();  // (the buffers of the step before are free after it)
+                    const double p = 1.0 / row[k], f = col[r];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const double x = c + j == k ? p : row[c + j] * p;
+                        d[j] = r == k ? x : c + j == k ? -f * p : fma(-f, x, d[j]);
+                    }
                 }
 #pragma unroll
-                for (int i = 0; i < kTile; ++i) S.d[i][tid] = d[i];
+                for (int j = 0; j < 4; ++j) S.d[r][c + j] = d[j];
             }
             __syncthreads();
-            for (int q = first; q < nt * nt; q += stride) {
-                const int ti = q / nt, tj = q % nt;
-                const int i0 = ti * kTile, j0 = tj * kTile;
-                gj_barrier(group);
-                for (int e = t; e < kTile * kTile; e += kTileThreads) {
-                    const int r = e / kTile, c = e % kTile;
-                    W.u[r][c] = from(i0 + r, k0 + c);
-                    W.v[r][c] = from(k0 + r, j0 + c);
-                }
-                gj_barrier(group);
+            int have = -1;  // W.u holds -G_ik D of this row of tiles
+            for (int q = q0; q < q1; ++q) {
+                const int ti = q / nt, tj = q % nt, i0 = ti * kTile, j0 = tj * kTile;
                 double acc[4][4] = {};
-                if (ti == step && tj == step) {
+                if (ti != step && ti != have) {
+                    gj_barrier(group);
+                    for (int e = t; e < kTile * kTile; e += kTileThreads)
+                        W.u[e / kTile][e % kTile] = from(i0 + e / kTile, k0 + e % kTile);
+                    gj_barrier(group);
+                    gj_product(W.u, S.d, r0, c0, acc);
+                    gj_barrier(group);
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) acc[i][j] = S.d[r0 + i][c0 + j];
-                } else if (ti == step) {
-                    gj_product(S.d, W.v, r0, c0, acc);
+                        for (int j = 0; j < 4; ++j) W.u[r0 + i][c0 + j] = -acc[i][j];
+                    have = ti;
+                }
+                const double (*x)[kTile + 1] = ti == step ? S.d : W.u;
+                if (tj == step) {  // (the thread's own entries of u)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[i][j] = x[r0 + i][c0 + j];
                 } else {
-                    gj_product(W.u, S.d, r0, c0, acc);  // G_ik D
-                    if (tj == step) {
+                    gj_barrier(group);
+                    for (int e = t; e < kTile * kTile; e += kTileThreads)
+                        W.v[e / kTile][e % kTile] = from(k0 + e / kTile, j0 + e % kTile);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) acc[i][j] = -acc[i][j];
-                    } else {
-                        gj_barrier(group);  // every thread has read u
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                W.u[r0 + i][c0 + j] = -acc[i][j];
-                                acc[i][j] = from(i0 + r0 + i, j0 + c0 + j);
-                            }
-                        gj_barrier(group);
-                        gj_product(W.u, W.v, r0, c0, acc);
-                    }
+                        for (int j = 0; j < 4; ++j)
+                            acc[i][j] = ti == step ? 0.0 : from(i0 + r0 + i, j0 + c0 + j);
+                    gj_barrier(group);
+                    gj_product(x, W.v, r0, c0, acc);
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
