@@ -1007,12 +1007,15 @@ __device__ __forceinline__ void sheet_store(const InstDesc& d, uint32_t i, doubl
     }
 }
 
-// FP64 simulations: every panel term.  A work item is 64 blobs, four threads per
-// blob with a quarter of the panels each (their sums added in order): with two
-// blobs per thread and all panels in turn, a simulation of 2000 blobs was four
-// blocks' work (222 us a call at 128 panels; 49 now).
-constexpr uint32_t kSheetItem = 64;
-constexpr int kSheetParts = 4;
+// FP64 simulations: every panel term.  A work item is 16 blobs, 16 threads per blob
+// with a sixteenth of the panels each (their sums added in order): a thread's chain
+// of logarithms and arctangents bounds a call until the items fill the chip some
+// times over.  128 panels and 2000, 5000, 20 000, 100 000 blobs, a call: items of 64
+// blobs and four threads each 49, 61, 62, 166 us, of 32 and eight 39, 40, 52, 165,
+// of 16 and 16 28, 29, 50, 167; two blobs per thread and all panels in turn 222 us
+// at 2000.
+constexpr uint32_t kSheetItem = 16;
+constexpr int kSheetParts = 16;
 constexpr size_t kSheetSmemPerPanel = 72;  // nine FP64 arrays
 
 __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restrict__ table,
