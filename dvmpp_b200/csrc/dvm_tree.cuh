@@ -282,11 +282,6 @@ struct BinomialTable {
 };
 static __device__ const BinomialTable g_binomial = BinomialTable();
 
-__device__ __forceinline__ void binomial_row(double (&row)[kTerms], int l) {
-#pragma unroll
-    for (int k = 0; k < kTerms; ++k) row[k] = __ldg(&g_binomial.c[k][l]);
-}
-
 // Value of a node's moments at an offset (dx, dz) from its centre outside
 // R / kTheta; A: the moments in shared memory.
 __device__ __forceinline__ Cplx moment_value(const Cplx* __restrict__ A, double s, double dx,
@@ -301,10 +296,13 @@ __device__ __forceinline__ Cplx moment_value(const Cplx* __restrict__ A, double 
 
 // Moment-to-local translations by a warp, kBatch nodes at a time.  Four lanes per
 // node first write c_k = a_k (s_node / d)^k and f_l = (-s_group / d)^l / d to
-// shared memory, a quarter of the powers each; then lane l adds f_l times its row
-// of the translation matrix times c, two nodes side by side.  (Forming both powers
-// in every lane for one node at a time took 500 instructions per node, walk
-// included; this takes 210, 36 % of them FP64.)
+// shared memory, a quarter of the powers each; then the constant translation matrix
+// times the c of four nodes (real and imaginary parts: eight columns) goes to the
+// FP64 matrix instruction, and a lane adds f_l times its share.  Every lane with
+// a row of the matrix in registers, multiplying two nodes' c read from shared memory,
+// was bound by those reads (82 % of the L1 pipe, FP64 34 %): k_far at 262 144 blobs 146
+// us against 98, where latency bounds it (four warps per scheduler).  One buffer for c
+// and f, for a fifth, spills: 125 us.
 constexpr int kBatch = 8;
 constexpr int kPowStride = kTerms + 1;  // 400-byte rows: the quarters' stores meet no bank twice
 struct TransBuf {
@@ -312,12 +310,56 @@ struct TransBuf {
     Cplx f[kBatch][kPowStride];
 };
 
+// The lane's entries of the translation matrix, as m8n8k4 takes them: rows l = 8 i +
+// lane / 4, columns k = 6 (lane % 4) + s (any order of the k will do, the same for c;
+// this one reads c without bank conflicts).
+struct Binomials {
+    double a[kTerms / 8][kTerms / 4];
+};
+__device__ __forceinline__ Binomials binomials(int lane) {
+    Binomials t;
+#pragma unroll
+    for (int i = 0; i < kTerms / 8; ++i)
+#pragma unroll
+        for (int s = 0; s < kTerms / 4; ++s)
+            t.a[i][s] = __ldg(&g_binomial.c[(lane & 3) * (kTerms / 4) + s][8 * i + (lane >> 2)]);
+    return t;
+}
+
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+// A local expansion while it is summed: coefficient 8 i + lane / 4, the share of the
+// nodes at places lane % 4 (mod 4) of their batches.
+struct LocalSum {
+    Cplx b[kTerms / 8];
+};
+// Lane l < kTerms: coefficient l.
+__device__ __forceinline__ Cplx local_total(const LocalSum& t, int lane) {
+    Cplx out{0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < kTerms / 8; ++i) {
+        Cplx v = t.b[i];
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        const Cplx w = cshfl(v, (lane & 7) << 2);
+        if ((lane >> 3) == i) out = w;
+    }
+    return out;
+}
+
 // Nodes list[0 .. cnt), cnt <= kBatch; N, mom: the simulation's.
 __device__ __forceinline__ void translate(const TreeNode* __restrict__ N,
                                           const double2* __restrict__ mom, uint32_t C,
                                           const uint32_t* __restrict__ list, int cnt,
-                                          const TargetBox& t, const double (&row)[kTerms],
-                                          TransBuf& buf, int lane, Cplx& b) {
+                                          const TargetBox& t, const Binomials& mat,
+                                          TransBuf& buf, int lane, LocalSum& sum) {
     constexpr int Q = kTerms / 4;
     const int n = lane >> 2, part = lane & 3;
     __syncwarp();  // the previous batch's reads
@@ -350,23 +392,25 @@ __device__ __forceinline__ void translate(const TreeNode* __restrict__ N,
             pn = cmul(pn, qn);
             pt = cmul(pt, qt);
         }
+    } else if (n < ((cnt + 3) & ~3)) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) buf.c[n][part * Q + k] = buf.f[n][part * Q + k] = Cplx{0.0, 0.0};
     }
     __syncwarp();
-    for (int q = 0; q < cnt; q += 2) {  // two nodes side by side (an odd last one twice, once unused)
-        const int p = min(q + 1, cnt - 1);
-        Cplx s0{0.0, 0.0}, s1{0.0, 0.0};
 #pragma unroll
-        for (int k = 0; k < kTerms; ++k) {
-            const Cplx c0 = buf.c[q][k], c1 = buf.c[p][k];
-            s0.x = fma(row[k], c0.x, s0.x);
-            s0.y = fma(row[k], c0.y, s0.y);
-            s1.x = fma(row[k], c1.x, s1.x);
-            s1.y = fma(row[k], c1.y, s1.y);
+    for (int j = 0; j < kBatch / 4; ++j) {
+        if (4 * j >= cnt) break;
+        const Cplx* c = &buf.c[4 * j + (lane >> 3)][part * Q];
+        double d[kTerms / 8][2] = {};
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            const double v = (lane & 4) ? c[s].y : c[s].x;
+#pragma unroll
+            for (int i = 0; i < kTerms / 8; ++i) mma_f64(d[i], mat.a[i][s], v);
         }
-        if (lane < kTerms) {
-            b = cfma(s0, buf.f[q][lane], b);
-            if (p > q) b = cfma(s1, buf.f[p][lane], b);
-        }
+#pragma unroll
+        for (int i = 0; i < kTerms / 8; ++i)
+            sum.b[i] = cfma(Cplx{d[i][0], d[i][1]}, buf.f[4 * j + part][8 * i + n], sum.b[i]);
     }
 }
 

@@ -657,7 +657,7 @@ __device__ __forceinline__ void kahan(float& s, float& c, float x) {
 // that reach over hundreds of leaves) has kNearOver as its count, and k_self_f32
 // walks again.
 constexpr int kFarWarps = 4;
-constexpr int kFarBlocks = 4;  // blocks per SM (the translation matrix's row: 48 registers)
+constexpr int kFarBlocks = 4;  // blocks per SM (the translation matrix: 36 registers)
 constexpr int kFarList = 64;   // at least kBatch + 32
 struct FarShared {
     TreeWalk walk;
@@ -686,8 +686,7 @@ __global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
     const unsigned total = s_pre[nlist];
     const int lane = threadIdx.x & 31;
     FarShared& S = reinterpret_cast<FarShared*>(s_far)[threadIdx.x >> 5];
-    double row[kTerms];
-    binomial_row(row, lane);
+    const Binomials mat = binomials(lane);
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(work, 1u);
@@ -710,7 +709,7 @@ __global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
         int sp = walk_begin(S.walk, N, C, nl, level, idx, c == 0 ? (int)min((uint32_t)kLeaf, n - t0) : 0,
                             S.at, lane);
         const TargetBox tb = S.walk.chain[0];
-        Cplx b{0.0, 0.0};  // lane l: local coefficient l
+        LocalSum sum{};
         int nfar = 0, nnear = 0, nmid = 0;
         while (sp > 0) {
             uint32_t id;
@@ -731,9 +730,10 @@ __global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
             while (nfar >= kBatch || (sp == 0 && nfar > 0)) {  // from the list's end
                 const int m = min(kBatch, nfar);
                 nfar -= m;
-                translate(N, A, C, S.far + nfar, m, tb, row, S.buf, lane, b);
+                translate(N, A, C, S.far + nfar, m, tb, mat, S.buf, lane, sum);
             }
         }
+        const Cplx b = local_total(sum, lane);
         if (lane < kTerms)
             loc[(e.noff + node_level(C, level) + idx) * kTerms + lane] = make_double2(b.x, b.y);
         if (row_out && lane == 0) {
@@ -1505,9 +1505,8 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     const uint64_t TXH = f2pack(txh, txh), TXL = f2pack(txl, txl);
     const uint64_t TZH = f2pack(tzh, tzh), TZL = f2pack(tzl, tzl);
     __syncthreads();
-    double row[kTerms];
-    binomial_row(row, lane);
-    Cplx b{0.0, 0.0};            // lane l: local coefficient l, this warp's share
+    const Binomials mat = binomials(lane);
+    LocalSum sum{};              // this warp's share
     double nu = 0.0, sw = 0.0;   // -u and w at the lane's point, near and mid
     int sp = nl ? walk_begin(W.walk, nl, tb, kWalkTop, (uint32_t)wid, kRhsWarps, lane) : 0;
     int nfar = 0;
@@ -1522,7 +1521,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
         while (nfar >= kBatch || (sp == 0 && nfar > 0)) {
             const int m = min(kBatch, nfar);
             nfar -= m;
-            translate(N, A, C, W.far + nfar, m, tb, row, W.buf, lane, b);
+            translate(N, A, C, W.far + nfar, m, tb, mat, W.buf, lane, sum);
         }
         for (unsigned todo = __ballot_sync(all, kind == kWalkMid); todo; todo &= todo - 1) {
             const uint32_t q = __shfl_sync(all, id, __ffs(todo) - 1);
@@ -1586,6 +1585,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     }
     __syncwarp();
     W.sum[lane] = make_double2(nu, sw);
+    Cplx b = local_total(sum, lane);
     if (lane < kTerms) W.buf.c[0][lane] = b;
     __syncthreads();
     if (wid != 0) return;

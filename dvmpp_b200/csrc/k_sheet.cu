@@ -1115,8 +1115,7 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
     const unsigned total = s_pre[nlist], all = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[threadIdx.x >> 5];
-    double row[kTerms];
-    binomial_row(row, lane);
+    const Binomials mat = binomials(lane);
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(work, 1u);
@@ -1136,7 +1135,7 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
         tb.n = (int)min((uint32_t)kLeaf, n - t0);
         tb.at = S.at;
         const double2 pa = S.at[lane], pb = S.at[lane + 32];
-        Cplx b{0.0, 0.0};
+        LocalSum sum{};
         double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
         int sp = walk_begin(S.walk, nl, tb, 1u, 0u, 1u, lane), nfar = 0;
         bool any_far = false;
@@ -1152,7 +1151,7 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
             while (nfar >= kBatch || (sp == 0 && nfar > 0)) {
                 const int m = min(kBatch, nfar);
                 nfar -= m;
-                translate(N, A, C, S.far + nfar, m, tb, row, S.buf, lane, b);
+                translate(N, A, C, S.far + nfar, m, tb, mat, S.buf, lane, sum);
             }
             for (unsigned todo = __ballot_sync(all, kind == kWalkMid); todo; todo &= todo - 1) {
                 const uint32_t q = __shfl_sync(all, id, __ffs(todo) - 1);
@@ -1180,6 +1179,7 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
             }
         }
         if (any_far) {  // warp-uniform
+            const Cplx b = local_total(sum, lane);
             __syncwarp();
             if (lane < kTerms) S.buf.c[0][lane] = b;
             __syncwarp();
