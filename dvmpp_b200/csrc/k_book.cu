@@ -256,44 +256,52 @@ __device__ __forceinline__ void load_contour(const InstDesc& d, double* sx, doub
 // items of 256 or 1024, each warp going through its own 32, they were one or a few
 // blocks' work (1024 panels, RK3, DELETE: 231 us, 31 now; 128 panels, 2 k blobs,
 // REFLECT: 22-43 us, 12-29 now).
-constexpr uint32_t kCrossItem = 64;
+// An item costs four barriers and a counter's turn, though, so from 2^20 blobs
+// (capacity) on, where there are plenty of them, items are 256 (4 M blobs, REFLECT
+// and the whole DELETE: 0.51 and 0.56 ms in items of 64, 0.24 and 0.38 in these).
+constexpr uint32_t kCrossItem = 64, kCrossMost = 256;
+constexpr uint64_t kCrossLarge = 1u << 20;
+template <int ITEM>
 struct CrossQueue {
-    double2 at[kCrossItem];
-    uint32_t slot[kCrossItem];
+    double2 at[ITEM];
+    uint32_t slot[ITEM];
     uint32_t count;
 };
 
-// Fills the queue from blobs i0 .. i0 + 63 (every thread calls it; ends with a
+// Fills the queue from blobs i0 .. i0 + ITEM - 1 (every thread calls it; ends with a
 // barrier).
-__device__ __forceinline__ void cross_candidates(CrossQueue& Q, const InstDesc& d, uint32_t i0,
+template <int ITEM>
+__device__ __forceinline__ void cross_candidates(CrossQueue<ITEM>& Q, const InstDesc& d, uint32_t i0,
                                                  uint32_t n) {
     if (threadIdx.x == 0) Q.count = 0;
     __syncthreads();
-    if (threadIdx.x < kCrossItem) {
-        const uint32_t i = i0 + threadIdx.x;
+#pragma unroll
+    for (uint32_t t = threadIdx.x; t < ITEM; t += 256) {
+        const uint32_t i = i0 + t;
         const bool valid = i < n;
         const double px = valid ? d.x[i] : 0.0, pz = valid ? d.z[i] : 0.0;
         if (valid && in_bbox(d, px, pz)) {
             const uint32_t q = atomicAdd(&Q.count, 1u);  // (their order does not matter)
             Q.at[q] = make_double2(px, pz);
-            Q.slot[q] = threadIdx.x;
+            Q.slot[q] = t;
         }
     }
     __syncthreads();
 }
 
 // REFLECT / ABSORB (src/VortexSheet.cpp:345-405): each blob moves independently.
+template <int ITEM>
 __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ table,
                                                  const InstState* __restrict__ st,
                                                  const ListEntry* __restrict__ list, int nlist,
                                                  unsigned* __restrict__ work) {
     extern __shared__ double s_c[];
     __shared__ unsigned s_pre[1025];
-    __shared__ CrossQueue Q;
+    __shared__ CrossQueue<ITEM> Q;
     __shared__ unsigned s_item;
     list_prefix(s_pre, nlist, [&](int k) {
         const InstState& S = st[list[k].inst];
-        return S.status ? 0u : (S.n + kCrossItem - 1) / kCrossItem;
+        return S.status ? 0u : (S.n + ITEM - 1) / ITEM;
     });
     const unsigned total = s_pre[nlist];
     int loaded = -1;
@@ -310,7 +318,7 @@ __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ ta
         double* sz = sx + (np + 1);
         double* snx = sz + (np + 1);
         double* snz = snx + np;
-        const uint32_t i0 = (item - s_pre[k]) * kCrossItem;
+        const uint32_t i0 = (item - s_pre[k]) * ITEM;
         cross_candidates(Q, d, i0, st[e.inst].n);
         const uint32_t count = Q.count;
         if (count && loaded != k) {  // block-uniform
@@ -371,6 +379,7 @@ __global__ void __launch_bounds__(256) k_reflect(const InstDesc* __restrict__ ta
 // (tile_counts starts at zero).
 constexpr int kDelTile = 1024;
 
+template <int ITEM>
 __global__ void __launch_bounds__(256) k_del_flags(const InstDesc* __restrict__ table,
                                                    const InstState* __restrict__ st,
                                                    const ListEntry* __restrict__ list, int nlist,
@@ -379,12 +388,12 @@ __global__ void __launch_bounds__(256) k_del_flags(const InstDesc* __restrict__ 
                                                    unsigned* __restrict__ work) {
     extern __shared__ double s_c[];
     __shared__ unsigned s_pre[1025];
-    __shared__ CrossQueue Q;
-    __shared__ uint8_t s_in[kCrossItem];
+    __shared__ CrossQueue<ITEM> Q;
+    __shared__ uint8_t s_in[ITEM];
     __shared__ unsigned s_item;
     list_prefix(s_pre, nlist, [&](int k) {
         const InstState& S = st[list[k].inst];
-        return S.status ? 0u : (S.n + kCrossItem - 1) / kCrossItem;
+        return S.status ? 0u : (S.n + ITEM - 1) / ITEM;
     });
     const unsigned total = s_pre[nlist];
     int loaded = -1;
@@ -396,10 +405,10 @@ __global__ void __launch_bounds__(256) k_del_flags(const InstDesc* __restrict__ 
         const int k = locate(s_pre, nlist, item);
         const ListEntry e = list[k];
         const InstDesc& d = table[e.inst];
-        const uint32_t n = st[e.inst].n, i0 = (item - s_pre[k]) * kCrossItem;
+        const uint32_t n = st[e.inst].n, i0 = (item - s_pre[k]) * ITEM;
         double* sx = s_c;
         double* sz = sx + (d.np + 1);
-        if (threadIdx.x < kCrossItem) s_in[threadIdx.x] = 0;
+        for (uint32_t t = threadIdx.x; t < ITEM; t += 256) s_in[t] = 0;
         cross_candidates(Q, d, i0, n);
         const uint32_t count = Q.count;
         if (count && loaded != k) {  // block-uniform
@@ -415,9 +424,9 @@ __global__ void __launch_bounds__(256) k_del_flags(const InstDesc* __restrict__ 
             if ((threadIdx.x & 31) == 0 && in) s_in[Q.slot[c]] = 1;
         }
         __syncthreads();
-        if (threadIdx.x < kCrossItem) {  // two warps
-            const uint32_t i = i0 + threadIdx.x;
-            const bool keep = i < n && !s_in[threadIdx.x];
+        for (uint32_t t = threadIdx.x; t < ITEM; t += 256) {  // whole warps
+            const uint32_t i = i0 + t;
+            const bool keep = i < n && !s_in[t];
             if (i < n) flags[e.coff + i] = keep ? 1 : 0;
             const unsigned b = __ballot_sync(0xffffffffu, keep);
             if ((threadIdx.x & 31) == 0 && b)
@@ -621,9 +630,13 @@ void release(const InstDesc* table, InstState* st, const ListEntry* list, int nl
 void reflect(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, int max_np,
              const Workspace& ws, int sms, cudaStream_t s) {
     const size_t smem = contour_smem(max_np);
-    cudaFuncSetAttribute(k_reflect, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_reflect<kCrossItem>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_reflect<kCrossMost>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaMemsetAsync(ws.work + 2, 0, sizeof(unsigned), s);
-    k_reflect<<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.work + 2);
+    if (ws.total_cap > kCrossLarge)
+        k_reflect<kCrossMost><<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.work + 2);
+    else
+        k_reflect<kCrossItem><<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.work + 2);
 }
 
 void delete_inside(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
@@ -631,7 +644,11 @@ void delete_inside(const InstDesc* table, InstState* st, const ListEntry* list, 
     const size_t smem = sizeof(double) * (2 * (size_t)max_np + 2);
     cudaMemsetAsync(ws.tile_counts, 0, sizeof(uint32_t) * (ws.total_cap / kDelTile + 1), s);
     cudaMemsetAsync(ws.work + 3, 0, 2 * sizeof(unsigned), s);
-    k_del_flags<<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.flags, ws.tile_counts,
+    if (ws.total_cap > kCrossLarge)
+        k_del_flags<kCrossMost><<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.flags, ws.tile_counts,
+                                           ws.work + 4);
+    else
+        k_del_flags<kCrossItem><<<sms * 4, 256, smem, s>>>(table, st, list, nlist, ws.flags, ws.tile_counts,
                                            ws.work + 4);
     k_del_scan<<<nlist, 1024, 0, s>>>(st, list, ws.tile_counts, ws.tile_base, ws.del_kept);
     cudaMemsetAsync(ws.del_ready, 0, sizeof(uint32_t) * (ws.total_cap / kDelTile + 1), s);
