@@ -54,6 +54,15 @@ constexpr size_t kPoolPerPlan = 6144;  // list entries per plan: 4 partitions + 
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Panels x capacity up to which a call that needs the FP32 right-hand side or sheet
+// velocity alone sums all pairs rather than sort the blobs and build their tree
+// (about 150 us at 131 k blobs; both grow with the blobs, so up to 128 panels the
+// sheet never builds one).  A solve of 1024 panels and 262 k blobs by pairs 250 us, 64
+// and 131 k 81; the sheet velocity of 131 k blobs from 64, 128, 256 panels by pairs
+// 54, 76, 126 us, by the tree 190, 200, 210; from 512 and 1024 by the tree 212 and 225,
+// by pairs 271 and 365.
+constexpr uint64_t kLonePairsRhs = 1ull << 28, kLonePairsSheet = 1ull << 26;
+
 // Source chunks of a simulation's FP64 pair kernel, at most.  Fixed by the capacity
 // alone, so a simulation's sums are associated the same way alone and inside
 // any batch: one chunk per 32 k sources (up to 32); for small simulations enough
@@ -220,7 +229,7 @@ void free_plan(dvm_ctx* c, Plan* pl) {
     delete pl;
 }
 
-// Drop the plans (and graphs) whose FP32 pair lists belong to shape class cls.
+// Drop the plans (and graphs) whose FP32 lists belong to shape class cls.
 void drop_plans_of_class(dvm_ctx* c, int cls) {
     for (auto it = c->plans.begin(); it != c->plans.end();) {
         if (it->second->eul_f32.cls == cls || it->second->rk3_f32.cls == cls) {
@@ -2022,15 +2031,21 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
             prof_end(c, pr);
             break;
         }
-        case DVM_PHASE_SOLVE:
-            if (prec == kF32) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
-            sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st);
+        // (a step has the blobs' tree from their own velocities; these two would have
+        // to build one: kLonePairsRhs, kLonePairsSheet)
+        case DVM_PHASE_SOLVE: {
+            const bool pairs = (uint64_t)np * s->h.cap <= kLonePairsRhs;
+            if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st, pairs);
             sheet_solve(T, S, L, 1, np, st);
             break;
-        case DVM_PHASE_SHEETBC:
-            if (prec == kF32) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
-            sheet_velocity(T, S, L, 1, 0, np, prec, ws, c->sms, st);
+        }
+        case DVM_PHASE_SHEETBC: {
+            const bool pairs = np <= 128 || (np <= 256 && (uint64_t)np * s->h.cap <= kLonePairsSheet);
+            if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            sheet_velocity(T, S, L, 1, 0, np, prec, ws, c->sms, st, pairs);
             break;
+        }
         case DVM_PHASE_CONVECT:
             for (int k = 0; k < (s->h.scheme == kRK3 ? 3 : 1); ++k) {
                 biot_savart_self(T, S, L, 1, prec, ws, c->sms, st,

@@ -37,11 +37,7 @@ enum Scheme : int { kEuler = 0, kRK3 = 1 };
 enum Cross : int { kDelete = 0, kAbsorb = 1, kReflect = 2 };
 enum Rng : int { kInject = 0, kPhilox = 1 };
 
-// N-body tiling (targets per work item, sources per shared-memory stage).
-constexpr int kBsThreads = 256;
-constexpr int kBsR = 4;                        // consecutive targets per thread
-constexpr int kBsTT = kBsThreads * kBsR;       // 1024 targets per item
-constexpr int kBsST = 256;                     // sources per stage (= sort tile)
+constexpr int kBsST = 256;                     // blobs per sort tile (FP64 pairs, at-target sums)
 constexpr int kAtChunk = 4096;                 // sources per item of the at-target kernels
 constexpr int kCapAlign = 1024;                // capacities are multiples of this
 constexpr int kMaxBatch = 1024;                // simulations per batched step
@@ -144,7 +140,7 @@ struct InstDesc {
     double rho, nu, dt, ux, uz, cutoff_exp, Ur, area;
     double bxmax, bzmin, bzmax;     // contour bounding box (x padded) for the crossing early-out
     double bxmin;
-    double kx0, kz0, kinv;          // Morton-key domain: cell = (x - kx0) * kinv
+    double kx0, kz0, kinv;          // sort-key domain: cell = (x - kx0) * kinv
     uint32_t M;                     // max_NumPanelVort
     int np;
     int scheme, cross, rng, precision, refine;
@@ -170,7 +166,7 @@ struct ListEntry {
     int inst;          // table index
     int chunks;        // N-body source chunks (fixed by capacity)
     int rhs_chunks;    // at-target source chunks = ceil(cap / rhs_chunk)
-    int npad;          // np rounded up to kBsThreads
+    int npad;          // np rounded up to 256
     uint32_t cap;
     uint32_t rhs_chunk;  // sources per at-target work item (rhs_chunk_for)
     uint64_t coff;     // offset in the concatenated capacity space (multiple of kCapAlign)
@@ -232,11 +228,11 @@ int report_error(int code, const char* msg);
 // ---- launchers (all asynchronous on `s`) ------------------------------------
 size_t cub_sort_bytes(uint64_t total);
 
-// Launch shape of the FP32 pair kernel.  None of it changes a result: the
-// source chunking (which does) is fixed by each simulation's capacity.
+// Launch shape of the FP32 near-field kernel.  None of it changes a result: a
+// leaf's sums are grouped by its own list of near leaves.
 struct PairConfig {
-    int tile = 256;  // targets per work item (one sort tile)
-    int ctas = 4;    // persistent CTAs per SM
+    int tile = 256;  // part of the public record only (an item is a leaf of kLeaf targets)
+    int ctas = 4;    // quarters of the persistent CTAs that fit an SM
     int order = 0;   // 0: list order; 1: costliest simulations' items first (the caller
                      // passes the list in that order)
 };
@@ -260,9 +256,10 @@ void biot_savart_finish(const InstDesc* table, InstState* st, const ListEntry* l
 void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const Workspace& ws,
                 int sms, cudaStream_t s);
 // Blob-on-collocation right-hand side b (src/VortexSheet.cpp:171-210).  FP32: from
-// the tree that biot_savart_prepare has built of the same positions.
+// the tree that biot_savart_prepare has built of the same positions, or pair by pair.
 void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
-               int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s);
+               int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s,
+               bool pairs = false);
 // Velocity at arbitrary targets from one blob set (src/VelocityKernel.cpp:69-109).
 void direct_at_raw(const double* x, const double* z, const double* circ, const double* sigma,
                    uint32_t ns, const double* tx, const double* tz, uint32_t nt, double* u,
@@ -331,14 +328,14 @@ void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, in
 // Sheet-on-blob velocity (src/VortexSheet.cpp:217-273), optionally fused with
 // the convection update of the Euler / RK3 stage (src/DVMBase.cpp:167-209), for
 // sims of one precision.  FP32: over the tree that biot_savart_prepare has built
-// of the same positions.
+// of the same positions, or (pairs) over all panels.
 //   mode 0: uvs/wvs only; 1: Euler update; 2+k: RK3 stage k (k = 0,1,2)
 void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, int max_np, int precision, const Workspace& ws, int sms,
-                    cudaStream_t s);
-// The FP32 panels' tree and records from gamma (k_biot_savart.cu).
+                    cudaStream_t s, bool pairs = false);
+// The FP32 panels' tree and records (or these alone) from gamma (k_biot_savart.cu).
 void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
-                int max_np, const Workspace& ws, int sms, cudaStream_t s);
+                int max_np, const Workspace& ws, int sms, cudaStream_t s, bool records = false);
 // x += (u + uvs + Ux) dt without recomputing uvs (used by the phase API).
 void convect_update(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, const Workspace& ws, int sms, cudaStream_t s);

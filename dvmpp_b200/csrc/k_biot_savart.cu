@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                 r.ez = d.zc[p] + dsp * d.sth[p];
                 pan[e.panoff + p] = r;
             }
+            if (!nodes) continue;  // the records are all that is wanted
         }
         uint32_t next[2];  // the next leaf's blobs, ahead of its gather
 #pragma unroll
@@ -642,13 +643,6 @@ __device__ __forceinline__ void leaf_sum(const StagedLeaf& __restrict__ src,
     }
 }
 
-__device__ __forceinline__ void kahan(float& s, float& c, float x) {
-    const float y = x - c;
-    const float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
 // Local expansions of every target group of every listed simulation, one warp per
 // group (the wide groups first, they have the most to translate).  A leaf's walk
 // also meets the leaves to be summed pair by pair and the nodes to be evaluated
@@ -751,7 +745,7 @@ __global__ void __launch_bounds__(32 * kFarWarps, kFarBlocks)
 // end.
 //
 // Measured (B200, wake of 2^20 blobs, sigma 0.0169): the whole velocity call
-// 1.99 ms, of which this kernel 1.15, k_far 0.49 and k_tree 0.17, against
+// 1.87 ms, of which this kernel 1.18, k_far 0.36 and k_tree 0.17, against
 // 215 ms for all pairs in mutual FP32x2 tiles at 80 % of the FP32 peak.  Relative
 // L2 error against FP64 1.3e-7 (all pairs: 5.7e-7 to 7.6e-7) at 2^18.  At 2^18
 // the MUFU pipe is 60 % and the FMA pipe 53 % busy, issue 57 %: latency bounds
@@ -1435,21 +1429,28 @@ __global__ void __launch_bounds__(256) k_rhs_combine(const InstDesc* __restrict_
 }
 
 // The same right-hand side for FP32 simulations, over the tree of the blobs: one
-// block per group of 32 collocation points, lane t of every warp at point t.
+// block per group of 32 collocation points, lane t of every warp at point t (of
+// eight points for bodies of up to 128 panels, whose few blocks would otherwise each
+// see half of the near leaves: lane t at point t % 8, with every fourth pair of
+// sources).
 // The tree's top nodes are dealt out to the warps, and each walks its own: far
 // nodes are translated, near leaves summed pair by pair as in k_at (offsets in
 // two parts, one compensated sum per half), their sums added in FP64; the
 // warps' results are added in order.  The circulations' sum is the root's first
 // moment.  Depends only on the simulation, never on the batch.
 //
-// Measured (B200, 250 k blobs, 1024 panels): 46 us for 240 us of all pairs
-// (and 12 us to combine their chunks); 2^17 blobs 38 for 122.
+// Near leaves go to a queue that all warps share out, or the warps with the
+// nearest top nodes would work alone.  Measured (B200, 2^17 blobs, RHS of a step):
+// 64, 128, 512, 1024 panels 29, 23, 27, 25 us; without the queue and with 32 points
+// per block throughout 142, 109, -, 39; all pairs 72, 70, 87, 129.
 constexpr int kRhsWarps = 8;
 constexpr int kRhsGroup = 32;
+constexpr int kRhsNear = 128;  // near leaves a warp leaves to all; more it sums at once
+__host__ __device__ __forceinline__ int rhs_group(int np) { return np <= 128 ? 8 : kRhsGroup; }
 struct RhsWarp {
     TreeWalk walk;
     TransBuf buf;
-    uint32_t far[kFarList];
+    uint32_t far[kFarList], near[kRhsNear];
     float4 pos_hi[kLeaf / 2], pos_lo[kLeaf / 2];  // (x a, x b, z a, z b) of sources 2i, 2i + 1
     float4 cst[kLeaf / 2];                        // (circ a, circ b, 10 sigma^2 a, b)
     float2 rs[kLeaf / 2];
@@ -1458,6 +1459,7 @@ struct RhsWarp {
 struct RhsShared {
     RhsWarp w[kRhsWarps];
     double2 at[kRhsGroup];
+    int nnear[kRhsWarps];
 };
 __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     k_rhs_tree(const InstDesc* __restrict__ table, InstState* __restrict__ st,
@@ -1468,7 +1470,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     RhsShared& S = *reinterpret_cast<RhsShared*>(s_raw);
     const ListEntry e = list[blockIdx.y];
     const InstDesc& d = table[e.inst];
-    const int i0 = (int)blockIdx.x * kRhsGroup;
+    const int group = rhs_group(d.np), i0 = (int)blockIdx.x * group;
     if (i0 >= d.np) return;  // block-uniform
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned all = 0xffffffffu;
@@ -1478,7 +1480,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     const double2* __restrict__ A = mom + e.noff * kTerms;
     const double2* __restrict__ X = pxz + e.coff;
     const float4* __restrict__ F = pf + e.coff;
-    const int i = min(i0 + lane, d.np - 1);
+    const int i = min(i0 + (lane & (group - 1)), d.np - 1);
     const double tx = d.xc[i], tz = d.zc[i];
     if (wid == 0) S.at[lane] = make_double2(tx, tz);
     double x0 = tx, x1 = tx, z0 = tz, z1 = tz;
@@ -1508,8 +1510,57 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     const Binomials mat = binomials(lane);
     LocalSum sum{};              // this warp's share
     double nu = 0.0, sw = 0.0;   // -u and w at the lane's point, near and mid
+    auto near_leaf = [&](uint32_t leaf) {  // sums a leaf's pairs with the 32 points
+        const uint32_t j0 = leaf * kLeaf;
+        // (padding: far away, no circulation)
+        float xh[2] = {1e18f, 1e18f}, xl[2] = {0.f, 0.f}, zh[2] = {0.f, 0.f}, zl[2] = {0.f, 0.f};
+        float g[2] = {0.f, 0.f}, thr[2] = {0.f, 0.f}, rs[2] = {0.f, 0.f};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t j = j0 + 2 * lane + h;
+            if (j < n) {
+                const double2 p = X[j];
+                const float4 f = F[j];
+                split_16(p.x - ox, xh[h], xl[h]);
+                split_16(p.y - oz, zh[h], zl[h]);
+                g[h] = f.x;
+                thr[h] = f.y;
+                rs[h] = f.z;
+            }
+        }
+        __syncwarp();
+        W.pos_hi[lane] = make_float4(xh[0], xh[1], zh[0], zh[1]);
+        W.pos_lo[lane] = make_float4(xl[0], xl[1], zl[0], zl[1]);
+        W.cst[lane] = make_float4(g[0], g[1], thr[0], thr[1]);
+        W.rs[lane] = make_float2(rs[0], rs[1]);
+        __syncwarp();
+        const uint64_t zero2 = f2pack(0.0f, 0.0f);
+        uint64_t snu = zero2, enu = zero2, s2 = zero2, e2 = zero2;
+#pragma unroll 4
+        for (int q = lane / group; q < kLeaf / 2; q += kRhsGroup / group) {
+            const float4 H = W.pos_hi[q], L = W.pos_lo[q], Cs = W.cst[q];
+            const uint64_t DX = f2add(f2sub(TXH, f2pack(H.x, H.y)), f2sub(TXL, f2pack(L.x, L.y)));
+            const uint64_t DZ = f2add(f2sub(TZH, f2pack(H.z, H.w)), f2sub(TZL, f2pack(L.z, L.w)));
+            const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
+            const float ra = f2lo(R2), rb = f2hi(R2);
+            float ka = rcp_approx(ra), kb = rcp_approx(rb);
+            const bool ca = ra < Cs.z, cb = rb < Cs.w;
+            if (__any_sync(all, ca || cb)) {
+                const float2 R = W.rs[q];
+                const float qa = core_kernel_expm1(ra, R.x, ka);
+                const float qb = core_kernel_expm1(rb, R.y, kb);
+                ka = ca ? qa : ka;
+                kb = cb ? qb : kb;
+            }
+            const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
+            kahan2_fma(snu, enu, G, DZ);
+            kahan2_fma(s2, e2, G, DX);
+        }
+        nu += ((double)f2lo(snu) + (double)f2lo(enu)) + ((double)f2hi(snu) + (double)f2hi(enu));
+        sw += ((double)f2lo(s2) + (double)f2lo(e2)) + ((double)f2hi(s2) + (double)f2hi(e2));
+    };
     int sp = nl ? walk_begin(W.walk, nl, tb, kWalkTop, (uint32_t)wid, kRhsWarps, lane) : 0;
-    int nfar = 0;
+    int nfar = 0, nnear = 0;
     while (sp > 0) {
         uint32_t id;
         const int kind = walk_step(W.walk, N, C, nl, sp, id, lane);
@@ -1530,59 +1581,24 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
             if (lane < kTerms) W.buf.c[0][lane] = Cplx{A[at * kTerms + lane].x, A[at * kTerms + lane].y};
             __syncwarp();
             const Cplx f = moment_value(W.buf.c[0], exp2_int(N[at].e), tx - N[at].cx, tz - N[at].cz);
-            nu -= f.y;
-            sw += f.x;
-        }
-        for (unsigned todo = __ballot_sync(all, kind == kWalkNear); todo; todo &= todo - 1) {
-            const uint32_t j0 = __shfl_sync(all, id, __ffs(todo) - 1) * kLeaf;
-            // (padding: far away, no circulation)
-            float xh[2] = {1e18f, 1e18f}, xl[2] = {0.f, 0.f}, zh[2] = {0.f, 0.f}, zl[2] = {0.f, 0.f};
-            float g[2] = {0.f, 0.f}, thr[2] = {0.f, 0.f}, rs[2] = {0.f, 0.f};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t j = j0 + 2 * lane + h;
-                if (j < n) {
-                    const double2 p = X[j];
-                    const float4 f = F[j];
-                    split_16(p.x - ox, xh[h], xl[h]);
-                    split_16(p.y - oz, zh[h], zl[h]);
-                    g[h] = f.x;
-                    thr[h] = f.y;
-                    rs[h] = f.z;
-                }
+            if (lane < group) {
+                nu -= f.y;
+                sw += f.x;
             }
-            __syncwarp();
-            W.pos_hi[lane] = make_float4(xh[0], xh[1], zh[0], zh[1]);
-            W.pos_lo[lane] = make_float4(xl[0], xl[1], zl[0], zl[1]);
-            W.cst[lane] = make_float4(g[0], g[1], thr[0], thr[1]);
-            W.rs[lane] = make_float2(rs[0], rs[1]);
-            __syncwarp();
-            const uint64_t zero2 = f2pack(0.0f, 0.0f);
-            uint64_t snu = zero2, enu = zero2, s2 = zero2, e2 = zero2;
-#pragma unroll 4
-            for (int q = 0; q < kLeaf / 2; ++q) {
-                const float4 H = W.pos_hi[q], L = W.pos_lo[q], Cs = W.cst[q];
-                const uint64_t DX = f2add(f2sub(TXH, f2pack(H.x, H.y)), f2sub(TXL, f2pack(L.x, L.y)));
-                const uint64_t DZ = f2add(f2sub(TZH, f2pack(H.z, H.w)), f2sub(TZL, f2pack(L.z, L.w)));
-                const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
-                const float ra = f2lo(R2), rb = f2hi(R2);
-                float ka = rcp_approx(ra), kb = rcp_approx(rb);
-                const bool ca = ra < Cs.z, cb = rb < Cs.w;
-                if (__any_sync(all, ca || cb)) {
-                    const float2 R = W.rs[q];
-                    const float qa = core_kernel_expm1(ra, R.x, ka);
-                    const float qb = core_kernel_expm1(rb, R.y, kb);
-                    ka = ca ? qa : ka;
-                    kb = cb ? qb : kb;
-                }
-                const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
-                kahan2_fma(snu, enu, G, DZ);
-                kahan2_fma(s2, e2, G, DX);
-            }
-            nu += ((double)f2lo(snu) + (double)f2lo(enu)) + ((double)f2hi(snu) + (double)f2hi(enu));
-            sw += ((double)f2lo(s2) + (double)f2lo(e2)) + ((double)f2hi(s2) + (double)f2hi(e2));
         }
+        int cnear;
+        const int place = warp_place(kind == kWalkNear, lane, cnear);
+        const bool kept = kind == kWalkNear && nnear + place < kRhsNear;
+        if (kept) W.near[nnear + place] = id;
+        for (unsigned todo = __ballot_sync(all, kind == kWalkNear && !kept); todo; todo &= todo - 1)
+            near_leaf(__shfl_sync(all, id, __ffs(todo) - 1));  // (no room)
+        nnear = min(nnear + cnear, kRhsNear);
     }
+    if (lane == 0) S.nnear[wid] = nnear;
+    __syncthreads();
+    for (int q = 0, at = 0; q < kRhsWarps; at += S.nnear[q++])  // every warp's, dealt out by place
+        for (int k = (wid - at) & (kRhsWarps - 1); k < S.nnear[q]; k += kRhsWarps)
+            near_leaf(S.w[q].near[k]);
     __syncwarp();
     W.sum[lane] = make_double2(nu, sw);
     Cplx b = local_total(sum, lane);
@@ -1598,13 +1614,17 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     }
     __syncwarp();
     const Cplx f = local_value(W.buf.c[0], tx - tb.cx, tz - tb.cz, tb.e);
-    nu -= f.y;
-    sw += f.x;
     for (int q = 1; q < kRhsWarps; ++q) {
         nu += S.w[q].sum[lane].x;
         sw += S.w[q].sum[lane].y;
     }
-    if (i0 + lane < d.np) {
+    for (int o = group; o < 32; o <<= 1) {  // a point's lanes
+        nu += __shfl_xor_sync(all, nu, o);
+        sw += __shfl_xor_sync(all, sw, o);
+    }
+    nu -= f.y;
+    sw += f.x;
+    if (lane < group && i0 + lane < d.np) {
         const double ui = dmul(-nu, kRpi2), wi = dmul(sw, kRpi2);
         d.b[i] = dadd(dmul(dadd(d.ux, ui), d.enx[i]), dmul(dadd(d.uz, wi), d.enz[i]));
     }
@@ -1725,11 +1745,13 @@ void biot_savart_self(const InstDesc* table, InstState* st, const ListEntry* lis
 }
 
 void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
-               int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s) {
-    if (precision == kF32) {
+               int max_np, int precision, const Workspace& ws, int sms, cudaStream_t s, bool pairs) {
+    if (precision == kF32 && !pairs) {
         cudaFuncSetAttribute(k_rhs_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(RhsShared));
-        k_rhs_tree<<<dim3((max_np + kRhsGroup - 1) / kRhsGroup, nlist), 32 * kRhsWarps,
+        // (a list's smaller bodies may have up to 16 groups of eight points)
+        k_rhs_tree<<<dim3(std::max((max_np + kRhsGroup - 1) / kRhsGroup,
+                                   std::min((max_np + 7) / 8, 16)), nlist), 32 * kRhsWarps,
                      sizeof(RhsShared), s>>>(
             table, st, list, reinterpret_cast<const double2*>(ws.packed),
             reinterpret_cast<const float4*>(ws.packed + ws.packed_cap / 2), ws.nodes, ws.mom);
@@ -1739,7 +1761,8 @@ void sheet_rhs(const InstDesc* table, InstState* st, const ListEntry* list, int 
     AtJob* jobs = reinterpret_cast<AtJob*>(ws.jobs);
     k_build_rhs_jobs<<<(nlist + 127) / 128, 128, 0, s>>>(table, st, list, nlist, ws.rhs_part,
                                                          ws.circ_part, jobs);
-    k_at<false><<<sms * 4, 256, 0, s>>>(jobs, nlist);
+    if (precision == kF32) k_at<true><<<sms * 4, 256, 0, s>>>(jobs, nlist);
+    else k_at<false><<<sms * 4, 256, 0, s>>>(jobs, nlist);
     k_rhs_combine<<<dim3((max_np + 31) / 32, nlist), 256, 0, s>>>(table, st, list, jobs);
 }
 
@@ -1760,11 +1783,12 @@ static unsigned combine_threads(uint64_t nchunk) {
 }
 
 void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
-                int max_np, const Workspace& ws, int sms, cudaStream_t s) {
+                int max_np, const Workspace& ws, int sms, cudaStream_t s, bool records) {
     const int shares = ((int)panel_leaves(max_np) + kFan - 1) / kFan;
-    cudaMemsetAsync(ws.parrived, 0, sizeof(unsigned) * ws.pnodes_used, s);
+    if (!records) cudaMemsetAsync(ws.parrived, 0, sizeof(unsigned) * ws.pnodes_used, s);
     k_tree<true><<<std::min(sms * 2, nlist * shares), 32 * kTreeWarps, 0, s>>>(
-        table, st, list, nlist, nullptr, nullptr, nullptr, ws.pnodes, ws.pmom, ws.parrived, ws.pan);
+        table, st, list, nlist, nullptr, nullptr, nullptr, records ? nullptr : ws.pnodes, ws.pmom,
+        ws.parrived, ws.pan);
 }
 
 size_t direct_at_part_elems(uint32_t ns, uint32_t nt) {

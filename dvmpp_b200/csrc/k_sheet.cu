@@ -1092,7 +1092,9 @@ __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restri
 // (or evaluated at every blob of a spread leaf), and only the near panels'
 // terms are evaluated, kPanelLeaf at a time.  All panels for all blobs took
 // 716 us for 250 k blobs and 1024 panels (FMA pipe and issue); 70 to 90 now, the
-// panels' tree included.
+// panels' tree included.  TREE false: every panel, for a call that has no tree of the
+// blobs and would take longer to build one (five blocks per SM at 94 registers are
+// slower than three: 131 k blobs and 256 panels 160 us, 141).
 constexpr int kSheetWarps = 4;
 struct SheetWarp {
     TreeWalk walk;
@@ -1102,6 +1104,7 @@ struct SheetWarp {
     PanelRec pan[kPanelLeaf];
 };
 
+template <bool TREE>
 __global__ void __launch_bounds__(32 * kSheetWarps, 3)
     k_sheet_f32(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
                 const ListEntry* __restrict__ list, int nlist, int mode,
@@ -1114,8 +1117,10 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
     list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
     const unsigned total = s_pre[nlist], all = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[threadIdx.x >> 5];
-    const Binomials mat = binomials(lane);
+    SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[TREE ? threadIdx.x >> 5 : 0];
+    PanelRec* near = TREE ? S.pan : reinterpret_cast<PanelRec*>(s_raw) + (threadIdx.x >> 5) * kPanelLeaf;
+    Binomials mat;
+    if (TREE) mat = binomials(lane);
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(work, 1u);
@@ -1129,6 +1134,24 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
         const TreeNode* __restrict__ N = pnodes + e.pnoff;
         const double2* __restrict__ A = pmom + e.pnoff * kTerms;
         __syncwarp();
+        auto panels = [&](int j0, double2 pa, double2 pb, double& ua, double& wa, double& ub, double& wb) {
+            const int m = min(kPanelLeaf, d.np - j0);
+            __syncwarp();
+            const double2* from = reinterpret_cast<const double2*>(pan + e.panoff + j0);
+            for (int q = lane; q < m * (int)(sizeof(PanelRec) / 16); q += 32)
+                reinterpret_cast<double2*>(near)[q] = from[q];
+            __syncwarp();
+            sheet_sum_f32x2(pa.x, pa.y, pb.x, pb.y, m, near, ua, wa, ub, wb);
+        };
+        if (!TREE) {  // every panel, blobs in their own order
+            const uint32_t ia = min(t0 + lane, n - 1), ib = min(t0 + 32 + lane, n - 1);
+            const double2 pa = make_double2(d.x[ia], d.z[ia]), pb = make_double2(d.x[ib], d.z[ib]);
+            double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
+            for (int j0 = 0; j0 < d.np; j0 += kPanelLeaf) panels(j0, pa, pb, ua, wa, ub, wb);
+            if (t0 + lane < n) sheet_store(d, ia, ua, wa, mode);
+            if (t0 + 32 + lane < n) sheet_store(d, ib, ub, wb, mode);
+            continue;
+        }
         for (int q = lane; q < kLeaf; q += 32) S.at[q] = pxz[e.coff + min(t0 + q, n - 1)];
         __syncwarp();
         TargetBox tb = target_box(nodes[e.noff + leaf]);
@@ -1167,16 +1190,8 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
                 ub += fb.y;
                 wb += fb.x;
             }
-            for (unsigned todo = __ballot_sync(all, kind == kWalkNear); todo; todo &= todo - 1) {
-                const int j0 = (int)__shfl_sync(all, id, __ffs(todo) - 1) * kPanelLeaf;
-                const int m = min(kPanelLeaf, d.np - j0);
-                __syncwarp();
-                const double2* from = reinterpret_cast<const double2*>(pan + e.panoff + j0);
-                for (int q = lane; q < m * (int)(sizeof(PanelRec) / 16); q += 32)
-                    reinterpret_cast<double2*>(S.pan)[q] = from[q];
-                __syncwarp();
-                sheet_sum_f32x2(pa.x, pa.y, pb.x, pb.y, m, S.pan, ua, wa, ub, wb);
-            }
+            for (unsigned todo = __ballot_sync(all, kind == kWalkNear); todo; todo &= todo - 1)
+                panels((int)__shfl_sync(all, id, __ffs(todo) - 1) * kPanelLeaf, pa, pb, ua, wa, ub, wb);
         }
         if (any_far) {  // warp-uniform
             const Cplx b = local_total(sum, lane);
@@ -1571,13 +1586,14 @@ void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, in
 
 void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, int max_np, int precision, const Workspace& ws, int sms,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool pairs) {
     cudaMemsetAsync(ws.work + 1, 0, sizeof(unsigned), s);
     if (precision == kF32) {
-        panel_tree(table, st, list, nlist, max_np, ws, sms, s);
-        constexpr size_t smem = sizeof(SheetWarp) * kSheetWarps;
-        cudaFuncSetAttribute(k_sheet_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_sheet_f32<<<sms * 3, 32 * kSheetWarps, smem, s>>>(
+        panel_tree(table, st, list, nlist, max_np, ws, sms, s, pairs);
+        const size_t smem = (pairs ? sizeof(PanelRec) * kPanelLeaf : sizeof(SheetWarp)) * kSheetWarps;
+        auto* kernel = pairs ? k_sheet_f32<false> : k_sheet_f32<true>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<sms * 3, 32 * kSheetWarps, smem, s>>>(
             table, st, list, nlist, mode, ws.perm, reinterpret_cast<const double2*>(ws.packed),
             ws.nodes, ws.pnodes, ws.pmom, ws.pan, ws.work + 1);
         return;

@@ -139,7 +139,7 @@ int dvm_ctx_launch_count(dvm_ctx* ctx, uint64_t* launches);
 #define DVM_PROF_DIFFREL 4    /* diffusion + release/append */
 #define DVM_PROF_CROSS 5      /* reflect / delete */
 #define DVM_PROF_LOADS 6      /* loads + step counter */
-#define DVM_PROF_SORT 7       /* Morton sort, pack, partial combine */
+#define DVM_PROF_SORT 7       /* curve sort, pack / far-field tree, partial combine */
 #define DVM_PROF_STEP 8       /* whole step */
 #define DVM_PROF_FAMILIES 9
 /* Pre-size the shared workspace for batches of up to max_sims simulations whose
@@ -390,15 +390,15 @@ int dvm_batch_wait_state(dvm_ctx* ctx, int nsims, double* const* x, double* cons
 /* ---- pair-kernel autotuning (no counterpart in the reference) ---------------------
  * The FP32 blob-on-blob kernel's launch shape: persistent CTAs per SM and the
  * order in which simulations' work items are handed out (a work item is one
- * 256-blob sort tile of targets against one source chunk).  Neither changes a
- * result (source chunking, which would, is fixed by each simulation's capacity),
- * so tuning never changes velocities.  Shapes are kept
+ * 64-blob leaf of targets with the leaves near it).  Neither changes a result
+ * (what is summed, and in which order, depends on the simulation alone), so
+ * tuning never changes velocities.  Shapes are kept
  * per batch-shape class (log2 of the summed capacity of the batch's FP32
  * simulations x a bucket of their count: 1, 2-8, 9-64, more); plans and graphs
  * built afterwards use them. */
 typedef struct dvm_pair_config {
-    int32_t tile;        /* targets per work item: 256 */
-    int32_t ctas_per_sm; /* 1..4 */
+    int32_t tile;        /* 256 (kept for the record's layout) */
+    int32_t ctas_per_sm; /* 1..4 quarters of the CTAs that fit an SM */
     int32_t order;       /* 0: list order; 1: costliest simulations' items first */
     int32_t reserved;
 } dvm_pair_config;
