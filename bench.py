@@ -518,7 +518,7 @@ def run_ours(args, dist):
     t_setup = time.perf_counter()
     instances = make_instances(args.instances, args.seed)
     ctx = N.Context(dist.local)
-    sms, ccmaj, ccmin = ctx.device_info()
+    _, ccmaj, ccmin = ctx.device_info()
     steps_total = args.warmup + args.steps + args.prof_steps + args.plain_steps + args.e2e_steps + 2
     prepush = args.warmup + args.steps + args.prof_steps + args.plain_steps + 1
     sims, bodies, sparams = [], [], []
@@ -581,9 +581,10 @@ def run_ours(args, dist):
     # ---- profiled steps (eager, CUDA events around every kernel family)
     ctx.set_profiling(True)
     ctx.profile_reset()
-    pairs = 0
+    pairs = blobs = 0
     for _ in range(args.prof_steps):
         ns = [s.n for s in sims]
+        blobs += sum(ns)
         pairs += sum(n * (n - 1) for n in ns)
         ctx.step_batch(sims, 1, use_graph=False)
     prof = ctx.profile()
@@ -592,11 +593,11 @@ def run_ours(args, dist):
     step_ms_prof = prof["step"][0] / max(prof["step"][1], 1)
     nbody_launch_ms = nb_ms / max(nb_n, 1)
     pairs_per_launch = pairs / max(nb_n, 1)
-    achieved_tflops = (12.0 * pairs_per_launch / (nbody_launch_ms / 1e3) / 1e12
-                       if nbody_launch_ms > 0 else 0.0)  # no profiled steps: not measured
-    pk = peaks()
-    sm_max = float(pk.get("sm_max_mhz", 1965.0))
-    fp32_peak = sms * 128 * 2 * sm_max * 1e6 / 1e12
+    # bytes the launch cannot do without: x, z, circulation, sigma in, u, w out, FP64
+    bytes_per_launch = 48.0 * blobs / max(nb_n, 1)
+    achieved_gbs = (bytes_per_launch / (nbody_launch_ms / 1e3) / 1e9
+                    if nbody_launch_ms > 0 else 0.0)  # no profiled steps: not measured
+    hbm_peak = float(peaks().get("hbm_gbs", 6650.0))
 
     # ---- accuracy of the timed arithmetic: FP64 on the identical state
     accuracy = None
@@ -720,23 +721,23 @@ def run_ours(args, dist):
         "plain_gpu": {"value": plain_value, "unit": UNIT, "steps": args.plain_steps,
                       "ratio_batched_over_plain": value / plain_value if plain_value else None,
                       "how": "each simulation stepped alone (its own launches, no batching)"},
-        "roofline": {"bound": "fp32", "kernel": "k_self_f32 (pair kernel)",
-                     "achieved": achieved_tflops, "peak": fp32_peak, "unit": "TFLOP/s",
-                     "frac": achieved_tflops / fp32_peak,
+        "roofline": {"bound": "latency", "kernel": "k_far + k_self_f32 (blob-on-blob)",
+                     "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
+                     "frac": achieved_gbs / hbm_peak,
+                     "frac_is": "bytes of the blobs' state per launch against the measured copy: "
+                                "expansions leave O(N) arithmetic, so no single pipe bounds it",
                      "traffic": args.traffic if args.traffic is not None else committed_traffic(),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one "
                                        "launch of this workload (profiles/"
                                        "bench_batched64_launches.md)",
-                     "flops_per_pair": 12, "pairs_per_launch": pairs_per_launch,
+                     "bytes_per_blob": 48, "pairs_represented_per_launch": pairs_per_launch,
                      "launch_ms": nbody_launch_ms,
-                     "peak_source": f"derived: {sms} SMs x 128 FP32 lanes x 2 x "
-                                    f"{sm_max:.0f} MHz (sm_max_mhz of MEASURED_PEAKS.json); "
-                                    f"that file has no FP32 figure",
+                     "peak_source": "hbm_gbs of MEASURED_PEAKS.json (copy)",
                      "share_of_step": nb_ms / max(prof["step"][0], 1e-9)},
         "profile_ms_per_step": {k: v[0] / max(args.prof_steps, 1) for k, v in prof.items()},
         "autotune": tune,
         "gpu_launches": int(launches),
-        "gpu_launches_note": "own kernels in the timed region; each step's Morton sort adds "
+        "gpu_launches_note": "own kernels in the timed region; each step's curve sort adds "
                              "the CUB radix-sort kernels compiled into the same library "
                              "(7 per step in the ncu launch list)",
         "clocks": clock_info,
@@ -763,8 +764,7 @@ def run_ours(args, dist):
         nb = cases.run_nbody(args.nbody_n, [N.F32], 2)
         r = nb["results"]["f32"]
         line["nbody"] = {"n": args.nbody_n, "pair_kernel_ms": r["pair_kernel_ms"],
-                         "gpairs_per_s": r["gpairs_per_s"], "tflops_12_per_pair": r["tflops_12_per_pair"],
-                         "fp32_peak_frac": r["fp32_peak_frac"]}
+                         "gpairs_per_s": r["gpairs_per_s"]}
     if args.serve_requests and dist.world == 1:
         from dvmpp_b200 import cases
 

@@ -38,7 +38,6 @@ from __future__ import annotations
 
 import argparse
 import json
-import os
 import time
 
 import numpy as np
@@ -49,20 +48,8 @@ from . import workloads as W
 SIGMA_CYL128 = 0.08188040878164335
 
 
-def _fp32_peak_tflops(sms: int) -> float:
-    mhz = 1965.0
-    try:
-        here = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-        with open(os.path.join(here, "MEASURED_PEAKS.json")) as f:
-            mhz = float(json.load(f).get("sm_max_mhz", mhz))
-    except (OSError, ValueError):
-        pass
-    return sms * 128 * 2 * mhz * 1e6 / 1e12
-
-
 def run_nbody(n: int, precs, reps: int, seed: int = 2):
     ctx = N.Context(0)
-    sms, _, _ = ctx.device_info()
     x, z, g, s = W.wake(n, seed, SIGMA_CYL128)
     bx, bz = W.circle(128)
     out = {"workload": "nbody", "n": n, "pairs": n * (n - 1), "results": {}}
@@ -81,11 +68,11 @@ def run_nbody(n: int, precs, reps: int, seed: int = 2):
         ms = prof["nbody"][0] / max(prof["nbody"][1], 1)
         d = sim.blobs()
         fields[prec] = (d["u"], d["w"])
-        tf = 12.0 * n * (n - 1) / (ms / 1e3) / 1e12
         out["results"]["f32" if prec == N.F32 else "f64"] = {
             "pair_kernel_ms": ms, "sort_pack_combine_ms": prof["sort"][0] / max(prof["sort"][1], 1),
-            "gpairs_per_s": n * (n - 1) / (ms / 1e3) / 1e9, "tflops_12_per_pair": tf,
-            "fp32_peak_frac": tf / _fp32_peak_tflops(sms)}
+            "gpairs_per_s": n * (n - 1) / (ms / 1e3) / 1e9}
+        if prec == N.F64:  # (every pair is evaluated; FP32 sums far ones by expansions)
+            out["results"]["f64"]["tflops_12_per_pair"] = 12.0 * n * (n - 1) / (ms / 1e3) / 1e12
         sim.close()
     if N.F32 in fields and N.F64 in fields:
         (uf, wf), (ud, wd) = fields[N.F32], fields[N.F64]
@@ -349,7 +336,6 @@ def run_sheet(n: int, npanels: int, reps: int, seed: int = 2):
     body), FP32 instance; blob velocities and the panel strengths are computed
     once, then the sheet-on-blob phase runs reps times (the first untimed)."""
     ctx = N.Context(0)
-    sms, _, _ = ctx.device_info()
     bx, bz = W.ellipse(npanels, incidence_deg=20.0)
     x, z, g, s = W.wake(n, seed, W.core_size(bx, bz))
     sim = ctx.sim(N.Params(capacity=n, precision=N.F32, rng=N.RNG_PHILOX, ux=1.0), bx, bz)
@@ -363,22 +349,19 @@ def run_sheet(n: int, npanels: int, reps: int, seed: int = 2):
     ctx.mark(1)
     ms = ctx.elapsed_ms(0, 1) / max(reps, 1)
     pairs = n * npanels
-    tf = 67.0 * pairs / (ms / 1e3) / 1e12
     sim.close()
     ctx.close()
     return {"workload": "sheet", "n": n, "panels": npanels, "pairs": pairs, "kernel_ms": ms,
-            "gpairs_per_s": pairs / (ms / 1e3) / 1e9, "tflops_67_per_pair": tf,
-            "fp32_peak_frac": tf / _fp32_peak_tflops(sms)}
+            "gpairs_per_s": pairs / (ms / 1e3) / 1e9}
 
 
 def run_rhs(n: int, npanels: int, reps: int, seed: int = 2):
     """Blob-on-collocation right-hand side alone (the at-target kernel of
     solvevortexsheet, src/VortexSheet.cpp:181-203): an ellipse (0.5, 0.25) at
     20 degrees with npanels panels and an n-blob wake, FP32 instance; the
-    profiled RHS family's CUDA-event time per launch, pairs/s and the FP32
-    fraction at 12 flop per pair."""
+    profiled RHS family's CUDA-event time per launch and the pairs it stands for
+    per second."""
     ctx = N.Context(0)
-    sms, _, _ = ctx.device_info()
     bx, bz = W.ellipse(npanels, incidence_deg=20.0)
     x, z, g, s = W.wake(n, seed, W.core_size(bx, bz))
     sim = ctx.sim(N.Params(capacity=n + 8 * npanels, precision=N.F32, rng=N.RNG_PHILOX, ux=1.0),
@@ -395,18 +378,16 @@ def run_rhs(n: int, npanels: int, reps: int, seed: int = 2):
     ctx.set_profiling(False)
     ms = prof["rhs"][0] / max(prof["rhs"][1], 1)
     pairs = n * npanels
-    tf = 12.0 * pairs / (ms / 1e3) / 1e12
     sim.close()
     ctx.close()
     return {"workload": "rhs", "n": n, "panels": npanels, "pairs": pairs, "kernel_ms": ms,
-            "gpairs_per_s": pairs / (ms / 1e3) / 1e9, "tflops_12_per_pair": tf,
-            "fp32_peak_frac": tf / _fp32_peak_tflops(sms)}
+            "gpairs_per_s": pairs / (ms / 1e3) / 1e9}
 
 
 def run_setup(panels=(64, 128, 256, 512, 1024), reps: int = 5):
-    """Per-body set-up (src/VortexSheet.cpp:78-165 plus the factorisation that
+    """Per-body set-up (src/VortexSheet.cpp:78-165 plus the pseudo-inverse that
     replaces the per-step LAPACK solve): wall time of creating a simulation on a
-    circle of np panels -- geometry, uploads, influence matrix, QR, P -- best of
+    circle of np panels -- geometry, uploads, influence matrix, P -- best of
     `reps` after one warm-up creation."""
     import time
     ctx = N.Context(0)
