@@ -390,19 +390,6 @@ def run_reference_arm(args, dist):
 # ---------------------------------------------------------------------------
 # our arm
 # ---------------------------------------------------------------------------
-def committed_traffic():
-    """DRAM bytes per pair-kernel launch on this workload, from the committed
-    ncu summary (one capture of the first timed step)."""
-    try:
-        with open(os.path.join(ROOT, "profiles", "bench_batched64_launches.md")) as f:
-            for ln in f:
-                if ln.strip().startswith("dram_bytes_per_launch:"):
-                    return float(ln.split(":")[1])
-    except (OSError, ValueError):
-        pass
-    return None
-
-
 def peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -726,10 +713,8 @@ def run_ours(args, dist):
                      "frac": achieved_gbs / hbm_peak,
                      "frac_is": "bytes of the blobs' state per launch against the measured copy: "
                                 "expansions leave O(N) arithmetic, so no single pipe bounds it",
-                     "traffic": args.traffic if args.traffic is not None else committed_traffic(),
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one "
-                                       "launch of this workload (profiles/"
-                                       "bench_batched64_launches.md)",
+                     "traffic": args.traffic,
+                     "traffic_source": "--traffic, from an ncu capture (null: not given)",
                      "bytes_per_blob": 48, "pairs_represented_per_launch": pairs_per_launch,
                      "launch_ms": nbody_launch_ms,
                      "peak_source": "hbm_gbs of MEASURED_PEAKS.json (copy)",
