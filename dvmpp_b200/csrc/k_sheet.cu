@@ -7,7 +7,7 @@
 // rounding per operation (dadd/dmul/...), so they round like the reference
 // compiled without FP contraction.  FP32 instances evaluate the near sheet-on-blob
 // panel terms in single precision (accumulated in FP64) and the far ones by FP64
-// expansions; the influence matrix, QR, solve, refinement and loads are FP64 for
+// expansions; the influence matrix, P, solve, refinement and loads are FP64 for
 // both.
 //
 // The solve: the reference forms A^T A and A^T b and solves with LAPACK every
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kTileThreads * kGjGroups) k_pinv_invert(const 
     }
 }
 
-// ---- Householder QR of A (column-major, m = np+1 rows), for nearly singular A ------------------------
+// ---- Householder QR of A (column-major, m = np+1 rows), for nearly singular A ----
 // M holds [A | Q^T]: columns 0..np-1 are A (overwritten by R on and above the
 // diagonal), columns np..np+m-1 receive Q^T.  Both paths are one cooperative
 // launch with one grid barrier per Householder step (a chain of np dependent

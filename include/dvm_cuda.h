@@ -59,7 +59,7 @@ extern "C" {
 
 /* arithmetic of the pair interactions */
 #define DVM_F64 0 /* FP64, the reference's formulas */
-#define DVM_F32 1 /* FP32 pair terms with compensated / FP64 sums; FP64 state, QR,
+#define DVM_F32 1 /* FP32 near pairs, FP64 far-field expansions; FP64 state, P,
                      refinement residual and Kelvin row */
 
 #define DVM_EULER 0 /* Scheme::Euler, src/DVMBase.hpp:27-30 */
@@ -229,10 +229,10 @@ int dvm_biot_savart_at_noalloc(const double* x, const double* z, const double* c
 int dvm_sim_create(dvm_ctx* ctx, const dvm_sim_params* p, const double* body_x,
                    const double* body_z, int npoints, dvm_sim** out);
 /* n simulations created together, as n calls of dvm_sim_create would create
- * them (same set-up arithmetic, bit for bit), but the once-per-body QR
- * factorisations of their influence matrices share cooperative launches (up to
- * 8 bodies per launch) and one wait covers them all: a serving loop admitting
- * several requests at once pays for about one factorisation chain instead of n.
+ * them (same set-up arithmetic, bit for bit), but the once-per-body
+ * pseudo-inverses of their influence matrices share launches (up to 8 bodies
+ * per launch): a serving loop admitting several requests at once pays for
+ * about one chain of dependent steps instead of n.
  * All or none: on any error no simulation is created and out[] stays NULL; an
  * argument error names the offending index.  The set-up scratch of all n
  * bodies (about 32 np^2 bytes each) is held at once and counts against the
@@ -472,7 +472,7 @@ typedef struct {
     double queue_p50_s, queue_p99_s;
     uint32_t peak_active;
     uint64_t peak_bytes;
-    /* host wall time spent admitting (simulation set-up, incl. the QR), issuing
+    /* host wall time spent admitting (simulation set-up included), issuing
      * and waiting for ticks, and retiring (results read back); tunings run */
     double admit_s, step_s, retire_s;
     uint32_t tunings;
