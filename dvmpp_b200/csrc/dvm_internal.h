@@ -48,7 +48,8 @@ constexpr int kTerms = 24;                     // terms of its expansions
 constexpr int kNodeSlack = 32;                 // nodes per simulation beyond 2 per leaf
 
 // Node of the far-field tree (dvm_tree.cuh): the box and circle around its
-// blobs, their largest 10 sigma^2, and the exponent of its moments' scale.
+// blobs (or panels), the squared gap from which it may be taken (their largest 10
+// sigma^2, or that of the panels' quadrature), and the exponent of its moments' scale.
 struct __align__(16) TreeNode {
     double cx, cz;  // centre of the box
     double R;       // radius around it

@@ -8,7 +8,8 @@
 // scaled by a power of two s >= its radius R (no over- or underflow at any
 // scale of the coordinates).  A target group (centre, radius R_t) takes a node
 // by one moment-to-local translation when
-//     R + R_t <= kTheta D   and the boxes are farther apart than the node's cores,
+//     R + R_t <= kTheta D   and the boxes are farther apart than the node's cores
+//     (a node of panels: than their quadrature needs),
 // D the distance of the centres, and otherwise looks at its two halves; a leaf
 // that is still too near is summed pair by pair (Greengard & Rokhlin,
 // J. Comput. Phys. 73 (1987) 325; the translations are theirs).  A group spread

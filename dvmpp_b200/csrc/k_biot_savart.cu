@@ -317,8 +317,15 @@ __device__ __forceinline__ void parent_node(const TreeNode& a, const TreeNode& b
     acc.y = ((sum[0].y + sum[1].y) + (sum[2].y + sum[3].y)) * fact;
 }
 
-// Gauss points and weights of four-point quadrature on [0, 1].  A leaf spans many
-// panels, so a panel's moments to order kTerms are as good as exact.
+// Gauss points and weights of four-point quadrature on [0, 1].  Seen from a gap of
+// 1, 2 or 3 of its lengths a panel is off by at most 6e-5, 6e-7 or 4e-8 of the sum of
+// its absolute contributions, whatever its two end strengths (against 200 points),
+// so the panels' nodes are taken from a gap of kPanelGap of their longest panel on (as
+// TreeNode::thr) and their boxes and radii hold the panels' ends.  A leaf of 16 equal
+// panels is farther away than that by its radius alone; one that a single panel
+// dominates (a remainder of one or two, a contour with long straight panels) is not,
+// and blobs near it were off by up to 2e-4 without the gap.
+constexpr double kPanelGap = 3.0;
 __device__ __constant__ const double kGaussT[kPanelPoints] = {
     0.06943184420297371, 0.33000947820757187, 0.66999052179242813, 0.93056815579702629};
 __device__ __constant__ const double kGaussW[kPanelPoints] = {
@@ -397,11 +404,12 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                 next[h] = !PANELS && i < n ? perm[e.coff + i] : 0u;
             }
             double px[2], pz[2], gc[2];
+            double ex[2], ez[2];  // PANELS: what the box holds, for a panel's outer points its ends
             double x0 = DBL_MAX, x1 = -DBL_MAX, z0 = DBL_MAX, z1 = -DBL_MAX, thr = 0.0;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t i = idx * kLeaf + h * 32 + lane;
-                px[h] = pz[h] = gc[h] = 0.0;
+                px[h] = pz[h] = gc[h] = ex[h] = ez[h] = 0.0;
                 if (i < n) {
                     if (PANELS) {
                         const uint32_t p = i / kPanelPoints;
@@ -411,6 +419,11 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                         px[h] = fma(dsp * t, d.cth[p], d.xc[p]);
                         pz[h] = fma(dsp * t, d.sth[p], d.zc[p]);
                         gc[h] = -(w * dsp) * fma(g1 - g0, t, g0);
+                        const int q = i % kPanelPoints;
+                        const double te = q == 0 ? 0.0 : q == kPanelPoints - 1 ? 1.0 : t;
+                        ex[h] = fma(dsp * te, d.cth[p], d.xc[p]);
+                        ez[h] = fma(dsp * te, d.sth[p], d.zc[p]);
+                        thr = fmax(thr, (kPanelGap * dsp) * (kPanelGap * dsp));
                     } else {
                         const uint32_t p = here[h];
                         const double sg = d.sigma[p], s2 = sg * sg;
@@ -422,10 +435,11 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                             make_float4((float)gc[h], (float)(10.0 * s2), (float)(1.0 / s2), 0.f);
                         thr = fmax(thr, 10.0 * s2);
                     }
-                    x0 = fmin(x0, px[h]);
-                    x1 = fmax(x1, px[h]);
-                    z0 = fmin(z0, pz[h]);
-                    z1 = fmax(z1, pz[h]);
+                    const double bx = PANELS ? ex[h] : px[h], bz = PANELS ? ez[h] : pz[h];
+                    x0 = fmin(x0, bx);
+                    x1 = fmax(x1, bx);
+                    z0 = fmin(z0, bz);
+                    z1 = fmax(z1, bz);
                 }
             }
 #pragma unroll
@@ -448,7 +462,8 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
                 if (idx * kLeaf + h * 32 + lane < n) {
                     px[h] -= m.cx;
                     pz[h] -= m.cz;
-                    r2 = fmax(r2, px[h] * px[h] + pz[h] * pz[h]);
+                    const double bx = PANELS ? ex[h] - m.cx : px[h], bz = PANELS ? ez[h] - m.cz : pz[h];
+                    r2 = fmax(r2, bx * bx + bz * bz);
                 }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(all, r2, o));
