@@ -1193,32 +1193,72 @@ __device__ __forceinline__ void kahan2_fma(uint64_t& s, uint64_t& e, uint64_t a,
 //
 // FP32 jobs pack two SOURCES per FP32x2 instruction, so no lane idles however few
 // targets a job has.  Offsets are formed without per-pair conversions: every
-// position is taken relative to the tile's first target in FP64 and split into an
-// FP32 pair, hi of 16 bits and lo = the remainder (40 bits together); dx = (t_hi -
-// s_hi) + (t_lo - s_lo), where the first difference is exact unless one
-// position is 2^8 times farther out than the other, so dx is rounded once (hi of
-// 24 bits rounds it twice: error against 64 bits 4 % up, this 7 % down against
-// FP64 differences rounded once).  Each pair keeps its compensated update (the
-// right-hand side is the small residual normal velocity, so its rounding must
-// stay relative to the few large near-blob terms, not compound): one Kahan
-// sum per half, the halves added at the end.  The core kernel runs for both
-// halves when any lane of the warp has a pair inside a core.  Sources are
-// staged as packed pairs (two 16-byte loads bring positions, two more the
-// circulations and core constants).  Where close pairs are skipped, a pair with
-// not r2 > 1e-15 (NaN included) adds nothing.
+// position is taken relative to the tile's first target in FP64
+// and split into an FP32 pair, hi of 16 bits and lo = the remainder (40 bits
+// together); dx = (t_hi - s_hi) + (t_lo - s_lo), where the first difference is exact
+// unless one position is 2^8 times farther out than the other, so dx is rounded
+// once (hi of 24 bits rounds it twice: error against 64 bits 4 % up, this 7 % down
+// against FP64 differences rounded once).  40 bits are not enough for a pair much
+// closer than its distance from the origin: below kSplitClose of that distance (where
+// the split's own error is 3e-8 at most) dx and dz come from the FP64 positions.
+// Targets need not lie together, so a tile may span everything; without this
+// offsets of 1e-4 were off by 3e-7 to 1.8e-5 at 10 to 1000 from the origin.
+// Each pair keeps its compensated update (the right-hand side is the small residual
+// normal velocity, so its rounding must stay relative to the few large near-blob
+// terms, not compound): one Kahan sum per half, the halves added at the end.  The
+// core kernel runs for both halves when any lane of the warp has a pair inside a
+// core.  Sources are staged as packed pairs (two 16-byte loads bring positions, two
+// more the circulations and core constants).  Where close pairs are skipped, a pair
+// with not r2 > 1e-15 (NaN included) adds nothing.
+constexpr double kSplitClose = 1.0 / 8192.0;
 __device__ __forceinline__ void split_16(double v, float& hi, float& lo) {
     hi = __int_as_float((__float_as_int((float)v) + 0x80) & ~0xFF);
     lo = (float)(v - (double)hi);
 }
+// Squared distance below which a target's pairs need FP64 offsets; dx, dz: from the
+// origin.  A source's, twice over, is above that of any target it is so close to, so
+// the larger of it and 10 sigma^2 settles for most pairs with one comparison that
+// neither matters (comparisons of their own: 4 % of the call).
+__device__ __forceinline__ float split_close2(double dx, double dz) {
+    return (float)(fma(dx, dx, dz * dz) * (kSplitClose * kSplitClose));
+}
+__device__ __forceinline__ float look_closer2(double dx, double dz, float thr) {
+    return fmaxf(thr, 2.0f * split_close2(dx, dz));
+}
+// The pair loops' r2 of one source (hi, lo: its entries of AtStage, z two further on),
+// bit for bit.
+__device__ __forceinline__ float split_dist2(float txh, float txl, float tzh, float tzl, const float* hi,
+                                             const float* lo) {
+    const float dx = __fadd_rn(__fsub_rn(txh, hi[0]), __fsub_rn(txl, lo[0]));
+    const float dz = __fadd_rn(__fsub_rn(tzh, hi[2]), __fsub_rn(tzl, lo[2]));
+    return __fmaf_rn(dx, dx, __fmul_rn(dz, dz));
+}
+// One pair from its FP64 offsets, added to half h of the packed sums; the caller's own
+// term for it is zero.
+__device__ __forceinline__ void close_pair(double ddx, double ddz, float rs, float thr, float circ, int h,
+                                           bool skip, uint64_t& snu, uint64_t& enu, uint64_t& sw,
+                                           uint64_t& ew) {
+    const float dx = (float)ddx, dz = (float)ddz, r2 = fmaf(dx, dx, dz * dz);
+    if (skip && !(r2 > 1e-15f)) return;
+    float k = rcp_approx(r2);
+    if (r2 < thr) k = core_kernel_expm1(r2, rs, k);
+    const float g = k * circ;
+    const uint64_t G = h ? f2pack(0.0f, g) : f2pack(g, 0.0f);
+    kahan2_fma(snu, enu, G, f2pack(dz, dz));
+    kahan2_fma(sw, ew, G, f2pack(dx, dx));
+}
 struct AtStage {
     float4 pos_hi[128];  // (x_hi a, x_hi b, z_hi a, z_hi b) of sources 2i, 2i+1
     float4 pos_lo[128];  // (x_lo a, x_lo b, z_lo a, z_lo b)
-    float4 cst[128];     // (circ a, circ b, 10 sigma^2 a, 10 sigma^2 b)
-    float2 rs[128];      // (1/sigma^2 a, 1/sigma^2 b)
+    float4 cst[128];     // (circ a, circ b, squared distance a, b below which to look closer)
+    float4 core[128];    // (1/sigma^2 a, 1/sigma^2 b, 10 sigma^2 a, 10 sigma^2 b)
 };
 
+// (FP32: three blocks fit an SM by themselves, but told so the compiler's loop is 4 %
+// faster: 256 targets against 2^20 sources 288 us, 300.  FP64: four, at 64 registers; at 68
+// a probe of 3001 points and 60 k blobs took 478 us instead of 416)
 template <bool F32>
-__global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(256, F32 ? 3 : 4) k_at(const AtJob* __restrict__ jobs, int njobs) {
     __shared__ unsigned s_pre[kMaxList + 1];
     // FP64: x, z, circ, 10 sigma^2 and 1 / sigma^2; FP32: packed pairs
     __shared__ union Stage {
@@ -1251,6 +1291,7 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
         split_16(tz - oz, tzh, tzl);
         const uint64_t TXH = f2pack(txh, txh), TXL = f2pack(txl, txl);
         const uint64_t TZH = f2pack(tzh, tzh), TZL = f2pack(tzl, tzl);
+        const float close2 = split_close2(tx - ox, tz - oz);
         const uint32_t j0 = c * J.chunk, j1 = min(ns, j0 + J.chunk);
         double uu = 0.0, ww = 0.0, csum = 0.0;
         const uint64_t zero2 = f2pack(0.0f, 0.0f);
@@ -1261,7 +1302,7 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
             if (F32) {
                 // slot (pair i = tid / 2, half h = tid % 2); a slot past the
                 // chunk holds a far, circulation-free source (it adds 0)
-                float xh = 1.0e18f, xl = 0.f, zh = 0.f, zl = 0.f, cf = 0.f, thr = 0.f, rsf = 0.f;
+                float xh = 1.0e18f, xl = 0.f, zh = 0.f, zl = 0.f, cf = 0.f, thr = 0.f, rsf = 0.f, look = 0.f;
                 if (j < j1) {
                     const double sg = J.ss[j];
                     const double s2 = dmul(sg, sg);
@@ -1270,20 +1311,22 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
                     cf = (float)J.sc[j];
                     thr = (float)dmul(10.0, s2);
                     rsf = (float)ddiv(1.0, s2);
+                    look = look_closer2(J.sx[j] - ox, J.sz[j] - oz, thr);
                     if (ttile == 0) csum += J.sc[j];
                 }
                 const int i = threadIdx.x >> 1, h = threadIdx.x & 1;
                 float* ph = reinterpret_cast<float*>(&S.f.pos_hi[i]);
                 float* pl = reinterpret_cast<float*>(&S.f.pos_lo[i]);
                 float* pc = reinterpret_cast<float*>(&S.f.cst[i]);
-                float* pr = reinterpret_cast<float*>(&S.f.rs[i]);
+                float* pr = reinterpret_cast<float*>(&S.f.core[i]);
                 ph[h] = xh;
                 ph[2 + h] = zh;
                 pl[h] = xl;
                 pl[2 + h] = zl;
                 pc[h] = cf;
-                pc[2 + h] = thr;
+                pc[2 + h] = look;
                 pr[h] = rsf;
+                pr[2 + h] = thr;
             } else if (j < j1) {
                 const double sg = J.ss[j];
                 const double s2 = dmul(sg, sg);
@@ -1294,6 +1337,7 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
             __syncthreads();
             const int cnt = (int)min(256u, j1 - s0);
             if (F32) {
+                int first = 256, last = -1;  // of the pairs with a source that is too close
 #pragma unroll 4
                 for (int i = 0; i < (cnt + 1) / 2; ++i) {
                     const float4 H = S.f.pos_hi[i], L = S.f.pos_lo[i], Cs = S.f.cst[i];
@@ -1302,13 +1346,19 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
                     const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
                     const float ra = f2lo(R2), rb = f2hi(R2);
                     float ka = rcp_approx(ra), kb = rcp_approx(rb);
-                    const bool ca = ra < Cs.z, cb = rb < Cs.w;
-                    if (__any_sync(0xffffffffu, ca || cb)) {
-                        const float2 R = S.f.rs[i];
+                    if (__any_sync(0xffffffffu, ra < Cs.z || rb < Cs.w)) {
+                        const float4 R = S.f.core[i];
+                        const bool ca = ra < R.z, cb = rb < R.w;
                         const float qa = core_kernel_expm1(ra, R.x, ka);
                         const float qb = core_kernel_expm1(rb, R.y, kb);
                         ka = ca ? qa : ka;
                         kb = cb ? qb : kb;
+                        if (fminf(ra, rb) < close2) {  // left to the loop below
+                            ka = ra < close2 ? 0.0f : ka;
+                            kb = rb < close2 ? 0.0f : kb;
+                            first = min(first, i);
+                            last = i;
+                        }
                     }
                     if (skip) {  // computeInducedAt (src/VelocityKernel.cpp:89)
                         const bool oa = ra > 1e-15f, ob = rb > 1e-15f;
@@ -1320,6 +1370,16 @@ __global__ void __launch_bounds__(256) k_at(const AtJob* __restrict__ jobs, int 
                     const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
                     kahan2_fma(snu, enu, G, DZ);
                     kahan2_fma(sw, ew, G, DX);
+                }
+#pragma unroll 1
+                for (int h = 2 * first; h < min(2 * last + 2, cnt); ++h) {
+                    const float* hi = reinterpret_cast<const float*>(&S.f.pos_hi[h >> 1]) + (h & 1);
+                    const float* lo = reinterpret_cast<const float*>(&S.f.pos_lo[h >> 1]) + (h & 1);
+                    const float* co = reinterpret_cast<const float*>(&S.f.core[h >> 1]) + (h & 1);
+                    if (split_dist2(txh, txl, tzh, tzl, hi, lo) < close2)
+                        close_pair(tx - J.sx[s0 + h], tz - J.sz[s0 + h], co[0], co[2],
+                                   reinterpret_cast<const float*>(&S.f.cst[h >> 1])[h & 1], h & 1, skip, snu,
+                                   enu, sw, ew);
                 }
             } else {
                 for (int jj = 0; jj < cnt; ++jj) {
@@ -1467,8 +1527,7 @@ struct RhsWarp {
     TransBuf buf;
     uint32_t far[kFarList], near[kRhsNear];
     float4 pos_hi[kLeaf / 2], pos_lo[kLeaf / 2];  // (x a, x b, z a, z b) of sources 2i, 2i + 1
-    float4 cst[kLeaf / 2];                        // (circ a, circ b, 10 sigma^2 a, b)
-    float2 rs[kLeaf / 2];
+    float4 cst[kLeaf / 2], core[kLeaf / 2];       // (as AtStage's)
     double2 sum[kRhsGroup];
 };
 struct RhsShared {
@@ -1521,6 +1580,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
     split_16(tz - oz, tzh, tzl);
     const uint64_t TXH = f2pack(txh, txh), TXL = f2pack(txl, txl);
     const uint64_t TZH = f2pack(tzh, tzh), TZL = f2pack(tzl, tzl);
+    const float close2 = split_close2(tx - ox, tz - oz);
     __syncthreads();
     const Binomials mat = binomials(lane);
     LocalSum sum{};              // this warp's share
@@ -1529,7 +1589,7 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
         const uint32_t j0 = leaf * kLeaf;
         // (padding: far away, no circulation)
         float xh[2] = {1e18f, 1e18f}, xl[2] = {0.f, 0.f}, zh[2] = {0.f, 0.f}, zl[2] = {0.f, 0.f};
-        float g[2] = {0.f, 0.f}, thr[2] = {0.f, 0.f}, rs[2] = {0.f, 0.f};
+        float g[2] = {0.f, 0.f}, thr[2] = {0.f, 0.f}, rs[2] = {0.f, 0.f}, look[2] = {0.f, 0.f};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t j = j0 + 2 * lane + h;
@@ -1541,16 +1601,18 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
                 g[h] = f.x;
                 thr[h] = f.y;
                 rs[h] = f.z;
+                look[h] = look_closer2(p.x - ox, p.y - oz, f.y);
             }
         }
         __syncwarp();
         W.pos_hi[lane] = make_float4(xh[0], xh[1], zh[0], zh[1]);
         W.pos_lo[lane] = make_float4(xl[0], xl[1], zl[0], zl[1]);
-        W.cst[lane] = make_float4(g[0], g[1], thr[0], thr[1]);
-        W.rs[lane] = make_float2(rs[0], rs[1]);
+        W.cst[lane] = make_float4(g[0], g[1], look[0], look[1]);
+        W.core[lane] = make_float4(rs[0], rs[1], thr[0], thr[1]);
         __syncwarp();
         const uint64_t zero2 = f2pack(0.0f, 0.0f);
         uint64_t snu = zero2, enu = zero2, s2 = zero2, e2 = zero2;
+        int first = kLeaf, last = -1;  // (as in k_at)
 #pragma unroll 4
         for (int q = lane / group; q < kLeaf / 2; q += kRhsGroup / group) {
             const float4 H = W.pos_hi[q], L = W.pos_lo[q], Cs = W.cst[q];
@@ -1559,18 +1621,35 @@ __global__ void __launch_bounds__(32 * kRhsWarps, 2)
             const uint64_t R2 = f2fma(DX, DX, f2mul(DZ, DZ));
             const float ra = f2lo(R2), rb = f2hi(R2);
             float ka = rcp_approx(ra), kb = rcp_approx(rb);
-            const bool ca = ra < Cs.z, cb = rb < Cs.w;
-            if (__any_sync(all, ca || cb)) {
-                const float2 R = W.rs[q];
+            if (__any_sync(all, ra < Cs.z || rb < Cs.w)) {
+                const float4 R = W.core[q];
+                const bool ca = ra < R.z, cb = rb < R.w;
                 const float qa = core_kernel_expm1(ra, R.x, ka);
                 const float qb = core_kernel_expm1(rb, R.y, kb);
                 ka = ca ? qa : ka;
                 kb = cb ? qb : kb;
+                if (fminf(ra, rb) < close2) {  // left to the loop below
+                    ka = ra < close2 ? 0.0f : ka;
+                    kb = rb < close2 ? 0.0f : kb;
+                    first = min(first, q);
+                    last = q;
+                }
             }
             const uint64_t G = f2mul(f2pack(ka, kb), f2pack(Cs.x, Cs.y));
             kahan2_fma(snu, enu, G, DZ);
             kahan2_fma(s2, e2, G, DX);
         }
+#pragma unroll 1
+        for (int q = first; q <= last; q += kRhsGroup / group)
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t j = j0 + 2 * q + h;
+                const float* hi = reinterpret_cast<const float*>(&W.pos_hi[q]) + h;
+                const float* lo = reinterpret_cast<const float*>(&W.pos_lo[q]) + h;
+                const float* co = reinterpret_cast<const float*>(&W.core[q]) + h;
+                if (j < n && split_dist2(txh, txl, tzh, tzl, hi, lo) < close2)
+                    close_pair(tx - X[j].x, tz - X[j].y, co[0], co[2],
+                               reinterpret_cast<const float*>(&W.cst[q])[h], h, false, snu, enu, s2, e2);
+            }
         nu += ((double)f2lo(snu) + (double)f2lo(enu)) + ((double)f2hi(snu) + (double)f2hi(enu));
         sw += ((double)f2lo(s2) + (double)f2lo(e2)) + ((double)f2hi(s2) + (double)f2hi(e2));
     };
