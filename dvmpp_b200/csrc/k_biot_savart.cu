@@ -1193,7 +1193,7 @@ __device__ __forceinline__ void kahan2_fma(uint64_t& s, uint64_t& e, uint64_t a,
 //
 // FP32 jobs pack two SOURCES per FP32x2 instruction, so no lane idles however few
 // targets a job has.  Offsets are formed without per-pair conversions: every
-// position is taken relative to the tile's first target in FP64
+// position is taken relative to the tile's origin (its first finite target) in FP64
 // and split into an FP32 pair, hi of 16 bits and lo = the remainder (40 bits
 // together); dx = (t_hi - s_hi) + (t_lo - s_lo), where the first difference is exact
 // unless one position is 2^8 times farther out than the other, so dx is rounded
@@ -1212,7 +1212,13 @@ __device__ __forceinline__ void kahan2_fma(uint64_t& s, uint64_t& e, uint64_t a,
 // with not r2 > 1e-15 (NaN included) adds nothing.
 constexpr double kSplitClose = 1.0 / 8192.0;
 __device__ __forceinline__ void split_16(double v, float& hi, float& lo) {
-    hi = __int_as_float((__float_as_int((float)v) + 0x80) & ~0xFF);
+    const float f = (float)v;
+    if (!(fabsf(f) <= FLT_MAX)) {  // infinite or NaN: all of it
+        hi = f;
+        lo = 0.0f;
+        return;
+    }
+    hi = __int_as_float((__float_as_int(f) + 0x80) & ~0xFF);
     lo = (float)(v - (double)hi);
 }
 // Squared distance below which a target's pairs need FP64 offsets; dx, dz: from the
@@ -1285,7 +1291,10 @@ __global__ void __launch_bounds__(256, F32 ? 3 : 4) k_at(const AtJob* __restrict
         const uint32_t ttile = local / nchunk, c = local % nchunk;
         const uint32_t t = ttile * 256 + threadIdx.x;
         const double tx = t < J.nt ? J.tx[t] : 0.0, tz = t < J.nt ? J.tz[t] : 0.0;
-        const double ox = J.tx[ttile * 256], oz = J.tz[ttile * 256];  // the tile's origin
+        uint32_t o = ttile * 256;  // the tile's origin (block-uniform)
+        if (F32)
+            while (o + 1 < min(J.nt, ttile * 256 + 256) && !(isfinite(J.tx[o]) && isfinite(J.tz[o]))) ++o;
+        const double ox = J.tx[o], oz = J.tz[o];
         float txh, txl, tzh, tzl;
         split_16(tx - ox, txh, txl);
         split_16(tz - oz, tzh, tzl);

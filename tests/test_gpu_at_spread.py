@@ -1,10 +1,12 @@
-"""FP32 velocities at targets that do not lie together.  A block holds its 256 targets'
-offsets from one of them; a far neighbour must not cost a target precision.
+"""FP32 velocities at targets that do not lie together, and at sets with non-finite
+targets.  A block holds its 256 targets' offsets from one of them, so a far neighbour
+must not cost a target precision, nor a NaN its result.
 
-Bound: a lone source's term is rounded in its two offsets (2^-24 each), r^2, the
+Bounds: a lone source's term is rounded in its two offsets (2^-24 each), r^2, the
 reciprocal (2^-22), the core kernel and the products: below 16 x 2^-24 = 1e-6
 relative for the sources 1e-4 from their targets, whose pair dominates everything else
-by the ratio of the distances."""
+by the ratio of the distances.  A target among non-finite ones gives what it gives
+among finite ones to the FP32 bar of 1e-5."""
 import numpy as np
 import pytest
 
@@ -27,6 +29,21 @@ def test_far_neighbours_cost_nothing(ctx, spread, r, nt):
     u, w = ctx.biot_savart_at(sx, sz, g, s, tx, tz, N.F32)
     u0, w0 = ctx.biot_savart_at(sx, sz, g, s, tx, tz, N.F64)
     assert np.max(np.hypot(u - u0, w - w0) / np.hypot(u0, w0)) <= 1e-6
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("where", [[0], [0, 1, 2, 256], [255, 256], [40]])
+def test_non_finite_targets_spoil_only_themselves(ctx, where, bad):
+    x, z, g, s = W.wake(700, 3, 0.06)
+    tx, tz = W.collocation_circle(300)
+    u0, w0 = ctx.biot_savart_at(x, z, g, s, tx, tz, N.F64)
+    bx, bz = tx.copy(), tz.copy()
+    bx[where] = bad
+    bz[where[-1]] = bad
+    u, w = ctx.biot_savart_at(x, z, g, s, bx, bz, N.F32)
+    ok = np.setdiff1d(np.arange(300), where)
+    assert np.linalg.norm(u[ok] - u0[ok]) <= 1e-5 * np.linalg.norm(u0[ok])
+    assert np.linalg.norm(w[ok] - w0[ok]) <= 1e-5 * np.linalg.norm(w0[ok])
 
 
 @pytest.mark.parametrize("npan,n", [(3, 100), (15, 1000), (16, 1), (17, 65), (31, 3000), (33, 3000),
