@@ -1015,10 +1015,15 @@ __device__ __forceinline__ double rcp_f64(double v) {
     return h - 0x03d00000u < 0x78000000u ? rcp_newton(v) : __drcp_rn(v);
 }
 
-// K(r2) of src/VelocityKernel.cpp:51-57 with rs = 1 / sigma^2, thr = 10 sigma^2.
+// K(r2) of src/VelocityKernel.cpp:51-57 with rs = 1 / sigma^2, thr = 10 sigma^2.  Where
+// the reciprocal overflows (r2 < 5.6e-309) a core's factor may be 0 and their product
+// NaN, so both are scaled there; r2 = 0 gives NaN, as the reference's division does.
 __device__ __forceinline__ double kernel_f64(double r2, double thr, double rs) {
     const double y = rcp_f64(r2);
-    return r2 < thr ? dmul(dsub(1.0, exp(dmul(-r2, rs))), y) : y;
+    if (!(r2 < thr)) return y;
+    const double num = dsub(1.0, exp(dmul(-r2, rs)));
+    if (y > DBL_MAX) return dmul(dmul(num, 0x1p200), __drcp_rn(dmul(r2, 0x1p200)));
+    return dmul(num, y);
 }
 
 // Every pair, over the 256-blob tiles of the sorted order; each pair is the
