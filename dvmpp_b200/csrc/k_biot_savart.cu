@@ -658,6 +658,26 @@ __device__ __forceinline__ void leaf_sum(const StagedLeaf& __restrict__ src,
     }
 }
 
+// The same from the FP64 positions, for a leaf whose sum came out non-finite: two blobs of
+// different leaves that lie closer than their FP32 offsets resolve give r2 == 0 there, and
+// with a core size below that 1/0 times 0 (a blob's own leaf skips such pairs, above).  Pairs
+// whose squared distance is below FP32's range and that no core covers add nothing; what
+// is non-finite by its inputs stays so.
+__device__ __forceinline__ void leaf_sum_close(const double2* __restrict__ X, const float4* __restrict__ F,
+                                               uint32_t j0, uint32_t j1, double2 p, double& nu, double& w) {
+#pragma unroll 1
+    for (uint32_t j = j0; j < j1; ++j) {
+        const float4 f = F[j];
+        const float dx = (float)(p.x - X[j].x), dz = (float)(p.y - X[j].y);
+        const float r2 = fmaf(dx, dx, dz * dz);
+        float k = r2 >= FLT_MIN ? rcp_approx(r2) : 0.0f;
+        if (r2 < f.y && r2 > 0.0f) k = core_kernel_expm1(r2, f.z, k);
+        const double g = (double)k * f.x;
+        nu += g * dz;
+        w += g * dx;
+    }
+}
+
 // Local expansions of every target group of every listed simulation, one warp per
 // group (the wide groups first, they have the most to translate).  A leaf's walk
 // also meets the leaves to be summed pair by pair and the nodes to be evaluated
@@ -946,8 +966,13 @@ __global__ void __launch_bounds__(32 * WARPS, kNearThreads / (32 * WARPS))
                     }
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
-                        su[t] += (double)(f2lo(nu2[t]) + f2hi(nu2[t]));
-                        sw[t] += (double)(f2lo(w2[t]) + f2hi(w2[t]));
+                        const float fu = f2lo(nu2[t]) + f2hi(nu2[t]), fw = f2lo(w2[t]) + f2hi(w2[t]);
+                        if (fabsf(fu) <= FLT_MAX && fabsf(fw) <= FLT_MAX) {
+                            su[t] += (double)fu;
+                            sw[t] += (double)fw;
+                        } else {
+                            leaf_sum_close(X, F, j0, min(n, j0 + kLeaf), S.at[t * 32 + lane], su[t], sw[t]);
+                        }
                     }
                 }
 #pragma unroll
