@@ -1033,22 +1033,21 @@ __device__ __forceinline__ double rcp_newton(double v) {
     y = fma(y, fma(-v, y, 1.0), y);
     return fma(y, fma(-v, y, 1.0), y);
 }
-// The same for any v: IEEE where the iteration has no range (zero, infinite, NaN or
-// near the ends of the exponents).
-__device__ __forceinline__ double rcp_f64(double v) {
-    const unsigned h = (unsigned)__double2hiint(v);
-    return h - 0x03d00000u < 0x78000000u ? rcp_newton(v) : __drcp_rn(v);
-}
 
-// K(r2) of src/VelocityKernel.cpp:51-57 with rs = 1 / sigma^2, thr = 10 sigma^2.  Where
-// the reciprocal overflows (r2 < 5.6e-309) a core's factor may be 0 and their product
-// NaN, so both are scaled there; r2 = 0 gives NaN, as the reference's division does.
+// K(r2) of src/VelocityKernel.cpp:51-57 with rs = 1 / sigma^2, thr = 10 sigma^2; a division
+// where the iteration has no range (zero, infinite, NaN or near the ends of the
+// exponents: below 5.6e-309 a reciprocal overflows and would make NaN of a core's 0).
+// Called, not inlined: with it in line, or a test of the common path's result, a probe of
+// 3001 points and 60 k blobs takes 430 us instead of 400 (an IEEE reciprocal in line 418),
+// velocities of 40 k blobs 1515 instead of 1481 (1511).
+__device__ __noinline__ double kernel_f64_any(double r2, double thr, double rs) {
+    return ddiv(r2 < thr ? dsub(1.0, exp(dmul(-r2, rs))) : 1.0, r2);
+}
 __device__ __forceinline__ double kernel_f64(double r2, double thr, double rs) {
-    const double y = rcp_f64(r2);
-    if (!(r2 < thr)) return y;
-    const double num = dsub(1.0, exp(dmul(-r2, rs)));
-    if (y > DBL_MAX) return dmul(dmul(num, 0x1p200), __drcp_rn(dmul(r2, 0x1p200)));
-    return dmul(num, y);
+    const unsigned h = (unsigned)__double2hiint(r2);
+    if (h - 0x03d00000u >= 0x78000000u) return kernel_f64_any(r2, thr, rs);
+    const double y = rcp_newton(r2);
+    return r2 < thr ? dmul(dsub(1.0, exp(dmul(-r2, rs))), y) : y;
 }
 
 // Every pair, over the 256-blob tiles of the sorted order; each pair is the
@@ -1292,7 +1291,7 @@ struct AtStage {
 
 // (FP32: three blocks fit an SM by themselves, but told so the compiler's loop is 4 %
 // faster: 256 targets against 2^20 sources 288 us, 300.  FP64: four, at 64 registers; at 68
-// a probe of 3001 points and 60 k blobs took 478 us instead of 416)
+// a probe of 3001 points and 60 k blobs took 478 us instead of 416, before kernel_f64_any)
 template <bool F32>
 __global__ void __launch_bounds__(256, F32 ? 3 : 4) k_at(const AtJob* __restrict__ jobs, int njobs) {
     __shared__ unsigned s_pre[kMaxList + 1];
