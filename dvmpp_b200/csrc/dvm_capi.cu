@@ -1305,26 +1305,37 @@ int dvm_sim_set_blobs(dvm_sim* s, uint64_t n, const double* x, const double* z, 
     SIM_LOCK(s);
     dvm_ctx* c = s->ctx;
     cudaStream_t st = c->stream;
+    const InstDesc& h = s->h;
+    const BlobArrays to{h.x, h.z, h.circ, h.sigma, h.u, h.w, h.uvs, h.wvs, h.id};
+    const double* src[4] = {x, z, circ, sigma};
+    cudaError_t up = cudaSuccess;
+    uint32_t bad = UINT32_MAX;
     // Uploaded to scratch, checked and taken over on the device: a set with a
     // non-finite value leaves the simulation as it was.
     double* v = nullptr;
-    const cudaError_t e = pool_alloc(c, reinterpret_cast<void**>(&v), 32 * n + 16);
-    if (e != cudaSuccess) return fail(DVM_ERR_OOM, std::string("blob upload: ") + cudaGetErrorString(e));
-    uint32_t* d_bad = reinterpret_cast<uint32_t*>(v + 4 * n);
-    const double* src[4] = {x, z, circ, sigma};
-    cudaError_t up = cudaSuccess;
-    for (int k = 0; k < 4 && n && up == cudaSuccess; ++k)
-        up = cudaMemcpyAsync(v + k * n, src[k], 8 * n, cudaMemcpyHostToDevice, st);
-    const InstDesc& h = s->h;
-    if (up == cudaSuccess)
-        take_blobs(v, (uint32_t)n, d_bad,
-                   BlobArrays{h.x, h.z, h.circ, h.sigma, h.u, h.w, h.uvs, h.wvs, h.id},
-                   &c->d_state[s->slot].n, st);
-    g_launches += 2;
-    uint32_t bad = UINT32_MAX;
-    if (up == cudaSuccess)
-        up = cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, st);
-    pool_free(c, v);
+    if (pool_alloc(c, reinterpret_cast<void**>(&v), 32 * n + 16) == cudaSuccess) {
+        uint32_t* d_bad = reinterpret_cast<uint32_t*>(v + 4 * n);
+        for (int k = 0; k < 4 && n && up == cudaSuccess; ++k)
+            up = cudaMemcpyAsync(v + k * n, src[k], 8 * n, cudaMemcpyHostToDevice, st);
+        if (up == cudaSuccess) {
+            take_blobs(v, (uint32_t)n, d_bad, to, &c->d_state[s->slot].n, st);
+            up = cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, st);
+        }
+        g_launches += 2;
+        pool_free(c, v);
+    } else {  // no room for it: checked here and uploaded in place
+        cudaGetLastError();
+        for (uint64_t i = 0; i < n && bad == UINT32_MAX; ++i)
+            if (!std::isfinite(x[i]) || !std::isfinite(z[i]) || !std::isfinite(circ[i]) || !std::isfinite(sigma[i]))
+                bad = (uint32_t)i;
+        if (bad == UINT32_MAX) {
+            double* const dst[4] = {to.x, to.z, to.circ, to.sigma};
+            for (int k = 0; k < 4 && n && up == cudaSuccess; ++k)
+                up = cudaMemcpyAsync(dst[k], src[k], 8 * n, cudaMemcpyHostToDevice, st);
+            if (up == cudaSuccess) fresh_blobs((uint32_t)n, to, &c->d_state[s->slot].n, st);
+            g_launches += 1;
+        }
+    }
     const cudaError_t end = cudaStreamSynchronize(st);
     if (up == cudaSuccess) up = end;
     if (up != cudaSuccess) return fail(DVM_ERR_CUDA, std::string("blob upload: ") + cudaGetErrorString(up));

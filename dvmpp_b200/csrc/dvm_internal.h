@@ -312,6 +312,8 @@ void soa_to_aos(const double* x, const double* z, const double* c, const double*
 // value is not finite: *bad is then the first such blob, else the largest value.
 void take_blobs(const double* v, uint32_t n, uint32_t* bad, const BlobArrays& a, uint32_t* count,
                 cudaStream_t s);
+// The rest of that for a set that is in the arrays already: zero velocities, IDs, count.
+void fresh_blobs(uint32_t n, const BlobArrays& a, uint32_t* count, cudaStream_t s);
 // u += uvs + ux, w += wvs + uz for v = u, w, uvs, wvs.
 void probe_total(double* v, uint32_t n, double ux, double uz, cudaStream_t s);
 // One descriptor, state and list entry, by value.

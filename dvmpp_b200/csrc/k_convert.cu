@@ -58,6 +58,14 @@ __global__ void k_take_blobs(const double* __restrict__ v, uint32_t n,
     if (blockIdx.x == 0 && threadIdx.x == 0) *count = n;
 }
 
+__global__ void k_fresh_blobs(uint32_t n, BlobArrays a, uint32_t* __restrict__ count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        a.u[i] = a.w[i] = a.uvs[i] = a.wvs[i] = 0.0;
+        a.id[i] = i;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = n;
+}
+
 // Probe results: v = u, w, uvs, wvs of n points; u and w become the totals.
 __global__ void k_probe_total(double* __restrict__ v, uint32_t n, double ux, double uz) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -97,6 +105,10 @@ void take_blobs(const double* v, uint32_t n, uint32_t* bad, const BlobArrays& a,
     cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), s);
     if (n) k_check_finite<<<blocks_for(n), 256, 0, s>>>(v, n, bad);
     k_take_blobs<<<n ? blocks_for(n) : 1, 256, 0, s>>>(v, n, bad, a, count);
+}
+
+void fresh_blobs(uint32_t n, const BlobArrays& a, uint32_t* count, cudaStream_t s) {
+    k_fresh_blobs<<<n ? blocks_for(n) : 1, 256, 0, s>>>(n, a, count);
 }
 
 void probe_total(double* v, uint32_t n, double ux, double uz, cudaStream_t s) {

@@ -1,0 +1,61 @@
+"""Calls on a device whose memory is taken.  Setting a simulation's blobs has room of its own
+in the simulation's arrays; without scratch beside them it still gives the same
+state, and still refuses a non-finite value with the simulation left as it was."""
+import numpy as np
+import pytest
+
+from dvmpp_b200 import native as N
+from dvmpp_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _fill(torch):
+    """Takes the device's free memory in blocks (what other allocators keep unused is
+    given back to it on the way) but for 96 to 224 MB."""
+    spare, blocks, size = torch.empty(96 << 20, dtype=torch.uint8, device="cuda"), [], 32 << 30
+    while size >= 128 << 20:
+        try:
+            blocks.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size //= 2
+    del spare
+    torch.cuda.empty_cache()
+    return blocks
+
+
+def test_set_blobs_without_scratch():
+    torch = pytest.importorskip("torch")
+    n = 1 << 23  # 256 MB of blobs
+    rng = np.random.default_rng(5)
+    sets = [[rng.normal(0.0, 1.0, n), rng.normal(0.0, 1.0, n), rng.normal(0.0, 1e-3, n), rng.uniform(0.01, 0.02, n)]
+            for _ in range(2)]
+    with N.Context(0) as c:
+        sim = c.sim(N.Params(capacity=n, precision=N.F32, ux=1.0), *W.circle(16))
+        try:
+            small = [v[:10] for v in sets[0]]
+            sim.set_blobs(*small)  # (the code is on the device)
+            blocks = _fill(torch)
+            try:
+                with pytest.raises(torch.OutOfMemoryError):
+                    torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
+                sim.set_blobs(*sets[0])
+                got = sim.blobs()
+                assert sim.n == n
+                for k, v in zip(("x", "z", "circ", "sigma"), sets[0]):
+                    assert np.array_equal(got[k], v)
+                for k in ("u", "w", "uvs", "wvs"):
+                    assert not np.any(got[k])
+                assert np.array_equal(got["id"], np.arange(n))
+                bad = [v.copy() for v in sets[1]]
+                bad[2][n - 3] = np.inf
+                with pytest.raises(N.DvmError, match=f"blob {n - 3}"):
+                    sim.set_blobs(*bad)
+                assert sim.n == n and np.array_equal(sim.blobs()["circ"], sets[0][2])
+                sim.set_blobs(*sets[1])
+                assert np.array_equal(sim.blobs()["x"], sets[1][0])
+            finally:
+                del blocks
+                torch.cuda.empty_cache()
+        finally:
+            sim.close()
