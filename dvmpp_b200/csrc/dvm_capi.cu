@@ -2271,7 +2271,7 @@ int dvm_ctx_autotune(dvm_ctx* c, dvm_sim* const* sims, int nsims, int reps, dvm_
 }
 
 // ---- plugin seam ---------------------------------------------------------------------
-static int raw_reserve(dvm_ctx* c, size_t bytes) {
+static int raw_reserve(dvm_ctx* c, size_t bytes, bool room_to_grow = true) {
     if (bytes <= c->raw_bytes) return DVM_OK;
     CK(cudaStreamSynchronize(c->stream));
     if (c->raw_block) {
@@ -2280,12 +2280,55 @@ static int raw_reserve(dvm_ctx* c, size_t bytes) {
         c->raw_block = nullptr;
         c->raw_bytes = 0;
     }
-    bytes = align_up(bytes + bytes / 4, 1 << 20);
+    bytes = align_up(room_to_grow ? bytes + bytes / 4 : bytes, 1 << 20);
     if (c->in_use + bytes > c->budget) return fail(DVM_ERR_OOM, "plugin scratch exceeds the HBM budget");
     CK(cudaMalloc(&c->raw_block, bytes));
     c->raw_bytes = bytes;
     c->in_use += bytes;
     return DVM_OK;
+}
+
+// Host calls convert particles on the device, as they are in the caller's memory, through
+// a stage of up to kStage of them (32 MiB), or a quarter of all in place of the room to
+// grow where the budget does not hold both.  Reserves fixed + per * stage bytes for n of them.
+constexpr uint64_t kStage = 1u << 20;
+static int stage_reserve(dvm_ctx* c, size_t fixed, size_t per, uint64_t n, uint64_t* stage) {
+    *stage = std::min(n, kStage);
+    int rc = raw_reserve(c, fixed + per * *stage);
+    if (rc != DVM_ERR_OOM) return rc;
+    *stage = std::min((n + 3) / 4, kStage);
+    return raw_reserve(c, fixed + per * *stage, false);
+}
+
+// n particles into x z circ sigma, n each, at d.
+static int upload_particles(dvm_ctx* c, const dvm_particle* p, uint64_t n, double* d, void* at,
+                            uint64_t stage) {
+    for (uint64_t i = 0; i < n; i += stage) {
+        const uint64_t m = std::min(stage, n - i);
+        CK(cudaMemcpyAsync(at, p + i, sizeof(dvm_particle) * m, cudaMemcpyHostToDevice, c->stream));
+        aos_to_soa(at, (uint32_t)m, d + i, n, c->stream);
+        g_launches += 1;
+    }
+    return DVM_OK;
+}
+
+// n velocities from u and w on the device.
+static int download_velocities(dvm_ctx* c, const double* u, const double* w, uint64_t n,
+                               dvm_velocity* out, void* at, uint64_t stage) {
+    for (uint64_t i = 0; i < n; i += stage) {
+        const uint64_t m = std::min(stage, n - i);
+        velocity_pairs(u + i, w + i, (uint32_t)m, at, c->stream);
+        g_launches += 1;
+        CK(cudaMemcpyAsync(out + i, at, sizeof(dvm_velocity) * m, cudaMemcpyDeviceToHost, c->stream));
+    }
+    return DVM_OK;
+}
+
+static int raw_workspace(dvm_ctx* c, uint64_t n, int precision) {
+    const uint64_t cap = align_up(n, kCapAlign);
+    const uint64_t part =  // FP64 partials
+        precision == kF32 ? 1 : (uint64_t)nbody_chunks((uint32_t)cap) * cap;
+    return ensure_workspace(c, cap, part, 256, 1, 1, 1, false);
 }
 
 // Runs the batched self-induced kernel on caller buffers through table slot 0.
@@ -2317,8 +2360,7 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     e.rhs_chunks = 1;
     e.rhs_chunk = kAtChunk;
     e.npad = 256;
-    const uint64_t part = precision == kF32 ? 1 : (uint64_t)e.chunks * cap;  // FP64 partials
-    int rc = ensure_workspace(c, cap, part, 256, 1, 1, 1, false);
+    const int rc = raw_workspace(c, n, precision);
     if (rc) return rc;
     ListEntry* d_list = reinterpret_cast<ListEntry*>(c->ws.jobs);
     InstState st0;
@@ -2354,19 +2396,17 @@ int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velo
     if (n > 0xF0000000ull) return fail(DVM_ERR_ARG, "too many particles");
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    int rc = raw_reserve(c, 8 * 8 * n);
+    // x z circ sigma | particles staged, then u w | velocities staged
+    uint64_t stage = 0;
+    int rc = raw_workspace(c, n, precision);  // (first: the stage may be smaller)
+    if (!rc) rc = stage_reserve(c, 8 * 6 * n, 16, n, &stage);
     if (rc) return rc;
-    // x z circ sigma | particles, then u w and the velocity pairs in their place
     double* d = static_cast<double*>(c->raw_block);
-    double* aos = d + 4 * n;
-    double* pairs = aos + 2 * n;
-    CK(cudaMemcpyAsync(aos, p, sizeof(dvm_particle) * n, cudaMemcpyHostToDevice, c->stream));
-    aos_to_soa(aos, (uint32_t)n, d, c->stream);
-    rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, aos, aos + n, precision, 0.0, 0.0, 0.0);
+    double* u = d + 4 * n;
+    rc = upload_particles(c, p, n, d, u, stage);
+    if (!rc) rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, u, u + n, precision, 0.0, 0.0, 0.0);
+    if (!rc) rc = download_velocities(c, u, u + n, n, out, u + 2 * n, stage);
     if (rc) return rc;
-    velocity_pairs(aos, aos + n, (uint32_t)n, pairs, c->stream);
-    g_launches += 2;
-    CK(cudaMemcpyAsync(out, pairs, sizeof(dvm_velocity) * n, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return DVM_OK;
 }
@@ -2559,18 +2599,18 @@ int dvm_remesh(dvm_ctx* c, const dvm_particle* in, uint64_t n, const dvm_remesh_
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    // particles in, x z circ sigma | x z circ sigma out, particles out | count
+    // x z circ sigma | x z circ sigma out | count | particles staged
     const size_t in_b = align_up(8 * 4 * (size_t)n, 256), out_b = align_up(8 * 4 * (size_t)out_cap, 256);
-    const size_t data = 2 * in_b + 2 * out_b + 256;
-    rc = raw_reserve(c, data);
+    uint64_t stage = 0;
+    rc = stage_reserve(c, in_b + out_b + 256, sizeof(dvm_particle), std::max(n, out_cap), &stage);
     if (rc) return rc;
     char* base = static_cast<char*>(c->raw_block);
-    double* din = reinterpret_cast<double*>(base + in_b);
-    double* dout = reinterpret_cast<double*>(base + 2 * in_b);
-    char* aos_out = base + 2 * in_b + out_b;
-    uint32_t* dneed = reinterpret_cast<uint32_t*>(base + data - 256);
-    if (n) CK(cudaMemcpyAsync(base, in, sizeof(dvm_particle) * n, cudaMemcpyHostToDevice, c->stream));
-    aos_to_soa(base, (uint32_t)n, din, c->stream);
+    double* din = reinterpret_cast<double*>(base);
+    double* dout = reinterpret_cast<double*>(base + in_b);
+    uint32_t* dneed = reinterpret_cast<uint32_t*>(base + in_b + out_b);
+    void* at = base + in_b + out_b + 256;
+    rc = upload_particles(c, in, n, din, at, stage);
+    if (rc) return rc;
     void* scratch = nullptr;
     const cudaError_t e = pool_alloc(c, &scratch, remesh_scratch_bytes(g, (uint32_t)n, (uint32_t)out_cap));
     if (e != cudaSuccess) return fail(DVM_ERR_OOM, std::string("remesh scratch: ") + cudaGetErrorString(e));
@@ -2579,19 +2619,24 @@ int dvm_remesh(dvm_ctx* c, const dvm_particle* in, uint64_t n, const dvm_remesh_
     remesh_run(g, din, din + n, din + 2 * n, din + 3 * n, (uint32_t)n, (uint32_t)out_cap, d,
                nullptr, scratch, c->sms, c->stream);
     pool_free(c, scratch);
-    soa_to_aos(dout, dout + out_cap, dout + 2 * out_cap, dout + 3 * out_cap, dneed,
-               (uint32_t)out_cap, aos_out, c->stream);
-    g_launches += 9;
+    auto particles = [&](uint64_t i) {  // the stage's fill from blob i on
+        soa_to_aos(dout, dout + out_cap, dout + 2 * out_cap, dout + 3 * out_cap, dneed, (uint32_t)i,
+                   (uint32_t)std::min(stage, out_cap - i), at, c->stream);
+    };
+    particles(0);
+    g_launches += 8;
     uint32_t need = 0;
     CK(cudaMemcpyAsync(&need, dneed, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     *n_out = need;
     if (need > out_cap)
         return fail(DVM_ERR_CAPACITY, "remesh: " + std::to_string(need) + " blobs do not fit out_cap");
-    if (need) {
-        CK(cudaMemcpyAsync(out, aos_out, sizeof(dvm_particle) * need, cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
+    for (uint64_t i = 0; i < need; i += stage) {
+        if (i) particles(i);
+        CK(cudaMemcpyAsync(out + i, at, sizeof(dvm_particle) * std::min<uint64_t>(stage, need - i),
+                           cudaMemcpyDeviceToHost, c->stream));
     }
+    if (need) CK(cudaStreamSynchronize(c->stream));
     return DVM_OK;
 }
 
@@ -2640,26 +2685,26 @@ int dvm_biot_savart_at(dvm_ctx* c, const dvm_particle* p, uint64_t ns, const dou
     CK(cudaSetDevice(c->device));
     const size_t elems = direct_at_part_elems((uint32_t)ns, (uint32_t)nt);
     const size_t part_bytes = align_up(16 * elems, 256);
-    // x z circ sigma | tx tz | u w | particles, later velocities
-    const size_t aos = std::max<size_t>(sizeof(dvm_particle) * ns, sizeof(dvm_velocity) * nt);
-    const size_t data_bytes = align_up(8 * (4 * ns + 4 * nt), 256) + aos;
-    int rc = raw_reserve(c, part_bytes + data_bytes);
+    // partials | x z circ sigma | tx tz | u w | particles, later velocities staged
+    uint64_t stage = 0;
+    int rc = stage_reserve(c, part_bytes + align_up(8 * (4 * ns + 4 * nt), 256), sizeof(dvm_particle),
+                           std::max(ns, (nt + 1) / 2), &stage);
     if (rc) return rc;
     char* base = static_cast<char*>(c->raw_block);
     double* d = reinterpret_cast<double*>(base + part_bytes);
-    void* d_aos = base + part_bytes + align_up(8 * (4 * ns + 4 * nt), 256);
+    void* at = base + part_bytes + align_up(8 * (4 * ns + 4 * nt), 256);
     double* dt = d + 4 * ns;
-    if (ns) CK(cudaMemcpyAsync(d_aos, p, sizeof(dvm_particle) * ns, cudaMemcpyHostToDevice, c->stream));
-    aos_to_soa(d_aos, (uint32_t)ns, d, c->stream);
+    rc = upload_particles(c, p, ns, d, at, stage);
+    if (rc) return rc;
     CK(cudaMemcpyAsync(dt, tx, 8 * nt, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(dt + nt, tz, 8 * nt, cudaMemcpyHostToDevice, c->stream));
     double* du = dt + 2 * nt;
     double* dw = du + nt;
     direct_at_raw(d, d + ns, d + 2 * ns, d + 3 * ns, (uint32_t)ns, dt, dt + nt, (uint32_t)nt, du, dw,
                   precision, 1, reinterpret_cast<double2*>(base), c->sms, c->stream);
-    velocity_pairs(du, dw, (uint32_t)nt, d_aos, c->stream);
-    g_launches += 4;
-    CK(cudaMemcpyAsync(out, d_aos, sizeof(dvm_velocity) * nt, cudaMemcpyDeviceToHost, c->stream));
+    g_launches += 2;
+    rc = download_velocities(c, du, dw, nt, out, at, 2 * stage);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
     return DVM_OK;
 }

@@ -301,13 +301,14 @@ struct BlobArrays {
     double *x, *z, *circ, *sigma, *u, *w, *uvs, *wvs;
     uint32_t* id;
 };
-// n particles (x, z, circ, sigma) to four arrays.
-void aos_to_soa(const void* in, uint32_t n, double* out, cudaStream_t s);
+// m particles (x, z, circ, sigma) to the first m places of four arrays, or from out's
+// place in them on.
+void aos_to_soa(const void* in, uint32_t m, double* out, uint64_t n, cudaStream_t s);
 // n pairs (u, w).
 void velocity_pairs(const double* u, const double* w, uint32_t n, void* out, cudaStream_t s);
-// min(*n, cap) particles.
+// Particles first .. min(*n, first + cap) - 1.
 void soa_to_aos(const double* x, const double* z, const double* c, const double* sg,
-                const uint32_t* n, uint32_t cap, void* out, cudaStream_t s);
+                const uint32_t* n, uint32_t first, uint32_t cap, void* out, cudaStream_t s);
 // Blob set v (x, z, circ, sigma) into a simulation's arrays and count, unless a
 // value is not finite: *bad is then the first such blob, else the largest value.
 void take_blobs(const double* v, uint32_t n, uint32_t* bad, const BlobArrays& a, uint32_t* count,

@@ -7,13 +7,14 @@
 namespace dvmk {
 namespace {
 
-__global__ void k_aos_to_soa(const double4* __restrict__ in, uint32_t n, double* __restrict__ out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+__global__ void k_aos_to_soa(const double4* __restrict__ in, uint32_t m, double* __restrict__ out,
+                             size_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
         const double4 v = in[i];
         out[i] = v.x;
-        out[n + (size_t)i] = v.y;
-        out[2 * (size_t)n + i] = v.z;
-        out[3 * (size_t)n + i] = v.w;
+        out[n + i] = v.y;
+        out[2 * n + i] = v.z;
+        out[3 * n + i] = v.w;
     }
 }
 
@@ -25,11 +26,13 @@ __global__ void k_pairs(const double* __restrict__ u, const double* __restrict__
 
 __global__ void k_soa_to_aos(const double* __restrict__ x, const double* __restrict__ z,
                              const double* __restrict__ c, const double* __restrict__ s,
-                             const uint32_t* __restrict__ n, uint32_t cap,
+                             const uint32_t* __restrict__ n, uint32_t first, uint32_t cap,
                              double4* __restrict__ out) {
-    const uint32_t m = min(n[0], cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-        out[i] = make_double4(x[i], z[i], c[i], s[i]);
+    const uint32_t m = n[0] > first ? min(n[0] - first, cap) : 0u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const size_t j = (size_t)first + i;
+        out[i] = make_double4(x[j], z[j], c[j], s[j]);
+    }
 }
 
 // Least index with a non-finite value in any of four arrays of n (bad starts at
@@ -87,8 +90,8 @@ unsigned blocks_for(uint64_t n) {
 
 }  // namespace
 
-void aos_to_soa(const void* in, uint32_t n, double* out, cudaStream_t s) {
-    if (n) k_aos_to_soa<<<blocks_for(n), 256, 0, s>>>(static_cast<const double4*>(in), n, out);
+void aos_to_soa(const void* in, uint32_t m, double* out, uint64_t n, cudaStream_t s) {
+    if (m) k_aos_to_soa<<<blocks_for(m), 256, 0, s>>>(static_cast<const double4*>(in), m, out, n);
 }
 
 void velocity_pairs(const double* u, const double* w, uint32_t n, void* out, cudaStream_t s) {
@@ -96,8 +99,9 @@ void velocity_pairs(const double* u, const double* w, uint32_t n, void* out, cud
 }
 
 void soa_to_aos(const double* x, const double* z, const double* c, const double* sg,
-                const uint32_t* n, uint32_t cap, void* out, cudaStream_t s) {
-    if (cap) k_soa_to_aos<<<blocks_for(cap), 256, 0, s>>>(x, z, c, sg, n, cap, static_cast<double4*>(out));
+                const uint32_t* n, uint32_t first, uint32_t cap, void* out, cudaStream_t s) {
+    if (cap)
+        k_soa_to_aos<<<blocks_for(cap), 256, 0, s>>>(x, z, c, sg, n, first, cap, static_cast<double4*>(out));
 }
 
 void take_blobs(const double* v, uint32_t n, uint32_t* bad, const BlobArrays& a, uint32_t* count,
