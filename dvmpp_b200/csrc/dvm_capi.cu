@@ -80,6 +80,25 @@ int nbody_chunks(uint32_t cap) {
     return std::max(1, std::min(most, std::max(by_size, by_fill)));
 }
 
+// Upper bound of the FP64 partials, sum chunks * cap, of up to `sims` simulations whose
+// capacities sum up to `total`: the least over some slopes of slope * total + sims *
+// the most by which one simulation's partials exceed slope * cap.  Chunks are 32 from
+// 2^20 blobs on, so beyond it the largest capacity alone need be looked at.
+uint64_t nbody_part_bound(uint64_t total, uint64_t sims) {
+    uint64_t best = UINT64_MAX;
+    for (uint64_t slope = 8; slope <= 256; slope += 8) {
+        uint64_t over = 0;
+        auto look = [&](uint64_t cap) {
+            const uint64_t part = (uint64_t)nbody_chunks((uint32_t)cap) * cap;
+            if (part > slope * cap) over = std::max(over, part - slope * cap);
+        };
+        for (uint64_t cap = kCapAlign; cap <= std::min<uint64_t>(total, 1u << 20); cap += kCapAlign) look(cap);
+        look(std::min<uint64_t>(total, UINT32_MAX / kCapAlign * kCapAlign));
+        best = std::min(best, slope * total + sims * over);
+    }
+    return best;
+}
+
 }  // namespace
 
 struct SubList {
@@ -906,12 +925,17 @@ int dvm_ctx_reserve(dvm_ctx* c, uint64_t total_capacity, int max_sims, int max_p
     CK(cudaSetDevice(c->device));
     const uint64_t S = (uint64_t)max_sims;
     const uint64_t T = align_up(total_capacity, kCapAlign) + S * kCapAlign;
-    // bounds of the per-list sums: chunks*cap <= 16 cap + 2^21; rhs chunks per
+    // bounds of the per-list sums: FP64 partials (nbody_part_bound); rhs chunks per
     // simulation <= 601 or cap / kAtChunk + 1 (rhs_chunk_for)
-    const uint64_t part = 16 * T + S * (2u << 20);
+    const uint64_t part = nbody_part_bound(T, S), enough = 16 * T + S * (2u << 20);
     const uint64_t rchunks = T / kAtChunk + S * 602;
-    return ensure_workspace(c, T, part, rchunks * align_up((size_t)max_panels, 256), rchunks,
-                            S * (uint64_t)max_panels, max_sims, with_delete != 0);
+    auto size = [&](uint64_t part) {
+        return ensure_workspace(c, T, part, rchunks * align_up((size_t)max_panels, 256), rchunks,
+                                S * (uint64_t)max_panels, max_sims, with_delete != 0);
+    };
+    // (a budget that does not hold every batch's partials may hold those there will be)
+    const int rc = size(part);
+    return rc == DVM_ERR_OOM && enough < part ? size(enough) : rc;
 }
 
 int dvm_ctx_pool_reserve(dvm_ctx* c, uint64_t bytes) {
