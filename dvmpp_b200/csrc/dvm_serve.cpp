@@ -210,8 +210,7 @@ int dvm_server_run(dvm_server* s, int serial, int realtime) {
         for (Request* r : pre) {
             slabs.push_back(r->bytes);
             const uint64_t np = r->bx.size() - 1;  // influence + factorisation scratch
-            scratch = std::max<uint64_t>(
-                scratch, 8 * (2 * np * np + dvmk::pseudo_inverse_work_doubles((int)np)));
+            scratch = std::max<uint64_t>(scratch, 8 * dvmk::pseudo_inverse_work_doubles((int)np));
         }
         std::sort(slabs.rbegin(), slabs.rend());
         uint64_t want = scratch;

@@ -27,3 +27,32 @@ def test_first_step_after_reserve(caps):
         assert c.memory()[0] == before
         for s in sims:
             s.close()
+
+
+def test_server_reserves_one_set_up():
+    """A server's run holds device memory for its workspace, the largest simulations and one
+    body's set-up scratch (about 32 np^2 bytes), with 48 MB for the pool's
+    granularity and a context's own tables."""
+    torch = pytest.importorskip("torch")
+    npan = 2047
+
+    def run(c, panels):
+        srv = N.Server(c)
+        p = N.Params(capacity=1024 + 4 * panels, precision=N.F32, rng=N.RNG_PHILOX, ux=1.0, dt=0.02)
+        srv.submit(p, *W.circle(panels), 1)
+        srv.run()
+        assert srv.stats()["completed"] == 1
+        srv.close()
+        return N.sim_bytes(p, panels)
+
+    with N.Context(0) as c:
+        run(c, 300)  # (code on the device)
+    with N.Context(0) as c:
+        free0 = torch.cuda.mem_get_info()[0]
+        slab = run(c, npan)
+        taken = free0 - torch.cuda.mem_get_info()[0]
+        ws = N.C.c_uint64()
+        assert c.lib.dvm_ctx_workspace_bytes(c.h, N.C.byref(ws)) == 0
+        m = npan + 1
+        work = 8 * (2 * npan * npan + m * (npan + m) + 2 * m + 2 * npan + 8)
+        assert taken <= ws.value + slab + work + 48 * (1 << 20)
