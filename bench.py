@@ -12,7 +12,9 @@ each); value = simulation-steps per second over the whole job.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-One JSON line on rank 0.  Multi-GPU runs are replicas (each rank runs its own
+One short JSON line on rank 0 (a few kB: a log that keeps only the end of the output still
+holds all of it); the full record, with the accuracy of every simulation, the phases
+and the serving legs, goes to stderr or to --details FILE.  Multi-GPU runs are replicas (each rank runs its own
 copy of the batch; no data-path collective).
 """
 from __future__ import annotations
@@ -499,6 +501,34 @@ def run_f64(ctx, instances, steps_total, warmup, steps):
     return ms
 
 
+def short_line(line):
+    """What is printed of the full record: the measured figures, without the explanations
+    and the lists by simulation, request or phase."""
+    def pick(d, *keys):
+        return {k: d[k] for k in keys if k in d}
+
+    out = pick(line, "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+               "scaling", "vs_baseline", "dtype", "data", "config", "gpu_launches", "clocks", "setup_s", "f64_value",
+               "nbody")
+    for key, keys in (("plain_gpu", ("value", "unit", "ratio_batched_over_plain")),
+                      ("roofline", ("bound", "kernel", "achieved", "peak", "unit", "frac", "traffic", "launch_ms",
+                                    "share_of_step")),
+                      ("e2e", ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")),
+                      ("cpu_baseline", ("value", "unit", "cores", "kind")),
+                      ("accuracy", ("simulations", "pooled_rel_l2", "within_bounds"))):
+        if key in line:
+            out[key] = pick(line[key], *keys)
+    serving = line.get("serving", {})
+    if serving:
+        live = serving.get("realtime_live", {}).get("batched", {})
+        full = serving.get("saturated", {})
+        out["serving"] = {
+            **pick(serving, "requests"), **pick(live, "latency_p50_s", "latency_p99_s"),
+            **pick(full.get("batched", {}), "completed", "sim_steps_per_s"),
+            **pick(full, "ratio_batched_over_serial")}
+    return out
+
+
 def run_ours(args, dist):
     from dvmpp_b200 import native as N
 
@@ -780,7 +810,12 @@ def run_ours(args, dist):
             "panels": "U{64..512}", "budget_gb": 150.0, "max_active": 256,
             "bodies": "circle / ellipse / rounded square / Joukowski", **legs}
     if dist.rank == 0:
-        print(json.dumps(line))
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(line, f, indent=1)
+        else:
+            sys.stderr.write(json.dumps(line) + "\n")
+        print(json.dumps(short_line(line)))
     if accuracy and not accuracy["within_bounds"]:
         sys.stderr.write("accuracy outside its bounds: " + json.dumps(accuracy["worst"]) + "\n")
         sys.exit(3)
@@ -812,6 +847,8 @@ def main(argv=None):
                     help="range of the serving requests' step counts")
     ap.add_argument("--no-serial", action="store_true",
                     help="skip the serial plain-GPU serving run")
+    ap.add_argument("--details", metavar="FILE",
+                    help="where the full record goes (stderr without it)")
     ap.add_argument("--traffic", type=float, default=None,
                     help="dram bytes per pair-kernel launch from an ncu capture")
     args = ap.parse_args(argv)
