@@ -5,7 +5,7 @@ Workload ("batched", the metric's configuration): 64 independent bodies --
 circle R=0.5, ellipses of aspect U[1,4], rounded squares (side 1, corner
 radius 0.05) -- with panel counts log-uniform in [64, 512], each pre-seeded
 with a wake of log-uniform 1e4..4e5 blobs (seeded synthetic data), Euler,
-dt = 0.005, nu = 1e-3, ux = 1, REFLECT, FP32 compensated pair sums.
+dt = 0.005, nu = 1e-3, ux = 1, REFLECT, FP32 mode.
 
 A "step" advances all 64 simulations by one time step (DVMBase::compute_step
 each); value = simulation-steps per second over the whole job.
@@ -425,11 +425,11 @@ def evaluate(sim, N):
 
 
 def accuracy_vs_f64(ctx, sims, bodies, params):
-    """The timed FP32-compensated arithmetic against FP64 on the identical
+    """The timed FP32 arithmetic against FP64 on the identical
     state of every simulation of the batch: each FP32 simulation evaluates its
-    current state in place (the same kernels and source chunking as its
+    current state in place (the same kernels as its
     batched step); an FP64 copy of that state (same body and capacity) does
-    the same in the reference's operation order.  Per simulation: rel-L2 and
+    the same with the reference's formulas.  Per simulation: rel-L2 and
     max-norm errors of u, w (blob-on-blob), uvs, wvs (sheet-on-blob), the total
     induced velocity (u + uvs, w + wvs) and gamma; Cd and Cl errors relative to
     the force coefficient's magnitude |(Cd, Cl)|."""
@@ -468,7 +468,7 @@ def accuracy_vs_f64(ctx, sims, bodies, params):
     ok = (all(worst[k + "_rel_l2"] <= ACC_REL_L2 for k in sq)
           and worst["cd_err"] <= ACC_FORCE_REL and worst["cl_err"] <= ACC_FORCE_REL)
     return {"simulations": len(per), "blobs": int(sum(r["n"] for r in per)),
-            "how": "FP32 step arithmetic vs FP64 (reference operation order) on the identical "
+            "how": "FP32 step arithmetic vs FP64 (the reference's formulas, all pairs) on the identical "
                    "state of every simulation after the timed steps; rel-L2 per simulation (worst "
                    "shown) and pooled over all blobs; Cd / Cl error relative to |(Cd, Cl)| of FP64",
             "bounds": {"rel_l2": ACC_REL_L2, "cd_cl": ACC_FORCE_REL},
@@ -477,7 +477,7 @@ def accuracy_vs_f64(ctx, sims, bodies, params):
 
 
 def run_f64(ctx, instances, steps_total, warmup, steps):
-    """The same batch with every pair sum in FP64 (reference operation order):
+    """The same batch with every pair summed in FP64 (the reference's formulas):
     fresh simulations from the same initial state, Philox walk; graph-replayed
     batched steps timed with CUDA events on the library's stream."""
     from dvmpp_b200 import native as N
@@ -718,18 +718,18 @@ def run_ours(args, dist):
         f64 = {"value": dist.world * args.instances * args.f64_steps / (f64_ms / 1e3), "unit": UNIT,
                "steps": args.f64_steps, "ms_per_step": f64_ms / args.f64_steps,
                "how": "the same 64 simulations from the same initial state with every pair "
-                      "sum in FP64 in the reference's operation order (the arithmetic of the "
-                      "reference arm), Philox walk, graph-replayed batched steps after one "
+                      "summed in FP64 with the reference's formulas (the reference arm's "
+                      "arithmetic), Philox walk, graph-replayed batched steps after one "
                       "warm-up step; CUDA events"}
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": dist.world,
         "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_max / args.steps, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 pair sums (Kahan), f64 state/sheet",
+        "vs_baseline": None, "dtype": "f32 near pairs, f64 far field and state",
         "data": "synthetic (seeded bodies and wakes)",
         "config": {"workload": "batched: 64 mixed bodies (circle / ellipse aspect U[1,4] / "
                                "rounded square), panels log-U[64,512], wakes log-U[1e4,4e5] "
-                               "blobs, Euler dt=0.005, nu=1e-3, ux=1, REFLECT, FP32 compensated",
+                               "blobs, Euler dt=0.005, nu=1e-3, ux=1, REFLECT, FP32 mode",
                    "instances": args.instances, "blobs_total": int(sum(nblobs)),
                    "panels_total": int(sum(s.np for s in sims)),
                    "parallelism": f"replicas x{dist.world}" if dist.world > 1 else "single GPU",

@@ -6,20 +6,20 @@ nbody: the standalone regularised Biot-Savart workload -- N blobs, 70 % in a
 wake x ~ U[0.5, 20], z ~ N(0, 1), 30 % in the annulus 0.5 < r < 1.5,
 Gamma ~ N(0, 1e-3) summing to zero, sigma = 0.081880 (ds^0.675 of the
 128-panel R = 0.5 circle), seed 2.  Prints one JSON line with the pair
-kernel's CUDA-event time, pairs/s, FP32-pipe fraction and (with both
+kernels' CUDA-event time, the pairs it stands for per second and (with both
 precisions) the FP32-vs-FP64 error.
 
     python -m dvmpp_b200.cases precision [--steps 20] [--n-wake 524288] [--panels 1024]
                                          [--eval-every 50] [--f64-steps 150]
 
 precision: ellipse (0.5, 0.25) at 20 degrees, 1024 panels (a 1025 x 1024
-influence matrix), a 2^19-blob wake, RK3 dt = 0.002; the FP32-compensated run
-(FP64 QR, FP64 refinement and Kelvin row) against an all-FP64 run.
+influence matrix), a 2^19-blob wake, RK3 dt = 0.002; the FP32 run
+(FP64 pseudo-inverse, refinement and Kelvin row) against an all-FP64 run.
 
     python -m dvmpp_b200.cases sheet [--n 131072] [--panels 1024] [--reps 3]
 
 sheet: the FP32 sheet-on-blob velocity alone (ellipse at 20 degrees, wake of
-n blobs); prints its CUDA-event time, pairs/s and FP32 fraction (67 flop/pair).
+n blobs); prints its CUDA-event time and the pairs it stands for per second.
 
     python -m dvmpp_b200.cases book [--n 4194304] [--panels 256] [--inside 0.02]
 
@@ -28,7 +28,7 @@ book: the Philox walk, REFLECT and DELETE alone on one simulation (CUDA events).
     python -m dvmpp_b200.cases rhs [--n 131072] [--panels 1024] [--reps 3]
 
 rhs: the blob-on-collocation right-hand side alone (same body and wake);
-prints its CUDA-event time per launch, pairs/s and FP32 fraction (12 flop/pair).
+prints its CUDA-event time per launch and the pairs it stands for per second.
 
     python -m dvmpp_b200.cases serve [--requests 100] [--serial] [--realtime] [--live]
 
@@ -216,8 +216,7 @@ def run_precision(steps: int, n_wake: int, npanels: int = 1024, seed: int = 2,
     """Sheet-solve precision: an ellipse (semi-axes 0.5, 0.25) at the given
     incidence, npanels panels, a wake of n_wake blobs (the N-body distribution,
     core size ds^0.675 of this body), RK3 with dt = 0.002, nu = 1e-3, ux = 1.
-    One run with FP32 compensated pair sums (FP64 QR + FP64 refinement,
-    Kelvin row in FP64) for `steps` steps beside an all-FP64 run from the same
+    One run in FP32 mode (FP64 pseudo-inverse, refinement and Kelvin row) for `steps` steps beside an all-FP64 run from the same
     state and the same Philox stream for the first `f64_steps` of them (all by
     default).  Reports per-step gamma / Cd / Cl differences while both run,
     the blob counts, the least-squares solvers against each other on one

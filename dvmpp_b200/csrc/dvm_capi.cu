@@ -2357,8 +2357,7 @@ static int raw_workspace(dvm_ctx* c, uint64_t n, int precision) {
 
 // Runs the batched self-induced kernel on caller buffers through table slot 0.
 static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* circ,
-                    const double* sigma, uint64_t n, double* u, double* w, int precision,
-                    double kx0, double kz0, double kinv) {  // kinv 0: domain from the blobs
+                    const double* sigma, uint64_t n, double* u, double* w, int precision) {
     if (n == 0) return DVM_OK;
     if (n > 0xF0000000ull) return fail(DVM_ERR_ARG, "too many particles");
     const uint64_t cap = align_up(n, kCapAlign);
@@ -2372,9 +2371,6 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     h.w = w;
     h.cap = (uint32_t)cap;
     h.precision = precision;
-    h.kx0 = kx0;
-    h.kz0 = kz0;
-    h.kinv = kinv;
     h.np = 1;
     ListEntry e;
     std::memset(&e, 0, sizeof(e));
@@ -2394,7 +2390,7 @@ static int raw_self(dvm_ctx* c, const double* x, const double* z, const double* 
     Workspace ws = c->ws;
     ws.key_bits = key_bits_for(1);
     ws.total_cap = cap;
-    if (!(kinv > 0.0)) set_domain(c->d_table, x, z, (uint32_t)n, ws, c->sms, c->stream);
+    set_domain(c->d_table, x, z, (uint32_t)n, ws, c->sms, c->stream);
     biot_savart_self(c->d_table, c->d_state, d_list, 1, precision, ws, c->sms, c->stream,
                      tuned_config(c, shape_class(cap, 1)));
     g_launches += 4;  // keys, pack, pair kernel, combine
@@ -2409,7 +2405,7 @@ int dvm_biot_savart_self_device(dvm_ctx* c, const double* x, const double* z, co
     if (precision != DVM_F64 && precision != DVM_F32) return fail(DVM_ERR_ARG, "bad precision");
     std::lock_guard<std::mutex> lk(c->mu);
     CK(cudaSetDevice(c->device));
-    return raw_self(c, x, z, circ, sigma, n, u, w, precision, 0.0, 0.0, 0.0);
+    return raw_self(c, x, z, circ, sigma, n, u, w, precision);
 }
 
 int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velocity* out,
@@ -2428,7 +2424,7 @@ int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velo
     double* d = static_cast<double*>(c->raw_block);
     double* u = d + 4 * n;
     rc = upload_particles(c, p, n, d, u, stage);
-    if (!rc) rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, u, u + n, precision, 0.0, 0.0, 0.0);
+    if (!rc) rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, u, u + n, precision);
     if (!rc) rc = download_velocities(c, u, u + n, n, out, u + 2 * n, stage);
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));

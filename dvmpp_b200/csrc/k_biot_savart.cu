@@ -8,11 +8,12 @@
 // FP32 path (the throughput path): blobs of every listed simulation are sorted
 // along a Hilbert curve, packed as FP64 (x, z) + FP32 (Gamma, 10 sigma^2,
 // 1/sigma^2) and cut into leaves of 64 blobs.  A binary tree over the leaves
-// carries FP64 expansions of the field outside the cores (dvm_tree.cuh).  A block
-// takes one leaf of targets: it walks the tree, translates every node that is
-// far enough into a local expansion about the leaf, and sums the few leaves
-// that remain pair by pair in packed FP32x2 arithmetic, each with the core
-// test only where a core can reach.  Coordinates are FP32 offsets from the
+// carries FP64 expansions of the field outside the cores (dvm_tree.cuh).  k_far, a
+// warp per group of targets, walks the tree, translates every node that is far
+// enough into a local expansion about the group and lists the few leaves that
+// remain; k_self_f32, a block per leaf of targets, sums those pair by pair in packed
+// FP32x2 arithmetic, each with the core test only where a core can reach, and
+// adds the local expansions.  Coordinates are FP32 offsets from the
 // target leaf's first blob; sums are FP32 within a source leaf and FP64 across
 // leaves, in an order that the simulation's own blobs fix: deterministic, and
 // independent of the batch a simulation runs in and of the launch shape.
@@ -224,8 +225,8 @@ __device__ __forceinline__ int scale_exp(double R) {  // 2^e > R, clamped
 }
 
 // Gather the blobs in sorted order, and build the tree bottom up.  A block makes
-// 32 consecutive leaves (box, radius, moments; one warp each at a time) and the
-// five levels above them in shared memory, one warp per node (moment-to-moment
+// 16 consecutive leaves (box, radius, moments; one warp each at a time) and the
+// four levels above them in shared memory, one warp per node (moment-to-moment
 // translations as a convolution with the factorials divided out).  Of 16
 // neighbouring blocks the one that finishes last goes on with their 16 top nodes
 // in the same way, and so on up to the root; nobody waits.  A node is always
@@ -235,8 +236,8 @@ __device__ __forceinline__ int scale_exp(double R) {  // 2^e > R, clamped
 // What bounds it is latency (a gather, then a chain of small FP64 steps), so the
 // levels inside a block meet no memory fence: with one arrival counter per
 // node and a fence at each the kernel took 284 us for 2^20 blobs, 93 for 250 k and
-// 38 for 5003, against 174, 55 and 29 us this way (32 leaves per block: 143, 75
-// and 36).
+// 38 for 5003, against 174, 55 and 29 us this way (32 leaves and five levels per
+// block: 143, 75 and 36).
 constexpr int kFan = 16;  // nodes of the lowest level of a block's share
 constexpr int kFanLevels = 4;
 struct TreeShared {
@@ -1202,7 +1203,7 @@ struct AtJob {
     const uint32_t* pns;  // source count on the device, or null -> ns
     uint32_t ns;
     int npad;             // partial row length
-    uint32_t chunk;       // sources per work item (a multiple of 256)
+    uint32_t chunk;       // sources per work item (64, 128 or a multiple of 256)
     double2* part;        // [chunk][npad]
     double* circ_part;    // [chunk], or null
 };

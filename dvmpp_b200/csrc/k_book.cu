@@ -256,8 +256,8 @@ __device__ __forceinline__ void load_contour(const InstDesc& d, double* sx, doub
 // items of 256 or 1024, each warp going through its own 32, they were one or a few
 // blocks' work (1024 panels, RK3, DELETE: 231 us, 31 now; 128 panels, 2 k blobs,
 // REFLECT: 22-43 us, 12-29 now).
-// An item costs four barriers and a counter's turn, though, so from 2^20 blobs
-// (capacity) on, where there are plenty of them, items are 256 (4 M blobs, REFLECT
+// An item costs four barriers and a counter's turn, though, so in batches of more than
+// 2^20 blobs of capacity in all, where there are plenty of them, items are 256 (4 M blobs, REFLECT
 // and the whole DELETE: 0.51 and 0.56 ms in items of 64, 0.24 and 0.38 in these).
 constexpr uint32_t kCrossItem = 64, kCrossMost = 256;
 constexpr uint64_t kCrossLarge = 1u << 20;

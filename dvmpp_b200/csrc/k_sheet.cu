@@ -3,9 +3,9 @@
 // velocity fused with the convection update (src/VortexSheet.cpp:217-273,
 // src/DVMBase.cpp:167-209) and the pressure loads (src/VortexSheet.cpp:487-514).
 //
-// FP64 instances: pair formulas keep the reference's operation order with one
-// rounding per operation (dadd/dmul/...), so they round like the reference
-// compiled without FP contraction.  FP32 instances evaluate the near sheet-on-blob
+// FP64 instances: the reference's pair formulas, one rounding per operation
+// (dadd/dmul/...); A in its operation order, the sheet velocity with a panel's length
+// divided by as its reciprocal and a blob's panels summed in sixteen parts.  FP32 instances evaluate the near sheet-on-blob
 // panel terms in single precision (accumulated in FP64) and the far ones by FP64
 // expansions; the influence matrix, P, solve, refinement and loads are FP64 for
 // both.

@@ -6,7 +6,7 @@
 // complete when solve() / run() return).  The random walk uses the reference's stream
 // (constants/seed through std::mt19937) unless algorithms/diffusion_rng is
 // "philox".  algorithms/velocity_kernel selects the pair arithmetic:
-// "direct" (default, FP64) or "cuda" (FP32 with compensated sums).
+// "direct" (default, FP64) or "cuda" (FP32 near pairs, FP64 far field).
 #ifndef DVMPP_B200_DVMBASE_HPP
 #define DVMPP_B200_DVMBASE_HPP
 

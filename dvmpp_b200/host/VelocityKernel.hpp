@@ -1,9 +1,9 @@
 // The reference's velocity-kernel plugin seam (src/VelocityKernel.hpp:12-62)
 // with GPU implementations behind it:
 //   create("direct")  DirectKernel -- the reference's direct O(N^2) sum,
-//                     FP64 on the GPU (same operation order)
-//   create("cuda")    CudaKernel   -- FP32 pair sums with compensated
-//                     accumulation on the GPU
+//                     FP64 on the GPU (the same formulas)
+//   create("cuda")    CudaKernel   -- on the GPU: near pairs in FP32, far ones
+//                     by FP64 expansions; at targets compensated FP32 pairs
 //   create("cuda64")  CudaKernel in FP64
 // Unknown names throw dvm::AlgorithmException, as the reference's factory does.
 #ifndef DVMPP_B200_VELOCITYKERNEL_HPP
