@@ -2475,6 +2475,15 @@ int dvm_biot_savart_at_device(dvm_ctx* c, const double* x, const double* z, cons
 }
 
 // ---- vortex merging ----------------------------------------------------------------------
+static cudaError_t merge_scratch(dvm_ctx* c, uint32_t n, void** scratch, bool* rounds) {
+    *rounds = true;
+    const cudaError_t e = pool_alloc(c, scratch, merge_scratch_bytes(n, true));
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    *rounds = false;
+    return pool_alloc(c, scratch, merge_scratch_bytes(n, false));
+}
+
 int dvm_sim_merge(dvm_sim* s, double threshold, uint64_t* merged) {
     if (!s) return fail(DVM_ERR_ARG, "sim is null");
     dvm_ctx* c = s->ctx;
@@ -2487,14 +2496,15 @@ int dvm_sim_merge(dvm_sim* s, double threshold, uint64_t* merged) {
                            c->stream));
         CK(cudaStreamSynchronize(c->stream));
         void* scratch = nullptr;
-        const cudaError_t e = pool_alloc(c, &scratch, merge_scratch_bytes(n));
+        bool rounds = false;
+        const cudaError_t e = merge_scratch(c, n, &scratch, &rounds);
         if (e != cudaSuccess)
             return fail(DVM_ERR_OOM, std::string("merge scratch: ") + cudaGetErrorString(e));
         const InstDesc& h = s->h;
         uint32_t* cdev =
             reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + merge_count_offset(n));
         merge_run(MergeArrays{h.x, h.z, h.circ, h.sigma, h.u, h.w, h.uvs, h.wvs}, h.id, n,
-                  threshold, &c->d_state[s->slot].n, cdev, scratch, c->sms, c->stream);
+                  threshold, &c->d_state[s->slot].n, cdev, scratch, rounds, c->sms, c->stream);
         CK(cudaMemcpyAsync(&cnt, cdev, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
         pool_free(c, scratch);
         g_launches += 4;
@@ -2523,11 +2533,12 @@ int dvm_merge_blobs(dvm_ctx* c, double* x, double* z, double* circ, double* sigm
         CK(cudaMemcpyAsync(d + k * n, host[k], 8 * n, cudaMemcpyHostToDevice, c->stream));
     void* scratch = nullptr;
     const uint32_t nn = (uint32_t)n;
-    const cudaError_t e = pool_alloc(c, &scratch, merge_scratch_bytes(nn));
+    bool rounds = false;
+    const cudaError_t e = merge_scratch(c, nn, &scratch, &rounds);
     if (e != cudaSuccess) return fail(DVM_ERR_OOM, std::string("merge scratch: ") + cudaGetErrorString(e));
     uint32_t* cdev = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + merge_count_offset(nn));
     merge_run(MergeArrays{d, d + n, d + 2 * n, d + 3 * n, d + 4 * n, d + 5 * n, d + 6 * n, d + 7 * n},
-              nullptr, nn, threshold, nullptr, cdev, scratch, c->sms, c->stream);
+              nullptr, nn, threshold, nullptr, cdev, scratch, rounds, c->sms, c->stream);
     uint32_t cnt = 0;
     CK(cudaMemcpyAsync(&cnt, cdev, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     pool_free(c, scratch);

@@ -286,14 +286,16 @@ void remesh_run(const RemeshGrid& g, const double* x, const double* z, const dou
                 int* status, void* scratch, int sms, cudaStream_t s);
 
 // Vortex merging (k_merge.cu), in place on 8 SoA arrays of n blobs; the merge
-// count goes to scratch + merge_count_offset(n), the new length to n_dev.
+// count goes to scratch + merge_count_offset(n), the new length to n_dev.  rounds: scratch has
+// room for the parallel rounds, else for the ordered walk alone (the same result).
 struct MergeArrays {
     double *x, *z, *circ, *sigma, *u, *w, *uvs, *wvs;
 };
-size_t merge_scratch_bytes(uint32_t n);
+size_t merge_scratch_bytes(uint32_t n, bool rounds);
 size_t merge_count_offset(uint32_t n);
 void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
-               uint32_t* n_dev, uint32_t* count_dev, void* scratch, int sms, cudaStream_t s);
+               uint32_t* n_dev, uint32_t* count_dev, void* scratch, bool rounds,
+               int sms, cudaStream_t s);
 
 // Conversions between host and device layouts (k_convert.cu).  Arrays "of four" are
 // n values each, one after another.

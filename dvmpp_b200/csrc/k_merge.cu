@@ -20,7 +20,7 @@
 // not settle, or the second one takes more than kOrderedShare of all blobs (long
 // chains, which one warp each would go through again and again), one block
 // walks the absorbers in order instead, searching together for each
-// (k_merge_greedy).
+// (k_merge_greedy); so it does when there is no memory for the rounds' lists.
 // Then merged blobs are removed (stable) and IDs renumbered.  Every arithmetic
 // step is the reference's, in FP64 with one rounding per operation, so the merged
 // state is bit-identical.  A division-free pre-test rejects pairs that cannot
@@ -161,22 +161,24 @@ __device__ __forceinline__ uint32_t search(const Blobs& B, const MergeGrid& G, u
 }
 
 // Partners of every blob in its original state, in no particular order; nl[i] =
-// their number, or kLong when there are more than kList.  One warp per blob.
+// their number, or kLong when there are more than kList (without lists: more than
+// none).  One warp per blob.
 __global__ void __launch_bounds__(256) k_mg_lists(Blobs B, uint32_t n, double thr, MergeGrid G,
                                                   uint32_t* __restrict__ nl,
                                                   uint32_t* __restrict__ lists) {
     const unsigned all = 0xffffffffu;
+    const uint32_t room = lists ? kList : 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = warp; i < n; i += warps) {
         const double xi = B.x[i], zi = B.z[i], gi = B.circ[i];
-        uint32_t* __restrict__ out = lists + (uint64_t)i * kList;
+        uint32_t* __restrict__ out = lists + (uint64_t)i * room;
         uint32_t m = 0;  // warp-uniform
         auto add = [&](bool hit, uint32_t j) {
             const unsigned b = __ballot_sync(all, hit);
             const uint32_t at = m + __popc(b & ((1u << lane) - 1u));
-            if (hit && at < (uint32_t)kList) out[at] = j;
+            if (hit && at < room) out[at] = j;
             m += __popc(b);
         };
         auto look = [&](uint32_t q, bool in) {
@@ -191,20 +193,20 @@ __global__ void __launch_bounds__(256) k_mg_lists(Blobs B, uint32_t n, double th
         };
         long long cx0, cx1, cz0, cz1;
         if (!cell_range(G, xi, zi, gi, thr, cx0, cx1, cz0, cz1)) {
-            for (uint32_t j = i + 1; j < n && m <= (uint32_t)kList; j += 32) {
+            for (uint32_t j = i + 1; j < n && m <= room; j += 32) {
                 const uint32_t q = j + lane;
                 add(q < n && merge_test(xi, zi, gi, B.x[q], B.z[q], B.circ[q], thr), q);
             }
         } else {
-            for (long long cz = cz0; cz <= cz1 && m <= (uint32_t)kList; ++cz) {
+            for (long long cz = cz0; cz <= cz1 && m <= room; ++cz) {
                 const uint64_t r = (uint64_t)cz * G.nxc;
                 const uint32_t q1 = G.cbegin[r + cx1 + 1];
                 for (uint32_t q = G.cbegin[r + cx0]; q < q1; q += 32) look(q + lane, q + lane < q1);
             }
-            for (uint32_t q = G.cbegin[(uint64_t)G.nxc * G.nzc]; q < n && m <= (uint32_t)kList; q += 32)
+            for (uint32_t q = G.cbegin[(uint64_t)G.nxc * G.nzc]; q < n && m <= room; q += 32)
                 look(q + lane, q + lane < n);
         }
-        if (lane == 0) nl[i] = m > (uint32_t)kList ? kLong : m;
+        if (lane == 0) nl[i] = m > room ? kLong : m;
     }
 }
 
@@ -519,7 +521,10 @@ int sort_bits(uint64_t v) {
     return b;
 }
 
-MLayout mlayout(uint32_t n) {
+// Scratch of a merge (about 300 bytes per blob), or, without room for the rounds' lists, of
+// the ordered walk alone (half of that; the candidates then lie where the merged
+// blobs are gathered later).
+MLayout mlayout(uint32_t n, bool rounds) {
     const uint64_t ncells = (uint64_t)kGridMax * kGridMax;
     size_t scan_b = 0, sk_b = 0, sp_b = 0, sel_b = 0;
     const int64_t nn = (int64_t)std::max<uint32_t>(n, 1);
@@ -550,17 +555,19 @@ MLayout mlayout(uint32_t n) {
     L.skeys = take(8ull * n + 8);
     L.vals = take(4ull * n + 4);
     L.svals = take(4ull * n + 4);
-    L.cand = take(32ull * n + 32);
+    L.cand = rounds ? take(32ull * n + 32) : L.t;
     L.cbegin = take(4 * (ncells + 1));
     L.part = take(sizeof(double4) * kStatBlocks);
     L.scal = take(128);
-    L.len = take(4ull * n + 4);
-    L.after = take(32ull * n + 32);
     L.alist = take(4ull * n + 4);
     L.nl = take(4ull * n + 4);
-    L.lists = take(4ull * kList * n + 4);
-    L.own = take(8ull * n + 8);
-    L.flags = take(4 * (kRoundsMax + 2));
+    if (rounds) {
+        L.len = take(4ull * n + 4);
+        L.after = take(32ull * n + 32);
+        L.lists = take(4ull * kList * n + 4);
+        L.own = take(8ull * n + 8);
+        L.flags = take(4 * (kRoundsMax + 2));
+    }
     L.bytes = off;
     return L;
 }
@@ -626,12 +633,13 @@ MergeGrid build_grid(const MergeArrays& a, uint32_t n, double thr, uint32_t smal
 
 }  // namespace
 
-size_t merge_scratch_bytes(uint32_t n) { return mlayout(n).bytes; }
-size_t merge_count_offset(uint32_t n) { return mlayout(n).count; }
+size_t merge_scratch_bytes(uint32_t n, bool rounds) { return mlayout(n, rounds).bytes; }
+size_t merge_count_offset(uint32_t n) { return mlayout(n, false).count; }
 
 void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
-               uint32_t* n_dev, uint32_t* count_dev, void* scratch, int sms, cudaStream_t s) {
-    const MLayout L = mlayout(n);
+               uint32_t* n_dev, uint32_t* count_dev, void* scratch, bool rounds, int sms,
+               cudaStream_t s) {
+    const MLayout L = mlayout(n, rounds);
     char* b = static_cast<char*>(scratch);
     uint32_t* keep = reinterpret_cast<uint32_t*>(b + L.keep);
     uint32_t* pos = reinterpret_cast<uint32_t*>(b + L.pos);
@@ -654,7 +662,7 @@ void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
     uint32_t* n_abs = reinterpret_cast<uint32_t*>(b + L.scal) + 4;
     const Blobs B{a.x, a.z, a.circ, a.sigma};
     uint32_t* nl = reinterpret_cast<uint32_t*>(b + L.nl);
-    uint32_t* lists = reinterpret_cast<uint32_t*>(b + L.lists);
+    uint32_t* lists = rounds ? reinterpret_cast<uint32_t*>(b + L.lists) : nullptr;
     uint32_t* own[2] = {reinterpret_cast<uint32_t*>(b + L.own),
                         reinterpret_cast<uint32_t*>(b + L.own) + n};
     uint32_t* flags = reinterpret_cast<uint32_t*>(b + L.flags) + 1;  // one per round
@@ -663,12 +671,14 @@ void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
     size_t sb = L.tmp_bytes;
     cub::DeviceSelect::Flagged(b + L.tmp, sb, cub::CountingInputIterator<uint32_t>(0), nl, alist,
                                n_abs, (int64_t)n, s);
-    cudaMemsetAsync(flags - 1, 1, 4, s);  // (anything but 0: the first round runs)
-    cudaMemsetAsync(flags, 0, 4 * (kRoundsMax + 1), s);
-    cudaMemsetAsync(own[0], 0xff, 4 * (size_t)n, s);
-    k_mg_guess<<<sms * 2, 256, 0, s>>>(alist, n_abs, nl, lists, own[0]);
+    if (rounds) {
+        cudaMemsetAsync(flags - 1, 1, 4, s);  // (anything but 0: the first round runs)
+        cudaMemsetAsync(flags, 0, 4 * (kRoundsMax + 1), s);
+        cudaMemsetAsync(own[0], 0xff, 4 * (size_t)n, s);
+        k_mg_guess<<<sms * 2, 256, 0, s>>>(alist, n_abs, nl, lists, own[0]);
+    }
     bool settled = false;
-    for (int r = 0; r < kRoundsMax && !settled;) {
+    for (int r = 0; rounds && r < kRoundsMax && !settled;) {
         for (const int end = std::min(kRoundsMax, r == 0 ? 2 : r + 4); r < end; ++r) {
             uint32_t *from = own[r & 1], *to = own[(r + 1) & 1];
             k_mg_clear<<<sms * 2, 256, 0, s>>>(n, flags + r, to);

@@ -1,6 +1,7 @@
 """Calls on a device whose memory is taken.  Setting a simulation's blobs has room of its own
 in the simulation's arrays; without scratch beside them it still gives the same
-state, and still refuses a non-finite value with the simulation left as it was."""
+state, and still refuses a non-finite value with the simulation left as it was.
+Merging without room for its lists gives the same blobs by the ordered walk."""
 import numpy as np
 import pytest
 
@@ -10,11 +11,11 @@ from dvmpp_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-def _fill(torch):
+def _fill(torch, spare=96, step=128):
     """Takes the device's free memory in blocks (what other allocators keep unused is
-    given back to it on the way) but for 96 to 224 MB."""
-    spare, blocks, size = torch.empty(96 << 20, dtype=torch.uint8, device="cuda"), [], 32 << 30
-    while size >= 128 << 20:
+    given back to it on the way) but for spare to spare + step MB."""
+    spare, blocks, size = torch.empty(spare << 20, dtype=torch.uint8, device="cuda"), [], 32 << 30
+    while size >= step << 20:
         try:
             blocks.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
         except torch.OutOfMemoryError:
@@ -57,5 +58,35 @@ def test_set_blobs_without_scratch():
             finally:
                 del blocks
                 torch.cuda.empty_cache()
+        finally:
+            sim.close()
+
+
+def test_merge_without_room_for_lists():
+    """3 million blobs: 900 MB with the lists, 450 without; 480 to 608 MB left."""
+    torch = pytest.importorskip("torch")
+    n = 3_000_000
+    x, z, g, s = W.wake(n, 9, 0.02)
+    rng = np.random.default_rng(9)
+    for a in (x, z):
+        a[100:n:500] = a[99:n - 1:500]  # some share a place, which is all that merges
+    x[100:n:500] += 1e-12 * rng.normal(size=x[100:n:500].size)
+    threshold = 1e-13
+    with N.Context(0) as c:
+        sim = c.sim(N.Params(capacity=n, precision=N.F32, ux=1.0), *W.circle(16))
+        try:
+            got = []
+            for full in (False, True):
+                sim.set_blobs(x, z, g, s)
+                blocks = _fill(torch, 480, 128) if full else []
+                try:
+                    count = sim.merge(threshold)
+                finally:
+                    del blocks
+                    torch.cuda.empty_cache()
+                got.append((count, sim.blobs()))
+            assert got[0][0] == got[1][0] >= 1000
+            for k in got[0][1]:
+                assert np.array_equal(got[0][1][k], got[1][1][k])
         finally:
             sim.close()
