@@ -20,7 +20,8 @@
 // not settle, or the second one takes more than kOrderedShare of all blobs (long
 // chains, which one warp each would go through again and again), one block
 // walks the absorbers in order instead, searching together for each
-// (k_merge_greedy); so it does when there is no memory for the rounds' lists.
+// (k_merge_greedy); so it does for a few blobs, for lists that are mostly long, and when there
+// is no memory for them.
 // Then merged blobs are removed (stable) and IDs renumbered.  Every arithmetic
 // step is the reference's, in FP64 with one rounding per operation, so the merged
 // state is bit-identical.  A division-free pre-test rejects pairs that cannot
@@ -61,6 +62,12 @@ constexpr uint32_t kFirstMost = 32;    // members in the first two rounds: at a 
 // Share of the blobs taken in the second round from which the ordered walk is the
 // faster one (20 k blobs: 32 % merged, rounds 10 ms, walk 62; 58 %, 178 and 73).
 constexpr double kOrderedShare = 0.45;
+// Share of the blobs with more than kList partners from which that is so in advance (wakes of
+// 3000 to 20 000: from 0.67 on the second round takes 49 % and more, at 0.49 32 %).
+constexpr double kLongShare = 0.6;
+constexpr uint32_t kRoundsMin = 256;   // blobs below which the walk takes less than the rounds' launches
+                                       // (10, 100: 180, 190 us against 235, 230; 300: 212, 235 at a
+                                       // threshold that merges little, 388 and 336 at one that does)
 constexpr int kRoundsMax = 64;         // rounds before the ordered pass takes over
 constexpr uint32_t kLong = 0xFFu;      // as a list's length: more than kList
 constexpr uint32_t kSmallList = 2048;  // blobs kept out of the grid, at most
@@ -71,6 +78,7 @@ struct MergeGrid {
     double x0, z0, inv_h, h, g_cut;
     int nxc, nzc, enabled;
     const double4* cand;     // (x, z, circ, index), cell-sorted; from cbegin[cells] on the short list
+    const uint32_t* svals;   // their indices alone
     const uint32_t* cbegin;  // first candidate of each cell, and of the short list
 };
 
@@ -165,9 +173,11 @@ __device__ __forceinline__ uint32_t search(const Blobs& B, const MergeGrid& G, u
 // none).  One warp per blob.
 __global__ void __launch_bounds__(256) k_mg_lists(Blobs B, uint32_t n, double thr, MergeGrid G,
                                                   uint32_t* __restrict__ nl,
-                                                  uint32_t* __restrict__ lists) {
+                                                  uint32_t* __restrict__ lists,
+                                                  uint32_t* __restrict__ n_long) {
     const unsigned all = 0xffffffffu;
     const uint32_t room = lists ? kList : 0;
+    uint32_t many = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -207,7 +217,9 @@ __global__ void __launch_bounds__(256) k_mg_lists(Blobs B, uint32_t n, double th
                 look(q + lane, q + lane < n);
         }
         if (lane == 0) nl[i] = m > room ? kLong : m;
+        many += m > room;
     }
+    if (n_long && lane == 0 && many) atomicAdd(n_long, many);
 }
 
 // First guess of the owners: as if every blob took all its partners.
@@ -226,8 +238,17 @@ __global__ void k_mg_guess(const uint32_t* __restrict__ who, const uint32_t* __r
 // absorbs, given the owners, and claims what it takes (one warp per blob); owners
 // compared.  flags[0]: some owner changed; flags[-1]: in the round before (when
 // none had, there is nothing to do, and both owner arrays stay as they are).
-__global__ void k_mg_clear(uint32_t n, const uint32_t* __restrict__ flags, uint32_t* __restrict__ next) {
-    if (flags[-1] == 0) return;
+// Nor is there when too many blobs have long lists.
+struct Tally {  // of a merge
+    uint32_t taken;   // blobs owned after the second round
+    uint32_t n_long;  // blobs with more than kList partners
+};
+__device__ __forceinline__ bool idle(const uint32_t* flags, const Tally* t, uint32_t n) {
+    return flags[-1] == 0 || t->n_long > kLongShare * n;
+}
+__global__ void k_mg_clear(uint32_t n, const uint32_t* __restrict__ flags, const Tally* __restrict__ tally,
+                           uint32_t* __restrict__ next) {
+    if (idle(flags, tally, n)) return;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
         next[p] = UINT32_MAX;
 }
@@ -241,8 +262,9 @@ __global__ void __launch_bounds__(256) k_mg_round(Blobs B, uint32_t n, double th
                                                   uint32_t* __restrict__ next,
                                                   uint32_t* __restrict__ len,
                                                   double4* __restrict__ after, uint32_t most,
-                                                  uint32_t* __restrict__ flags) {
-    if (flags[-1] == 0) return;
+                                                  uint32_t* __restrict__ flags,
+                                                  const Tally* __restrict__ tally) {
+    if (idle(flags, tally, n)) return;
     const unsigned all = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31, m = n_who[0];
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -276,16 +298,16 @@ __global__ void __launch_bounds__(256) k_mg_round(Blobs B, uint32_t n, double th
 
 __global__ void k_mg_compare(uint32_t n, const uint32_t* __restrict__ own,
                              const uint32_t* __restrict__ next, uint32_t* __restrict__ flags,
-                             uint32_t* __restrict__ taken) {
-    if (flags[-1] == 0) return;
+                             Tally* tally, bool second) {
+    if (idle(flags, tally, n)) return;
     uint32_t mine = 0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         if (own[p] != next[p]) flags[0] = 1;
         mine += next[p] != UINT32_MAX;
     }
-    if (taken) {
+    if (second) {
         mine = __reduce_add_sync(0xffffffffu, mine);
-        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(taken, mine);
+        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&tally->taken, mine);
     }
 }
 
@@ -334,23 +356,26 @@ __global__ void __launch_bounds__(kMergeThreads, 1)
                     }
                 }
             } else {
-                // one warp per cell, so the cells' bounds are loaded concurrently
+                // One warp per cell, so the cells' bounds are loaded concurrently.  Most of the
+                // blobs that this walk meets are merged already, so whether one is left comes
+                // before its position and the test (10 k, 20 k blobs, 98, 82 % merged: 215 and
+                // 135 ms the other way round, 135 and 123 so).
                 const long long ncx = cx1 - cx0 + 1, ncell = ncx * (cz1 - cz0 + 1);
                 const uint32_t warp = tid >> 5, lane = tid & 31;
                 for (long long k = warp; k < ncell; k += kMergeThreads / 32) {
                     const uint64_t c = (uint64_t)(cz0 + k / ncx) * G.nxc + (cx0 + k % ncx);
                     for (uint32_t q = G.cbegin[c] + lane; q < G.cbegin[c + 1]; q += 32) {
-                        const double4 v = G.cand[q];  // (a later blob is as it was)
-                        const uint32_t j = (uint32_t)__double_as_longlong(v.w);
-                        if (j < j0 || j >= best) continue;
-                        if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr) && keep[j]) best = j;
+                        const uint32_t j = G.svals[q];
+                        if (j < j0 || j >= best || !keep[j]) continue;
+                        const double4 v = G.cand[q];
+                        if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr)) best = j;
                     }
                 }
                 for (uint32_t q = n_grid + tid; q < n; q += kMergeThreads) {
+                    const uint32_t j = G.svals[q];
+                    if (j < j0 || j >= best || !keep[j]) continue;
                     const double4 v = G.cand[q];
-                    const uint32_t j = (uint32_t)__double_as_longlong(v.w);
-                    if (j < j0 || j >= best) continue;
-                    if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr) && keep[j]) best = j;
+                    if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr)) best = j;
                 }
             }
             best = Reduce(red).Reduce(best, cub::Min());
@@ -566,7 +591,7 @@ MLayout mlayout(uint32_t n, bool rounds) {
         L.after = take(32ull * n + 32);
         L.lists = take(4ull * kList * n + 4);
         L.own = take(8ull * n + 8);
-        L.flags = take(4 * (kRoundsMax + 2));
+        L.flags = take(4 * (kRoundsMax + 1) + sizeof(Tally));
     }
     L.bytes = off;
     return L;
@@ -627,6 +652,7 @@ MergeGrid build_grid(const MergeArrays& a, uint32_t n, double thr, uint32_t smal
     k_mg_cells<<<592, 256, 0, s>>>(a.x, a.z, a.circ, skeys, svals, n, ncells, cand, cbegin);
     G.cand = cand;
     G.cbegin = cbegin;
+    G.svals = svals;
     G.enabled = 1;
     return G;
 }
@@ -651,6 +677,7 @@ void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
         cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
         return;
     }
+    rounds = rounds && n >= kRoundsMin;
     // a warp's search likes a short list and about four cells per blob
     const int root = (int)std::sqrt((double)n);
     const MergeGrid G =
@@ -666,14 +693,16 @@ void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
     uint32_t* own[2] = {reinterpret_cast<uint32_t*>(b + L.own),
                         reinterpret_cast<uint32_t*>(b + L.own) + n};
     uint32_t* flags = reinterpret_cast<uint32_t*>(b + L.flags) + 1;  // one per round
-    uint32_t* taken = flags + kRoundsMax;
-    k_mg_lists<<<sms * 8, 256, 0, s>>>(B, n, threshold, G, nl, lists);
+    Tally* tally = reinterpret_cast<Tally*>(flags + kRoundsMax);
+    if (rounds) {
+        cudaMemsetAsync(flags - 1, 1, 4, s);  // (anything but 0: the first round runs)
+        cudaMemsetAsync(flags, 0, 4 * kRoundsMax + sizeof(Tally), s);
+    }
+    k_mg_lists<<<sms * 8, 256, 0, s>>>(B, n, threshold, G, nl, lists, rounds ? &tally->n_long : nullptr);
     size_t sb = L.tmp_bytes;
     cub::DeviceSelect::Flagged(b + L.tmp, sb, cub::CountingInputIterator<uint32_t>(0), nl, alist,
                                n_abs, (int64_t)n, s);
     if (rounds) {
-        cudaMemsetAsync(flags - 1, 1, 4, s);  // (anything but 0: the first round runs)
-        cudaMemsetAsync(flags, 0, 4 * (kRoundsMax + 1), s);
         cudaMemsetAsync(own[0], 0xff, 4 * (size_t)n, s);
         k_mg_guess<<<sms * 2, 256, 0, s>>>(alist, n_abs, nl, lists, own[0]);
     }
@@ -681,18 +710,19 @@ void merge_run(const MergeArrays& a, uint32_t* id, uint32_t n, double threshold,
     for (int r = 0; rounds && r < kRoundsMax && !settled;) {
         for (const int end = std::min(kRoundsMax, r == 0 ? 2 : r + 4); r < end; ++r) {
             uint32_t *from = own[r & 1], *to = own[(r + 1) & 1];
-            k_mg_clear<<<sms * 2, 256, 0, s>>>(n, flags + r, to);
+            k_mg_clear<<<sms * 2, 256, 0, s>>>(n, flags + r, tally, to);
             k_mg_round<<<sms * 8, 256, 0, s>>>(B, n, threshold, G, alist, n_abs, nl, lists, from, to,
                                                len, after, r < 2 ? kFirstMost : UINT32_MAX,
-                                               flags + r);
-            k_mg_compare<<<sms * 2, 256, 0, s>>>(n, from, to, flags + r, r == 1 ? taken : nullptr);
+                                               flags + r, tally);
+            k_mg_compare<<<sms * 2, 256, 0, s>>>(n, from, to, flags + r, tally, r == 1);
         }
-        uint32_t last = 1, h_taken = 0;
+        uint32_t last = 1;
+        Tally t{};
         cudaMemcpyAsync(&last, flags + r - 1, 4, cudaMemcpyDeviceToHost, s);
-        if (r == 2) cudaMemcpyAsync(&h_taken, taken, 4, cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) break;
+        if (r == 2) cudaMemcpyAsync(&t, tally, sizeof(t), cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess || t.n_long > kLongShare * n) break;
         settled = last == 0;
-        if (!settled && (double)h_taken > kOrderedShare * n) break;
+        if (!settled && (double)t.taken > kOrderedShare * n) break;
     }
     if (settled) {
         cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
