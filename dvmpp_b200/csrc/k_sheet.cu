@@ -106,6 +106,9 @@ constexpr double kSchulzExact = 1e-12, kSchulzDone = 1e-8, kSchulzStart = 1e-5;
 // there at once.
 constexpr double kThinCond = 1e5, kThinCondSmall = 5e3;
 constexpr int kThinSmall = 100;
+// So do the smallest: 3, 8, 12, 16, 20, 24 panels 76, 90, 102, 116, 116, 144 us, by products
+// 110, 110, 114, 117, 115, 118 (110 to 132 when nearly flat).
+constexpr int kTinyPanels = 16;
 
 struct PinvBody {
     const double* A;  // m x np
@@ -1472,7 +1475,7 @@ cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, do
         hw.push_back(w);
     };
     for (int i = 0; i < n; ++i) {
-        if (cond[i] > (np[i] < kThinSmall ? kThinCondSmall : kThinCond)) {
+        if (np[i] <= kTinyPanels || cond[i] > (np[i] < kThinSmall ? kThinCondSmall : kThinCond)) {
             householder(A[i], np[i], P[i], work[i]);
             continue;
         }
@@ -1481,15 +1484,18 @@ cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, do
         gP.push_back(P[i]);
         gw.push_back(work[i]);
     }
-    int dev = 0, sms = 0, per_sm = 0;
+    const int ng = (int)gA.size();
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_pinv_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GjShared));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pinv_invert, kTileThreads * kGjGroups,
-                                                  sizeof(GjShared));
-    if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+    if (ng > 0) {
+        int per_sm = 0;
+        cudaFuncSetAttribute(k_pinv_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GjShared));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pinv_invert, kTileThreads * kGjGroups,
+                                                      sizeof(GjShared));
+        if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+    }
     const int most = sms;  // blocks of the inversion, all resident, one per SM
-    const int ng = (int)gA.size();
     for (int first = 0; first < ng; first += kPinvMaxBodies) {
         PinvGroup Q{};
         Q.nb = std::min(kPinvMaxBodies, ng - first);
