@@ -54,14 +54,18 @@ constexpr size_t kPoolPerPlan = 6144;  // list entries per plan: 4 partitions + 
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Panels x capacity up to which a call that needs the FP32 right-hand side or sheet
-// velocity alone sums all pairs rather than sort the blobs and build their tree
-// (about 150 us at 131 k blobs; both grow with the blobs, so up to 128 panels the
-// sheet never builds one).  A solve of 1024 panels and 262 k blobs by pairs 250 us, 64
-// and 131 k 81; the sheet velocity of 131 k blobs from 64, 128, 256 panels by pairs
-// 54, 76, 126 us, by the tree 190, 200, 210; from 512 and 1024 by the tree 212 and 225,
-// by pairs 271 and 365.
-constexpr uint64_t kLonePairsRhs = 1ull << 28, kLonePairsSheet = 1ull << 26;
+// When a call that needs the FP32 right-hand side or sheet velocity alone sums all pairs
+// rather than sort the blobs and build their tree, which takes 60 to 400 us with the
+// capacity.  Pairs grow with the blobs, so where the capacity does not settle it their
+// count is read (10 us).  Measured, pairs against tree: solves of 131, 300, 600 k blobs with
+// 256 panels 79, 204; 111, 245; 174, 355 us, 512 panels 101, 191; 176, 215; 300, 300, 1024
+// 149, 190; 297, 209; 541, 285; of 300 k in a capacity of 1.2 M 171, 269; 226, 238; 411, 234.
+// Sheet velocity of 5, 131, 300, 600 k blobs with 256 panels 70, 190; 114, 219; 195, 241; 379, 313,
+// 512 panels 117, 201; 201, 242; 358, 256; 680, 325, 1024 panels of 1, 5 k 218, 143; 290, 221;
+// 128 panels of 600 k 213, 303.
+constexpr uint64_t kLonePairsRhs = 1ull << 28, kLoneFewRhs = 5ull << 25, kLoneFewRhsLarge = 1ull << 25;
+constexpr uint64_t kLonePairsSheet = 3ull << 25;
+constexpr int kLoneRhsLarge = 512, kLoneSheetAlways = 128, kLoneSheetMost = 640;
 
 // Source chunks of a simulation's FP64 pair kernel, at most.  Fixed by the capacity
 // alone, so a simulation's sums are associated the same way alone and inside
@@ -2052,6 +2056,12 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
     cudaStream_t st = c->stream;
     const ListEntry* L = pl->all.d_list;
     const int np = s->h.np, prec = s->h.precision;
+    auto few = [&](uint64_t most) {  // whether panels x blobs are within it
+        if ((uint64_t)np * s->h.cap <= most) return true;
+        uint32_t n = UINT32_MAX;
+        cudaMemcpyAsync(&n, &S[s->slot].n, sizeof(n), cudaMemcpyDeviceToHost, st);
+        return cudaStreamSynchronize(st) == cudaSuccess && (uint64_t)np * n <= most;
+    };
     switch (phase) {
         case DVM_PHASE_BIOTSAVART: {
             int pr = prof_begin(c, DVM_PROF_SORT);
@@ -2067,16 +2077,18 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
             break;
         }
         // (a step has the blobs' tree from their own velocities; these two would have
-        // to build one: kLonePairsRhs, kLonePairsSheet)
+        // to build one: kLonePairsRhs, ...)
         case DVM_PHASE_SOLVE: {
-            const bool pairs = (uint64_t)np * s->h.cap <= kLonePairsRhs;
+            const bool pairs = prec == kF32 && ((uint64_t)np * s->h.cap <= kLonePairsRhs ||
+                                                few(np <= kLoneRhsLarge ? kLoneFewRhs : kLoneFewRhsLarge));
             if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
             sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st, pairs);
             sheet_solve(T, S, L, 1, np, st);
             break;
         }
         case DVM_PHASE_SHEETBC: {
-            const bool pairs = np <= 128 || (np <= 256 && (uint64_t)np * s->h.cap <= kLonePairsSheet);
+            const bool pairs = prec == kF32 && (np <= kLoneSheetAlways ||
+                                                (np <= kLoneSheetMost && few(kLonePairsSheet)));
             if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
             sheet_velocity(T, S, L, 1, 0, np, prec, ws, c->sms, st, pairs);
             break;

@@ -339,9 +339,9 @@ void sheet_solve(const InstDesc* table, InstState* st, const ListEntry* list, in
 void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, int max_np, int precision, const Workspace& ws, int sms,
                     cudaStream_t s, bool pairs = false);
-// The FP32 panels' tree and records (or these alone) from gamma (k_biot_savart.cu).
+// The FP32 panels' tree and records from gamma (k_biot_savart.cu).
 void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
-                int max_np, const Workspace& ws, int sms, cudaStream_t s, bool records = false);
+                int max_np, const Workspace& ws, int sms, cudaStream_t s);
 // x += (u + uvs + Ux) dt without recomputing uvs (used by the phase API).
 void convect_update(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
                     int mode, const Workspace& ws, int sms, cudaStream_t s);

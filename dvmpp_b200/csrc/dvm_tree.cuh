@@ -98,6 +98,25 @@ __device__ __forceinline__ void list_prefix(unsigned* s_pre, int n, F count) {
     __syncthreads();
 }
 
+// Panel p as the FP32 sheet sums read it.
+__device__ __forceinline__ PanelRec panel_record(const InstDesc& d, int p) {
+    auto dup = [](double v) {
+        const float f = (float)v;
+        return f2pack(f, f);
+    };
+    const double ds = d.ds[p], g0 = d.gamma[p], g1 = d.gamma[p + 1 == d.np ? 0 : p + 1];
+    PanelRec r;
+    r.cs = make_ulonglong2(dup(d.cth[p]), dup(d.sth[p]));
+    r.dd = make_ulonglong2(dup(ds), dup(1.0 / ds));
+    r.cc = make_ulonglong2(dup(d.c2th[p]), dup(d.s2th[p]));
+    r.gd = make_ulonglong2(dup(g0), dup(g1 - g0));
+    r.xc = d.xc[p];
+    r.zc = d.zc[p];
+    r.ex = d.xc[p] + ds * d.cth[p];
+    r.ez = d.zc[p] + ds * d.sth[p];
+    return r;
+}
+
 // A group of targets: centre, radius, half extents of its box, scale exponent.
 struct TargetBox {
     double cx, cz, R, hx, hz;

@@ -368,27 +368,9 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 2)
         double2* __restrict__ A = mom + noff * kTerms;
         uint32_t g = item - s_pre[k];  // the block's share: nodes kFan g .. of its lowest level
         if (PANELS) {
-            auto dup = [](double v) {
-                const float f = (float)v;
-                return f2pack(f, f);
-            };
             const uint32_t p = g * (kFan * kPanelLeaf) + threadIdx.x;
             static_assert(kFan * kPanelLeaf == 32 * kTreeWarps, "a record per thread");
-            if (p < (uint32_t)d.np) {
-                const double dsp = d.ds[p], g0 = d.gamma[p];
-                const double g1 = d.gamma[p + 1 == (uint32_t)d.np ? 0 : p + 1];
-                PanelRec r;
-                r.cs = make_ulonglong2(dup(d.cth[p]), dup(d.sth[p]));
-                r.dd = make_ulonglong2(dup(dsp), dup(1.0 / dsp));
-                r.cc = make_ulonglong2(dup(d.c2th[p]), dup(d.s2th[p]));
-                r.gd = make_ulonglong2(dup(g0), dup(g1 - g0));
-                r.xc = d.xc[p];
-                r.zc = d.zc[p];
-                r.ex = d.xc[p] + dsp * d.cth[p];
-                r.ez = d.zc[p] + dsp * d.sth[p];
-                pan[e.panoff + p] = r;
-            }
-            if (!nodes) continue;  // the records are all that is wanted
+            if (p < (uint32_t)d.np) pan[e.panoff + p] = panel_record(d, (int)p);
         }
         uint32_t next[2];  // the next leaf's blobs, ahead of its gather
 #pragma unroll
@@ -1924,11 +1906,11 @@ static unsigned combine_threads(uint64_t nchunk) {
 }
 
 void panel_tree(const InstDesc* table, const InstState* st, const ListEntry* list, int nlist,
-                int max_np, const Workspace& ws, int sms, cudaStream_t s, bool records) {
+                int max_np, const Workspace& ws, int sms, cudaStream_t s) {
     const int shares = ((int)panel_leaves(max_np) + kFan - 1) / kFan;
-    if (!records) cudaMemsetAsync(ws.parrived, 0, sizeof(unsigned) * ws.pnodes_used, s);
+    cudaMemsetAsync(ws.parrived, 0, sizeof(unsigned) * ws.pnodes_used, s);
     k_tree<true><<<std::min(sms * 2, nlist * shares), 32 * kTreeWarps, 0, s>>>(
-        table, st, list, nlist, nullptr, nullptr, nullptr, records ? nullptr : ws.pnodes, ws.pmom,
+        table, st, list, nlist, nullptr, nullptr, nullptr, ws.pnodes, ws.pmom,
         ws.parrived, ws.pan);
 }
 

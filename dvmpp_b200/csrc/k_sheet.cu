@@ -1095,9 +1095,7 @@ __global__ void __launch_bounds__(256) k_sheet_velocity(const InstDesc* __restri
 // (or evaluated at every blob of a spread leaf), and only the near panels'
 // terms are evaluated, kPanelLeaf at a time.  All panels for all blobs took
 // 716 us for 250 k blobs and 1024 panels (FMA pipe and issue); 70 to 90 now, the
-// panels' tree included.  TREE false: every panel, for a call that has no tree of the
-// blobs and would take longer to build one (five blocks per SM at 94 registers are
-// slower than three: 131 k blobs and 256 panels 160 us, 141).
+// panels' tree included.
 constexpr int kSheetWarps = 4;
 struct SheetWarp {
     TreeWalk walk;
@@ -1107,7 +1105,6 @@ struct SheetWarp {
     PanelRec pan[kPanelLeaf];
 };
 
-template <bool TREE>
 __global__ void __launch_bounds__(32 * kSheetWarps, 3)
     k_sheet_f32(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
                 const ListEntry* __restrict__ list, int nlist, int mode,
@@ -1120,10 +1117,8 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
     list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kLeaf - 1) / kLeaf; });
     const unsigned total = s_pre[nlist], all = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[TREE ? threadIdx.x >> 5 : 0];
-    PanelRec* near = TREE ? S.pan : reinterpret_cast<PanelRec*>(s_raw) + (threadIdx.x >> 5) * kPanelLeaf;
-    Binomials mat;
-    if (TREE) mat = binomials(lane);
+    SheetWarp& S = reinterpret_cast<SheetWarp*>(s_raw)[threadIdx.x >> 5];
+    const Binomials mat = binomials(lane);
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(work, 1u);
@@ -1142,19 +1137,10 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
             __syncwarp();
             const double2* from = reinterpret_cast<const double2*>(pan + e.panoff + j0);
             for (int q = lane; q < m * (int)(sizeof(PanelRec) / 16); q += 32)
-                reinterpret_cast<double2*>(near)[q] = from[q];
+                reinterpret_cast<double2*>(S.pan)[q] = from[q];
             __syncwarp();
-            sheet_sum_f32x2(pa.x, pa.y, pb.x, pb.y, m, near, ua, wa, ub, wb);
+            sheet_sum_f32x2(pa.x, pa.y, pb.x, pb.y, m, S.pan, ua, wa, ub, wb);
         };
-        if (!TREE) {  // every panel, blobs in their own order
-            const uint32_t ia = min(t0 + lane, n - 1), ib = min(t0 + 32 + lane, n - 1);
-            const double2 pa = make_double2(d.x[ia], d.z[ia]), pb = make_double2(d.x[ib], d.z[ib]);
-            double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
-            for (int j0 = 0; j0 < d.np; j0 += kPanelLeaf) panels(j0, pa, pb, ua, wa, ub, wb);
-            if (t0 + lane < n) sheet_store(d, ia, ua, wa, mode);
-            if (t0 + 32 + lane < n) sheet_store(d, ib, ub, wb, mode);
-            continue;
-        }
         for (int q = lane; q < kLeaf; q += 32) S.at[q] = pxz[e.coff + min(t0 + q, n - 1)];
         __syncwarp();
         TargetBox tb = target_box(nodes[e.noff + leaf]);
@@ -1210,6 +1196,52 @@ __global__ void __launch_bounds__(32 * kSheetWarps, 3)
         }
         if (t0 + lane < n) sheet_store(d, perm[e.coff + t0 + lane], ua, wa, mode);
         if (t0 + 32 + lane < n) sheet_store(d, perm[e.coff + t0 + 32 + lane], ub, wb, mode);
+    }
+}
+
+// Every panel for every blob, for a call that has no tree of the blobs and would take
+// longer to build one: a block takes 256 blobs, two per lane, against 128 panels at a
+// time, whose records its threads make (one set for all its items where it is all
+// the panels).  Few blobs are a chain of np panels, many fill the FMA pipe: 256 panels and 5,
+// 131, 300 k blobs 70, 114, 195 us, at three blocks per SM 86, 119, 205, at five 72, 135, 210;
+// 512 panels and 5 k 117, 153, 121.
+constexpr int kPairPanels = 32 * kSheetWarps;
+constexpr uint32_t kPairBlobs = 2 * 32 * kSheetWarps;
+__global__ void __launch_bounds__(32 * kSheetWarps, 4)
+    k_sheet_pairs(const InstDesc* __restrict__ table, const InstState* __restrict__ st,
+                  const ListEntry* __restrict__ list, int nlist, int mode, unsigned* __restrict__ work) {
+    __shared__ unsigned s_pre[1025];
+    __shared__ PanelRec s_pan[kPairPanels];
+    __shared__ unsigned s_item;
+    list_prefix(s_pre, nlist, [&](int k) { return (st[list[k].inst].n + kPairBlobs - 1) / kPairBlobs; });
+    const unsigned total = s_pre[nlist];
+    const uint32_t tid = threadIdx.x;
+    int loaded = -1;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_item = atomicAdd(work, 1u);
+        __syncthreads();
+        const unsigned item = s_item;
+        if (item >= total) break;
+        const int k = locate(s_pre, nlist, item);
+        const InstDesc& d = table[list[k].inst];
+        const uint32_t n = st[list[k].inst].n;
+        const uint32_t t0 = (item - s_pre[k]) * kPairBlobs + 2 * (tid & ~31u);  // the warp's first
+        const uint32_t ia = t0 + (tid & 31), ib = ia + 32, a = min(ia, n - 1), b = min(ib, n - 1);
+        const double xa = d.x[a], za = d.z[a], xb = d.x[b], zb = d.z[b];
+        double ua = 0.0, wa = 0.0, ub = 0.0, wb = 0.0;
+        for (int j0 = 0; j0 < d.np; j0 += kPairPanels) {
+            const int m = min(kPairPanels, d.np - j0);
+            if (loaded != k || d.np > kPairPanels) {  // block-uniform
+                __syncthreads();
+                if ((int)tid < m) s_pan[tid] = panel_record(d, j0 + (int)tid);
+                __syncthreads();
+            }
+            if (t0 < n) sheet_sum_f32x2(xa, za, xb, zb, m, s_pan, ua, wa, ub, wb);
+        }
+        loaded = k;
+        if (ia < n) sheet_store(d, ia, ua, wa, mode);
+        if (ib < n) sheet_store(d, ib, ub, wb, mode);
     }
 }
 
@@ -1595,11 +1627,14 @@ void sheet_velocity(const InstDesc* table, InstState* st, const ListEntry* list,
                     cudaStream_t s, bool pairs) {
     cudaMemsetAsync(ws.work + 1, 0, sizeof(unsigned), s);
     if (precision == kF32) {
-        panel_tree(table, st, list, nlist, max_np, ws, sms, s, pairs);
-        const size_t smem = (pairs ? sizeof(PanelRec) * kPanelLeaf : sizeof(SheetWarp)) * kSheetWarps;
-        auto* kernel = pairs ? k_sheet_f32<false> : k_sheet_f32<true>;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<sms * 3, 32 * kSheetWarps, smem, s>>>(
+        if (pairs) {
+            k_sheet_pairs<<<sms * 4, 32 * kSheetWarps, 0, s>>>(table, st, list, nlist, mode, ws.work + 1);
+            return;
+        }
+        panel_tree(table, st, list, nlist, max_np, ws, sms, s);
+        const size_t smem = sizeof(SheetWarp) * kSheetWarps;
+        cudaFuncSetAttribute(k_sheet_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_sheet_f32<<<sms * 3, 32 * kSheetWarps, smem, s>>>(
             table, st, list, nlist, mode, ws.perm, reinterpret_cast<const double2*>(ws.packed),
             ws.nodes, ws.pnodes, ws.pmom, ws.pan, ws.work + 1);
         return;
