@@ -69,6 +69,7 @@ constexpr uint32_t kRoundsMin = 256;   // blobs below which the walk takes less 
                                        // (10, 100: 180, 190 us against 235, 230; 300: 212, 235 at a
                                        // threshold that merges little, 388 and 336 at one that does)
 constexpr int kRoundsMax = 64;         // rounds before the ordered pass takes over
+constexpr uint32_t kLookFirst = 32768; // blobs up to which the walk looks who is left first
 constexpr uint32_t kLong = 0xFFu;      // as a list's length: more than kList
 constexpr uint32_t kSmallList = 2048;  // blobs kept out of the grid, at most
 constexpr int kGridMax = 1024;         // cells per axis, at most (and about two per sqrt(n))
@@ -344,6 +345,23 @@ __global__ void __launch_bounds__(kMergeThreads, 1)
         while (j0 < n) {
             const double xi = si[0], zi = si[1], gi = si[2];
             uint32_t best = UINT32_MAX;
+            // Most of the blobs that this walk meets are merged already, so whether one is left
+            // comes before its position and the test, as long as `keep` stays in the L1
+            // cache (10 k, 20 k blobs, 98, 82 % merged: 215 and 135 ms the other way round, 134 and
+            // 122 so; 60 k, 95 %: 4.6 s and 5.2).
+            auto look = [&](uint32_t q) {
+                if (n <= kLookFirst) {
+                    const uint32_t j = G.svals[q];
+                    if (j < j0 || j >= best || !keep[j]) return;
+                    const double4 v = G.cand[q];
+                    if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr)) best = j;
+                } else {
+                    const double4 v = G.cand[q];  // (a later blob is as it was)
+                    const uint32_t j = (uint32_t)__double_as_longlong(v.w);
+                    if (j < j0 || j >= best) return;
+                    if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr) && keep[j]) best = j;
+                }
+            };
             // cell range of this pass (the same decision in every thread)
             long long cx0 = 0, cx1 = -1, cz0 = 0, cz1 = -1;
             const bool full = !cell_range(G, xi, zi, gi, thr, cx0, cx1, cz0, cz1);
@@ -356,26 +374,17 @@ __global__ void __launch_bounds__(kMergeThreads, 1)
                     }
                 }
             } else {
-                // One warp per cell, so the cells' bounds are loaded concurrently.  Most of the
-                // blobs that this walk meets are merged already, so whether one is left comes
-                // before its position and the test (10 k, 20 k blobs, 98, 82 % merged: 215 and
-                // 135 ms the other way round, 135 and 123 so).
+                // one warp per cell, so the cells' bounds are loaded concurrently
                 const long long ncx = cx1 - cx0 + 1, ncell = ncx * (cz1 - cz0 + 1);
                 const uint32_t warp = tid >> 5, lane = tid & 31;
                 for (long long k = warp; k < ncell; k += kMergeThreads / 32) {
                     const uint64_t c = (uint64_t)(cz0 + k / ncx) * G.nxc + (cx0 + k % ncx);
                     for (uint32_t q = G.cbegin[c] + lane; q < G.cbegin[c + 1]; q += 32) {
-                        const uint32_t j = G.svals[q];
-                        if (j < j0 || j >= best || !keep[j]) continue;
-                        const double4 v = G.cand[q];
-                        if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr)) best = j;
+                        look(q);
                     }
                 }
                 for (uint32_t q = n_grid + tid; q < n; q += kMergeThreads) {
-                    const uint32_t j = G.svals[q];
-                    if (j < j0 || j >= best || !keep[j]) continue;
-                    const double4 v = G.cand[q];
-                    if (merge_test(xi, zi, gi, v.x, v.y, v.z, thr)) best = j;
+                    look(q);
                 }
             }
             best = Reduce(red).Reduce(best, cub::Min());
