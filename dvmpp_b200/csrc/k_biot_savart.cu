@@ -91,15 +91,51 @@ __global__ void __launch_bounds__(256) k_domain(const double* __restrict__ x,
     }
 }
 
-// The sort domain of a simulation's descriptor from k_domain's box.
-__global__ void k_set_domain(InstDesc* __restrict__ d, const unsigned long long* __restrict__ dom) {
-    if (dom[0] == 0ull) return;  // no finite point: the domain is as good as any
-    const double x1 = from_ordered_bits(dom[0]), z1 = from_ordered_bits(dom[1]);
-    const double x0 = -from_ordered_bits(dom[2]), z0 = -from_ordered_bits(dom[3]);
-    const double L = fmax(x1 - x0, z1 - z0);
-    d->kx0 = x0;
-    d->kz0 = z0;
+// The sort domain of a simulation's descriptor from the largest x, z, -x and -z (-DBL_MAX:
+// no finite point, and any domain will do).
+__device__ __forceinline__ void set_domain_of(InstDesc* d, const double (&m)[4]) {
+    if (m[0] == -DBL_MAX) return;
+    const double L = fmax(m[0] + m[2], m[1] + m[3]);
+    d->kx0 = -m[2];
+    d->kz0 = -m[3];
     d->kinv = L > 0.0 ? 65535.0 / L : 1.0;
+}
+__global__ void k_set_domain(InstDesc* __restrict__ d, const unsigned long long* __restrict__ dom) {
+    if (dom[0] == 0ull) return;
+    const double m[4] = {from_ordered_bits(dom[0]), from_ordered_bits(dom[1]), from_ordered_bits(dom[2]),
+                         from_ordered_bits(dom[3])};
+    set_domain_of(d, m);
+}
+
+// Both by one block, for a few blobs.
+constexpr uint32_t kDomainOne = 8192;
+__global__ void __launch_bounds__(1024) k_domain_one(const double* __restrict__ x, const double* __restrict__ z,
+                                                     uint32_t n, InstDesc* __restrict__ d) {
+    __shared__ double s_m[4][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double m[4] = {-DBL_MAX, -DBL_MAX, -DBL_MAX, -DBL_MAX};
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const double a = x[i], b = z[i];
+        if (fabs(a) < 1e300 && fabs(b) < 1e300) {
+            m[0] = fmax(m[0], a);
+            m[1] = fmax(m[1], b);
+            m[2] = fmax(m[2], -a);
+            m[3] = fmax(m[3], -b);
+        }
+    }
+    for (int pass = 0; pass < 2; ++pass) {  // within the warps, then over them
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            for (int o = 16; o > 0; o >>= 1) m[k] = fmax(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+            if (pass == 0 && lane == 0) s_m[k][wid] = m[k];
+        }
+        if (pass == 1) break;
+        __syncthreads();
+        if (wid != 0) return;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) m[k] = s_m[k][lane];
+    }
+    if (lane == 0) set_domain_of(d, m);
 }
 
 __device__ __forceinline__ int entry_of_slot(const ListEntry* list, int nlist, uint64_t g) {
@@ -1789,6 +1825,10 @@ __global__ void k_build_rhs_jobs(const InstDesc* __restrict__ table, InstState* 
 
 void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const Workspace& ws,
                 int sms, cudaStream_t s) {
+    if (n <= kDomainOne) {
+        k_domain_one<<<1, 1024, 0, s>>>(x, z, n, d);
+        return;
+    }
     unsigned long long* dom = reinterpret_cast<unsigned long long*>(ws.work + 32);
     cudaMemsetAsync(dom, 0, 4 * sizeof(*dom), s);
     k_domain<<<std::min<uint32_t>((n + 1023) / 1024, sms * 4), 256, 0, s>>>(x, z, n, dom);
