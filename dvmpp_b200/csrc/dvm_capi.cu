@@ -48,6 +48,9 @@ namespace {
             return fail(DVM_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Host calls on so few particles, points or blobs pack and convert them here: a launch or a
+// copy of its own costs more than a loop over them.
+constexpr uint64_t kHostSmall = 512;
 constexpr size_t kMaxPlans = 32;       // cached batch plans per context (LRU)
 constexpr size_t kPoolPerPlan = 6144;  // list entries per plan: 4 partitions + 1 reordered
                                        // pair-kernel list, x 1024 sims
@@ -1341,7 +1344,7 @@ int dvm_sim_set_blobs(dvm_sim* s, uint64_t n, const double* x, const double* z, 
     // Uploaded to scratch, checked and taken over on the device: a set with a
     // non-finite value leaves the simulation as it was.
     double* v = nullptr;
-    if (pool_alloc(c, reinterpret_cast<void**>(&v), 32 * n + 16) == cudaSuccess) {
+    if (n > kHostSmall && pool_alloc(c, reinterpret_cast<void**>(&v), 32 * n + 16) == cudaSuccess) {
         uint32_t* d_bad = reinterpret_cast<uint32_t*>(v + 4 * n);
         for (int k = 0; k < 4 && n && up == cudaSuccess; ++k)
             up = cudaMemcpyAsync(v + k * n, src[k], 8 * n, cudaMemcpyHostToDevice, st);
@@ -1351,7 +1354,7 @@ int dvm_sim_set_blobs(dvm_sim* s, uint64_t n, const double* x, const double* z, 
         }
         g_launches += 2;
         pool_free(c, v);
-    } else {  // no room for it: checked here and uploaded in place
+    } else {  // few, or no room for it: checked here and uploaded in place
         cudaGetLastError();
         for (uint64_t i = 0; i < n && bad == UINT32_MAX; ++i)
             if (!std::isfinite(x[i]) || !std::isfinite(z[i]) || !std::isfinite(circ[i]) || !std::isfinite(sigma[i]))
@@ -2339,6 +2342,17 @@ static int stage_reserve(dvm_ctx* c, size_t fixed, size_t per, uint64_t n, uint6
 // n particles into x z circ sigma, n each, at d.
 static int upload_particles(dvm_ctx* c, const dvm_particle* p, uint64_t n, double* d, void* at,
                             uint64_t stage) {
+    if (n <= kHostSmall) {
+        double h[4 * kHostSmall];
+        for (uint64_t i = 0; i < n; ++i) {
+            h[i] = p[i].x;
+            h[n + i] = p[i].z;
+            h[2 * n + i] = p[i].circ;
+            h[3 * n + i] = p[i].sigma;
+        }
+        if (n) CK(cudaMemcpyAsync(d, h, 32 * n, cudaMemcpyHostToDevice, c->stream));
+        return DVM_OK;
+    }
     for (uint64_t i = 0; i < n; i += stage) {
         const uint64_t m = std::min(stage, n - i);
         CK(cudaMemcpyAsync(at, p + i, sizeof(dvm_particle) * m, cudaMemcpyHostToDevice, c->stream));
@@ -2348,15 +2362,23 @@ static int upload_particles(dvm_ctx* c, const dvm_particle* p, uint64_t n, doubl
     return DVM_OK;
 }
 
-// n velocities from u and w on the device.
-static int download_velocities(dvm_ctx* c, const double* u, const double* w, uint64_t n,
-                               dvm_velocity* out, void* at, uint64_t stage) {
+// n velocities from u and, n values further on, w on the device; ends with the stream's wait.
+static int download_velocities(dvm_ctx* c, const double* u, uint64_t n, dvm_velocity* out, void* at,
+                               uint64_t stage) {
+    if (n <= kHostSmall) {
+        double h[2 * kHostSmall];
+        CK(cudaMemcpyAsync(h, u, 16 * n, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        for (uint64_t i = 0; i < n; ++i) out[i] = dvm_velocity{h[i], h[n + i]};
+        return DVM_OK;
+    }
     for (uint64_t i = 0; i < n; i += stage) {
         const uint64_t m = std::min(stage, n - i);
-        velocity_pairs(u + i, w + i, (uint32_t)m, at, c->stream);
+        velocity_pairs(u + i, u + n + i, (uint32_t)m, at, c->stream);
         g_launches += 1;
         CK(cudaMemcpyAsync(out + i, at, sizeof(dvm_velocity) * m, cudaMemcpyDeviceToHost, c->stream));
     }
+    CK(cudaStreamSynchronize(c->stream));
     return DVM_OK;
 }
 
@@ -2437,10 +2459,8 @@ int dvm_biot_savart_self(dvm_ctx* c, const dvm_particle* p, uint64_t n, dvm_velo
     double* u = d + 4 * n;
     rc = upload_particles(c, p, n, d, u, stage);
     if (!rc) rc = raw_self(c, d, d + n, d + 2 * n, d + 3 * n, n, u, u + n, precision);
-    if (!rc) rc = download_velocities(c, u, u + n, n, out, u + 2 * n, stage);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(c->stream));
-    return DVM_OK;
+    if (!rc) rc = download_velocities(c, u, n, out, u + 2 * n, stage);
+    return rc;
 }
 
 int dvm_random_walk(dvm_ctx* c, double* x, double* z, uint64_t n, const double* R, double nu,
@@ -2702,8 +2722,17 @@ int dvm_sim_probe(dvm_sim* s, const double* px, const double* pz, uint64_t n, do
     if (rc) return rc;
     double* d = reinterpret_cast<double*>(static_cast<char*>(c->raw_block) + part_bytes);
     double *dx = d, *dz = d + n, *dres = d + 2 * n;  // dres: u, w, uvs, wvs
-    CK(cudaMemcpyAsync(dx, px, 8 * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(dz, pz, 8 * n, cudaMemcpyHostToDevice, c->stream));
+    // (a few points in one copy each way: five of the six cost their calls' 4 us each)
+    const bool packed = n <= kHostSmall;
+    std::vector<double> host(packed ? 4 * n : 0);
+    if (packed) {
+        std::copy(px, px + n, host.begin());
+        std::copy(pz, pz + n, host.begin() + n);
+        CK(cudaMemcpyAsync(dx, host.data(), 16 * n, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CK(cudaMemcpyAsync(dx, px, 8 * n, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(dz, pz, 8 * n, cudaMemcpyHostToDevice, c->stream));
+    }
     // blobs: the at-target sum (pairs closer than r^2 = 1e-15 skipped, as in
     // src/VelocityKernel.cpp:89), in the simulation's precision
     direct_at_raw(s->h.x, s->h.z, s->h.circ, s->h.sigma, ns, dx, dz, nt, dres, dres + n,
@@ -2712,10 +2741,13 @@ int dvm_sim_probe(dvm_sim* s, const double* px, const double* pz, uint64_t n, do
     probe_total(dres, nt, s->h.ux, s->h.uz, c->stream);
     g_launches += ns ? 4 : 2;
     double* const out[4] = {u, w, uvs, wvs};
-    for (int k = 0; k < 4; ++k)
+    if (packed) CK(cudaMemcpyAsync(host.data(), dres, 32 * n, cudaMemcpyDeviceToHost, c->stream));
+    for (int k = 0; k < 4 && !packed; ++k)
         if (out[k])
             CK(cudaMemcpyAsync(out[k], dres + k * n, 8 * n, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < 4 && packed; ++k)
+        if (out[k]) std::copy(host.begin() + k * n, host.begin() + (k + 1) * n, out[k]);
     return DVM_OK;
 }
 
@@ -2739,17 +2771,21 @@ int dvm_biot_savart_at(dvm_ctx* c, const dvm_particle* p, uint64_t ns, const dou
     double* dt = d + 4 * ns;
     rc = upload_particles(c, p, ns, d, at, stage);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(dt, tx, 8 * nt, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(dt + nt, tz, 8 * nt, cudaMemcpyHostToDevice, c->stream));
+    if (nt <= kHostSmall) {
+        double h[2 * kHostSmall];
+        std::copy(tx, tx + nt, h);
+        std::copy(tz, tz + nt, h + nt);
+        CK(cudaMemcpyAsync(dt, h, 16 * nt, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CK(cudaMemcpyAsync(dt, tx, 8 * nt, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(dt + nt, tz, 8 * nt, cudaMemcpyHostToDevice, c->stream));
+    }
     double* du = dt + 2 * nt;
     double* dw = du + nt;
     direct_at_raw(d, d + ns, d + 2 * ns, d + 3 * ns, (uint32_t)ns, dt, dt + nt, (uint32_t)nt, du, dw,
                   precision, 1, reinterpret_cast<double2*>(base), c->sms, c->stream);
     g_launches += 2;
-    rc = download_velocities(c, du, dw, nt, out, at, 2 * stage);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(c->stream));
-    return DVM_OK;
+    return download_velocities(c, du, nt, out, at, 2 * stage);
 }
 
 }  // extern "C"
