@@ -103,8 +103,10 @@ constexpr int kTileDepth = 16;
 constexpr double kSchulzExact = 1e-12, kSchulzDone = 1e-8, kSchulzStart = 1e-5;
 // Bodies that would end in the Householder factorisation anyway, or whose extra
 // launches and waits outweigh the products (0.28 ms against 0.24 at 64 panels), go
-// there at once.
-constexpr double kThinCond = 1e5, kThinCondSmall = 5e3;
+// there at once.  (The residual grows with the panels too: of plates 0.5 to 0.05 % thick those up
+// to a product of 5.73e7 with the condition's estimate end by products, from 6.15e7 on
+// not; 720 and 750 panels, 0.2 %: 1.33 ms, and 7.5, by Householder at once 6.5.)
+constexpr double kThinCond = 1e5, kThinCondSmall = 5e3, kThinPanelCond = 5.9e7;
 constexpr int kThinSmall = 100;
 // So do the smallest: 3, 8, 12, 16, 20, 24 panels 76, 90, 102, 116, 116, 144 us, by products
 // 110, 110, 114, 117, 115, 118 (110 to 132 when nearly flat).
@@ -1507,7 +1509,8 @@ cudaError_t pseudo_inverse_many(int n, const double* const* A, const int* np, do
         hw.push_back(w);
     };
     for (int i = 0; i < n; ++i) {
-        if (np[i] <= kTinyPanels || cond[i] > (np[i] < kThinSmall ? kThinCondSmall : kThinCond)) {
+        if (np[i] <= kTinyPanels || cond[i] > (np[i] < kThinSmall ? kThinCondSmall : kThinCond) ||
+            cond[i] * np[i] > kThinPanelCond) {
             householder(A[i], np[i], P[i], work[i]);
             continue;
         }
