@@ -559,7 +559,7 @@ void issue_step(dvm_ctx* c, Plan& pl) {
     };
     const int pstep = prof_begin(c, DVM_PROF_STEP);
     int p = prof_begin(c, DVM_PROF_LOADS);
-    step_counter(S, pl.all.d_list, pl.all.n, s);
+    step_counter(T, S, pl.all.d_list, pl.all.n, s);
     prof_end(c, p);
     L += 1;
     stage(pl.eul_f32, kF32, 1);
@@ -2068,6 +2068,7 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
     switch (phase) {
         case DVM_PHASE_BIOTSAVART: {
             int pr = prof_begin(c, DVM_PROF_SORT);
+            domain_levels(T, S, L, 1, st);
             biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
             prof_end(c, pr);
             pr = prof_begin(c, DVM_PROF_NBODY);
@@ -2084,7 +2085,10 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
         case DVM_PHASE_SOLVE: {
             const bool pairs = prec == kF32 && ((uint64_t)np * s->h.cap <= kLonePairsRhs ||
                                                 few(np <= kLoneRhsLarge ? kLoneFewRhs : kLoneFewRhsLarge));
-            if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            if (prec == kF32 && !pairs) {
+                domain_levels(T, S, L, 1, st);
+                biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            }
             sheet_rhs(T, S, L, 1, np, prec, ws, c->sms, st, pairs);
             sheet_solve(T, S, L, 1, np, st);
             break;
@@ -2092,11 +2096,15 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
         case DVM_PHASE_SHEETBC: {
             const bool pairs = prec == kF32 && (np <= kLoneSheetAlways ||
                                                 (np <= kLoneSheetMost && few(kLonePairsSheet)));
-            if (prec == kF32 && !pairs) biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            if (prec == kF32 && !pairs) {
+                domain_levels(T, S, L, 1, st);
+                biot_savart_prepare(T, S, L, 1, prec, ws, c->sms, st);
+            }
             sheet_velocity(T, S, L, 1, 0, np, prec, ws, c->sms, st, pairs);
             break;
         }
         case DVM_PHASE_CONVECT:
+            domain_levels(T, S, L, 1, st);
             for (int k = 0; k < (s->h.scheme == kRK3 ? 3 : 1); ++k) {
                 biot_savart_self(T, S, L, 1, prec, ws, c->sms, st,
                                  tuned_config(c, shape_class(s->h.cap, 1)));
@@ -2112,7 +2120,7 @@ int dvm_sim_phase(dvm_sim* s, int phase) {
             else reflect(T, S, L, 1, np, ws, c->sms, st);
             break;
         case DVM_PHASE_LOADS: loads(T, S, L, 1, np, st); break;
-        case DVM_PHASE_INCREMENT: step_counter(S, L, 1, st); break;
+        case DVM_PHASE_INCREMENT: step_counter(T, S, L, 1, st); break;
         case DVM_PHASE_REFLECT: reflect(T, S, L, 1, np, ws, c->sms, st); break;
         case DVM_PHASE_DELETE: delete_inside(T, S, L, 1, np, ws, c->sms, st); break;
         default: return fail(DVM_ERR_ARG, "bad phase");

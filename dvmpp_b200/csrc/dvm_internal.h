@@ -141,7 +141,7 @@ struct InstDesc {
     double rho, nu, dt, ux, uz, cutoff_exp, Ur, area;
     double bxmax, bzmin, bzmax;     // contour bounding box (x padded) for the crossing early-out
     double bxmin;
-    double kx0, kz0, kinv;          // sort-key domain: cell = (x - kx0) * kinv
+    double kx0, kz0, kinv;          // sort-key domain: cell = (x - kx0) * kinv (InstState::level 0)
     uint32_t M;                     // max_NumPanelVort
     int np;
     int scheme, cross, rng, precision, refine;
@@ -156,7 +156,7 @@ struct InstState {
     uint32_t step;     // DVMBase::m_step
     uint64_t cursor;   // next uniform to consume (inject mode)
     int status;        // first error raised on the device for this instance
-    int pad;
+    int level;         // the sort's domain is this many times doubled (domain_level)
     double fx, fz, cd, cl;  // last loads
     double totalcirc;       // last Kelvin sum (sum of circ)
 };
@@ -358,7 +358,9 @@ void delete_inside(const InstDesc* table, InstState* st, const ListEntry* list, 
                    int max_np, const Workspace& ws, int sms, cudaStream_t s);
 void loads(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, int max_np,
            cudaStream_t s);
-void step_counter(InstState* st, const ListEntry* list, int nlist, cudaStream_t s);
+void domain_levels(const InstDesc* table, InstState* st, const ListEntry* list, int nlist,
+                   cudaStream_t s);  // (a step does it with its counter)
+void step_counter(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, cudaStream_t s);
 
 // Body set-up, once per body (FP64).
 void influence_matrix(const double* xp, const double* zp, const double* xc, const double* zc,

@@ -91,20 +91,49 @@ __global__ void __launch_bounds__(256) k_domain(const double* __restrict__ x,
     }
 }
 
+// The lane with the r-th smallest value of a warp's.
+__device__ __forceinline__ int ranked_lane(double v, int r, int lane) {
+    int mine = 0;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        const double o = __shfl_sync(0xffffffffu, v, k);
+        mine += o < v || (o == v && k < lane);
+    }
+    return __ffs(__ballot_sync(0xffffffffu, mine == r)) - 1;
+}
 // The sort domain of a simulation's descriptor from the largest x, z, -x and -z (-DBL_MAX:
-// no finite point, and any domain will do).
-__device__ __forceinline__ void set_domain_of(InstDesc* d, const double (&m)[4]) {
+// no finite point, and any domain will do), by a warp.  Of 32 blobs taken at equal
+// distances in their order, s holds all but three around their median; where the box is
+// far wider than that (64 s to a side), a few strays make it so, and it would put all others in a
+// few cells: the domain is then 16 s to each side, and the strays share its edge cells (200 k blobs
+// of a wake, one at 1e6: 18.9 ms by the box, 0.47 without that one).
+__device__ __forceinline__ void set_domain_of(InstDesc* d, const double (&m)[4], const double* __restrict__ x,
+                                              const double* __restrict__ z, uint32_t n, int lane) {
     if (m[0] == -DBL_MAX) return;
-    const double L = fmax(m[0] + m[2], m[1] + m[3]);
-    d->kx0 = -m[2];
-    d->kz0 = -m[3];
+    double x0 = -m[2], z0 = -m[3], L = fmax(m[0] + m[2], m[1] + m[3]);
+    const uint32_t i = (uint32_t)((uint64_t)lane * n / 32);
+    // (a non-finite one counts as a stray)
+    const double sx = isfinite(x[i]) ? x[i] : 1e300, sz = isfinite(z[i]) ? z[i] : 1e300;
+    const double cx = __shfl_sync(0xffffffffu, sx, ranked_lane(sx, 16, lane));
+    const double cz = __shfl_sync(0xffffffffu, sz, ranked_lane(sz, 16, lane));
+    const double r = fmax(fabs(sx - cx), fabs(sz - cz));
+    const double s = __shfl_sync(0xffffffffu, r, ranked_lane(r, 28, lane));
+    if (n >= 64 && s > 0.0 && L > 128.0 * s) {
+        x0 = cx - 16.0 * s;
+        z0 = cz - 16.0 * s;
+        L = 32.0 * s;
+    }
+    if (lane != 0) return;
+    d->kx0 = x0;
+    d->kz0 = z0;
     d->kinv = L > 0.0 ? 65535.0 / L : 1.0;
 }
-__global__ void k_set_domain(InstDesc* __restrict__ d, const unsigned long long* __restrict__ dom) {
+__global__ void k_set_domain(InstDesc* __restrict__ d, const unsigned long long* __restrict__ dom,
+                             const double* __restrict__ x, const double* __restrict__ z, uint32_t n) {
     if (dom[0] == 0ull) return;
     const double m[4] = {from_ordered_bits(dom[0]), from_ordered_bits(dom[1]), from_ordered_bits(dom[2]),
                          from_ordered_bits(dom[3])};
-    set_domain_of(d, m);
+    set_domain_of(d, m, x, z, n, (int)threadIdx.x);
 }
 
 // Both by one block, for a few blobs.
@@ -135,7 +164,7 @@ __global__ void __launch_bounds__(1024) k_domain_one(const double* __restrict__ 
 #pragma unroll
         for (int k = 0; k < 4; ++k) m[k] = s_m[k][lane];
     }
-    if (lane == 0) set_domain_of(d, m);
+    set_domain_of(d, m, x, z, n, lane);
 }
 
 __device__ __forceinline__ int entry_of_slot(const ListEntry* list, int nlist, uint64_t g) {
@@ -160,7 +189,17 @@ __global__ void k_keys(const InstDesc* __restrict__ table, const InstState* __re
         const uint32_t i = (uint32_t)(g - e.coff);
         const InstDesc& d = table[e.inst];
         uint32_t mk = 0xFFFFFFFFu;
-        if (i < st[e.inst].n) mk = curve_key(d.x[i], d.z[i], d.kx0, d.kz0, d.kinv);
+        const InstState& S = st[e.inst];
+        if (i < S.n) {
+            double x0 = d.kx0, z0 = d.kz0, inv = d.kinv;
+            if (S.level) {
+                const double grow = 32768.0 / inv * (exp2_int(S.level) - 1.0);
+                x0 -= grow;
+                z0 -= grow;
+                inv *= exp2_int(-S.level);
+            }
+            mk = curve_key(d.x[i], d.z[i], x0, z0, inv);
+        }
         keys[g] = ((uint64_t)k << 32) | mk;
         vals[g] = i;
     }
@@ -566,6 +605,7 @@ __device__ __forceinline__ uint32_t chunk_count(uint32_t n, int chunks) {
 // out of shared memory as register pairs (no duplicating moves), the targets'
 // are duplicated once per item.
 constexpr int kNearThreads = 640;  // per SM at full occupancy (96 registers)
+constexpr double kStray = 64.0;
 constexpr int kNearSlots = 8;   // partial sums of an item: list entries q, q + 8, ...
 
 __device__ __forceinline__ void split_hi_lo(double v, float& hi, float& lo) {
@@ -626,7 +666,8 @@ __device__ __forceinline__ float core_kernel_expm1(float r2, float rs, float rcp
 // Accumulates -u and w, even and odd sources apart.
 //
 // WIDE: for a target leaf much wider than the source leaf, or than its
-// neighbours (blobs of two distant clusters, a sparse fringe).  Offsets from
+// neighbours (blobs of two distant clusters, a sparse fringe; against every source leaf
+// when a stray makes it kStray times wider than a neighbour).  Offsets from
 // its first blob would carry the rounding of its extent into close pairs, so
 // they are kept in two FP32 parts, hi + low: dx = (t_hi - s_hi) + (t_low -
 // s_low), exact before its last rounding for close pairs.
@@ -869,9 +910,10 @@ __global__ void __launch_bounds__(32 * WARPS, kNearThreads / (32 * WARPS))
         if (tid < kLeaf) S.at[tid] = X[min(t0 + tid, n - 1)];
         for (int q = tid; q < kNearSlots * kLeaf; q += 32 * WARPS)
             S.sum[q / kLeaf][q % kLeaf] = make_double2(0.0, 0.0);
-        const TargetBox tb = target_box(N[leaf]);
+        TargetBox tb = target_box(N[leaf]);
         const double nr = fmin(leaf > 0 ? N[leaf - 1].R : DBL_MAX,
                                leaf + 1 < nl ? N[leaf + 1].R : DBL_MAX);
+        if (tb.R > kStray * nr) tb.R = DBL_MAX;  // (only `wide` below reads it)
         int sp = 0;
         if (over) {
             __syncthreads();  // S.at is complete
@@ -1832,7 +1874,7 @@ void set_domain(InstDesc* d, const double* x, const double* z, uint32_t n, const
     unsigned long long* dom = reinterpret_cast<unsigned long long*>(ws.work + 32);
     cudaMemsetAsync(dom, 0, 4 * sizeof(*dom), s);
     k_domain<<<std::min<uint32_t>((n + 1023) / 1024, sms * 4), 256, 0, s>>>(x, z, n, dom);
-    k_set_domain<<<1, 1, 0, s>>>(d, dom);
+    k_set_domain<<<1, 32, 0, s>>>(d, dom, x, z, n);
 }
 
 size_t cub_sort_bytes(uint64_t total) {

@@ -1345,10 +1345,38 @@ __global__ void __launch_bounds__(kLoadThreads) k_loads(const InstDesc* __restri
     s.cl = ddiv(fz, den);
 }
 
-__global__ void k_step_counter(InstState* __restrict__ st, const ListEntry* __restrict__ list,
-                               int nlist) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nlist) st[list[k].inst].step += 1;
+// How many times a simulation's sort domain is to be doubled about its centre so that the
+// blobs fit: all but two of 32 taken at equal distances in their order (a stray blob or two
+// must not cost the others their resolution).  Beyond the domain blobs share its edge
+// cells, and leaves of such blobs are spread over all of them: 60 k blobs a hundred times
+// wider than a wake took 1.92 ms a step, 0.46 in the domain.  By a warp.
+__device__ __forceinline__ int domain_level(const InstDesc& d, uint32_t n, int lane) {
+    if (n == 0) return 0;
+    const uint32_t i = (uint32_t)((uint64_t)lane * n / 32);
+    const double half = 32768.0 / d.kinv;
+    const double m = fmax(fabs(d.x[i] - (d.kx0 + half)), fabs(d.z[i] - (d.kz0 + half))) / half;
+    const int mine = m > 1.0 ? min(ilogb(m), 59) + 1 : 0;
+    int level = 0;
+    while (__popc(__ballot_sync(0xffffffffu, mine <= level)) < 30) ++level;
+    return level;
+}
+// A step's beginning: its number, and the sort's domain.  A warp per simulation.
+__global__ void k_step_counter(const InstDesc* __restrict__ table, InstState* __restrict__ st,
+                               const ListEntry* __restrict__ list, int nlist) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= nlist) return;
+    InstState& s = st[list[k].inst];
+    const int level = domain_level(table[list[k].inst], s.n, lane);
+    if (lane == 0) {
+        s.step += 1;
+        s.level = level;
+    }
+}
+__global__ void k_domain_levels(const InstDesc* __restrict__ table, InstState* __restrict__ st,
+                                const ListEntry* __restrict__ list) {
+    InstState& s = st[list[blockIdx.x].inst];
+    const int level = domain_level(table[list[blockIdx.x].inst], s.n, (int)threadIdx.x);
+    if (threadIdx.x == 0) s.level = level;
 }
 
 }  // namespace
@@ -1666,8 +1694,12 @@ void loads(const InstDesc* table, InstState* st, const ListEntry* list, int nlis
     k_loads<<<nlist, kLoadThreads, sizeof(double) * (max_np + 1), s>>>(table, st, list);
 }
 
-void step_counter(InstState* st, const ListEntry* list, int nlist, cudaStream_t s) {
-    k_step_counter<<<(nlist + 127) / 128, 128, 0, s>>>(st, list, nlist);
+void step_counter(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, cudaStream_t s) {
+    k_step_counter<<<(nlist + 3) / 4, 128, 0, s>>>(table, st, list, nlist);
+}
+
+void domain_levels(const InstDesc* table, InstState* st, const ListEntry* list, int nlist, cudaStream_t s) {
+    k_domain_levels<<<nlist, 32, 0, s>>>(table, st, list);
 }
 
 }  // namespace dvmk
