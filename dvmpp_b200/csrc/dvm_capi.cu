@@ -285,7 +285,8 @@ PairConfig tuned_config(const dvm_ctx* c, int cls) {
 }
 
 // Stream-ordered allocation from the context's pool; on exhaustion the pool's
-// cached memory is released to the device and the allocation retried once.
+// cached memory is released to the device and the allocation retried once.  A failure is
+// the caller's to report and leaves no error behind for the next call to meet.
 cudaError_t pool_alloc(dvm_ctx* c, void** p, size_t bytes) {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->mempool, c->stream);
     if (e == cudaErrorMemoryAllocation) {
@@ -294,6 +295,7 @@ cudaError_t pool_alloc(dvm_ctx* c, void** p, size_t bytes) {
         cudaMemPoolTrimTo(c->mempool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, c->mempool, c->stream);
     }
+    if (e != cudaSuccess) cudaGetLastError();
     return e;
 }
 
@@ -381,12 +383,6 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
     panels = std::max(panels, c->ws_panels);
     const uint64_t lists = std::max<uint64_t>({(uint64_t)nlist, c->ws_lists, 64});
     need_delete = need_delete || c->ws_delete;
-    CK(cudaStreamSynchronize(c->stream));
-    if (c->ws_block) {
-        cudaFree(c->ws_block);
-        c->in_use -= c->ws_bytes;
-        c->ws_block = nullptr;
-    }
     const size_t cub = cub_sort_bytes(cap);
     const uint64_t nodes = 2 * cap / kLeaf + (uint64_t)kNodeSlack * lists;
     const uint64_t pnodes = panel_nodes_bound(panels, lists);
@@ -411,11 +407,27 @@ int ensure_workspace(dvm_ctx* c, uint64_t cap, uint64_t part, uint64_t rhs, uint
                  o_ready = take(4 * (cap / 1024 + 1)),
                  o_jobs = take(256 * lists);
     const uint64_t bytes = off;
-    if (c->in_use + bytes > c->budget)
+    // (a refusal leaves the workspace as it was; once freed, it is as if there never was one)
+    if (c->in_use - (c->ws_block ? c->ws_bytes : 0) + bytes > c->budget)
         return fail(DVM_ERR_OOM, "workspace of " + std::to_string(bytes) +
                                      " B exceeds the HBM budget");
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->ws_block) {
+        cudaFree(c->ws_block);
+        c->in_use -= c->ws_bytes;
+        c->ws_block = nullptr;
+        c->ws_bytes = c->ws_cap = c->ws_part = c->ws_rhs = c->ws_circ = c->ws_panels = c->ws_lists = 0;
+        c->ws_delete = false;
+        c->ws = Workspace();
+        c->ws_generation++;  // graphs that hold its addresses are captured anew
+    }
     void* blk = nullptr;
-    CK(cudaMalloc(&blk, bytes));
+    const cudaError_t e = cudaMalloc(&blk, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(e == cudaErrorMemoryAllocation ? DVM_ERR_OOM : DVM_ERR_CUDA,
+                    std::string("workspace: ") + cudaGetErrorString(e));
+    }
     c->ws_block = blk;
     c->ws_bytes = bytes;
     c->in_use += bytes;
@@ -1355,7 +1367,6 @@ int dvm_sim_set_blobs(dvm_sim* s, uint64_t n, const double* x, const double* z, 
         g_launches += 2;
         pool_free(c, v);
     } else {  // few, or no room for it: checked here and uploaded in place
-        cudaGetLastError();
         for (uint64_t i = 0; i < n && bad == UINT32_MAX; ++i)
             if (!std::isfinite(x[i]) || !std::isfinite(z[i]) || !std::isfinite(circ[i]) || !std::isfinite(sigma[i]))
                 bad = (uint32_t)i;
@@ -2320,6 +2331,9 @@ int dvm_ctx_autotune(dvm_ctx* c, dvm_sim* const* sims, int nsims, int reps, dvm_
 // ---- plugin seam ---------------------------------------------------------------------
 static int raw_reserve(dvm_ctx* c, size_t bytes, bool room_to_grow = true) {
     if (bytes <= c->raw_bytes) return DVM_OK;
+    bytes = align_up(room_to_grow ? bytes + bytes / 4 : bytes, 1 << 20);
+    if (c->in_use - c->raw_bytes + bytes > c->budget)
+        return fail(DVM_ERR_OOM, "plugin scratch exceeds the HBM budget");
     CK(cudaStreamSynchronize(c->stream));
     if (c->raw_block) {
         cudaFree(c->raw_block);
@@ -2327,9 +2341,13 @@ static int raw_reserve(dvm_ctx* c, size_t bytes, bool room_to_grow = true) {
         c->raw_block = nullptr;
         c->raw_bytes = 0;
     }
-    bytes = align_up(room_to_grow ? bytes + bytes / 4 : bytes, 1 << 20);
-    if (c->in_use + bytes > c->budget) return fail(DVM_ERR_OOM, "plugin scratch exceeds the HBM budget");
-    CK(cudaMalloc(&c->raw_block, bytes));
+    const cudaError_t e = cudaMalloc(&c->raw_block, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        c->raw_block = nullptr;
+        return fail(e == cudaErrorMemoryAllocation ? DVM_ERR_OOM : DVM_ERR_CUDA,
+                    std::string("plugin scratch: ") + cudaGetErrorString(e));
+    }
     c->raw_bytes = bytes;
     c->in_use += bytes;
     return DVM_OK;
@@ -2519,7 +2537,6 @@ static cudaError_t merge_scratch(dvm_ctx* c, uint32_t n, void** scratch, bool* r
     *rounds = true;
     const cudaError_t e = pool_alloc(c, scratch, merge_scratch_bytes(n, true));
     if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
     *rounds = false;
     return pool_alloc(c, scratch, merge_scratch_bytes(n, false));
 }

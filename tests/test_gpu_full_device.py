@@ -90,3 +90,27 @@ def test_merge_without_room_for_lists():
                 assert np.array_equal(got[0][1][k], got[1][1][k])
         finally:
             sim.close()
+
+
+def test_a_refusal_leaves_nothing_behind():
+    """A call that does not fit fails with DVM_ERR_OOM; the next one, which does, is as ever."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 23
+    x, z, g, s = W.wake(1000, 3, 0.05)
+    big = [np.zeros(n)] * 4
+    mesh = N.RemeshParams(-1.0, 22.0, -5.0, 5.0, 0.0025, 0.0025, 0.05, 0.0, 0)  # 37 million nodes
+    with N.Context(0) as c:
+        u0, w0 = c.biot_savart_self(x, z, g, s, N.F32)
+        c.remesh(x, z, g, s, N.RemeshParams(-1.0, 22.0, -5.0, 5.0, 0.5, 0.5, 0.05, 0.0, 0))
+        blocks = _fill(torch)
+        try:
+            for refused in (lambda: c.biot_savart_self(*big, N.F32), lambda: c.remesh(x, z, g, s, mesh, 1000),
+                            lambda: c.merge_blobs(dict(x=big[0], z=big[0], circ=big[0], sigma=big[0], u=big[0], w=big[0],
+                                                       uvs=big[0], wvs=big[0]), 1e-9)):
+                with pytest.raises(N.DvmError, match=r"^\[2\]"):
+                    refused()
+                u, w = c.biot_savart_self(x, z, g, s, N.F32)
+                assert np.array_equal(u, u0) and np.array_equal(w, w0)
+        finally:
+            del blocks
+            torch.cuda.empty_cache()

@@ -56,3 +56,16 @@ def test_server_reserves_one_set_up():
         m = npan + 1
         work = 8 * (2 * npan * npan + m * (npan + m) + 2 * m + 2 * npan + 8)
         assert taken <= ws.value + slab + work + 48 * (1 << 20)
+
+
+def test_a_refused_workspace_leaves_the_old_one():
+    """A reservation that the budget does not hold, and a call on the workspace after it."""
+    x, z, g, s = W.wake(5000, 3, 0.05)
+    with N.Context(0, budget_bytes=200 << 20) as c:
+        u0, w0 = c.biot_savart_self(x, z, g, s, N.F32)
+        held = c.memory()[0]
+        with pytest.raises(N.DvmError, match=r"^\[2\]"):
+            c.reserve(1 << 26, 4, 64)
+        assert c.memory()[0] == held
+        u, w = c.biot_savart_self(x, z, g, s, N.F32)
+        assert np.array_equal(u, u0) and np.array_equal(w, w0)
